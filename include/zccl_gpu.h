@@ -382,7 +382,7 @@ typedef struct zccl_gpu_batch {
     size_t clear_bytes; /* leading bytes of d_mem zeroed before every run */
     size_t jobs_off, map_off, tile0_off; /* tables inside d_mem */
     unsigned tb;      /* blocks per tile */
-    unsigned smem[6]; /* shared-memory layout of the launch */
+    unsigned smem[6]; /* reserved */
     int qprev_valid;  /* sums: every input carries its tile starting values */
     size_t rows_off;  /* compress: the jobs' tensor maps inside d_mem, 0 = none */
 } zccl_gpu_batch;

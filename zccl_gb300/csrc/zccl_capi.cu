@@ -72,17 +72,17 @@ int make_geom(size_t n, int L, int T, ZGeom *g)
     return ZCCL_GPU_OK;
 }
 
-/* Side index: size | tile_off[ntiles] | tile_qprev[ntiles] | widths[nblocks] */
+/* Side index: size | grp_off[ngroups] | grp_qprev[ngroups] | widths[nblocks] */
 struct IndexLayout {
-    size_t tile_off, qprev, widths, total;
+    size_t off, qprev, widths, total;
 };
 
 IndexLayout index_layout(const ZGeom &g)
 {
     IndexLayout l;
-    l.tile_off = 16;
-    l.qprev = align16(l.tile_off + 8 * g.ntiles);
-    l.widths = align16(l.qprev + 4 * g.ntiles);
+    l.off = 16;
+    l.qprev = align16(l.off + 8 * g.ngroups);
+    l.widths = align16(l.qprev + 4 * g.ngroups);
     l.total = align16(l.widths + g.nblocks) + 16;
     return l;
 }
@@ -93,8 +93,8 @@ ZIndex bind_index(void *mem, const ZGeom &g)
     uint8_t *p = (uint8_t *)mem;
     ZIndex z;
     z.size = (uint64_t *)p;
-    z.tile_off = (uint64_t *)(p + l.tile_off);
-    z.tile_qprev = (int32_t *)(p + l.qprev);
+    z.grp_off = (uint64_t *)(p + l.off);
+    z.grp_qprev = (int32_t *)(p + l.qprev);
     z.widths = p + l.widths;
     return z;
 }
@@ -149,8 +149,9 @@ ZWork bind_ws(void *ws)
     w.err = (uint32_t *)p;
     w.walk_err = (uint32_t *)(p + 4);
     w.ticket = (uint32_t *)(p + 8);
+    w.role = (uint32_t *)(p + 12);
     w.status = (uint64_t *)(p + 16);
-    w.lb_spin = LB_SPIN_LIMIT;
+    w.spin = SCAN_SPIN_LIMIT;
     return w;
 }
 
@@ -215,44 +216,6 @@ int walk_stream(zccl_gpu_stream *s, const ZGeom &g, void *ws, cudaStream_t st)
 
 bool valid_stream(const zccl_gpu_stream *s) { return s && s->bytes && s->index; }
 
-/* Shared-memory layouts, with room for the kernels' copies of their jobs:
- * two compute slots (the tile in progress and the one just claimed) and the
- * placer's. */
-ZSmem compress_smem(const ZGeom &g)
-{
-    return zg_smem(0, g.L, g.TB, (uint32_t)(2 * sizeof(CompressJob) + sizeof(ZPlace)));
-}
-
-/* The add's layout.  Two CTAs share an SM (registers allow no more), so
- * the shared memory they leave unused goes to the ring of packed sums: the
- * longer the ring, the longer a tile may wait there for its look-back before
- * the adding warps run out of room. */
-ZSmem homadd_smem(const ZGeom &g)
-{
-    ZSmem m = zg_smem(2, g.L, g.TB, homadd_job_bytes(g.TB));
-    static int per_cta = -1;
-    if (per_cta < 0) {
-        int dev = 0, sm = 0, rsv = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
-            cudaGetLastError();
-            sm = 0;
-        }
-        per_cta = sm > 0 ? sm / 2 - rsv - 1024 : 0; /* a kilobyte of margin */
-    }
-    if (per_cta > (int)m.total) {
-        const uint32_t extra = ((uint32_t)per_cta - m.total) & ~15u;
-        m.jobs += extra;
-        m.total += extra;
-    }
-    return m;
-}
-
-/* The decompressor's layout (padded rows, one input buffer) with room for
- * the copy of the job in progress. */
-ZSmem decompress_jobs_smem(const ZGeom &g) { return zg_smem(1, g.L, g.TB, (uint32_t)sizeof(DecompressJob)); }
-
 } // namespace
 
 /* ==================================================================== */
@@ -304,16 +267,14 @@ static int compress_fmt(zccl_gpu_stream *out, const float *d_in, size_t n, float
     a.job.inv = 1.0f / eb; /* float division, as ZCCL/src/ZCCL_float.c:540 */
     a.job.idx = bind_index(out->index, g);
     a.w = bind_ws(d_ws);
-    a.job.status = a.w.status;
     a.wt = width_table();
-    a.sm = compress_smem(g);
     if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     if (test_stall_tile0()) {
         static const uint32_t one = 1;
         if (cudaMemcpyAsync(a.w.ticket, &one, 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return ZCCL_GPU_ECUDA;
-        a.w.lb_spin = 4096;
+        a.w.spin = 4096;
     }
     int rc = cuda_status(launch_compress(a, st));
     if (rc == ZCCL_GPU_OK) {
@@ -360,15 +321,15 @@ static int decompress_fmt(float *d_out, zccl_gpu_stream *in, size_t n, float eb,
         if (rc) return rc;
     }
     DecompressArgs a;
-    a.in = in->bytes;
-    a.avail = in->capacity;
-    a.y = d_out;
-    a.g = g;
-    a.eb = eb;
-    a.idx = bind_index(in->index, g);
+    memset(&a, 0, sizeof(a));
+    a.job.g = g;
+    a.job.in = in->bytes;
+    a.job.avail = in->capacity;
+    a.job.y = d_out;
+    a.job.idx = bind_index(in->index, g);
+    a.job.eb = eb;
     a.qprev_valid = in->qprev_valid;
     a.w = w;
-    a.sm = zg_smem(1, g.L, g.TB, 0);
     int rc = cuda_status(launch_decompress(a, st));
     if (rc == ZCCL_GPU_OK) in->qprev_valid = 1;
     return rc;
@@ -395,7 +356,7 @@ extern "C" int zccl_gpu_decompress_accumulate(float *d_acc, const zccl_gpu_strea
         return ZCCL_GPU_EINVAL;
     cudaStream_t st = (cudaStream_t)cuda_stream;
     if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
-    DecompressJobsArgs a;
+    DecompressArgs a;
     memset(&a, 0, sizeof(a));
     a.job.g = g;
     a.job.in = in->bytes;
@@ -404,9 +365,9 @@ extern "C" int zccl_gpu_decompress_accumulate(float *d_acc, const zccl_gpu_strea
     a.job.idx = bind_index(in->index, g);
     a.job.eb = eb;
     a.job.accumulate = 1;
+    a.qprev_valid = 1;
     a.w = bind_ws(d_ws);
-    a.sm = decompress_jobs_smem(g);
-    return cuda_status(launch_decompress_jobs(a, st));
+    return cuda_status(launch_decompress(a, st));
 }
 
 /* The add of P inputs given by their bytes and index arrays (which need
@@ -425,11 +386,9 @@ static int homadd_inputs(zccl_gpu_stream *out, const HomInput *in, int P, int qv
     a.job.cap = out->capacity;
     a.job.idx = bind_index(out->index, g);
     a.job.g = g;
-    a.job.status = w.status;
     a.cases = d_cases;
     a.w = w;
     a.wt = width_table();
-    a.sm = homadd_smem(g);
     int rc = cuda_status(launch_homadd(a, st));
     if (rc == ZCCL_GPU_OK) {
         out->indexed = 1;
@@ -460,8 +419,8 @@ extern "C" int zccl_gpu_homadd_cases(zccl_gpu_stream *out, zccl_gpu_stream *ins,
         in[p].bytes = ins[p].bytes;
         in[p].avail = ins[p].capacity;
         in[p].widths = ix.widths;
-        in[p].tile_off = ix.tile_off;
-        in[p].tile_qprev = ix.tile_qprev;
+        in[p].grp_off = ix.grp_off;
+        in[p].grp_qprev = ix.grp_qprev;
         qv &= ins[p].qprev_valid ? 1 : 0;
     }
     return homadd_inputs(out, in, P, qv, g, d_ws, d_cases, st);
@@ -611,12 +570,11 @@ extern "C" int zccl_gpu_batch_plan(zccl_gpu_batch *b, int kind, const zccl_gpu_b
     const BatchLayout lay = batch_layout(kind, njobs, ntiles);
     if (bytes < lay.total) return ZCCL_GPU_ECAPACITY;
     uint8_t *base = static_cast<uint8_t *>(d_mem);
-    uint64_t *status = reinterpret_cast<uint64_t *>(base + 16);
     std::vector<uint16_t> map(ntiles);
     std::vector<uint64_t> tile0(njobs);
     std::vector<CompressJob> cj(kind == ZCCL_GPU_BATCH_COMPRESS ? njobs : 0);
     /* compress: a rows-of-32-floats tensor map per job whose full tiles can
-     * arrive as TMA boxes (L = 32, 256-block tiles, 16-byte-aligned input) */
+     * arrive as TMA boxes (L = 32) */
     struct alignas(64) RowsMap { CUtensorMap m; };
     std::vector<RowsMap> rmaps(kind == ZCCL_GPU_BATCH_COMPRESS ? njobs : 0);
     const size_t rows_off = kind == ZCCL_GPU_BATCH_COMPRESS
@@ -640,10 +598,9 @@ extern "C" int zccl_gpu_batch_plan(zccl_gpu_batch *b, int kind, const zccl_gpu_b
             c.out = J.out->bytes;
             c.cap = J.out->capacity;
             c.idx = bind_index(J.out->index, g);
-            c.status = status + t0;
             c.inv = 1.0f / J.eb; /* float division, as ZCCL/src/ZCCL_float.c:540 */
             memset(&rmaps[j], 0, sizeof(RowsMap));
-            c.boxed = L == 32 && g.TB == 256 && zk_rows_map(&rmaps[j].m, J.d_in, g.n, 256) ? 1u : 0u;
+            c.boxed = L == 32 && zk_rows_map(&rmaps[j].m, J.d_in, g.n) ? 1u : 0u;
             any_boxed |= c.boxed != 0;
         } else if (kind == ZCCL_GPU_BATCH_DECOMPRESS) {
             DecompressJob &d = dj[j];
@@ -665,8 +622,8 @@ extern "C" int zccl_gpu_batch_plan(zccl_gpu_batch *b, int kind, const zccl_gpu_b
                 h.in[p].bytes = J.ins[p].bytes;
                 h.in[p].avail = J.ins[p].capacity;
                 h.in[p].widths = ix.widths;
-                h.in[p].tile_off = ix.tile_off;
-                h.in[p].tile_qprev = ix.tile_qprev;
+                h.in[p].grp_off = ix.grp_off;
+                h.in[p].grp_qprev = ix.grp_qprev;
                 jq &= J.ins[p].qprev_valid ? 1 : 0;
             }
             h.P = (uint32_t)J.P;
@@ -674,7 +631,6 @@ extern "C" int zccl_gpu_batch_plan(zccl_gpu_batch *b, int kind, const zccl_gpu_b
             h.out = J.out->bytes;
             h.cap = J.out->capacity;
             h.idx = bind_index(J.out->index, g);
-            h.status = status + t0;
             qv &= jq;
         }
         t0 += g.ntiles;
@@ -704,11 +660,6 @@ extern "C" int zccl_gpu_batch_plan(zccl_gpu_batch *b, int kind, const zccl_gpu_b
     b->tile0_off = lay.tile0;
     b->rows_off = any_boxed ? rows_off : 0;
     b->tb = gs[0].TB;
-    const ZSmem sm = kind == ZCCL_GPU_BATCH_COMPRESS ? compress_smem(gs[0])
-                     : kind == ZCCL_GPU_BATCH_HOMADD ? homadd_smem(gs[0])
-                                                     : decompress_jobs_smem(gs[0]);
-    static_assert(sizeof(sm) == sizeof(b->smem), "layout fields");
-    memcpy(b->smem, &sm, sizeof(sm));
     b->qprev_valid = kind == ZCCL_GPU_BATCH_HOMADD ? qv : 1;
     if (kind != ZCCL_GPU_BATCH_DECOMPRESS)
         for (size_t j = 0; j < njobs; j++) {
@@ -732,39 +683,38 @@ extern "C" int zccl_gpu_batch_run(const zccl_gpu_batch *b, void *cuda_stream)
     bt.njobs = (uint32_t)b->njobs;
     bt.ntiles = b->ntiles;
     bt.maps = b->kind == ZCCL_GPU_BATCH_COMPRESS && b->rows_off ? base + b->rows_off : nullptr;
-    ZSmem sm;
-    memcpy(&sm, b->smem, sizeof(sm));
     if (b->kind == ZCCL_GPU_BATCH_COMPRESS) {
         CompressArgs a;
         memset(&a, 0, sizeof(a));
         a.job.g.L = (uint32_t)b->L; /* the batch's shared L and tile size */
         a.job.g.TB = b->tb;
+        a.job.g.GB = b->tb / ZG_SUB;
         a.batch = bt;
         a.w = bind_ws(base);
         a.wt = width_table();
-        a.sm = sm;
         a.grid = b->grid;
         return cuda_status(launch_compress(a, st));
     }
     if (b->kind == ZCCL_GPU_BATCH_DECOMPRESS) {
-        DecompressJobsArgs a;
+        DecompressArgs a;
         memset(&a, 0, sizeof(a));
         a.job.g.L = (uint32_t)b->L;
         a.job.g.TB = b->tb;
+        a.job.g.GB = b->tb / ZG_SUB;
         a.batch = bt;
+        a.qprev_valid = 1;
         a.w = bind_ws(base);
-        a.sm = sm;
         a.grid = b->grid;
-        return cuda_status(launch_decompress_jobs(a, st));
+        return cuda_status(launch_decompress(a, st));
     }
     HomAddArgs a;
     memset(&a, 0, sizeof(a));
     a.job.g.L = (uint32_t)b->L;
     a.job.g.TB = b->tb;
+    a.job.g.GB = b->tb / ZG_SUB;
     a.batch = bt;
     a.w = bind_ws(base);
     a.wt = width_table();
-    a.sm = sm;
     a.grid = b->grid;
     return cuda_status(launch_homadd(a, st));
 }
@@ -1543,8 +1493,8 @@ int pipe_homadd(DropCtx *c, unsigned char *out, size_t *out_size, const unsigned
                 hi[i].bytes = ib;
                 hi[i].avail = both.capacity;
                 hi[i].widths = ix.widths + (size_t)i * q.g.nblocks;
-                hi[i].tile_off = ix.tile_off + (size_t)i * q.g.ntiles;
-                hi[i].tile_qprev = ix.tile_qprev + (size_t)i * q.g.ntiles;
+                hi[i].grp_off = ix.grp_off + (size_t)i * q.g.ngroups;
+                hi[i].grp_qprev = ix.grp_qprev + (size_t)i * q.g.ngroups;
             }
             if ((rc = homadd_inputs(&sum, hi, 2, 0, q.g, ws, nullptr, st))) break;
         } else {

@@ -3,16 +3,16 @@
  *
  *   quantize*()          bit-exact stand-ins for (int)((double)x * (double)inv)
  *   width_of()           bit-exact stand-in for (int)log2f((float)m) + 1
- *   encode_full/decode_full   one 32-element block, registers <-> packed bytes
- *   encode_small/decode_small/decode_add_full   the same for widths below 16
- *   encode_mid/decode_mid     the same for widths 16..23 (two high bytes)
- *   encode_block32/decode_block32   the fastest of these for a block's width
+ *   encode_block         one block of up to 32 elements, registers -> packed bytes
+ *   decode_small_f/decode_mid_f   its inverse as floats, widths below 16 / 16..23
+ *   decode_add_any       any width, added to integers
+ *   decode_octet         eight elements of any block
  *   encode_any/decode_any     any block, one element at a time
  *   Packer / Reader      MSB-first bit streams in shared memory
  *   tma_load_superset()  TMA bulk copy global -> shared
  *   store_realign()      shared -> global at any byte alignment
  *   cta_excl_scan()      block-wide exclusive scan
- *   lb_publish/resolve   single-pass decoupled look-back across tiles
+ *   scan_publish/scan_wait/scan_tiles   the tiles' places while they are made
  */
 #ifndef ZCCL_GB300_ZDEV_CUH
 #define ZCCL_GB300_ZDEV_CUH
@@ -72,26 +72,6 @@ __device__ __forceinline__ int32_t quantize(float x, float inv, uint32_t &bad)
     return (int32_t)((uint32_t)__float2int_rz(p) + (uint32_t)__float2int_rz(c));
 }
 
-/* The same truncation when the caller knows |x * inv| < 2^24 (see
- * tile_fast_ok()): one rounded-toward-zero multiply and a truncating
- * conversion. */
-__device__ __forceinline__ int32_t quantize_fast(float x, float inv)
-{
-    return __float2int_rz(__fmul_rz(x, inv));
-}
-
-/* max over |x| as raw float bits: NaN ranks above +inf, so a NaN also fails
- * the fast-quantization test. */
-__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
-
-/* Fast quantization is exact for the whole tile when the rounded-toward-
- * zero product of its largest magnitude stays below 2^24. */
-__device__ __forceinline__ bool tile_fast_ok(uint32_t amax_bits, float inv)
-{
-    float am = __uint_as_float(amax_bits);
-    return am == am && fabsf(__fmul_rz(am, inv)) < 16777216.0f;
-}
-
 __device__ __forceinline__ uint32_t bswap32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
 
 /* ---------------------------------------------------------------------
@@ -146,96 +126,9 @@ struct Packer {
     }
 };
 
-/* Reads MSB-first bits from byte offset o of a shared word array.  After
- * refill() at least 33 bits are buffered.  Loads whole aligned words, so it
- * may read up to 8 bytes past the last bit it returns (buffers carry slack). */
-struct Reader {
-    const uint32_t *w;
-    uint32_t wi, nacc;
-    uint64_t acc; /* valid bits left-aligned */
-
-    __device__ __forceinline__ void init(const uint32_t *words, uint32_t o)
-    {
-        w = words;
-        wi = o >> 2;
-        const uint32_t skip = (o & 3u) * 8u;
-        acc = ((uint64_t)bswap32(w[wi]) << 32) << skip;
-        nacc = 32u - skip;
-        wi++;
-        refill();
-    }
-    __device__ __forceinline__ void refill()
-    {
-        if (nacc <= 32u) {
-            acc |= (uint64_t)bswap32(w[wi]) << (32u - nacc);
-            wi++;
-            nacc += 32u;
-        }
-    }
-    __device__ __forceinline__ uint32_t get(uint32_t n) /* 1 <= n <= 32 */
-    {
-        uint32_t v = (uint32_t)(acc >> 32) >> (32u - n);
-        acc <<= n;
-        nacc -= n;
-        return v;
-    }
-};
-
-/* One full block of 32 elements: magnitudes m[] (m[j] >> b == 0), the sign
- * mask (element j at bit 31 - j) and the width b, packed at byte o of the
- * zeroed shared buffer at sbase.  Straight-line code: the header and the 32
- * sign bits, then the B = b/8 high bytes of each element (little-endian per
- * element, four elements per word when B == 1), then the r = b%8 low bits of
- * each element (four r-bit fields merged per put).  A zero-width block is a
- * single 0x00 byte, already in the buffer. */
-__device__ __forceinline__ void encode_full(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask,
-                                            const uint32_t (&m)[32], uint32_t fmt = ZG_FASTMODE1)
-{
-    if (b == 0) return;
-    uint32_t B, r;
-    zg_split(fmt, b, &B, &r);
-    Packer pk;
-    pk.init(sbase, o);
-    pk.put(b, 8);
-    pk.flush();
-    pk.put(smask, 32);
-    pk.flush();
-    if (B == 1) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            uint32_t h = (((m[j] >> r) * 256u + (m[j + 1] >> r)) * 256u + (m[j + 2] >> r)) * 256u +
-                         (m[j + 3] >> r);
-            pk.put(h, 32);
-            pk.flush();
-        }
-    } else if (B > 1) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            pk.put(bswap32(m[j] >> r) >> (32u - 8u * B), 8u * B);
-            pk.flush();
-        }
-    }
-    if (r) {
-        const uint32_t p = 1u << r, mask = p - 1u;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            uint32_t v0 = m[j], v1 = m[j + 1], v2 = m[j + 2], v3 = m[j + 3];
-            if (B) {
-                v0 &= mask;
-                v1 &= mask;
-                v2 &= mask;
-                v3 &= mask;
-            }
-            pk.put(((v0 * p + v1) * p + v2) * p + v3, 4u * r);
-            pk.flush();
-        }
-    }
-    pk.finish();
-}
-
-/* The width byte and the four sign bytes of a 32-element fastmode1 block as
- * one 40-bit little-endian value placed at byte o of the zeroed packing
- * buffer (two word ORs). */
+/* The width byte and the sign bytes (element j at bit 31 - j of smask) of a
+ * block as one 40-bit little-endian value placed at byte o of the zeroed
+ * packing buffer (two word ORs). */
 __device__ __forceinline__ void put_head(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask)
 {
     const uint32_t q = o >> 2, s8 = (o & 3u) * 8u;
@@ -244,84 +137,77 @@ __device__ __forceinline__ void put_head(uint32_t sbase, uint32_t o, uint32_t b,
     sh_or(sbase + 4u * q + 4u, (uint32_t)(v >> 32));
 }
 
-/* The r low bits of the 32 magnitudes m, MSB-first from byte lb (four r-bit
- * fields merged per put). */
+/* The r low bits of the 32 magnitudes m, MSB-first from byte lb: every group
+ * of eight elements is r whole bytes, one 64-bit value (its two halves of
+ * four fields joined by one wide multiply-add) ORed into the one to three
+ * words it touches.  No chain from group to group. */
 __device__ __forceinline__ void put_low_bits(uint32_t sbase, uint32_t lb, uint32_t r, const uint32_t (&m)[32])
 {
-    const uint32_t p = 1u << r, mask = p - 1u;
-    Packer pk;
-    pk.init(sbase, lb);
+    const uint32_t p = 1u << r, mask = p - 1u, p4 = 1u << (4u * r), up = 64u - 8u * r;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-        const uint32_t v0 = m[j] & mask, v1 = m[j + 1] & mask, v2 = m[j + 2] & mask, v3 = m[j + 3] & mask;
-        pk.put(((v0 * p + v1) * p + v2) * p + v3, 4u * r);
-        pk.flush();
+    for (int g = 0; g < 4; g++) {
+        auto f = [&](int k) { return m[8 * g + k] & mask; };
+        const uint32_t h0 = ((f(0) * p + f(1)) * p + f(2)) * p + f(3), h1 = ((f(4) * p + f(5)) * p + f(6)) * p + f(7);
+        const uint64_t v = ((uint64_t)h0 * p4 + h1) << up;
+        const uint32_t lo = bswap32((uint32_t)(v >> 32)), hi = bswap32((uint32_t)v); /* bytes 0 .. 3, 4 .. 7 */
+        const uint32_t at = lb + (uint32_t)g * r, q = sbase + (at & ~3u), sh = (at & 3u) * 8u;
+        const uint32_t end = (at & 3u) + r; /* bytes from q to the group's end */
+        sh_or(q, lo << sh);
+        if (end > 4u) sh_or(q + 4u, __funnelshift_l(lo, hi, sh));
+        if (end > 8u) sh_or(q + 8u, __funnelshift_l(hi, 0u, sh));
     }
-    pk.finish();
 }
 
-/* encode_full for a width of 1..15 bits (B = b/8 <= 1 whole byte per
- * magnitude), the common case at the error bounds the collectives use, with
- * whole words instead of the bit packer where the layout allows: the header
- * and the four sign bytes by put_head, and for B = 1 the 32 high bytes as
- * eight little-endian words realigned to their byte offset by funnel shifts
- * (nine word ORs); the low bits go through the packer as in encode_full.
- * Same bytes as encode_full in the fastmode1 layout. */
-__device__ __forceinline__ void encode_small(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask,
-                                             const uint32_t (&m)[32])
+/* A full block of 32 elements: magnitudes m[] (bits from the 24th on are
+ * ignored for b <= 24), the sign mask (element j at bit 31 - j) and the width
+ * b, packed at byte o of the zeroed shared buffer at sbase: the header and
+ * the sign bytes, the B = b/8 high bytes of each element, then the r = b%8
+ * low bits of each element.  Whole words where the layout allows: one-byte
+ * high parts as eight words of four elements, two-byte ones as sixteen words
+ * of two, realigned to their byte offset by funnel shifts.  A zero-width
+ * block is a single 0x00 byte, already in the buffer. */
+__device__ __forceinline__ void encode_block(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask,
+                                             const uint32_t (&m)[32], uint32_t fmt = ZG_FASTMODE1)
 {
-    const uint32_t B = b >> 3, r = b & 7u;
+    if (b == 0) return;
+    uint32_t B, r;
+    zg_split(fmt, b, &B, &r);
     put_head(sbase, o, b, smask);
     const uint32_t hb = o + 5u;
-    if (B) {
-        const uint32_t q = hb >> 2, sh = (hb & 3u) * 8u;
+    if (B == 1) {
+        const uint32_t q = sbase + (hb & ~3u), sh = (hb & 3u) * 8u;
         uint32_t prev = 0;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const uint32_t lo2 = __byte_perm(m[4 * k] >> r, m[4 * k + 1] >> r, 0x0040u);
             const uint32_t hi2 = __byte_perm(m[4 * k + 2] >> r, m[4 * k + 3] >> r, 0x0040u);
             const uint32_t W = __byte_perm(lo2, hi2, 0x5410u); /* bytes of elements 4k .. 4k + 3 */
-            sh_or(sbase + 4u * (q + (uint32_t)k), __funnelshift_l(prev, W, sh));
+            sh_or(q + 4u * (uint32_t)k, __funnelshift_l(prev, W, sh));
             prev = W;
         }
-        if (sh) sh_or(sbase + 4u * (q + 8u), prev >> (32u - sh));
+        if (sh) sh_or(q + 32u, prev >> (32u - sh));
+    } else if (B == 2) {
+        const uint32_t q = sbase + (hb & ~3u), sh = (hb & 3u) * 8u;
+        uint32_t prev = 0;
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const uint32_t W = __byte_perm(m[2 * k] >> r, m[2 * k + 1] >> r, 0x5410u); /* elements 2k, 2k + 1 */
+            sh_or(q + 4u * (uint32_t)k, __funnelshift_l(prev, W, sh));
+            prev = W;
+        }
+        if (sh) sh_or(q + 64u, prev >> (32u - sh));
+    } else if (__builtin_expect(B > 2, 0)) {
+        const uint32_t keep = B == 3 ? 0xFFFFFFu : 0xFFFFFFFFu;
+#pragma unroll
+        for (int j = 0; j < 32; j++) { /* B bytes each, in two words */
+            const uint32_t at = hb + B * (uint32_t)j, H = (m[j] >> r) & keep;
+            if (H) {
+                sh_or(sbase + (at & ~3u), H << ((at & 3u) * 8u));
+                sh_or(sbase + (at & ~3u) + 4u, __funnelshift_l(H, 0u, (at & 3u) * 8u));
+            }
+        }
     }
     if (r) put_low_bits(sbase, hb + 32u * B, r, m);
-}
-
-/* encode_full for a width of 16..23 bits (B = 2 whole bytes per magnitude):
- * the header by put_head, the 32 two-byte high parts (little-endian per
- * element) as sixteen words of two elements each, realigned to their byte
- * offset by funnel shifts (seventeen word ORs), the low bits through the
- * packer.  Same bytes as encode_full in the fastmode1 layout. */
-__device__ __forceinline__ void encode_mid(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask,
-                                           const uint32_t (&m)[32])
-{
-    const uint32_t r = b & 7u;
-    put_head(sbase, o, b, smask);
-    const uint32_t hb = o + 5u, q = hb >> 2, sh = (hb & 3u) * 8u;
-    uint32_t prev = 0;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const uint32_t W = __byte_perm(m[2 * k] >> r, m[2 * k + 1] >> r, 0x5410u); /* elements 2k, 2k + 1 */
-        sh_or(sbase + 4u * (q + (uint32_t)k), __funnelshift_l(prev, W, sh));
-        prev = W;
-    }
-    if (sh) sh_or(sbase + 4u * (q + 16u), prev >> (32u - sh));
-    if (r) put_low_bits(sbase, hb + 64u, r, m);
-}
-
-/* The fastmode1 encoder for a full 32-element block of width b: the word
- * forms for widths 1..23, encode_full otherwise. */
-__device__ __forceinline__ void encode_block32(uint32_t sbase, uint32_t o, uint32_t b, uint32_t smask,
-                                               const uint32_t (&m)[32])
-{
-    if (__builtin_expect(b - 1u < 15u, 1))
-        encode_small(sbase, o, b, smask, m);
-    else if (b >= 16 && b < 24)
-        encode_mid(sbase, o, b, smask, m);
-    else
-        encode_full(sbase, o, b, smask, m);
 }
 
 /* Bytes a .. a + 7 of the shared words w as a 64-bit big-endian value
@@ -334,247 +220,64 @@ __device__ __forceinline__ void be64_at(const uint32_t *w, uint32_t a, uint32_t 
     lo = __funnelshift_l(w2, w1, sh);
 }
 
-/* prmt.b32 with a selector whose nibbles may ask for the sign of a byte
- * replicated (nibble bit 3), which __byte_perm does not offer. */
-__device__ __forceinline__ uint32_t prmt_sign(uint32_t a, uint32_t sel)
+/* The deltas of a fastmode1 block of n <= 32 elements and any width b at byte
+ * o added into acc (acc[j] += delta j, wrapping; garbage from element n on):
+ * the homomorphic add's form for sums that floats cannot hold.  The same code for every width (a magnitude's bytes
+ * are read by two words each), so that it stays small beside the float
+ * forms. */
+__device__ __forceinline__ void decode_add_any(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n,
+                                               uint32_t (&acc)[32])
 {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(a), "r"(sel));
-    return r;
-}
-
-/* Inverse of encode_full for a block of width b at byte o of the shared
- * words w: d[j] = the int32 delta of element j (as uint32).  Returns the
- * wrapped sum of the deltas.  Branch-free in the width's low part, so the
- * threads of a warp stay together whatever their blocks' widths:
- *   - the high bytes (B = b / 8 == 1, the common case) come from nine
- *     aligned words realigned by funnel shifts, one byte per element;
- *   - the r = b % 8 low bits of eight consecutive elements fill r whole
- *     bytes (byte g r on for group g), read as one big-endian window whose
- *     two 4r-bit halves give four fields each;
- *   - element j's sign (bit 31 - j of the sign word) becomes a mask by
- *     replicating the sign of byte j / 8 of the sign word shifted by j % 8.
- * Reads up to 12 bytes past the block (buffers carry slack). */
-__device__ __forceinline__ uint32_t decode_full(const uint32_t *w, uint32_t o, uint32_t b,
-                                                uint32_t (&d)[32], uint32_t fmt = ZG_FASTMODE1)
-{
-    if (b == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) d[j] = 0;
-        return 0;
-    }
-    uint32_t B, r;
-    zg_split(fmt, b, &B, &r);
-    uint32_t sg, unused;
-    be64_at(w, o + 1, sg, unused);
-    const uint32_t hb = o + 5, lb = hb + 32u * B;
-    if (B == 1) {
-        const uint32_t k0 = hb >> 2, sh = (hb & 3u) * 8u;
-        uint32_t prev = w[k0];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t next = w[k0 + k + 1];
-            const uint32_t A = __funnelshift_r(prev, next, sh); /* bytes hb + 4k .. hb + 4k + 3 */
-            prev = next;
-#pragma unroll
-            for (int i = 0; i < 4; i++) d[4 * k + i] = __byte_perm(A, 0, 0x4440 | i) << r;
-        }
-    } else if (B > 1) {
-        Reader rd;
-        rd.init(w, hb);
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            rd.refill();
-            d[j] = bswap32(rd.get(8u * B) << (32u - 8u * B)) << r;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; j++) d[j] = 0;
-    }
-    if (r) {
-        const uint32_t mask = (1u << r) - 1u;
-        const uint32_t s1 = 32u - r, s2 = s1 - r, s3 = s2 - r, s4 = s3 - r; /* >= 4 */
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-            uint32_t hi, lo;
-            be64_at(w, lb + (uint32_t)g * r, hi, lo);
-            const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r); /* fields 4 .. 7 on top */
-            d[8 * g + 0] |= (hi >> s1) & mask;
-            d[8 * g + 1] |= (hi >> s2) & mask;
-            d[8 * g + 2] |= (hi >> s3) & mask;
-            d[8 * g + 3] |= (hi >> s4) & mask;
-            d[8 * g + 4] |= (h2 >> s1) & mask;
-            d[8 * g + 5] |= (h2 >> s2) & mask;
-            d[8 * g + 6] |= (h2 >> s3) & mask;
-            d[8 * g + 7] |= (h2 >> s4) & mask;
-        }
-    }
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const uint32_t t = sg << k; /* element 8m + k's sign is the top bit of byte 3 - m */
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const uint32_t s = prmt_sign(t, 0x1111u * (8u | (3u - (uint32_t)m))); /* all ones when negative */
-            const int j = 8 * m + k;
-            d[j] = (d[j] ^ s) - s;
-            sum += d[j];
-        }
-    }
-    return sum;
-}
-
-/* decode_full for a fastmode1 block of width 0..15 (B <= 1), the same
- * instructions for every such width so that a warp whose blocks mix one- and
- * zero-byte magnitudes does not split: the high byte of element 8g + k is
- * byte k of the realigned words of group g, replaced by zero when B = 0; its
- * r low bits are field k of the group's r-byte window; the sign mask comes as
- * in decode_full.  Returns the wrapped sum of the deltas. */
-__device__ __forceinline__ uint32_t decode_small(const uint32_t *w, uint32_t o, uint32_t b, uint32_t (&d)[32])
-{
-    if (b == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) d[j] = 0;
-        return 0;
-    }
     const uint32_t B = b >> 3, r = b & 7u;
     uint32_t sg, unused;
     be64_at(w, o + 1, sg, unused);
-    const uint32_t hb = o + 5, lb = hb + 32u * B;
-    const uint32_t k0 = hb >> 2, sh = (hb & 3u) * 8u;
-    const uint32_t zsel = B ? 0u : 4u; /* selector nibble 4..7: a byte of the zero operand */
-    uint32_t tk[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) tk[k] = sg << k; /* element 8g + k's sign: top bit of byte 3 - g */
-    const uint32_t r1 = r, r2 = 2u * r, r3 = 3u * r;
-    uint32_t prev = w[k0], sum = 0;
+    const uint32_t hb = o + 1u + ((n + 7u) >> 3), lb = hb + n * B;
+    const uint32_t bmask = B >= 4 ? 0xFFFFFFFFu : (1u << (8u * B)) - 1u;
 #pragma unroll
     for (int g = 0; g < 4; g++) {
-        const uint32_t n1 = w[k0 + 2 * g + 1], n2 = w[k0 + 2 * g + 2];
-        const uint32_t A0 = __funnelshift_r(prev, n1, sh), A1 = __funnelshift_r(n1, n2, sh);
-        prev = n2;
-        uint32_t hi, lo;
+        uint32_t hi = 0, lo = 0;
         be64_at(w, lb + (uint32_t)g * r, hi, lo);
-        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r); /* fields 4 .. 7 on top */
-        const uint32_t sel = 0x1111u * (8u | (3u - (uint32_t)g));
+        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r);
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const uint32_t A = k < 4 ? A0 : A1;
-            const uint32_t H = __byte_perm(A, 0, 0x4440u | (uint32_t)(k & 3) | zsel);
+            const uint32_t a = hb + (uint32_t)(8 * g + k) * B; /* element 8g + k's little-endian bytes */
+            const uint32_t H = __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], (a & 3u) * 8u) & bmask;
             const uint32_t src = k < 4 ? hi : h2;
-            const uint32_t s1 = (k & 3) == 0 ? 0u : (k & 3) == 1 ? r1 : (k & 3) == 2 ? r2 : r3;
-            const uint32_t m = __funnelshift_l(src << s1, H, r);
-            const uint32_t s = prmt_sign(tk[k], sel); /* all ones when negative */
-            d[8 * g + k] = (m ^ s) - s;
-            sum += d[8 * g + k];
+            const uint32_t m = __funnelshift_l(src << ((uint32_t)(k & 3) * r), H, r);
+            const uint32_t s = (uint32_t)((int32_t)(sg << (8 * g + k)) >> 31); /* all ones when negative */
+            acc[8 * g + k] += (m ^ s) - s;
         }
     }
-    return sum;
 }
 
-/* decode_full for a fastmode1 block of width 16..23 (B = 2), the form of
- * decode_small with two bytes per magnitude: group g's sixteen high bytes are
- * four realigned words, two elements each (little-endian halves); the low
- * bits and signs come as in decode_small.  ADD: d[j] += delta j (the
- * homomorphic add's accumulation, returns 0); otherwise d[j] = delta j and
- * the wrapped sum of the deltas is returned. */
-template <bool ADD>
-__device__ __forceinline__ uint32_t decode_mid(const uint32_t *w, uint32_t o, uint32_t b, uint32_t (&d)[32])
-{
-    const uint32_t r = b & 7u;
-    uint32_t sg, unused;
-    be64_at(w, o + 1, sg, unused);
-    const uint32_t hb = o + 5, lb = hb + 64u;
-    const uint32_t k0 = hb >> 2, sh = (hb & 3u) * 8u;
-    uint32_t tk[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) tk[k] = sg << k; /* element 8g + k's sign: top bit of byte 3 - g */
-    const uint32_t r1 = r, r2 = 2u * r, r3 = 3u * r;
-    uint32_t prev = w[k0], sum = 0;
-#pragma unroll
-    for (int g = 0; g < 4; g++) {
-        uint32_t A[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t nx = w[k0 + 4 * g + i + 1];
-            A[i] = __funnelshift_r(prev, nx, sh); /* bytes hb + 16g + 4i .. + 3: elements 8g + 2i, 8g + 2i + 1 */
-            prev = nx;
-        }
-        uint32_t hi, lo;
-        be64_at(w, lb + (uint32_t)g * r, hi, lo);
-        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r); /* fields 4 .. 7 on top */
-        const uint32_t sel = 0x1111u * (8u | (3u - (uint32_t)g));
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t H = __byte_perm(A[k >> 1], 0, (k & 1) ? 0x4432u : 0x4410u);
-            const uint32_t src = k < 4 ? hi : h2;
-            const uint32_t s1 = (k & 3) == 0 ? 0u : (k & 3) == 1 ? r1 : (k & 3) == 2 ? r2 : r3;
-            const uint32_t m = __funnelshift_l(src << s1, H, r);
-            const uint32_t s = prmt_sign(tk[k], sel); /* all ones when negative */
-            const uint32_t v = (m ^ s) - s;
-            if (ADD) {
-                d[8 * g + k] += v;
-            } else {
-                d[8 * g + k] = v;
-                sum += v;
-            }
-        }
-    }
-    return sum;
-}
+/* Integer work on the float pipe.  The codec kernels are bound by the ALU
+ * pipe, which takes a warp's logic, shift, permute, add or conversion every
+ * second cycle, while the float pipe takes an add or multiply-add every
+ * cycle; and floats hold the integers below 2^24 exactly.  So a magnitude is
+ * put together under the exponent of 2^23 (0x4B000000 | m is the float
+ * 2^23 + m), which costs nothing: the permute that selects its high byte
+ * takes the exponent's bytes from a second operand, 0x4B000000 >> r, so that
+ * the funnel shift by r completes both. */
+#define ZF_TWO23 8388608.0f
+#define ZF_EXP23 0x4B000000u
 
-/* The fastmode1 decoder for a full 32-element block of width b: the word
- * forms for widths 0..23, decode_full otherwise.  Returns the wrapped sum. */
-__device__ __forceinline__ uint32_t decode_block32(const uint32_t *w, uint32_t o, uint32_t b, uint32_t (&d)[32])
+/* The magnitudes of a fastmode1 block of n <= 32 elements and width b <= 15
+ * as floats, their signs in sg (element j at bit 31 - j): each(j, m, sg) for
+ * all 32, garbage from element n on.  The same instructions for every
+ * such width, so a warp whose blocks mix them does not split; a zero-width
+ * block reads (and discards) what follows its header.  Reads up to 150 bytes
+ * past a block's first byte (buffers carry slack). */
+template <class Each>
+__device__ __forceinline__ void decode_small_f(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, Each each)
 {
-    if (b < 16) return decode_small(w, o, b, d);
-    if (b < 24) return decode_mid<false>(w, o, b, d);
-    return decode_full(w, o, b, d);
-}
-
-/* The deltas of a fastmode1 block of width b at byte o added into acc
- * (acc[j] += delta j), for the homomorphic add.  Widths 1..15 take the
- * width-uniform path of decode_small, 16..23 decode_mid; 24..32 read three
- * or four whole bytes per magnitude group by group, so that no second array
- * of 32 values is live. */
-__device__ __forceinline__ void decode_add_full(const uint32_t *w, uint32_t o, uint32_t b, uint32_t (&acc)[32])
-{
-    if (b == 0) return;
     const uint32_t B = b >> 3, r = b & 7u;
     uint32_t sg, unused;
-    if (__builtin_expect(b >= 16, 0)) { /* rare at the bounds the collectives use: out of the hot path */
-        if (b < 24) {
-            decode_mid<true>(w, o, b, acc);
-            return;
-        }
-        be64_at(w, o + 1, sg, unused);
-        const uint32_t hb = o + 5, lb = hb + 32u * B;
-        const uint32_t bmask = B >= 4 ? 0xFFFFFFFFu : (1u << (8u * B)) - 1u;
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-            uint32_t hi = 0, lo = 0;
-            be64_at(w, lb + (uint32_t)g * r, hi, lo);
-            const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t a = hb + (uint32_t)(8 * g + k) * B; /* element 8g + k's little-endian bytes */
-                const uint32_t H = __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], (a & 3u) * 8u) & bmask;
-                const uint32_t src = k < 4 ? hi : h2;
-                const uint32_t m = __funnelshift_l(src << ((uint32_t)(k & 3) * r), H, r);
-                const uint32_t s = (uint32_t)((int32_t)(sg << (8 * g + k)) >> 31); /* all ones when negative */
-                acc[8 * g + k] += (m ^ s) - s;
-            }
-        }
-        return;
-    }
     be64_at(w, o + 1, sg, unused);
-    const uint32_t hb = o + 5, lb = hb + 32u * B;
+    const uint32_t hb = o + 1u + ((n + 7u) >> 3), lb = hb + n * B;
     const uint32_t k0 = hb >> 2, sh = (hb & 3u) * 8u;
-    const uint32_t zsel = B ? 0u : 4u;
-    uint32_t tk[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) tk[k] = sg << k;
-    const uint32_t r1 = r, r2 = 2u * r, r3 = 3u * r;
+    const uint32_t bk = B ? 1u : 0u, s0 = B ? 0x7650u : 0x7654u; /* byte 0: high byte k, or the exponent word's zero byte */
+    const uint32_t ex = ZF_EXP23 >> r;             /* its low 17 bits are zero */
+    const uint32_t p1 = 1u << r, p2 = p1 * p1, p3 = p2 * p1;
     uint32_t prev = w[k0];
 #pragma unroll
     for (int g = 0; g < 4; g++) {
@@ -583,25 +286,233 @@ __device__ __forceinline__ void decode_add_full(const uint32_t *w, uint32_t o, u
         prev = n2;
         uint32_t hi, lo;
         be64_at(w, lb + (uint32_t)g * r, hi, lo);
-        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r);
-        const uint32_t sel = 0x1111u * (8u | (3u - (uint32_t)g));
+        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r); /* fields 4 .. 7 on top */
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const uint32_t A = k < 4 ? A0 : A1;
-            const uint32_t H = __byte_perm(A, 0, 0x4440u | (uint32_t)(k & 3) | zsel);
+            const uint32_t H = __byte_perm(k < 4 ? A0 : A1, ex, s0 + (uint32_t)(k & 3) * bk);
             const uint32_t src = k < 4 ? hi : h2;
-            const uint32_t s1 = (k & 3) == 0 ? 0u : (k & 3) == 1 ? r1 : (k & 3) == 2 ? r2 : r3;
-            const uint32_t m = __funnelshift_l(src << s1, H, r);
-            const uint32_t s = prmt_sign(tk[k], sel);
-            acc[8 * g + k] += (m ^ s) - s;
+            const uint32_t f = (k & 3) == 0 ? src : src * ((k & 3) == 1 ? p1 : (k & 3) == 2 ? p2 : p3);
+            const float m = __uint_as_float(__funnelshift_l(f, H, r)) - ZF_TWO23;
+            each(8 * g + k, m, sg);
         }
     }
 }
 
-/* Any block (n elements, any width), one element at a time: separate
- * streams for the header, the sign bits, the high bytes and the low bits.
- * Used for short tail blocks, block sizes above 32 and tiles that need the
- * exact slow quantization path.  elem(j, neg, mag) gives element j. */
+/* The same for a width of 16 .. 23 (two high bytes per magnitude). */
+template <class Each>
+__device__ __forceinline__ void decode_mid_f(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, Each each)
+{
+    const uint32_t r = b & 7u;
+    uint32_t sg, unused;
+    be64_at(w, o + 1, sg, unused);
+    const uint32_t hb = o + 1u + ((n + 7u) >> 3), lb = hb + 2u * n;
+    const uint32_t k0 = hb >> 2, sh = (hb & 3u) * 8u;
+    const uint32_t ex = ZF_EXP23 >> r; /* its low 16 bits are zero */
+    const uint32_t p1 = 1u << r, p2 = p1 * p1, p3 = p2 * p1;
+    uint32_t prev = w[k0];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        uint32_t hi, lo;
+        be64_at(w, lb + (uint32_t)g * r, hi, lo);
+        const uint32_t h2 = __funnelshift_l(lo, hi, 4u * r); /* fields 4 .. 7 on top */
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+            const uint32_t nx = w[k0 + 4 * g + (k >> 1) + 1];
+            const uint32_t A = __funnelshift_r(prev, nx, sh); /* the high bytes of elements 8g + k, 8g + k + 1 */
+            prev = nx;
+            const uint32_t src = k < 4 ? hi : h2;
+            const uint32_t f0 = (k & 3) == 0 ? src : src * p2, f1 = src * ((k & 3) == 0 ? p1 : p3);
+            each(8 * g + k, __uint_as_float(__funnelshift_l(f0, __byte_perm(A, ex, 0x7610), r)) - ZF_TWO23, sg);
+            each(8 * g + k + 1, __uint_as_float(__funnelshift_l(f1, __byte_perm(A, ex, 0x7632), r)) - ZF_TWO23,
+                 sg);
+        }
+    }
+}
+
+/* m, negated where sg has element j's sign bit (a select is cheaper here than
+ * a shift, a mask and a multiplication: the add 384^3 139 -> 134 us). */
+__device__ __forceinline__ float with_sign(float m, uint32_t sg, int j) { return (sg & (0x80000000u >> j)) ? -m : m; }
+
+/* 1.0f with the sign of bit 31 of s. */
+__device__ __forceinline__ float sign_of(uint32_t s) { return __uint_as_float((s & 0x80000000u) | 0x3F800000u); }
+
+/* N + 1 consecutive floats x become N deltas of their quantized values:
+ * m[j] = 0x4B000000 | |d_j| (the float 2^23 + |d_j|), the signs in smask (d_j
+ * at bit N - 1 - j), mx = max |d_j|, q0 = the first value.  One multiply-add
+ * rounded toward zero, |x| inv + 2^23, has trunc(|x| inv) in its low bits:
+ * the product enters it unrounded.  True when every product stayed below 2^23
+ * and every delta below 2^22, which makes all of this exact; otherwise
+ * (NaN and infinity included) the block is done again by quantize_exact. */
+template <int N, int X>
+__device__ __forceinline__ bool quantize_deltas(const float (&x)[X], float inv, uint32_t (&m)[N], uint32_t &smask,
+                                                uint32_t &mx, int32_t &q0)
+{
+    uint32_t seen = 0;
+    float mf = 0.f, qp = 0.f;
+    smask = 0;
+#pragma unroll
+    for (int j = 0; j <= N; j++) {
+        const float t = __fmaf_rz(fabsf(x[j]), inv, ZF_TWO23);
+        seen |= __float_as_uint(t);
+        const float q = __fmaf_rn(sign_of(__float_as_uint(x[j])), t - ZF_TWO23, 0.f); /* never -0 */
+        if (j == 0) {
+            q0 = __float2int_rn(q);
+        } else {
+            const float d = q - qp;
+            smask = __funnelshift_l(__float_as_uint(d), smask, 1);
+            mf = fmaxf(mf, fabsf(d));
+            m[j - 1] = __float_as_uint(fabsf(d) + ZF_TWO23);
+        }
+        qp = q;
+    }
+    mx = (uint32_t)mf;
+    /* an exponent above 2^23's has a bit that 2^23's lacks; NaN too */
+    return !(seen & ~(ZF_EXP23 | 0x7FFFFFu)) && mf < 4194304.f;
+}
+
+/* The same in integers, exact wherever the reference is defined; x(j) gives
+ * float j.  m[j] is the magnitude alone. */
+template <int N, class X>
+__device__ __forceinline__ void quantize_exact(X x, float inv, uint32_t (&m)[N], uint32_t &smask, uint32_t &mx,
+                                               int32_t &q0, uint32_t &bad)
+{
+    int32_t qp = q0 = quantize(x(0), inv, bad);
+    mx = smask = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const int32_t q = quantize(x(j + 1), inv, bad);
+        const int32_t d = (int32_t)((uint32_t)q - (uint32_t)qp);
+        qp = q;
+        smask = (smask << 1) | ((uint32_t)d >> 31);
+        m[j] = (uint32_t)abs(d); /* |INT_MIN| wraps to 2^31, as in the reference */
+        mx = max(mx, m[j]);
+    }
+}
+
+/* Eight elements of a block: octet g (elements 8g .. 8g + 7) of the block of
+ * n elements and width b at byte o of the shared words w: d[k] = the int32
+ * delta of element 8g + k, 0 past the block's end.  G = ceil(L / 8)
+ * neighbouring lanes hold a block, so a warp's shared reads are those of
+ * 32 / G consecutive blocks, each read as one run.
+ *   - the octet's signs are one byte;
+ *   - its r low bits per element fill r whole bytes (byte g r of the low
+ *     section on), read as one window whose two 4r-bit halves give four
+ *     fields each;
+ *   - its high bytes are 8 (B = 1) or 16 (B = 2) consecutive bytes, realigned
+ *     by funnel shifts; for B = 0 the byte permute selects a zero byte, so
+ *     lanes whose blocks mix B = 0 and 1 take the same instructions, and a
+ *     zero-width block reads (and discards) whatever follows its header.
+ * Reads up to n / 8 + 8G + 20 bytes past a block's end (buffers carry slack). */
+__device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, uint32_t g,
+                                             uint32_t fmt, uint32_t (&d)[8])
+{
+    uint32_t B = b >> 3, r = b & 7u;
+    if (fmt != ZG_FASTMODE1) {
+        B = b ? min(B + 1u, 4u) : 0u;
+        r = 0;
+    }
+    const uint32_t ns = (n + 7u) >> 3; /* a segment's last block may be shorter than L */
+    const uint32_t sg = (uint32_t)reinterpret_cast<const uint8_t *>(w)[o + 1u + g] << 24; /* element k: bit 31 - k */
+    const uint32_t hb = o + 1u + ns, la = hb + B * n + g * r;
+    uint32_t F0, F1;
+    {
+        const uint32_t k = la >> 2, sh = (la & 3u) * 8u;
+        const uint32_t w0 = w[k], w1 = w[k + 1], w2 = w[k + 2];
+        F0 = bswap32(__funnelshift_r(w0, w1, sh));
+        F1 = __funnelshift_l(bswap32(__funnelshift_r(w1, w2, sh)), F0, 4u * r); /* fields 4 .. 7 on top */
+    }
+    const uint32_t r2 = 2u * r, r3 = 3u * r;
+    auto put = [&](int k, uint32_t H) {
+        const uint32_t F = k < 4 ? F0 : F1;
+        const uint32_t f = (k & 3) == 0 ? F : F << ((k & 3) == 1 ? r : (k & 3) == 2 ? r2 : r3);
+        const uint32_t m = __funnelshift_l(f, H, r); /* H << r | the top r bits of f */
+        const uint32_t s = (uint32_t)((int32_t)(sg << k) >> 31);
+        d[k] = (m ^ s) - s;
+    };
+    if (B <= 1) {
+        const uint32_t a = hb + 8u * g, k0 = a >> 2, sh = (a & 3u) * 8u;
+        const uint32_t w0 = w[k0], w1 = w[k0 + 1], w2 = w[k0 + 2];
+        const uint32_t A0 = __funnelshift_r(w0, w1, sh), A1 = __funnelshift_r(w1, w2, sh);
+        const uint32_t zsel = B ? 0x4440u : 0x4444u; /* selector nibble 4: a byte of the zero operand */
+#pragma unroll
+        for (int k = 0; k < 8; k++) put(k, __byte_perm(k < 4 ? A0 : A1, 0, B ? 0x4440u | (uint32_t)(k & 3) : zsel));
+    } else if (B == 2) {
+        const uint32_t a = hb + 16u * g, k0 = a >> 2, sh = (a & 3u) * 8u;
+        uint32_t prev = w[k0];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t nx = w[k0 + i + 1];
+            const uint32_t A = __funnelshift_r(prev, nx, sh);
+            prev = nx;
+            put(2 * i, A & 0xFFFFu);
+            put(2 * i + 1, A >> 16);
+        }
+    } else {
+        const uint32_t bmask = B >= 4 ? 0xFFFFFFFFu : 0xFFFFFFu;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint32_t a = hb + (8u * g + (uint32_t)k) * B;
+            put(k, __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], (a & 3u) * 8u) & bmask);
+        }
+    }
+    if (8u * g + 8u > n) { /* the block's end, or a lane without an octet (n = 0) */
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (8u * g + (uint32_t)k >= n) d[k] = 0;
+    }
+}
+
+/* Bytes decode_octet may read past the last byte of a tile's last block. */
+__host__ __device__ __forceinline__ uint32_t octet_slack(uint32_t L) { return (L + 7u) / 8u + 8u * ((L + 7u) / 8u) + 24u; }
+
+/* v (its low bytes first) ORed into the zeroed buffer from byte at on. */
+__device__ __forceinline__ void or_bytes(uint32_t sbase, uint32_t at, uint64_t v)
+{
+    const uint32_t q = sbase + (at & ~3u), sh = (at & 3u) * 8u, lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+    const uint32_t w0 = lo << sh, w1 = __funnelshift_l(lo, hi, sh), w2 = __funnelshift_l(hi, 0u, sh);
+    if (w0) sh_or(q, w0);
+    if (w1) sh_or(q + 4u, w1);
+    if (w2) sh_or(q + 8u, w2);
+}
+
+/* The inverse of decode_octet: octet g of a block of n elements and width b
+ * into the zeroed buffer at sbase from byte o on; s8: its signs (element k at
+ * bit 7 - k); m: its magnitudes (bits from the 24th on are ignored for
+ * b <= 24); both 0 past the block's end.  Octet 0 writes the header. */
+__device__ __forceinline__ void encode_octet(uint32_t sbase, uint32_t o, uint32_t b, uint32_t n, uint32_t g,
+                                             uint32_t s8, const uint32_t (&m)[8], uint32_t fmt)
+{
+    if (b == 0) return;
+    uint32_t B, r;
+    zg_split(fmt, b, &B, &r);
+    if (g == 0)
+        or_bytes(sbase, o, b | s8 << 8);
+    else
+        or_bytes(sbase, o + 1u + g, s8);
+    const uint32_t hb = o + 1u + ((n + 7u) >> 3), at = hb + 8u * B * g;
+    if (B == 1) {
+        uint64_t v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) v |= (uint64_t)((m[k] >> r) & 0xFFu) << (8 * k);
+        or_bytes(sbase, at, v);
+    } else if (B > 1) {
+        const uint32_t keep = B == 2 ? 0xFFFFu : B == 3 ? 0xFFFFFFu : 0xFFFFFFFFu;
+#pragma unroll
+        for (int k = 0; k < 8; k++) or_bytes(sbase, at + (uint32_t)k * B, (m[k] >> r) & keep);
+    }
+    if (r) { /* r bytes, most significant bit first */
+        const uint32_t mask = (1u << r) - 1u;
+        uint64_t v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) v = v << r | (m[k] & mask);
+        v <<= 64u - 8u * r;
+        or_bytes(sbase, hb + B * n + g * r, (uint64_t)bswap32((uint32_t)v) << 32 | bswap32((uint32_t)(v >> 32)));
+    }
+}
+
+/* A block of n elements, one element at a time: separate streams for the
+ * header, the sign bits, the high bytes and the low bits (a segment's short
+ * last block).  elem(j, neg, mag) gives element j. */
 template <class Elem>
 __device__ __forceinline__ void encode_any(uint32_t sbase, uint32_t o, uint32_t b, uint32_t n,
                                            Elem elem, uint32_t fmt = ZG_FASTMODE1)
@@ -618,6 +529,7 @@ __device__ __forceinline__ void encode_any(uint32_t sbase, uint32_t o, uint32_t 
     ps.init(sbase, o + 1);
     pb.init(sbase, o + 1 + ns);
     pl.init(sbase, o + 1 + ns + B * n);
+#pragma unroll 1
     for (uint32_t j = 0; j < n; j++) {
         uint32_t neg, mg;
         elem(j, neg, mg);
@@ -637,48 +549,14 @@ __device__ __forceinline__ void encode_any(uint32_t sbase, uint32_t o, uint32_t 
     if (r) pl.finish();
 }
 
-/* Element-at-a-time decoder for any block; sink(j, delta). */
-template <class Sink>
-__device__ __forceinline__ void decode_any(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n,
-                                           Sink sink, uint32_t fmt = ZG_FASTMODE1)
-{
-    if (b == 0) {
-        for (uint32_t j = 0; j < n; j++) sink(j, 0u);
-        return;
-    }
-    uint32_t B, r;
-    zg_split(fmt, b, &B, &r);
-    const uint32_t ns = (n + 7) >> 3;
-    Reader rs, rh, rl;
-    rs.init(w, o + 1);
-    rh.init(w, o + 1 + ns);
-    rl.init(w, o + 1 + ns + B * n);
-    for (uint32_t j = 0; j < n; j++) {
-        rs.refill();
-        rh.refill();
-        rl.refill();
-        uint32_t v = B ? bswap32(rh.get(8u * B) << (32u - 8u * B)) << r : 0u;
-        if (r) v |= rl.get(r);
-        if (rs.get(1)) v = 0u - v;
-        sink(j, v);
-    }
-}
-
-/* v[j] and v[j] += x for a runtime j, as selects and predicated adds so
- * that the register array stays in registers (short tail blocks only). */
+/* v[j] for a runtime j, as selects so that the register array stays in
+ * registers (short tail blocks only). */
 __device__ __forceinline__ uint32_t pick(const uint32_t (&v)[32], uint32_t j)
 {
     uint32_t r = v[0];
 #pragma unroll
     for (int k = 1; k < 32; k++) r = (uint32_t)k == j ? v[k] : r;
     return r;
-}
-
-__device__ __forceinline__ void add_at(uint32_t (&v)[32], uint32_t j, uint32_t x)
-{
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-        if ((uint32_t)k == j) v[k] += x;
 }
 
 /* Barrier `id` (1..15) over the first n threads of the CTA (a multiple of
@@ -719,27 +597,40 @@ __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
 
+/* One try for phase `parity` of the barrier (the hardware may hold the
+ * thread for up to the given time, in ns, before it answers). */
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity, uint32_t ns)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n"
+        " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(addr), "r"(parity), "r"(ns)
+        : "memory");
+    return done != 0;
+}
+
 /* Wait for phase `parity` of the barrier to complete.  Gives up after about
  * 2^32 SM clock cycles (two seconds or more) and reports ZERR_TIMEOUT
  * instead of hanging; a wait that spans other stages of a pipeline (which
  * may themselves wait on other CTAs) stays well inside that limit. */
-__device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, uint32_t *err)
+static __device__ __noinline__ void mbar_wait_slow(uint32_t addr, uint32_t parity, uint32_t *err)
 {
-    uint32_t addr = smem_u32(bar);
     const long long t0 = clock64();
-    for (uint32_t it = 0; it < (1u << 30); it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n"
-            " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) return;
+    for (uint32_t it = 0; it < (1u << 26); it++) {
+#pragma unroll 1
+        for (uint32_t k = 0; k < 16; k++)
+            if (mbar_try(addr, parity, 20000u)) return;
         if (clock64() - t0 > (1ll << 32)) break;
     }
     atomicOr(err, ZERR_TIMEOUT);
+}
+__device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, uint32_t *err)
+{
+    const uint32_t addr = smem_u32(bar);
+    if (!mbar_try(addr, parity, 1000u)) mbar_wait_slow(addr, parity, err);
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem()
@@ -792,14 +683,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t sa, const void *map, int32_
         : "memory");
 }
 
-/* TMA tensor store of the box at (c0, c1) of a 2-D map from shared memory,
- * in the issuing thread's bulk group.  The writers of the shared box run
- * fence_proxy_async_smem() and a barrier before it. */
-__device__ __forceinline__ void tma_store_2d(const void *map, uint32_t sa, int32_t c0, int32_t c1)
+/* Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned)
+ * from shared memory to global, in the issuing thread's bulk group.  The
+ * writers of the shared bytes run fence_proxy_async_smem() and a barrier
+ * before it. */
+__device__ __forceinline__ void bulk_s2g(void *gdst, const void *ssrc, uint32_t bytes)
 {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                     (uint64_t)(uintptr_t)map),
-                 "r"(sa), "r"(c0), "r"(c1)
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
+                 "r"(bytes)
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -808,7 +699,7 @@ __device__ __forceinline__ void tma_store_2d(const void *map, uint32_t sa, int32
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-/* Thread 0 only: TMA bulk copy of the 16-byte-aligned superset
+/* One thread: TMA bulk copy of the 16-byte-aligned superset
  * [floor16(g), ceil16(g + nbytes)) into the 16-byte-aligned buffer s, arming
  * the barrier with its byte count.  The superset only adds bytes of 16-byte
  * chunks that already contain bytes of the range, so it never touches a page
@@ -817,7 +708,7 @@ __device__ __forceinline__ void tma_load_superset(uint8_t *s, const uint8_t *g, 
                                                   uint64_t *bar)
 {
     uintptr_t a0 = (uintptr_t)g & ~(uintptr_t)15u;
-    uintptr_t a1 = ((uintptr_t)g + nbytes + 15u) & ~(uintptr_t)15u;
+    uintptr_t a1 = nbytes ? ((uintptr_t)g + nbytes + 15u) & ~(uintptr_t)15u : a0; /* no bytes: g may be anywhere */
     fence_proxy_async_smem(); /* earlier generic accesses of s before the async write */
     mbar_expect_tx(bar, (uint32_t)(a1 - a0));
     if (a1 > a0) bulk_g2s(s, (const void *)a0, (uint32_t)(a1 - a0), bar);
@@ -846,22 +737,40 @@ __device__ __forceinline__ void store_realign(uint8_t *g, const uint8_t *s, uint
     const uint32_t nch = (uint32_t)((a1 - a0) >> 4), q = d >> 2, sh = (d & 3u) * 8u;
     const uint4 *s4 = reinterpret_cast<const uint4 *>(s);
     uint4 *g4 = reinterpret_cast<uint4 *>(a0);
-    for (uint32_t c = tid; c < nch; c += nt) {
-        uint4 lo = s4[c], hi = s4[c + 1];
-        uint32_t o0, o1, o2, o3, o4;
-        /* q is the same for every thread of the tile: a uniform branch */
-        switch (q) {
-        case 0: o0 = lo.x; o1 = lo.y; o2 = lo.z; o3 = lo.w; o4 = hi.x; break;
-        case 1: o0 = lo.y; o1 = lo.z; o2 = lo.w; o3 = hi.x; o4 = hi.y; break;
-        case 2: o0 = lo.z; o1 = lo.w; o2 = hi.x; o3 = hi.y; o4 = hi.z; break;
-        default: o0 = lo.w; o1 = hi.x; o2 = hi.y; o3 = hi.z; o4 = hi.w; break;
+    /* four chunks a thread in flight: one warp writes a tile alone */
+#pragma unroll 1
+    for (uint32_t c0 = tid; c0 < nch; c0 += 4u * nt) {
+        uint4 lo[4], hi[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const uint32_t c = min(c0 + u * nt, nch - 1u);
+            lo[u] = s4[c];
+            hi[u] = s4[c + 1];
         }
-        uint4 v;
-        v.x = __funnelshift_r(o0, o1, sh);
-        v.y = __funnelshift_r(o1, o2, sh);
-        v.z = __funnelshift_r(o2, o3, sh);
-        v.w = __funnelshift_r(o3, o4, sh);
-        g4[c] = v;
+        /* q is the same for every thread of the tile: uniform branches */
+        if (q & 1u) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                lo[u].x = lo[u].y, lo[u].y = lo[u].z, lo[u].z = lo[u].w, lo[u].w = hi[u].x;
+                hi[u].x = hi[u].y, hi[u].y = hi[u].z, hi[u].z = hi[u].w;
+            }
+        }
+        if (q & 2u) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                lo[u].x = lo[u].z, lo[u].y = lo[u].w, lo[u].z = hi[u].x, lo[u].w = hi[u].y;
+                hi[u].x = hi[u].z;
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            uint4 v;
+            v.x = __funnelshift_r(lo[u].x, lo[u].y, sh);
+            v.y = __funnelshift_r(lo[u].y, lo[u].z, sh);
+            v.z = __funnelshift_r(lo[u].z, lo[u].w, sh);
+            v.w = __funnelshift_r(lo[u].w, hi[u].x, sh);
+            if (c0 + u * nt < nch) g4[c0 + u * nt] = v;
+        }
     }
 }
 
@@ -952,18 +861,24 @@ __device__ __forceinline__ uint32_t cta_excl_scan(uint32_t v, uint32_t *wsum, ui
 }
 
 /* ---------------------------------------------------------------------
- * Decoupled look-back (Merrill & Garland 2016).  status[t] packs a 2-bit
- * flag (1 = aggregate of tile t only, 2 = inclusive prefix through t) over
- * a 62-bit value; values add modulo 2^62.  Tiles are taken in ticket order,
- * so every tile a CTA waits on belongs to a CTA that is already running and
- * never waits on a later tile.
+ * The tiles' places: an exclusive scan of their sizes while they are being
+ * made.  status[t] packs a 2-bit flag (1 = the size of tile t, 2 = the
+ * inclusive sum through t) over a 62-bit value.  Workers publish sizes (a
+ * stream's first tile its inclusive sum at once); one warp of the grid, in
+ * the CTA that started first, turns them into sums in ticket order, up to 256
+ * a round; each tile's placer polls its own word only.  (With a decoupled
+ * look-back in every CTA instead, every placer read its 256 predecessors and
+ * more each round, and its chain of look-back and write-out set the pace of
+ * the add: 384^3 floats in 111 us with all decoding left out.)  Tickets are
+ * handed out in order, so the tile that the scan waits for belongs to a CTA
+ * that is running and that waits for no later tile before it publishes.
  * ------------------------------------------------------------------- */
-/* Polls of a predecessor's word before the look-back gives up (about a
- * second at the 32 ns back-off; callers may pass a smaller limit). */
-#define LB_SPIN_LIMIT (1u << 22)
-#define LB_FLAG_A (1ull << 62)
-#define LB_FLAG_P (2ull << 62)
-#define LB_VAL (LB_FLAG_A - 1ull)
+/* Polls before a wait gives up (a second or more; callers may pass a
+ * smaller limit). */
+#define SCAN_SPIN_LIMIT (1u << 22)
+#define SCAN_SIZE (1ull << 62)
+#define SCAN_SUM (2ull << 62)
+#define SCAN_VAL (SCAN_SIZE - 1ull)
 
 /* A status word carries its flag and its value together, and a reader
  * uses nothing else that the writer produced, so relaxed device-scope
@@ -982,89 +897,89 @@ __device__ __forceinline__ uint64_t ld_flag(const uint64_t *p)
     return v;
 }
 
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v)
+/* One thread: tile t's size (its sum, for a stream's first tile). */
+__device__ __forceinline__ void scan_publish(uint64_t *status, uint64_t t, uint32_t size, bool first)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    st_flag(status + t, (first ? SCAN_SUM : SCAN_SIZE) | size);
 }
 
-/* Any lane of the publishing warp may call it; lane 0 stores: this tile's
- * aggregate, or, for a first tile (no predecessor in its scan), its
- * inclusive value start + agg. */
-__device__ __forceinline__ void lb_publish(uint64_t *status, uint64_t tile, uint64_t agg, bool first,
-                                           uint64_t start)
+/* All lanes of a warp: the inclusive sum through a tile, waiting for it;
+ * SCAN_NONE and ZERR_TIMEOUT after `limit` polls. */
+#define SCAN_NONE (~0ull)
+__device__ __forceinline__ uint64_t scan_wait(const uint64_t *word, uint32_t limit, uint32_t *err)
 {
-    if ((threadIdx.x & 31u) == 0)
-        st_flag(status + tile, first ? (LB_FLAG_P | ((start + agg) & LB_VAL))
-                                        : (LB_FLAG_A | (agg & LB_VAL)));
+    uint64_t v = ld_flag(word);
+    uint32_t i = 0;
+#pragma unroll 1
+    while ((v >> 62) != 2u) { /* every lane reads the same word, but not at the same time */
+        if (++i >= limit) {
+            atomicOr(err, ZERR_TIMEOUT);
+            break;
+        }
+        __nanosleep(64);
+        v = ld_flag(word);
+    }
+    return __shfl_sync(0xffffffffu, (v >> 62) == 2u ? v & SCAN_VAL : SCAN_NONE, 0);
 }
 
-/* Called by all lanes of one warp after lb_publish: returns the exclusive
- * prefix of the tile (the sum of every tile back to and including the
- * nearest one that published an inclusive value, or `start` for a first
- * tile) and publishes the tile's inclusive value.  Each round inspects 256
- * predecessors (lane l reads tiles pos - l - 32k, k < 8, all loads in flight
- * together): with a persistent grid several hundred tiles are in flight at
- * once, and the nearest inclusive value is typically that far back.  A
- * predecessor that never publishes makes the wait give up after a bounded
- * number of polls: ZERR_TIMEOUT is set, the missing value counts as 0 and
- * the inclusive value is still published, so successors never hang. */
-static __device__ __noinline__ uint64_t lb_resolve(uint64_t *status, uint64_t tile, uint64_t agg,
-                                                   bool first, uint64_t start, uint32_t *err,
-                                                   uint32_t spin_limit = LB_SPIN_LIMIT)
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v);
+
+/* The scanning warp, over n tiles.  A tile that never publishes makes it
+ * give up after `limit` polls: ZERR_TIMEOUT is set, the tile's size counts
+ * as 0 and the scan goes on, so that no placer waits forever.  While the tile
+ * waited for is not yet handed out (its CTA is still waiting for room on the
+ * device), polls count 64-fold less. */
+static __device__ __noinline__ void scan_tiles(uint64_t *status, uint64_t n, const uint32_t *ticket, uint32_t *err,
+                                               uint32_t limit)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    if (first) return start;
-    uint64_t prefix = 0;
-    int64_t pos = (int64_t)tile - 1;
-    uint32_t spins = 0;
-    for (;;) {
+    uint64_t pos = 0, run = 0; /* tiles summed, their sum (within a stream) */
+    uint32_t polls = 0, idle = 0;
+#pragma unroll 1
+    while (pos < n) {
         uint64_t v[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            int64_t idx = pos - (int64_t)(lane + 32u * k);
-            v[k] = idx >= 0 ? ld_flag(status + idx) : LB_FLAG_P; /* before tile 0: value 0 */
+            const uint64_t i = pos + 32u * (uint32_t)k + lane;
+            v[k] = i < n ? ld_flag(status + i) : 0ull;
         }
-        /* nearest inclusive value: smallest distance lane + 32k flagged P */
-        uint32_t kp = 8, fp = 31, pending = 0;
+        uint32_t done = 0;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const uint32_t flag = (uint32_t)(v[k] >> 62);
-            const uint32_t pm = __ballot_sync(0xffffffffu, flag == 2u);
-            const uint32_t xm = __ballot_sync(0xffffffffu, flag == 0u);
-            if (kp == 8) {
-                if (pm) {
-                    kp = k;
-                    fp = (uint32_t)(__ffs(pm) - 1);
-                    pending |= xm & ((1u << fp) - 1u);
-                } else {
-                    pending |= xm;
-                }
+            if (done == 32u * (uint32_t)k) { /* uniform: every tile before these was ready */
+                const uint32_t flag = (uint32_t)(v[k] >> 62);
+                const uint32_t gap = ~__ballot_sync(0xffffffffu, flag != 0u);
+                const uint32_t cnt = gap ? (uint32_t)__ffs(gap) - 1u : 32u; /* ready in a row */
+                const uint32_t sums = __ballot_sync(0xffffffffu, flag == 2u) & ((2u << lane) - 1u); /* up to this lane */
+                const uint32_t inc = warp_incl_scan(flag == 1u && lane < cnt ? (uint32_t)v[k] : 0u);
+                const uint32_t from = sums ? 31u - (uint32_t)__clz(sums) : 0u;
+                const uint64_t at = __shfl_sync(0xffffffffu, v[k] & SCAN_VAL, from);
+                const uint32_t at_inc = __shfl_sync(0xffffffffu, inc, from);
+                const uint64_t sum = sums ? at + (inc - at_inc) : run + inc;
+                if (flag == 1u && lane < cnt) st_flag(status + pos + 32u * (uint32_t)k + lane, SCAN_SUM | sum);
+                if (cnt) run = __shfl_sync(0xffffffffu, sum, cnt - 1u);
+                done += cnt;
             }
         }
-        if (pending) {
-            if (++spins < spin_limit) {
-                __nanosleep(32);
-                continue;
-            }
-            /* give up: missing values count as 0 */
-            if (lane == 0) atomicOr(err, ZERR_TIMEOUT);
+        pos += done;
+        if (done) {
+            polls = 0;
+            continue;
         }
-        uint64_t c = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const bool ready = (v[k] >> 62) != 0;
-            if ((uint32_t)k < kp || ((uint32_t)k == kp && lane <= fp))
-                c += ready ? (v[k] & LB_VAL) : 0ull;
+        __nanosleep(32);
+        if (++polls < limit) continue;
+        if (limit == SCAN_SPIN_LIMIT && *(volatile const uint32_t *)ticket <= pos && ++idle < 64u) {
+            polls = 0;
+            continue;
         }
-        prefix += warp_sum_u64(c);
-        if (kp < 8) break;
-        pos -= 256;
-        spins = 0;
+        if (lane == 0) { /* give up */
+            atomicOr(err, ZERR_TIMEOUT);
+            st_flag(status + pos, SCAN_SUM | run);
+        }
+        pos++;
+        limit = 16;
+        polls = 0;
     }
-    if (lane == 0) st_flag(status + tile, LB_FLAG_P | ((prefix + agg) & LB_VAL));
-    return prefix & LB_VAL;
 }
 
 #endif

@@ -14,7 +14,11 @@
  * On the device a segment is cut into tiles of up to TB consecutive blocks;
  * tile 0 of a segment also owns the segment's head.  Tiles are numbered in
  * stream order, so the byte offset of a tile is the exclusive prefix sum of
- * the byte sizes of all tiles before it.  One CUDA thread owns one block.
+ * the byte sizes of all tiles before it.  A tile's blocks are cut into ZG_SUB
+ * groups of GB = TB / ZG_SUB blocks, one per warp of a codec CTA; the side
+ * index has an entry per group.  Within a warp, G = ceil(L / 8) neighbouring
+ * lanes share a block, eight elements each, so 32 / G blocks are worked on
+ * at a time.
  */
 #ifndef ZCCL_GB300_ZGEOM_H
 #define ZCCL_GB300_ZGEOM_H
@@ -28,6 +32,7 @@
 #endif
 
 #define ZG_MAX_L 256 /* largest block size the kernels accept */
+#define ZG_SUB 8u    /* block groups per tile (compute warps of a codec CTA) */
 
 typedef struct ZGeom {
     uint64_t n;       /* elements */
@@ -42,8 +47,12 @@ typedef struct ZGeom {
     uint64_t nt_rm;   /* tiles of the extra segment (0 when rem == 0) */
     uint64_t nblocks; /* all blocks */
     uint64_t ntiles;  /* all tiles */
+    uint64_t gr_reg;  /* index groups per regular segment (at least 1: the head's) */
+    uint64_t ngroups; /* all index groups */
     uint32_t fmt;     /* block magnitude layout: ZG_FASTMODE1 or ZG_FIXED_BYTES */
-    uint32_t pad_;
+    uint32_t GB;      /* blocks per index group */
+    uint32_t nt_rcp;  /* floor(2^32 / nt_reg) (2^32 - 1 for 1): division of tile numbers */
+    uint32_t small;   /* n < 2^31: every element, block and group number fits 32 bits */
 } ZGeom;
 
 /* Block magnitude layouts.  fastmode1: B = b/8 whole bytes per magnitude
@@ -62,6 +71,7 @@ typedef struct ZTile {
     uint64_t gblk0;     /* first block of the tile, index within the stream */
     uint64_t e_first;   /* first element of the first block (head + 1 + blk0*L) */
     uint64_t e_end;     /* one past the last element of the tile's last block */
+    uint64_t grp0;      /* first index group of the tile, index within the stream */
     uint32_t seg;       /* segment index (T for the extra segment) */
     uint32_t nblk;      /* blocks in the tile (0 for a segment of length 1) */
     uint32_t has_head;  /* tile 0 of its segment */
@@ -105,11 +115,6 @@ ZG_HD uint32_t zg_block_bytes_f(uint32_t fmt, uint32_t b, uint32_t n)
     return 1 + (n + 7) / 8 + B * n + (r * n + 7) / 8;
 }
 
-/* Row stride (in 4-byte words) of the padded per-block shared-memory layout:
- * odd, so thread t reading word j of row t hits bank (t*stride + j) % 32,
- * distinct across a warp. */
-ZG_HD uint32_t zg_row_stride(uint32_t L) { return (L & 1) ? L + 2 : L + 1; }
-
 ZG_HD uint64_t zg_seg_blocks(uint64_t len, uint32_t L) { return len ? zg_div_up(len - 1, L) : 0; }
 
 ZG_HD int zg_init(ZGeom *g, uint64_t n, uint32_t L, uint32_t T)
@@ -119,7 +124,8 @@ ZG_HD int zg_init(ZGeom *g, uint64_t n, uint32_t L, uint32_t T)
     g->T = T;
     g->L = L;
     g->fmt = ZG_FASTMODE1;
-    g->pad_ = 0;
+    g->small = n < (1ull << 31);
+    g->GB = zg_tile_blocks(L) / ZG_SUB;
     g->tbs = n / T;
     g->rem = (uint32_t)(n % T);
     g->TB = zg_tile_blocks(L);
@@ -130,20 +136,33 @@ ZG_HD int zg_init(ZGeom *g, uint64_t n, uint32_t L, uint32_t T)
     g->nblocks = (uint64_t)T * g->nb_reg + g->nb_rm;
     g->ntiles = (uint64_t)T * g->nt_reg + g->nt_rm;
     if (g->ntiles >> 32) return -1; /* tile indices are 32-bit on the device */
+    g->gr_reg = g->nb_reg ? zg_div_up(g->nb_reg, g->GB) : 1;
+    g->ngroups = (uint64_t)T * g->gr_reg + (g->rem ? (g->nb_rm ? zg_div_up(g->nb_rm, g->GB) : 1) : 0);
+    g->nt_rcp = g->nt_reg > 1 ? (uint32_t)((1ull << 32) / g->nt_reg) : 0xFFFFFFFFu;
     return 0;
+}
+
+/* t / nt_reg for t < 2^32 by the reciprocal: its floor, floor(2^32 / nt_reg)
+ * t / 2^32, is at most one too small (t / 2^32 < 1 bounds the loss). */
+ZG_HD uint32_t zg_seg_of(const ZGeom *g, uint32_t t)
+{
+    uint32_t s = (uint32_t)(((uint64_t)t * g->nt_rcp) >> 32);
+    if (t - s * (uint32_t)g->nt_reg >= (uint32_t)g->nt_reg) s++;
+    return s;
 }
 
 ZG_HD void zg_tile(const ZGeom *g, uint64_t t, ZTile *z)
 {
     uint64_t k, nb;
     if (t < (uint64_t)g->T * g->nt_reg) {
-        uint64_t s = (uint32_t)t / (uint32_t)g->nt_reg; /* tiles and tiles per segment < 2^32 */
+        uint64_t s = zg_seg_of(g, (uint32_t)t); /* tiles and tiles per segment < 2^32 */
         k = t - s * g->nt_reg;
         z->seg = (uint32_t)s;
         z->seg_start = s * g->tbs;
         z->seg_len = g->tbs;
         nb = g->nb_reg;
         z->gblk0 = s * g->nb_reg + k * g->TB;
+        z->grp0 = s * g->gr_reg + k * ZG_SUB;
     } else {
         k = t - (uint64_t)g->T * g->nt_reg;
         z->seg = g->T;
@@ -151,6 +170,7 @@ ZG_HD void zg_tile(const ZGeom *g, uint64_t t, ZTile *z)
         z->seg_len = g->rem;
         nb = g->nb_rm;
         z->gblk0 = (uint64_t)g->T * g->nb_reg + k * g->TB;
+        z->grp0 = (uint64_t)g->T * g->gr_reg + k * ZG_SUB;
     }
     z->blk0 = k * g->TB;
     uint64_t left = nb > z->blk0 ? nb - z->blk0 : 0;
@@ -160,6 +180,54 @@ ZG_HD void zg_tile(const ZGeom *g, uint64_t t, ZTile *z)
     uint64_t last = (z->blk0 + z->nblk) * g->L; /* elements after the head, capped below */
     if (last > z->seg_len - 1) last = z->seg_len - 1;
     z->e_end = z->seg_start + 1 + last;
+}
+
+/* Group `sub` of tile t: blocks [gblk, gblk + nblk) of the stream, the last of
+ * nlast elements, the first starting at element e_first. */
+typedef struct ZGroup {
+    uint64_t e_first, gblk, grp;
+    uint32_t nblk, nlast, has_head;
+} ZGroup;
+
+ZG_HD void zg_group(const ZGeom *g, uint64_t t, uint32_t sub, ZGroup *c)
+{
+    const uint32_t GB = g->GB, L = g->L, b0 = sub * GB;
+    if (g->small) { /* the same in 32 bits: a warp of the decompressor does this for every group */
+        const uint32_t reg = g->T * (uint32_t)g->nt_reg;
+        uint32_t s, k, nb, len;
+        if ((uint32_t)t < reg) {
+            s = zg_seg_of(g, (uint32_t)t);
+            k = (uint32_t)t - s * (uint32_t)g->nt_reg;
+            nb = (uint32_t)g->nb_reg;
+            len = (uint32_t)g->tbs;
+        } else {
+            s = g->T;
+            k = (uint32_t)t - reg;
+            nb = (uint32_t)g->nb_rm;
+            len = g->rem;
+        }
+        const uint32_t blk = k * g->TB + b0, left = nb > blk ? nb - blk : 0u;
+        c->nblk = left < GB ? left : GB;
+        c->has_head = k == 0 && sub == 0;
+        c->gblk = s * (uint32_t)g->nb_reg + blk;
+        c->grp = s * (uint32_t)g->gr_reg + k * ZG_SUB + sub;
+        c->e_first = s * (uint32_t)g->tbs + 1u + blk * L;
+        c->nlast = left > GB || !left ? L : len - 1u - (blk + c->nblk - 1u) * L;
+        if (c->nlast > L) c->nlast = L;
+        return;
+    }
+    ZTile z;
+    zg_tile(g, t, &z);
+    c->nblk = z.nblk > b0 ? (z.nblk - b0 < GB ? z.nblk - b0 : GB) : 0u;
+    c->has_head = z.has_head && sub == 0;
+    c->gblk = z.gblk0 + b0;
+    c->grp = z.grp0 + sub;
+    c->e_first = z.e_first + (uint64_t)b0 * L;
+    c->nlast = L;
+    if (c->nblk) {
+        const uint32_t rest = (uint32_t)(z.e_end - z.e_first) - (b0 + c->nblk - 1u) * L;
+        if (rest < L) c->nlast = rest;
+    }
 }
 
 /* Elements of block j (index within the segment) of a segment of len. */
@@ -184,18 +252,6 @@ ZG_HD uint64_t zg_stream_worst(const ZGeom *g)
     return 8ull * g->T + (uint64_t)g->T * zg_seg_worst(g->tbs, g->L) + zg_seg_worst(g->rem, g->L);
 }
 
-/* Shared-memory layout of the codec kernels (bytes), all regions 16-byte
- * aligned:
- *   [0, 256)   mbarriers, scan scratch, broadcast slots
- *   [256, 512) look-back records
- *   rows       per-block rows, TB x row_stride 4-byte words (floats or ints)
- *   in0, in1   double-buffered TMA input (raw floats or tile bytes)
- *   out        packed output tile (compressor, homomorphic add)
- *   jobs       copies of the jobs in progress (job_bytes) */
-typedef struct ZSmem {
-    uint32_t rows, in0, in1, out, jobs, total;
-} ZSmem;
-
 ZG_HD uint32_t zg_a16(uint32_t v) { return (v + 15u) & ~15u; }
 
 /* Largest tile in bytes: head + TB blocks at width 32. */
@@ -207,58 +263,5 @@ ZG_HD uint32_t zg_tile_worst(uint32_t L, uint32_t TB) { return TB * zg_block_byt
  * behind the ring has that slack. */
 ZG_HD uint32_t zg_ring_need(uint32_t total) { return (total + 8u + 15u) & ~15u; }
 ZG_HD uint32_t zg_ring_bytes(uint32_t L, uint32_t TB) { return zg_ring_need(zg_tile_worst(L, TB)); }
-
-/* kind: 0 compressor, 1 decompressor, 2 homomorphic add.
- * The compressor stages one tile of floats at a time (in1 == in0) and keeps
- * a packed tile in out until the next tile has been quantized.  With
- * L <= 32 every warp holds its rows' floats in registers while they move
- * from the input into the rows, so the rows share the input's space
- * (rows == in0); longer blocks get separate regions.  The decompressor and
- * the homomorphic add double-buffer their input. */
-ZG_HD ZSmem zg_smem_base(uint32_t kind, uint32_t L, uint32_t TB);
-
-ZG_HD ZSmem zg_smem(uint32_t kind, uint32_t L, uint32_t TB, uint32_t job_bytes)
-{
-    ZSmem m = zg_smem_base(kind, L, TB);
-    m.jobs = m.total;
-    m.total = zg_a16(m.jobs + job_bytes);
-    return m;
-}
-
-ZG_HD ZSmem zg_smem_base(uint32_t kind, uint32_t L, uint32_t TB)
-{
-    ZSmem m;
-    const uint32_t rows_bytes = TB * zg_row_stride(L) * 4u;
-    const uint32_t raw_in = (TB * L + 1u) * 4u + 32u;     /* floats, 16-byte superset */
-    const uint32_t tile_in = zg_tile_worst(L, TB) + 48u;  /* bytes, superset + reader slack */
-    const uint32_t tile_out = zg_ring_bytes(L, TB) + 48u; /* the ring; readers look 32 past */
-    const int need_rows = kind != 2 || L > 32;
-    m.rows = 1024u;
-    if (kind == 0) {
-        if (L <= 32) {
-            m.in0 = m.rows;
-            m.in1 = m.in0;
-            m.out = zg_a16(m.rows + (rows_bytes > raw_in ? rows_bytes : raw_in));
-            m.total = zg_a16(m.out + tile_out);
-        } else {
-            m.in0 = zg_a16(m.rows + rows_bytes);
-            m.in1 = m.in0;
-            m.out = zg_a16(m.in0 + raw_in);
-            m.total = zg_a16(m.out + tile_out);
-        }
-        return m;
-    }
-    m.in0 = zg_a16(m.rows + (need_rows ? rows_bytes : 0u));
-    if (kind == 1) { /* one input buffer: three CTAs per SM instead of two buffers' two */
-        m.in1 = m.in0;
-        m.out = zg_a16(m.in0 + tile_in);
-        m.total = m.out;
-        return m;
-    }
-    m.in1 = zg_a16(m.in0 + tile_in);
-    m.out = zg_a16(m.in1 + tile_in);
-    m.total = zg_a16(m.out + tile_out);
-    return m;
-}
 
 #endif

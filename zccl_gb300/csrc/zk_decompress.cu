@@ -2,346 +2,385 @@
  * zk_decompress.cu -- decompressor.
  *
  * Replaces ZCCL_float_decompress_openmp_threadblock_arg
- * (ZCCL/src/ZCCLd_float.c:538-754) and produces the same floats.  Persistent
- * CTAs, one thread per block, mirroring the compressor.  With the index
- * holding every tile's starting value the tiles are independent: CTA c
- * takes tiles c, c + grid, ... and loads the index entries of the tile
- * after next while it works.  A stream that arrived as bytes gets those
- * values first: the same kernel in its SUMS form writes every tile's delta
- * sum into the index, and k_qprev_scan turns them, segment by segment, into
- * starting values from the segment's raw head.
- * Per tile:
- *   1. for the NEXT tile: block sizes from the width index, a block-wide
- *      scan for every block's offset, and one TMA bulk copy of its bytes,
- *      so the copy runs while the current tile is decoded (double buffer);
- *   2. every thread unpacks its block (sign bits, high bytes, low-bit
- *      stream, ZCCL/src/ZCCL_TypeManager.c:423-950) into int32 deltas;
- *   3. a block-wide scan of the per-block delta sums, started from the
- *      quantized value before the tile (from the index), restores the
- *      running values (ZCCLd_float.c:617-628);
- *   4. x = (float)q * eb (ZCCLd_float.c:624) into padded rows, written out
- *      row by row with coalesced stores.
+ * (ZCCL/src/ZCCLd_float.c:538-754) and produces the same floats, for one
+ * stream or a batch of them, written or added to the destination (the DOC
+ * reduce step's decompress-then-add, ZCCL/src/ZCCL_ring.c:1074-1076, in one
+ * pass with one rounding per sum).
+ *
+ * The side index holds, for every group of blocks, the quantized value
+ * before it, so groups are independent.  CTA c takes tiles c, c + grid, ...
+ * A producer warp does the work that is the same for a whole tile: its
+ * geometry, its blocks' widths and offsets (from the width index, requested
+ * a tile ahead), and one TMA bulk copy of its bytes.  Eight consumer warps
+ * take a group of the tile each, with no barrier and no wait on each other:
+ *   1. every lane decodes its block (sign bits, high bytes, low-bit stream,
+ *      ZCCL/src/ZCCL_TypeManager.c:423-950) into running sums, and a warp
+ *      scan of the blocks' sums restores the running values
+ *      (ZCCLd_float.c:617-628);
+ *   2. x = (float)q * eb (ZCCLd_float.c:624) goes through shared memory at
+ *      the destination's 16-byte phase and out in whole vectors.
+ * Groups with a short block, a block of another length than 32, the
+ * fixed-byte layout or a width above 15 go eight elements a lane instead
+ * (decode_octet).
+ * A stream that arrived as bytes gets its groups' starting values first: the
+ * same kernel in its SUMS form writes every group's delta sum into the
+ * index, and k_qprev_scan turns them, segment by segment, into starting
+ * values from the segment's raw head.
  */
 #include <cudaTypedefs.h>
 
-#include <cstring>
 #include <mutex>
 
 #include "zkern.cuh"
 
 namespace {
 
-/* Per-thread view of its block in a staged tile. */
-struct BlockSlot {
-    uint32_t b, n, off;
+constexpr uint32_t DEC_WARPS = ZG_SUB;            /* consumer warps */
+constexpr uint32_t DEC_THREADS = 32 * DEC_WARPS + 32; /* and the producer */
+
+/* A staged tile, written by the producer before its copy's barrier fires. */
+struct DTile {
+    uint64_t tile;    /* ZP_NONE: no more tiles */
+    float *y;         /* the tile's first block's first element */
+    int32_t *qout;    /* SUMS: the tile's groups' index entries */
+    uint32_t nblk, nlast, head;
+    uint32_t fmt, body; /* first block's place in shared memory, from the input buffer's start */
+    float eb;
+    uint32_t acc, pad;
+    uint32_t q0[ZG_SUB]; /* the value before each group */
 };
 
-/* The index entries one tile needs: this thread's block width, and on
- * thread 0 the tile's byte offset and the quantized value before it.  Loaded
- * a tile ahead of their use, so the loads' latency is hidden. */
-struct TileIdx {
-    uint32_t b;
-    uint64_t base;
-    uint32_t q0;
+struct DShared {
+    uint64_t full[2], empty[2];
+    DTile t[2];
+    uint32_t ent[2][256]; /* per block: offset from body << 8 | width */
 };
+constexpr uint32_t DEC_HEAD = (sizeof(DShared) + 127u) / 128u * 128u;
 
-__device__ __forceinline__ TileIdx load_idx(const DecompressArgs &a, uint64_t t, const ZTile &z)
+/* The producer warp.  The two tiles in flight share the input buffer, one
+ * at its start and one at its end (typical tiles are far below the largest,
+ * so two fit; one that does not waits for the other to be decoded). */
+template <bool L32, bool BATCH, bool QPREV>
+__device__ __forceinline__ void produce(const DecompressArgs &a, DShared *sh, uint8_t *buf, uint32_t room, uint32_t &bad)
 {
-    TileIdx r = {0, 0, 0};
-    if (t >= a.g.ntiles) return r;
-    if (threadIdx.x < z.nblk) r.b = a.idx.widths[z.gblk0 + threadIdx.x];
-    if (threadIdx.x == 0) {
-        r.base = a.idx.tile_off[t];
-        if (a.qprev_valid) r.q0 = (uint32_t)a.idx.tile_qprev[t];
-    }
-    return r;
-}
-
-/* Thread 0: the TMA copy of a tile's `total` bytes at the index's byte
- * offset (checked against the readable bytes) into buf; its offset and
- * starting value into *s_base and *s_q0. */
-__device__ __forceinline__ void issue_tile(const DecompressArgs &a, const TileIdx &ix, uint32_t total, uint8_t *buf,
-                                           uint64_t *bar, uint64_t *s_base, uint32_t *s_q0, uint32_t &bad)
-{
-    uint64_t base = ix.base;
-    uint32_t nload = total;
-    /* overflow-safe: base comes from the index and is not trusted */
-    if (base > a.avail || total > a.avail - base) {
-        bad |= ZERR_BOUNDS;
-        nload = base < a.avail ? (uint32_t)min((uint64_t)total, a.avail - base) : 0u;
-        if (base > a.avail) base = 0;
-    }
-    *s_base = base;
-    *s_q0 = ix.q0;
-    tma_load_superset(buf, a.in + base, nload, bar);
-}
-
-/* All threads: sizes of tile t's blocks (geometry z), their offsets, and
- * (thread 0) the TMA copy of the tile's bytes into buf.  Returns the slot of
- * this thread's block; the tile's byte offset lands in *s_base, its starting
- * value in *s_q0. */
-__device__ __forceinline__ BlockSlot stage_tile(const DecompressArgs &a, const ZTile &z, const TileIdx &ix,
-                                                uint8_t *buf, uint64_t *bar, uint32_t *wsum,
-                                                uint64_t *s_base, uint32_t *s_q0, uint32_t &bad)
-{
-    BlockSlot sl = {0, 0, 0};
-    uint32_t size = 0;
-    if (threadIdx.x < z.nblk) {
-        sl.n = zg_block_len(z.seg_len, a.g.L, z.blk0 + threadIdx.x);
-        sl.b = ix.b;
-        if (sl.b > 32) {
-            bad |= ZERR_CORRUPT;
-            sl.b = 0;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t ntiles = BATCH ? a.batch.ntiles : a.job.g.ntiles;
+    const DecompressJob *nj = nullptr; /* the requested tile: its job, geometry, index entries */
+    ZTile nz;
+    uint64_t nbase = 0;
+    uint32_t nq = 0, nw[3] = {0, 0, 0};
+    auto request = [&](uint64_t t) {
+        uint64_t local = t;
+        if (BATCH) nj = static_cast<const DecompressJob *>(a.batch.jobs) + batch_job(a.batch, t, &local);
+        const DecompressJob &J = BATCH ? *nj : a.job;
+        zg_tile(&J.g, local, &nz);
+        nbase = J.idx.grp_off[nz.grp0];
+        if (QPREV && (lane == 0 || (lane < ZG_SUB && lane * J.g.GB < nz.nblk))) nq = (uint32_t)J.idx.grp_qprev[nz.grp0 + lane];
+        load_widths(J.idx.widths + nz.gblk0, nz.nblk, nw);
+    };
+    uint64_t t = blockIdx.x;
+    if (t < ntiles) request(t);
+    uint32_t ppos = 0, plen = 0; /* the previous tile's place */
+    for (uint32_t seq = 0;; seq++, t += gridDim.x) {
+        const uint32_t s = seq & 1u;
+        if (t >= ntiles) {
+            if (seq >= 2) mbar_wait(&sh->empty[s], ((seq >> 1) + 1u) & 1u, a.w.err);
+            if (lane == 0) {
+                sh->t[s].tile = ZP_NONE;
+                mbar_arrive(&sh->full[s]);
+            }
+            return;
         }
-        size = a.g.fmt == ZG_FASTMODE1 && sl.n == 32 ? block32_bytes(sl.b) : zg_block_bytes_f(a.g.fmt, sl.b, sl.n);
+        const DecompressJob &J = BATCH ? *nj : a.job;
+        const ZTile z = nz;
+        uint64_t base = nbase;
+        const uint32_t wsh = widths_shift(J.idx.widths + nz.gblk0);
+        const uint32_t q = nq, w0 = __funnelshift_r(nw[0], nw[1], wsh), w1 = __funnelshift_r(nw[1], nw[2], wsh);
+        const uint32_t L = J.g.L;
+        if (t + gridDim.x < ntiles) request(t + gridDim.x);
+
+        const uint32_t nlast = z.nblk ? (uint32_t)(z.e_end - z.e_first) - (z.nblk - 1u) * L : 0u;
+        const uint32_t fmt = J.g.fmt;
+        uint4 e[2];
+        const uint32_t total = tile_entries<L32>(L, fmt, z.nblk, nlast, w0, w1, e, bad) + (z.has_head ? 4u : 0u);
+        const uint32_t len = ((uint32_t)((uintptr_t)(J.in + base) & 15u) + total + 15u) & ~15u; /* of the aligned superset */
+
+        if (seq >= 2) mbar_wait(&sh->empty[s], ((seq >> 1) + 1u) & 1u, a.w.err); /* tile seq - 2 is decoded */
+        uint32_t pos = 0;
+        if (seq >= 1) {
+            if (ppos == 0 ? plen + len <= room : len <= ppos)
+                pos = ppos == 0 ? room - len : 0u;
+            else /* no room beside it: wait for tile seq - 1 too */
+                mbar_wait(&sh->empty[s ^ 1u], ((seq - 1u) >> 1) & 1u, a.w.err);
+        }
+        ppos = pos;
+        plen = len;
+        uint32_t nload = total;
+        /* overflow-safe: base comes from the index and is not trusted */
+        if (base > J.avail || total > J.avail - base) {
+            bad |= ZERR_BOUNDS;
+            nload = base < J.avail ? (uint32_t)min((uint64_t)total, J.avail - base) : 0u;
+            if (base > J.avail) base = 0;
+        }
+        DTile &d = sh->t[s];
+        if (lane < ZG_SUB) d.q0[lane] = q;
+        uint4 *tab = reinterpret_cast<uint4 *>(&sh->ent[s][8u * lane]);
+        tab[0] = e[0];
+        tab[1] = e[1];
+        if (lane == 0) {
+            d.tile = t;
+            d.y = J.y + z.e_first;
+            d.qout = J.idx.grp_qprev + z.grp0;
+            d.nblk = z.nblk;
+            d.nlast = nlast;
+            d.head = z.has_head;
+            d.fmt = fmt;
+            d.body = pos + (uint32_t)((uintptr_t)(J.in + base) & 15u) + (z.has_head ? 4u : 0u);
+            d.eb = J.eb;
+            d.acc = J.accumulate != 0;
+        }
+        __syncwarp();
+        if (lane == 0) tma_load_superset(buf + pos, J.in + base, nload, &sh->full[s]);
     }
-    uint32_t total;
-    sl.off = cta_excl_scan(size, wsum, &total);
-    if (threadIdx.x == 0) issue_tile(a, ix, total + (z.has_head ? 4u : 0u), buf, bar, s_base, s_q0, bad);
-    return sl;
 }
 
-/* CTA c takes tiles c, c + grid, c + 2 grid, ..., with the index entries of
- * the tile after next already loading.  SUMS: only each tile's wrapped sum of
- * deltas, into the index's tile_qprev (k_qprev_scan completes it). */
-template <bool FAST, bool SUMS>
-__global__ void __launch_bounds__(256, 3) k_decompress(const DecompressArgs a, const __grid_constant__ CUtensorMap ymap)
+/* MODE 0: floats (or, by the job's flag, added floats); 1: only each
+ * group's wrapped sum of deltas, into the index's grp_qprev. */
+template <bool L32, int MODE, bool BATCH>
+__global__ void __launch_bounds__(DEC_THREADS, 3) k_decompress(const __grid_constant__ DecompressArgs a)
 {
-    extern __shared__ __align__(16) uint8_t smem[];
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem); /* [2] */
-    uint32_t *wsum = reinterpret_cast<uint32_t *>(smem + 16);
-    uint64_t *s_base = reinterpret_cast<uint64_t *>(smem + 192); /* [2] */
-    uint32_t *s_q0 = reinterpret_cast<uint32_t *>(smem + 208);   /* [2] */
-    uint32_t *ws1 = reinterpret_cast<uint32_t *>(smem + 320); /* [33] second scan scratch */
-    uint32_t *ws2 = reinterpret_cast<uint32_t *>(smem + 464); /* [33] the same pair, odd rounds */
-    uint32_t *ws3 = reinterpret_cast<uint32_t *>(smem + 608); /* [33] */
-    /* [4] geometry of the tiles in flight, each found once by thread 0 before
-     * a scan's barrier: the tile's (it % 4), the next one's, the one after
-     * (for its index entries); a slot is rewritten two rounds after its
-     * tile's, when every thread is past that tile */
-    ZTile *zs = reinterpret_cast<ZTile *>(smem + 752);
-    static_assert(752 + 4 * sizeof(ZTile) <= 1024, "the tile records fit below the rows");
-    float *rows = reinterpret_cast<float *>(smem + a.sm.rows);
-
-    const ZGeom &g = a.g;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
-    const uint32_t L = g.L, stride = zg_row_stride(L);
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    DShared *sh = reinterpret_cast<DShared *>(smem);
+    uint8_t *buf = smem + DEC_HEAD;
+    const uint32_t L = L32 ? 32u : a.job.g.L, GB = L32 ? 32u : a.job.g.GB; /* one L for the whole batch */
     uint32_t bad = 0;
-    /* Full tiles of L = 32 whose first element minus one starts a 128-byte
-     * row of y leave by TMA tensor stores, one per warp of 32 rows of 32
-     * floats (the element before the tile first), from a 1024-byte-aligned
-     * box with the 128-byte swizzle (16-byte chunk k of row r at chunk
-     * k ^ (r & 7)), so that each thread's vector stores of its row meet no
-     * bank conflict. */
-    const uint32_t rows_sa = smem_u32(rows);
-    const uint32_t box_sa = (rows_sa + 1023u) & ~1023u;
-    const bool rows_ok = FAST && a.rows_map && L == 32 && g.TB == 256 && blockDim.x == 256 &&
-                         box_sa + 32768u <= rows_sa + g.TB * stride * 4u;
     /* The index walk ran to completion before this launch, so every CTA sees
-     * the same word: after a failed walk no CTA touches the stream and no
-     * CTA waits on another. */
+     * the same word: after a failed walk no CTA touches the stream. */
     if (*(volatile const uint32_t *)a.w.walk_err) return;
-
-    uint64_t tile = blockIdx.x;
-    uint64_t tnext = tile + gridDim.x; /* the static order's next tile */
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        if (tile < g.ntiles) zg_tile(&g, tile, &zs[0]);
-        if (tnext < g.ntiles) zg_tile(&g, tnext, &zs[1]);
+        mbar_init(&sh->full[0], 1);
+        mbar_init(&sh->full[1], 1);
+        mbar_init(&sh->empty[0], DEC_WARPS);
+        mbar_init(&sh->empty[1], DEC_WARPS);
     }
     __syncthreads();
-    TileIdx ix = load_idx(a, tile, zs[0]);
-    BlockSlot cur = {0, 0, 0};
-    if (tile < g.ntiles) cur = stage_tile(a, zs[0], ix, smem + a.sm.in0, &bar[0], wsum, &s_base[0], &s_q0[0], bad);
-    ix = load_idx(a, tnext, zs[1]);
+    if (warp == DEC_WARPS) {
+        produce<L32, BATCH, MODE == 0>(a, sh, buf, a.room, bad);
+        if (bad) atomicOr(a.w.err, bad);
+        return;
+    }
 
-    /* One barrier a tile, the scan's (one more before the rows leave when a
-     * tile has short or long blocks).  The input buffer the next copy
-     * overwrites was last read before this tile's scan; the tile's byte
-     * offset and starting value (thread 0, at the copy) are visible through
-     * the copy's mbarrier; each warp writes and sends out only its own 32
-     * rows, and its box rows are free again once its lane 0 has seen its
-     * last store read them, before the scan. */
-    for (uint32_t it = 0;; it++) {
-        const uint32_t cb = it & 1u;
-        if (tile >= g.ntiles) break;
-        const ZTile &z = zs[it & 3u];
-
-        BlockSlot nxt = {0, 0, 0}; /* the next tile's block, found in step 3 */
-        uint32_t next_bytes = 0;  /* the next tile's bytes */
-        bool issue_now = true;    /* its copy starts right after the scan */
-        TileIdx ixn;              /* its index entries */
-
-        /* 2. unpack this tile's deltas */
-        mbar_wait(&bar[cb], (it >> 1) & 1u, a.w.err);
-        const uint8_t *buf = smem + (cb ? a.sm.in1 : a.sm.in0);
-        const uint32_t *sw = reinterpret_cast<const uint32_t *>(buf);
-        const uint32_t ph = (uint32_t)((uintptr_t)(a.in + s_base[cb]) & 15u);
-        int32_t head = 0;
-        if (z.has_head) {
-            uint32_t h = 0;
+    float *stage = reinterpret_cast<float *>(buf + a.in_bytes) + warp * ((GB * L + 31u) / 32u * 32u);
+    const uint32_t *sw = reinterpret_cast<const uint32_t *>(buf);
+    const uint32_t rb = smem_u32(stage) + lane * 128u, x4 = (lane & 7u) << 4;
+    const uint32_t sb = smem_u32(stage) + ((lane >> 3) << 7);
+    const uint64_t max_tiles = BATCH ? a.batch.ntiles : a.job.g.ntiles;
+    for (uint32_t seq = 0; seq <= max_tiles; seq++) { /* bounded even if a wait gave up */
+        const uint32_t s = seq & 1u;
+        mbar_wait(&sh->full[s], (seq >> 1) & 1u, a.w.err);
+        const DTile &D = sh->t[s];
+        if (D.tile == ZP_NONE) break;
+        const uint32_t tb = D.nblk, b0 = warp * GB;
+        const uint32_t nblk = tb > b0 ? min(GB, tb - b0) : 0u;
+        const uint32_t nlast = b0 + nblk == tb ? D.nlast : L; /* elements of the group's last block */
+        const uint32_t body = D.body, fmt = D.fmt, run0 = D.q0[warp];
+        const bool head = warp == 0 && D.head, acc = D.acc != 0;
+        const float eb = D.eb;
+        int32_t *qout = MODE == 1 ? D.qout : nullptr;
+        float *y = D.y + b0 * L;
+        auto put = [&](float *at, float x) { *at = acc ? __fadd_rn(*at, x) : x; };
+        uint32_t e = lane < nblk ? sh->ent[s][b0 + lane] : 0u;
+        const uint32_t b = e & 0xFFu, o = body + (e >> 8);
+        if (lane < nblk && buf[o] != b) bad |= ZERR_CORRUPT;
+        uint32_t sum = 0;
+        if (L32 && nblk == 32 && nlast == 32 && fmt == ZG_FASTMODE1 && __all_sync(0xffffffffu, b < 16)) {
+            /* running values from the block's start, then one scan of the
+             * blocks' sums.  In floats, which are exact while every value is
+             * an integer below 2^24: the 32 magnitudes of a block move the
+             * running value by less than 2^20, which leaves room for a
+             * starting value below 2^23. */
+            float v[32], f = 0.f;
+            decode_small_f(sw, o, b, 32u, [&](int j, float m, uint32_t sg) {
+                f += with_sign(m, sg, j);
+                v[j] = f;
+            });
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->empty[s]); /* this warp is done with the tile's bytes and entries */
+            sum = (uint32_t)__float2int_rn(f);
+            if (MODE == 0) {
+                const uint32_t q0 = run0 + warp_incl_scan(sum) - sum;
+                if (__all_sync(0xffffffffu, (uint32_t)abs((int32_t)q0) < (1u << 23))) {
+                    const float f0 = __int2float_rn((int32_t)q0);
 #pragma unroll
-            for (int k = 0; k < 4; k++) h |= (uint32_t)buf[ph + k] << (8 * k);
-            head = (int32_t)h;
-        }
-        const uint32_t headb = z.has_head ? 4u : 0u;
-        const uint32_t o = ph + headb + cur.off; /* this block, in buffer coordinates */
-        const uint32_t b = cur.b, n = cur.n;
-        const bool own = tid < z.nblk;
-        const bool full = FAST && own && n == 32;
-        uint32_t d[32];
-        uint32_t bsum = 0;
-        if (own && buf[o] != b) bad |= ZERR_CORRUPT;
-        if (full) {
-            bsum = g.fmt == ZG_FASTMODE1 ? decode_block32(sw, o, b, d) : decode_full(sw, o, b, d, g.fmt);
-        } else if (own) { /* short or long block: sum now, decode again for the values */
-            decode_any(sw, o, b, n, [&](uint32_t, uint32_t v) { bsum += v; }, g.fmt);
-        }
-
-        /* 3. starting value of every block.  In index order the next tile's
-         *    block offsets come from the same scan (its widths arrived a tile
-         *    ago), and its copy starts right after, into the other buffer. */
-        uint32_t tsum, pre;
-        {
-            const ZTile &zn = zs[(it + 1u) & 3u];
-            uint32_t sizen = 0;
-            if (tid == 0 && tnext + gridDim.x < g.ntiles) zg_tile(&g, tnext + gridDim.x, &zs[(it + 2u) & 3u]);
-            if (tnext < g.ntiles) {
-                if (tid < zn.nblk) {
-                    nxt.n = zg_block_len(zn.seg_len, L, zn.blk0 + tid);
-                    nxt.b = ix.b;
-                    if (nxt.b > 32) {
-                        bad |= ZERR_CORRUPT;
-                        nxt.b = 0;
-                    }
-                    sizen = g.fmt == ZG_FASTMODE1 && nxt.n == 32 ? block32_bytes(nxt.b)
-                                                                  : zg_block_bytes_f(g.fmt, nxt.b, nxt.n);
+                    for (int j = 0; j < 32; j++) v[j] = __fmul_rn(__fadd_rn(v[j], f0), eb);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        v[j] = __fmul_rn(__int2float_rn((int32_t)(q0 + (uint32_t)__float2int_rn(v[j]))), eb);
                 }
-            }
-            uint32_t totn;
-            if (!SUMS && lane == 0) bulk_wait_read0(); /* the warp's last box store has left the rows */
-            grp_excl_scan2_1(bsum, sizen, cb ? wsum : ws2, cb ? ws1 : ws3, pre, nxt.off, tsum, totn, blockDim.x, 0);
-            /* with one input buffer, a tile with short or long blocks reads
-             * it again for the values: its successor's copy waits for that */
-            next_bytes = totn + (tnext < g.ntiles && zn.has_head ? 4u : 0u);
-            issue_now = SUMS || a.sm.in0 != a.sm.in1 ||
-                        (FAST && L == 32 && z.nblk == g.TB && z.e_end - z.e_first == 32ull * g.TB);
-            if (tnext < g.ntiles && tid == 0 && issue_now)
-                issue_tile(a, ix, next_bytes, smem + (cb ? a.sm.in0 : a.sm.in1), &bar[cb ^ 1u], &s_base[cb ^ 1u],
-                           &s_q0[cb ^ 1u], bad);
-            ixn = ix;
-            ix = load_idx(a, tnext + gridDim.x, zs[(it + 2u) & 3u]);
-        }
-        if (SUMS) { /* the tile's delta sum; the values wait for the scan */
-            if (tid == 0) a.idx.tile_qprev[tile] = (int32_t)tsum;
-            cur = nxt;
-            tile = tnext;
-            tnext += gridDim.x;
-            continue;
-        }
-        const uint32_t q0 = z.has_head ? (uint32_t)head : s_q0[cb];
-        const bool box = rows_ok && z.nblk == 256 && z.e_end - z.e_first == 8192 && ((z.e_first - 1) & 31) == 0;
-
-        /* 4. values into rows, then out */
-        float *row = rows + tid * stride;
-        if (box) { /* every block is full: element e_first + 32 tid + j is box float 1 + 32 tid + j */
-            uint32_t q = q0 + pre;
-            /* the float before this block, the previous block's last (or the
-             * value before the tile: the head, or the previous tile's last
-             * element, stored there too with the same bits) */
-            const float prev = __fmul_rn(__int2float_rn((int32_t)q), a.eb);
-            float v[32];
+                /* rows of 32 floats at the destination's phase p: the last p
+                 * elements of the lane before, then this lane's; 16-byte
+                 * chunk k of row r at chunk k ^ (r & 7), so neither these
+                 * stores nor the reads below conflict */
+                const uint32_t p = (uint32_t)((uintptr_t)y >> 2) & 3u;
+                auto row = [&](int pc, float w0, float w1, float w2) {
+                    auto u = [&](int j) { return j >= pc ? v[j - pc] : j == pc - 1 ? w0 : j == pc - 2 ? w1 : w2; };
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                q += d[j];
-                v[j] = __fmul_rn(__int2float_rn((int32_t)q), a.eb);
-            }
-            const uint32_t rb = box_sa + tid * 128u, x4 = (tid & 7u) << 4;
-            st_shared_v4(rb | x4, prev, v[0], v[1], v[2]);
+                    for (int k = 0; k < 8; k++)
+                        st_shared_v4(rb | (((uint32_t)k << 4) ^ x4), u(4 * k), u(4 * k + 1), u(4 * k + 2), u(4 * k + 3));
+                };
+                auto before = [&](float x) { return __shfl_up_sync(0xffffffffu, x, 1); };
+                if (p == 1) /* uniform; first as the usual case: the element after a segment's head */
+                    row(1, before(v[31]), 0.f, 0.f);
+                else if (p == 0)
+                    row(0, 0.f, 0.f, 0.f);
+                else if (p == 2)
+                    row(2, before(v[31]), before(v[30]), 0.f);
+                else
+                    row(3, before(v[31]), before(v[30]), before(v[29]));
+                /* the first vector's elements from p on, and the p elements
+                 * past the last vector */
+                if (p && lane == 0) {
+                    put(y, v[0]);
+                    if (p < 3) put(y + 1, v[1]);
+                    if (p < 2) put(y + 2, v[2]);
+                }
+                if (p && lane == 31) {
+                    put(y + 1023, v[31]);
+                    if (p > 1) put(y + 1022, v[30]);
+                    if (p > 2) put(y + 1021, v[29]);
+                }
+                if (head && lane == 0) put(y - 1, __fmul_rn(__int2float_rn((int32_t)run0), eb));
+                __syncwarp();
+                float4 *y4 = reinterpret_cast<float4 *>(y - p) + lane;
+                const bool first = !p || lane; /* vector 0 is ragged unless p == 0 */
+                auto chunk = [&](uint32_t u) { /* vector lane + 32 u: chunk lane & 7 of row (lane >> 3) + 4 u */
+                    return ld_shared_v4(sb + u * 512u + (((lane & 7u) ^ (((lane >> 3) + 4u * u) & 7u)) << 4));
+                };
+                if (!acc) {
 #pragma unroll
-            for (uint32_t k = 1; k < 8; k++)
-                st_shared_v4(rb | ((k << 4) ^ x4), v[4 * k - 1], v[4 * k], v[4 * k + 1], v[4 * k + 2]);
-            if (tid == 255) a.y[z.e_end - 1] = v[31]; /* past the box; the others are the next rows' first */
-            fence_proxy_async_smem();
-            __syncwarp();
-            /* the warp's 32 rows leave by one TMA store */
-            if (lane == 0) tma_store_2d(&ymap, box_sa + warp * 4096u, 0, (int32_t)((z.e_first - 1) >> 5) + 32 * (int32_t)warp);
-        } else if (full) {
-            uint32_t q = q0 + pre;
+                    for (uint32_t u = 0; u < 8; u++) {
+                        const float4 x = chunk(u);
+                        if (u || first) y4[32u * u] = x;
+                    }
+                } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                q += d[j];
-                row[j] = __fmul_rn(__int2float_rn((int32_t)q), a.eb);
-            }
-        } else if (own) {
-            uint32_t q = q0 + pre;
-            decode_any(
-                sw, o, b, n,
-                [&](uint32_t j, uint32_t v) {
-                    q += v;
-                    row[j] = __fmul_rn(__int2float_rn((int32_t)q), a.eb);
-                },
-                g.fmt);
-        }
-        if (z.has_head && tid == 0) a.y[z.seg_start] = __fmul_rn(__int2float_rn(head), a.eb);
-        if (box) { /* each warp has sent its rows out above */
-        } else if (FAST && L == 32 && z.nblk == g.TB && z.e_end - z.e_first == 32ull * g.TB && nw * 32u == g.TB) {
-            /* a full tile: each warp stores its own 32 rows (no barrier),
-             * unrolled so that many stores are in flight */
-            __syncwarp();
-            float *dst = a.y + z.e_first + lane;
-#pragma unroll 8
-            for (uint32_t r = 0; r < 32; r++) {
-                const uint32_t k = warp * 32u + r;
-                dst[k * 32u] = rows[k * stride + lane];
+                    for (uint32_t h = 0; h < 2; h++) {
+                        float4 t[4];
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; u++) /* the loads ahead of the stores */
+                            t[u] = h || u || first ? y4[128u * h + 32u * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; u++) {
+                            const float4 x = chunk(4u * h + u);
+                            t[u].x = __fadd_rn(t[u].x, x.x);
+                            t[u].y = __fadd_rn(t[u].y, x.y);
+                            t[u].z = __fadd_rn(t[u].z, x.z);
+                            t[u].w = __fadd_rn(t[u].w, x.w);
+                            if (h || u || first) y4[128u * h + 32u * u] = t[u];
+                        }
+                    }
+                }
+                __syncwarp(); /* the stage is free again */
             }
         } else {
-            __syncthreads();
-            if (!issue_now && tnext < g.ntiles && tid == 0) /* every read of the one input buffer is done */
-                issue_tile(a, ixn, next_bytes, smem + (cb ? a.sm.in0 : a.sm.in1), &bar[cb ^ 1u], &s_base[cb ^ 1u],
-                           &s_q0[cb ^ 1u], bad);
-            for (uint32_t k = warp; k < z.nblk; k += nw) {
-                const uint32_t nk = zg_block_len(z.seg_len, L, z.blk0 + k);
-                float *dst = a.y + z.e_first + (uint64_t)k * L;
-                for (uint32_t j = lane; j < nk; j += 32) dst[j] = rows[k * stride + j];
+            /* G = ceil(L / 8) lanes share a block, BPI blocks at a time */
+            const uint32_t G = L32 ? 4u : (L + 7u) / 8u, BPI = 32u / G;
+            const uint32_t og = lane % G, bi = lane / G;
+            uint32_t run = run0;
+#pragma unroll 1
+            for (uint32_t k0 = 0; k0 < nblk; k0 += BPI) {
+                const uint32_t k = k0 + bi;
+                const bool has = bi < BPI && k < nblk;
+                e = has ? sh->ent[s][b0 + k] : 0u;
+                const uint32_t n = !has ? 0u : k + 1 < nblk ? L : nlast;
+                uint32_t d[8];
+                decode_octet(sw, body + (e >> 8), e & 0xFFu, n, og, fmt, d);
+                uint32_t tot = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) tot += d[j];
+                if (MODE == 1) {
+                    sum += tot;
+                    continue;
+                }
+                const uint32_t incl = warp_incl_scan(tot);
+                uint32_t q = run + incl - tot;
+                run += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    q += d[j];
+                    if (8u * og + (uint32_t)j < n)
+                        stage[k * L + 8u * og + (uint32_t)j] = __fmul_rn(__int2float_rn((int32_t)q), eb);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->empty[s]);
+            if (MODE == 0) {
+                if (head && lane == 0) put(y - 1, __fmul_rn(__int2float_rn((int32_t)run0), eb));
+                const uint32_t cnt = nblk ? (nblk - 1u) * L + nlast : 0u;
+                for (uint32_t i0 = lane; i0 < cnt; i0 += 256) { /* eight in flight */
+                    float t[8];
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u++) t[u] = acc && i0 + 32u * u < cnt ? y[i0 + 32u * u] : 0.f;
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u++)
+                        if (i0 + 32u * u < cnt) {
+                            const float x = stage[i0 + 32u * u];
+                            y[i0 + 32u * u] = acc ? __fadd_rn(t[u], x) : x;
+                        }
+                }
+                __syncwarp();
             }
         }
-        cur = nxt;
-        tile = tnext;
-        tnext += gridDim.x;
+        if (MODE == 1) {
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (lane == 0 && (nblk || head)) qout[warp] = (int32_t)sum;
+        }
     }
-    if (lane == 0) bulk_wait0();
     if (bad) atomicOr(a.w.err, bad);
 }
 
-/* One warp per segment: its tiles' delta sums (from k_decompress<_, true>)
- * become the quantized value before each tile, starting from the
- * segment's raw int32 head (the four bytes at its first tile's offset) and
- * wrapping like the reference's int32 running value (ZCCLd_float.c:582-628). */
-__global__ void k_qprev_scan(const DecompressArgs a)
+/* One CTA per segment: its groups' delta sums (from k_decompress in its SUMS
+ * form) become the quantized value before each group, starting from the
+ * segment's raw int32 head (the four bytes at its first group's offset) and
+ * wrapping like the reference's int32 running value (ZCCLd_float.c:582-628).
+ * Four groups a thread and one scan over the CTA a round: a segment of 64M
+ * floats is 16 rounds (a warp per segment took 2048 steps of one load's
+ * latency each). */
+__global__ void __launch_bounds__(1024) k_qprev_scan(const __grid_constant__ DecompressArgs a)
 {
-    const ZGeom &g = a.g;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t seg = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint64_t nseg = (uint64_t)g.T + (g.rem ? 1u : 0u);
-    if (seg >= nseg || *(volatile const uint32_t *)a.w.walk_err) return;
-    const uint64_t t0 = seg < g.T ? seg * g.nt_reg : (uint64_t)g.T * g.nt_reg;
-    const uint64_t nt = seg < g.T ? g.nt_reg : g.nt_rm;
-    const uint64_t off = a.idx.tile_off[t0];
+    __shared__ uint32_t ws[33];
+    const DecompressJob &J = a.job;
+    const ZGeom &g = J.g;
+    const uint64_t seg = blockIdx.x;
+    if (*(volatile const uint32_t *)a.w.walk_err) return;
+    const uint64_t g0 = seg * g.gr_reg;
+    const uint64_t ng = seg < g.T ? g.gr_reg : g.ngroups - (uint64_t)g.T * g.gr_reg;
+    const uint64_t off = J.idx.grp_off[g0];
     uint32_t run = 0;
-    if (off <= a.avail && a.avail - off >= 4) {
+    if (off <= J.avail && J.avail - off >= 4) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) run |= (uint32_t)a.in[off + k] << (8 * k);
-    } else if (lane == 0) {
+        for (int k = 0; k < 4; k++) run |= (uint32_t)J.in[off + k] << (8 * k);
+    } else if (threadIdx.x == 0) {
         atomicOr(a.w.err, ZERR_BOUNDS);
     }
-    for (uint64_t k0 = 0; k0 < nt; k0 += 32) {
-        const uint64_t k = k0 + lane;
-        const uint32_t v = k < nt ? (uint32_t)a.idx.tile_qprev[t0 + k] : 0u;
-        const uint32_t inc = warp_incl_scan(v);
-        if (k < nt) a.idx.tile_qprev[t0 + k] = (int32_t)(run + inc - v);
-        run += __shfl_sync(0xffffffffu, inc, 31);
+    for (uint64_t k0 = 0; k0 < ng; k0 += 4ull * blockDim.x) {
+        const uint64_t k = k0 + 4ull * threadIdx.x;
+        uint32_t v[4], s = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            v[i] = k + i < ng ? (uint32_t)J.idx.grp_qprev[g0 + k + i] : 0u;
+            s += v[i];
+        }
+        uint32_t tot;
+        uint32_t pre = run + cta_excl_scan(s, ws, &tot);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (k + i < ng) J.idx.grp_qprev[g0 + k + i] = (int32_t)pre;
+            pre += v[i];
+        }
+        run += tot;
     }
 }
 
@@ -365,50 +404,50 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_tiled()
 
 } // namespace
 
-bool zk_rows_map(CUtensorMap *map, const void *p, uint64_t n, uint32_t box_rows)
+bool zk_rows_map(CUtensorMap *map, const void *p, uint64_t n)
 {
-    const uint64_t nrows = n / 32u;
-    if (((uintptr_t)p & 15u) || nrows < 256u || nrows > 0x7fffffffull) return false;
+    const uint64_t before = ((uintptr_t)p & 15u) / 4u, nrows = (n + before) / 32u;
+    if (((uintptr_t)p & 3u) || nrows < 256u || nrows > 0x7fffffffull) return false;
     PFN_cuTensorMapEncodeTiled_v12000 enc = encode_tiled();
     if (!enc) return false;
     const cuuint64_t dim[2] = {32u, nrows};
     const cuuint64_t stride[1] = {128u};
-    const cuuint32_t box[2] = {32u, box_rows};
+    const cuuint32_t box[2] = {32u, 32u};
     const cuuint32_t estride[2] = {1u, 1u};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(p), dim, stride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(static_cast<const float *>(p) - before), dim, stride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-cudaError_t launch_decompress(const DecompressArgs &a, cudaStream_t st)
+cudaError_t launch_decompress(const DecompressArgs &a0, cudaStream_t st)
 {
-    const bool fast = a.g.L <= 32;
-    /* a stream without starting values: tile sums, then the scan per segment */
+    DecompressArgs a = a0;
+    const uint32_t L = a.job.g.L, GB = a.job.g.GB;
+    /* two typical tiles (at least one of the largest), room for the reads
+     * past a tile's end, and the floats */
+    a.room = zg_a16(zg_tile_worst(L, a.job.g.TB) + 15u);
+    a.in_bytes = (a.room + octet_slack(L) + 127u) / 128u * 128u;
+    const size_t smem = DEC_HEAD + a.in_bytes + DEC_WARPS * ((GB * L + 31u) / 32u * 128u);
+    const bool batch = a.batch.jobs != nullptr;
+    const uint64_t tiles = batch ? a.batch.ntiles : a.job.g.ntiles;
+    auto launch = [&](void (*k)(const DecompressArgs)) -> cudaError_t {
+        const cudaError_t e = set_max_smem((const void *)k, smem);
+        if (e != cudaSuccess) return e;
+        unsigned grid = persistent_grid((const void *)k, DEC_THREADS, smem, tiles);
+        if (a.grid && a.grid < grid) grid = a.grid;
+        k<<<grid, DEC_THREADS, smem, st>>>(a);
+        return cudaGetLastError();
+    };
+    /* a stream without starting values: group sums, then the scan per segment */
     if (!a.qprev_valid) {
-        const void *fs = fast ? (const void *)k_decompress<true, true> : (const void *)k_decompress<false, true>;
-        cudaError_t e = set_max_smem(fs, a.sm.total);
+        cudaError_t e = launch(L == 32 ? k_decompress<true, 1, false> : k_decompress<false, 1, false>);
         if (e != cudaSuccess) return e;
-        alignas(64) CUtensorMap none;
-        memset(&none, 0, sizeof none);
-        DecompressArgs b = a;
-        b.rows_map = 0;
-        void *args[] = {&b, &none};
-        e = cudaLaunchKernel(fs, dim3(persistent_grid(fs, a.g.TB, a.sm.total, a.g.ntiles)), dim3(a.g.TB), args,
-                             a.sm.total, st);
-        if (e != cudaSuccess) return e;
-        const unsigned nseg = a.g.T + (a.g.rem ? 1u : 0u);
-        k_qprev_scan<<<(nseg + 3) / 4, 128, 0, st>>>(a);
+        const unsigned nseg = a.job.g.T + (a.job.g.rem ? 1u : 0u);
+        const uint64_t most = a.job.g.gr_reg; /* groups of a segment (the extra one has fewer than T elements) */
+        const unsigned threads = most >= 4096 ? 1024u : (unsigned)((most + 127) / 128 * 32);
+        k_qprev_scan<<<nseg, threads < 32 ? 32 : threads, 0, st>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const void *fn = fast ? (const void *)k_decompress<true, false> : (const void *)k_decompress<false, false>;
-    cudaError_t e = set_max_smem(fn, a.sm.total);
-    if (e != cudaSuccess) return e;
-    unsigned grid = persistent_grid(fn, a.g.TB, a.sm.total, a.g.ntiles);
-    DecompressArgs b = a;
-    b.qprev_valid = 1;
-    alignas(64) CUtensorMap map;
-    memset(&map, 0, sizeof map);
-    b.rows_map = fast && zk_rows_map(&map, a.y, a.g.n, 32);
-    void *args[] = {&b, &map};
-    return cudaLaunchKernel(fn, dim3(grid), dim3(a.g.TB), args, a.sm.total, st);
+    if (batch) return launch(L == 32 ? k_decompress<true, 0, true> : k_decompress<false, 0, true>);
+    return launch(L == 32 ? k_decompress<true, 0, false> : k_decompress<false, 0, false>);
 }

@@ -40,6 +40,105 @@
 
 namespace {
 
+/* ---------------------------------------------------------------------
+ * Decoupled look-back (Merrill & Garland 2016).  status[t] packs a 2-bit
+ * flag (1 = aggregate of tile t only, 2 = inclusive prefix through t) over
+ * a 62-bit value; values add modulo 2^62.  Tiles are taken in ticket order,
+ * so every tile a CTA waits on belongs to a CTA that is already running and
+ * never waits on a later tile.
+ * ------------------------------------------------------------------- */
+/* Polls of a predecessor's word before the look-back gives up (about a
+ * second at the 32 ns back-off; callers may pass a smaller limit). */
+#define LB_SPIN_LIMIT (1u << 22)
+#define LB_FLAG_A (1ull << 62)
+#define LB_FLAG_P (2ull << 62)
+#define LB_VAL (LB_FLAG_A - 1ull)
+
+__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+/* Any lane of the publishing warp may call it; lane 0 stores: this tile's
+ * aggregate, or, for a first tile (no predecessor in its scan), its
+ * inclusive value start + agg. */
+__device__ __forceinline__ void lb_publish(uint64_t *status, uint64_t tile, uint64_t agg, bool first,
+                                           uint64_t start)
+{
+    if ((threadIdx.x & 31u) == 0)
+        st_flag(status + tile, first ? (LB_FLAG_P | ((start + agg) & LB_VAL))
+                                        : (LB_FLAG_A | (agg & LB_VAL)));
+}
+
+/* Called by all lanes of one warp after lb_publish: returns the exclusive
+ * prefix of the tile (the sum of every tile back to and including the
+ * nearest one that published an inclusive value, or `start` for a first
+ * tile) and publishes the tile's inclusive value.  Each round inspects 256
+ * predecessors (lane l reads tiles pos - l - 32k, k < 8, all loads in flight
+ * together): with a persistent grid several hundred tiles are in flight at
+ * once, and the nearest inclusive value is typically that far back.  A
+ * predecessor that never publishes makes the wait give up after a bounded
+ * number of polls: ZERR_TIMEOUT is set, the missing value counts as 0 and
+ * the inclusive value is still published, so successors never hang. */
+static __device__ __noinline__ uint64_t lb_resolve(uint64_t *status, uint64_t tile, uint64_t agg,
+                                                   bool first, uint64_t start, uint32_t *err,
+                                                   uint32_t spin_limit = LB_SPIN_LIMIT)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    if (first) return start;
+    uint64_t prefix = 0;
+    int64_t pos = (int64_t)tile - 1;
+    uint32_t spins = 0;
+    for (;;) {
+        uint64_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            int64_t idx = pos - (int64_t)(lane + 32u * k);
+            v[k] = idx >= 0 ? ld_flag(status + idx) : LB_FLAG_P; /* before tile 0: value 0 */
+        }
+        /* nearest inclusive value: smallest distance lane + 32k flagged P */
+        uint32_t kp = 8, fp = 31, pending = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint32_t flag = (uint32_t)(v[k] >> 62);
+            const uint32_t pm = __ballot_sync(0xffffffffu, flag == 2u);
+            const uint32_t xm = __ballot_sync(0xffffffffu, flag == 0u);
+            if (kp == 8) {
+                if (pm) {
+                    kp = k;
+                    fp = (uint32_t)(__ffs(pm) - 1);
+                    pending |= xm & ((1u << fp) - 1u);
+                } else {
+                    pending |= xm;
+                }
+            }
+        }
+        if (pending) {
+            if (++spins < spin_limit) {
+                __nanosleep(32);
+                continue;
+            }
+            /* give up: missing values count as 0 */
+            if (lane == 0) atomicOr(err, ZERR_TIMEOUT);
+        }
+        uint64_t c = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const bool ready = (v[k] >> 62) != 0;
+            if ((uint32_t)k < kp || ((uint32_t)k == kp && lane <= fp))
+                c += ready ? (v[k] & LB_VAL) : 0ull;
+        }
+        prefix += warp_sum_u64(c);
+        if (kp < 8) break;
+        pos -= 256;
+        spins = 0;
+    }
+    if (lane == 0) st_flag(status + tile, LB_FLAG_P | ((prefix + agg) & LB_VAL));
+    return prefix & LB_VAL;
+}
+
 constexpr uint32_t SZ_THREADS = 256;
 constexpr uint32_t SZ_CHUNK = 2048; /* sizes per CTA in the scan */
 constexpr uint32_t SZ_SCAN_BATCH = 8; /* rows loaded together in the y and x prefix sums */

@@ -21,7 +21,7 @@
  *       first block number.
  *   W3  per window, the path from its true entry, followed by one lane
  *       along 32 speculative sub-window walks run in parallel (see below),
- *       gives every block's width and every tile's offset, written by all
+ *       gives every block's width and every group's offset, written by all
  *       lanes at once; each chunk must end where the next starts.
  *   W4  the extra segment of the last chunk (N % T elements) and the total
  *       size.
@@ -100,7 +100,7 @@ __global__ void k_walk_setup(const WalkArgs a)
                     atomicOr(a.err, ZERR_BOUNDS);
                     ok = false;
                 } else {
-                    a.idx.tile_off[(uint64_t)s * g.nt_reg] = hdr + rel;
+                    a.idx.grp_off[(uint64_t)s * g.gr_reg] = hdr + rel;
                     P = hdr + rel + 4;
                     if (s + 1 < g.T) {
                         uint64_t rn = load_u64(a.in + 8ull * (s + 1));
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(32 * WARPS_W3, 3) k_walk_final(const WalkArgs 
         const uint32_t v = w.gwin[((uint64_t)gg * a.M + w.gentry[gg]) * WALK_G + k % WALK_G];
         const uint64_t b0 = w.gbase[gg] + (v >> 12);
         if (b0 >= nb) continue;
-        const uint64_t gblk0 = (uint64_t)s * g.nb_reg, tile0 = (uint64_t)s * g.nt_reg;
+        const uint64_t gblk0 = (uint64_t)s * g.nb_reg, grp0 = (uint64_t)s * g.gr_reg;
         const uint64_t start = w.seg_P[s] + (uint64_t)k * WALK_WW;
         load_exits(w.wexit + (uint64_t)wi * xb, reinterpret_cast<uint8_t *>(ex), xb);
         const uint8_t *bytes = load_window(a, start, area);
@@ -489,12 +489,12 @@ __global__ void __launch_bounds__(32 * WARPS_W3, 3) k_walk_final(const WalkArgs 
         true_path(bytes, ex, v & 0xFFFu, size, wp);
         __syncwarp();
         /* lane j records the true-path blocks of its sub-window; the
-         * next tile boundary at or after its first block is found once */
+         * next group boundary at or after its first block is found once */
         uint64_t blk = b0 + wp->pref[lane];
-        const uint64_t tq = blk / g.TB;
-        uint64_t tnext = tq * g.TB, tidx = tq;
+        const uint64_t tq = blk / g.GB;
+        uint64_t tnext = tq * g.GB, tidx = tq;
         if (tnext < blk) {
-            tnext += g.TB;
+            tnext += g.GB;
             tidx++;
         }
 #pragma unroll
@@ -516,8 +516,8 @@ __global__ void __launch_bounds__(32 * WARPS_W3, 3) k_walk_final(const WalkArgs 
                     break;
                 }
                 if (blk == tnext) {
-                    if (blk) a.idx.tile_off[tile0 + tidx] = gpos;
-                    tnext += g.TB;
+                    if (blk) a.idx.grp_off[grp0 + tidx] = gpos;
+                    tnext += g.GB;
                     tidx++;
                 }
                 a.idx.widths[gblk0 + blk] = (uint8_t)b;
@@ -550,15 +550,15 @@ __global__ void k_walk_finish(const WalkArgs a)
     }
     uint64_t pos = w.seg_end[g.T - 1];
     if (g.rem) {
-        const uint64_t tile0 = (uint64_t)g.T * g.nt_reg, gblk0 = (uint64_t)g.T * g.nb_reg;
+        const uint64_t grp0 = (uint64_t)g.T * g.gr_reg, gblk0 = (uint64_t)g.T * g.nb_reg;
         if (pos + 4 > a.avail) {
             atomicOr(a.err, ZERR_BOUNDS);
             return;
         }
-        a.idx.tile_off[tile0] = pos;
+        a.idx.grp_off[grp0] = pos;
         pos += 4;
         for (uint64_t j = 0; j < g.nb_rm; j++) {
-            if (j && j % g.TB == 0) a.idx.tile_off[tile0 + j / g.TB] = pos;
+            if (j && j % g.GB == 0) a.idx.grp_off[grp0 + j / g.GB] = pos;
             if (pos >= a.avail) {
                 atomicOr(a.err, ZERR_BOUNDS);
                 return;

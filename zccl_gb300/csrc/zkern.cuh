@@ -17,22 +17,25 @@
 #define ZH_MAXP 32 /* most inputs one homomorphic-add launch accepts */
 
 /* Per-call scratch in device memory, zeroed before every call:
- * err | walk_err | ticket | pad | status[ntiles]. */
+ * err | walk_err | ticket | role | status[ntiles]. */
 struct ZWork {
     uint32_t *err;      /* ZERR_* bits of the codec kernels */
     uint32_t *walk_err; /* ZERR_* bits of the index walk that ran before, if any */
     uint32_t *ticket;   /* next tile to hand out */
-    uint64_t *status;   /* decoupled look-back state, one word per tile */
-    uint32_t lb_spin;   /* polls before a look-back wait gives up */
+    uint32_t *role;     /* CTAs started: the first one scans */
+    uint64_t *status;   /* one word per tile (of all jobs): its size, then its place */
+    uint32_t spin;      /* polls before a wait on one gives up */
 };
 
 /* Side index of a resident stream: enough to find every block without
- * walking the 1-byte headers, and the quantized value before every tile so
- * decompression needs no scan. */
+ * walking the 1-byte headers, and the place of and quantized value before
+ * every group of blocks, so that decompression's warps, one per group, need
+ * nothing from each other.  (12 bytes per group of 32 blocks of 32 floats:
+ * 0.3 % of the floats' bytes.) */
 struct ZIndex {
     uint8_t *widths;     /* [nblocks] width byte of every block, stream order */
-    uint64_t *tile_off;  /* [ntiles]  byte offset (from stream start) of each tile's first unit */
-    int32_t *tile_qprev; /* [ntiles]  quantized value of the element before the tile's first block */
+    uint64_t *grp_off;   /* [ngroups] byte offset (from stream start) of each group's first unit */
+    int32_t *grp_qprev;  /* [ngroups] quantized value of the element before the group's first block */
     uint64_t *size;      /* [1]       total stream bytes */
 };
 
@@ -46,7 +49,6 @@ struct alignas(16) CompressJob {
     uint8_t *out;
     uint64_t cap; /* writable bytes at `out` */
     ZIndex idx;
-    uint64_t *status; /* this buffer's look-back words, one per tile */
     float inv;        /* 1.0f / eb, computed on the host in float */
     uint32_t boxed;   /* batch job: batch.maps[job] views x as rows of 32 floats */
 };
@@ -65,30 +67,17 @@ struct CompressArgs {
     ZBatch batch;
     ZWork w; /* err and ticket; status is per job */
     ZWidthTable wt;
-    ZSmem sm;
     uint32_t grid; /* CTAs to launch, 0 = as many as fit */
+    uint32_t ring; /* bytes of the ring of packed tiles (filled by the launcher) */
     int rows_map;  /* set by the launcher: its tensor map views job.x as rows of 32 floats */
-};
-
-struct DecompressArgs {
-    const uint8_t *in;
-    uint64_t avail; /* readable bytes at `in` */
-    float *y;
-    ZGeom g;
-    float eb;
-    ZIndex idx;      /* widths and tile_off must be valid */
-    int qprev_valid; /* tile_qprev valid; else recovered by look-back and written */
-    ZWork w;
-    ZSmem sm;
-    int rows_map;    /* set by the launcher: its tensor map views y as rows of 32 floats */
 };
 
 struct HomInput {
     const uint8_t *bytes;
     uint64_t avail;
     const uint8_t *widths;
-    const uint64_t *tile_off;
-    const int32_t *tile_qprev;
+    const uint64_t *grp_off;
+    const int32_t *grp_qprev;
 };
 
 /* One homomorphic sum of P streams. */
@@ -96,61 +85,32 @@ struct alignas(16) HomAddJob {
     ZGeom g;
     HomInput in[ZH_MAXP];
     uint32_t P;
-    int qprev_valid;  /* every input's tile_qprev is valid */
+    int qprev_valid;  /* every input's grp_qprev is valid */
     uint8_t *out;
     uint64_t cap;     /* writable bytes at `out` */
     ZIndex idx;       /* index of the output stream */
-    uint64_t *status; /* look-back words of the output, one per tile */
 };
 
-/* One indexed stream to decompress (with its tiles' starting values): the
- * floats go to y, or are added to y with accumulate. */
+/* One indexed stream to decompress: the floats go to y, or are added to y
+ * with accumulate. */
 struct alignas(16) DecompressJob {
     ZGeom g;
     const uint8_t *in;
     uint64_t avail; /* readable bytes at `in` */
     float *y;
-    ZIndex idx;
+    ZIndex idx; /* widths and grp_off must be valid */
     float eb;
     int accumulate;
 };
 
-struct DecompressJobsArgs {
+struct DecompressArgs {
     DecompressJob job; /* the single job (batch.jobs == null) */
     ZBatch batch;
-    ZWork w; /* err, walk_err */
-    ZSmem sm;
-    uint32_t grid; /* CTAs to launch, 0 = as many as fit */
+    int qprev_valid;   /* grp_qprev valid; else (single job) recovered first and written */
+    ZWork w;           /* err, walk_err */
+    uint32_t grid;     /* CTAs to launch, 0 = as many as fit */
+    uint32_t room, in_bytes; /* shared bytes for staged input, and with slack (filled by the launcher) */
 };
-
-/* One staged input tile of the homomorphic add: which tile and input it
- * is, and where its bytes start within the buffer (the TMA copy keeps the
- * source's 16-byte phase). */
-struct HStage {
-    uint64_t tile; /* within its job; ZP_NONE: no more tiles */
-    uint32_t job;
-    uint32_t p;    /* the input */
-    uint32_t ph;   /* the tile's first byte in the buffer */
-    uint32_t pad[3];
-};
-
-/* What the adding warps need of a claimed tile, written by the loader with
- * the tile's first input so that the adders read shared memory instead of
- * the job in device or parameter memory.  ZH_TILE_RECS records, by tile
- * count: the loader runs at most two input copies ahead of the adders, so a
- * record is reused only after its tile is packed. */
-struct HTile {
-    uint64_t gblk0;      /* first block of the tile in its stream */
-    uint8_t *widths;     /* the sum's width index */
-    int32_t *tile_qprev; /* the sum's tile starting values, or null */
-    uint64_t *status;    /* the sum's look-back words */
-    uint32_t P, nblk;
-    uint32_t nlast;      /* elements of the tile's last block */
-    uint32_t has_head;   /* tile 0 of its segment */
-    uint32_t qsum;       /* the inputs' starting values of the tile, summed */
-    uint32_t pad[3];
-};
-#define ZH_TILE_RECS 4u
 
 struct HomAddArgs {
     HomAddJob job; /* the single job (batch.jobs == null) */
@@ -158,8 +118,8 @@ struct HomAddArgs {
     unsigned long long *cases; /* optional [4]: both zero, first zero, second zero, both non-zero (P == 2) */
     ZWork w;
     ZWidthTable wt;
-    ZSmem sm;
     uint32_t grid; /* CTAs to launch, 0 = as many as fit */
+    uint32_t in_ring, in_bytes, ring; /* shared bytes of the input ring, with slack, and of the output ring (filled by the launcher) */
 };
 
 #define WALK_WW 4096u /* bytes per window of the parallel header walk */
@@ -206,19 +166,41 @@ size_t walk_w1_warp_bytes(uint32_t M);
 /* ------------------------------------------------------------------
  * Hand-off of packed tiles from the compute warps to the placer warp.
  *
- * The packed tiles wait in a ring of R bytes of shared memory (R holds
- * the largest tile; two typical tiles fit at once), so the compute warps
- * can pack tile k + 1 while the placer still writes out tile k.  Two
- * counters order the hand-off: `packed` (tiles packed, written by compute
- * thread 0) and `placed` (tiles written out, written by placer lane 0).
- * Tile k's size, ring position and index sit in slot k % 2.  All waits are
- * bounded: on time-out ZERR_TIMEOUT is set and the caller goes on.
+ * The packed tiles wait in a ring of shared memory with ZR_SLOTS slots, so
+ * that the compute warps can pack tile k + 1 while the placer still writes
+ * out tile k.  The loader describes tile k in slot k % ZR_SLOTS when it
+ * claims it (after the placer is done with the slot's previous tile); its
+ * size goes to the placer (mbarrier `sized`, one arrival by thread 0) right
+ * after the scan has found it, and `packed` (one arrival per packing warp)
+ * then hands over its bytes.  Ring space is counted in running bytes: a tile
+ * takes the next `need` bytes (skipping to the ring's start when it would
+ * not fit before the end) and may be written once the placer's running
+ * count of released bytes, `tail`, shows that the space is free.  Up to
+ * ZR_SLOTS tiles are between sizing and write-out at once (the ring's bytes
+ * hold one worst-case tile, far more typical ones), so the packing warps do
+ * not wait for a placer delayed by a slow look-back; 16 measured 3.7 %
+ * faster than 4 on the two-way add.  All waits are bounded: on time-out
+ * ZERR_TIMEOUT is set and the caller goes on.
  * ------------------------------------------------------------------ */
+#define ZR_SLOTS 16u
+
+struct ZSlot {
+    uint64_t ticket;    /* ZP_NONE ends the placer */
+    uint8_t *out;       /* the stream, its writable bytes */
+    uint64_t cap;
+    uint64_t *grp_off;  /* index: the tile's first group's offset */
+    uint8_t *hdr;       /* a segment's first tile: its chunk offset in the header, else null */
+    uint64_t *size;     /* the stream's last tile: where its size goes, else null */
+    uint32_t T8, ngrp;  /* bytes of the header; the tile's groups */
+    uint32_t total, pos, mend;
+    uint16_t goff[ZG_SUB]; /* where each of its groups starts in it (a tile is below 64 KB) */
+};
+
 struct ZRing {
-    uint32_t packed, placed;
-    uint32_t pos[2], total[2];
-    uint64_t tile[2]; /* the tile within its job */
-    uint32_t job[2];  /* its job in the batch (0 for a single job) */
+    uint32_t placed; /* tiles written out (placer lane 0, release) */
+    uint32_t tail;   /* running count of released ring bytes (release) */
+    uint64_t sized[ZR_SLOTS], packed[ZR_SLOTS]; /* mbarriers */
+    ZSlot slot[ZR_SLOTS];
 };
 
 __device__ __forceinline__ void ring_set(uint32_t *p, uint32_t v)
@@ -233,8 +215,8 @@ __device__ __forceinline__ uint32_t ring_get(const uint32_t *p)
     return v;
 }
 
-/* One thread: wait until *p >= v. */
-__device__ __forceinline__ void ring_wait(const uint32_t *p, uint32_t v, uint32_t *err)
+/* One thread: wait until *p >= v (counted with wrap-around). */
+static __device__ __noinline__ void ring_wait_slow(const uint32_t *p, uint32_t v, uint32_t *err)
 {
     for (uint32_t i = 0; i < (1u << 24); i++) {
         if ((int32_t)(ring_get(p) - v) >= 0) return;
@@ -242,84 +224,50 @@ __device__ __forceinline__ void ring_wait(const uint32_t *p, uint32_t v, uint32_
     }
     atomicOr(err, ZERR_TIMEOUT);
 }
-
-/* Compute thread 0, before packing tile k (0-based) of `need` bytes: its
- * ring position, after waiting until the placer has released the space.
- * end_prev / pos_prev describe tile k - 1 (updated here). */
-__device__ __forceinline__ uint32_t ring_reserve(ZRing *ring, uint32_t k, uint32_t need, uint32_t R,
-                                                 uint32_t &pos_prev, uint32_t &end_prev, uint32_t *err)
+__device__ __forceinline__ void ring_wait(const uint32_t *p, uint32_t v, uint32_t *err)
 {
-    const uint32_t pos = end_prev + need <= R ? end_prev : 0u;
-    /* tile k - 2 is always out of the way (its slot is reused); tile k - 1
-     * too when this tile wraps onto it */
-    uint32_t req = k >= 1 ? k - 1 : 0u;
-    if (k >= 1 && pos < end_prev && pos + need > pos_prev) req = k;
-    ring_wait(&ring->placed, req, err);
-    pos_prev = pos;
-    end_prev = pos + need;
-    return pos;
+    if ((int32_t)(ring_get(p) - v) < 0) ring_wait_slow(p, v, err);
 }
-
-/* Compute thread 0, after every compute thread has finished packing tile k
- * (pass ZP_NONE as `tile` once there are no more tiles). */
-__device__ __forceinline__ void ring_publish(ZRing *ring, uint32_t k, uint64_t tile, uint32_t job,
-                                             uint32_t total, uint32_t pos)
-{
-    ring->tile[k & 1u] = tile;
-    ring->job[k & 1u] = job;
-    ring->total[k & 1u] = total;
-    ring->pos[k & 1u] = pos;
-    ring_set(&ring->packed, k + 1);
-}
-
-/* ------------------------------------------------------------------
- * The same hand-off with early sizes and ZR_SLOTS slots.  A tile's identity and
- * size go to the placer (mbarrier `sized`, one arrival by thread 0) right
- * after the scan has found them, so the placer's look-back runs while the
- * tile is still being packed; `packed` (one arrival per packing warp) then
- * hands over its bytes.  Ring space is counted in running bytes: a tile
- * takes the next `need` bytes (skipping to the ring's start when it would
- * not fit before the end) and may be written once the placer's running
- * count of released bytes, `tail`, shows that the space is free.  Up to
- * ZR_SLOTS tiles are between sizing and write-out at once (the ring's bytes
- * hold one worst-case tile, far more typical ones), so the packing warps do
- * not wait for a placer delayed by a slow look-back; 16 measured 3.7 %
- * faster than 4 on the two-way add.  Its control block sits below the
- * rows at offset 1024 of shared memory.
- * ------------------------------------------------------------------ */
-#define ZR_SLOTS 16u
-
-struct ZRing4 {
-    uint32_t placed; /* tiles written out (placer lane 0, release) */
-    uint32_t tail;   /* running count of released ring bytes (release) */
-    uint32_t total[ZR_SLOTS], pos[ZR_SLOTS], mend[ZR_SLOTS], job[ZR_SLOTS];
-    uint64_t tile[ZR_SLOTS];
-    uint64_t sized[ZR_SLOTS], packed[ZR_SLOTS]; /* mbarriers */
-};
 
 /* Thread 0, before the CTA's first barrier. */
-__device__ __forceinline__ void ring4_init(ZRing4 *r, uint32_t packers)
+__device__ __forceinline__ void ring_init(ZRing *r, uint32_t packers)
 {
     r->placed = 0;
     r->tail = 0;
+#pragma unroll 1
     for (uint32_t i = 0; i < ZR_SLOTS; i++) {
         mbar_init(&r->sized[i], 1);
         mbar_init(&r->packed[i], packers);
     }
 }
 
-/* Thread 0: tile k's identity and size for the placer, once the placer is
- * done with tile k - ZR_SLOTS, the previous user of the slot.  ZP_NONE as
- * `tile` ends the placer. */
-__device__ __forceinline__ void ring4_sized(ZRing4 *r, uint32_t k, uint64_t tile, uint32_t job, uint32_t total,
-                                            uint32_t *err)
+/* The loader's lane 0: the slot of its k-th tile, free. */
+__device__ __forceinline__ ZSlot &ring_slot(ZRing *r, uint32_t k, uint32_t *err)
 {
     if (k >= ZR_SLOTS) ring_wait(&r->placed, k - ZR_SLOTS + 1, err);
-    const uint32_t s = k % ZR_SLOTS;
-    r->tile[s] = tile;
-    r->job[s] = job;
-    r->total[s] = total;
-    mbar_arrive(&r->sized[s]);
+    return r->slot[k % ZR_SLOTS];
+}
+
+/* ... and its description: batch ticket t, tile z (number `local`) of the
+ * stream that goes to out. */
+__device__ __forceinline__ void ring_describe(ZSlot &S, uint64_t t, uint64_t local, const ZTile &z, const ZGeom &g,
+                                              uint8_t *out, uint64_t cap, const ZIndex &idx)
+{
+    S.ticket = t;
+    S.out = out;
+    S.cap = cap;
+    S.grp_off = idx.grp_off + z.grp0;
+    S.hdr = z.has_head && z.seg < g.T ? out + 8ull * z.seg : nullptr;
+    S.size = local == g.ntiles - 1 ? idx.size : nullptr;
+    S.T8 = 8u * g.T;
+    S.ngrp = z.nblk ? (z.nblk + g.GB - 1u) / g.GB : 1u;
+}
+
+/* Thread 0: tile k's size for the placer. */
+__device__ __forceinline__ void ring_sized(ZRing *r, uint32_t k, uint32_t total)
+{
+    r->slot[k % ZR_SLOTS].total = total;
+    mbar_arrive(&r->sized[k % ZR_SLOTS]);
 }
 
 /* Every packing thread (the same result in each): the ring position of the
@@ -327,8 +275,8 @@ __device__ __forceinline__ void ring4_sized(ZRing4 *r, uint32_t k, uint64_t tile
  * the running count of ring bytes taken (compared with wrap-around) and hp
  * the ring position after the last tile; *mend receives the tile's running
  * end. */
-__device__ __forceinline__ uint32_t ring4_space(ZRing4 *r, uint32_t need, uint32_t R, uint32_t &H, uint32_t &hp,
-                                                uint32_t &mend, uint32_t *err)
+__device__ __forceinline__ uint32_t ring_space(ZRing *r, uint32_t need, uint32_t R, uint32_t &H, uint32_t &hp,
+                                               uint32_t &mend, uint32_t *err)
 {
     const uint32_t H0 = H;
     uint32_t M = H, pos = hp;
@@ -349,142 +297,64 @@ __device__ __forceinline__ uint32_t ring4_space(ZRing4 *r, uint32_t need, uint32
 }
 
 /* Thread 0, before its warp's `packed` arrival: where tile k lies. */
-__device__ __forceinline__ void ring4_where(ZRing4 *r, uint32_t k, uint32_t pos, uint32_t mend)
+__device__ __forceinline__ void ring_where(ZRing *r, uint32_t k, uint32_t pos, uint32_t mend)
 {
-    r->pos[k % ZR_SLOTS] = pos;
-    r->mend[k % ZR_SLOTS] = mend;
+    r->slot[k % ZR_SLOTS].pos = pos;
+    r->slot[k % ZR_SLOTS].mend = mend;
 }
 
-/* What the placer needs of a job. */
-struct ZPlace {
-    ZGeom g;
-    uint8_t *out;
-    uint64_t cap;
-    ZIndex idx;
-    uint64_t *status;
-};
-
-/* Shared bytes of the homomorphic add's job region: the placer's job, two
- * stage records, the tile records and two block tables (offset << 8 |
- * width per block). */
-static inline uint32_t homadd_job_bytes(uint32_t TB)
+/* Thread 0, when there is no tile k: ends the placers. */
+__device__ __forceinline__ void ring_end(ZRing *r, uint32_t k, uint32_t placers, uint32_t *err)
 {
-    return zg_a16((uint32_t)sizeof(ZPlace)) + 2u * (uint32_t)sizeof(HStage) + ZH_TILE_RECS * (uint32_t)sizeof(HTile) +
-           2u * TB * 4u;
-}
-
-
-/* The placer warp: for every packed tile, in order, the decoupled look-back
- * gives its byte offset in its stream; its bytes go out with 16-byte vector
- * stores realigned to that offset, with its offset in the side index, the
- * stream size after the stream's last tile and, for a segment's first tile,
- * the chunk offset in the header.  wait_packed(k) (all lanes) returns once
- * tile k is packed; fetch(job, ZPlace *) (lane 0) copies a job's placement
- * data into shared memory.  With `zero`, the ring bytes of a tile are set
- * back to zero once written out, so the packers find zeroed space. */
-template <class Wait, class Fetch>
-__device__ __forceinline__ void placer_loop(ZRing *ring, uint8_t *ringb, ZPlace *pj, uint32_t *err,
-                                            uint64_t max_tiles, uint32_t &bad, bool zero, uint32_t spin,
-                                            Wait wait_packed, Fetch fetch)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t cur_job = 0xFFFFFFFFu;
-    for (uint64_t k = 0; k <= max_tiles; k++) {
-        wait_packed(k);
-        __syncwarp();
-        const uint32_t slot = (uint32_t)k & 1u;
-        const uint64_t t = ring->tile[slot];
-        const uint32_t job = ring->job[slot];
-        const uint32_t total = ring->total[slot], pos = ring->pos[slot];
-        if (t == ZP_NONE) break;
-        if (job != cur_job) {
-            if (lane == 0) fetch(job, pj);
-            __syncwarp();
-            cur_job = job;
-        }
-        const ZGeom &g = pj->g;
-        const uint64_t base = 8ull * g.T + lb_resolve(pj->status, t, total, t == 0, 0, err, spin);
-        const bool fits = base + total <= pj->cap;
-        if (!fits) bad |= ZERR_CAPACITY;
-        if (lane == 0) {
-            ZTile z;
-            zg_tile(&g, t, &z);
-            pj->idx.tile_off[t] = base;
-            if (fits && z.has_head && z.seg < g.T) {
-                const uint64_t h = base - 8ull * g.T;
-#pragma unroll
-                for (int k8 = 0; k8 < 8; k8++) pj->out[8ull * z.seg + k8] = (uint8_t)(h >> (8 * k8));
-            }
-            if (t == g.ntiles - 1) *pj->idx.size = base + total;
-        }
-        if (fits) store_realign(pj->out + base, ringb + pos, total, lane, 32);
-        if (zero) {
-            __syncwarp(); /* every lane has read the tile */
-            uint4 *zr = reinterpret_cast<uint4 *>(ringb + pos);
-            for (uint32_t i = lane; i < zg_ring_need(total) / 16u; i += 32) zr[i] = make_uint4(0, 0, 0, 0);
-        }
-        __syncwarp();
-        if (lane == 0) ring_set(&ring->placed, (uint32_t)k + 1);
+#pragma unroll 1
+    for (uint32_t i = k; i < k + placers; i++) {
+        ring_slot(r, i, err).ticket = ZP_NONE;
+        mbar_arrive(&r->sized[i % ZR_SLOTS]);
     }
 }
 
-/* The placer warp on a ZRing4: for tile k, the look-back starts as soon
- * as its size is known; the side-index entries follow, and once the tile is
- * packed its bytes go out and its ring bytes are zeroed and released. */
-template <class Fetch>
-__device__ __forceinline__ void placer_loop4(ZRing4 *r, uint8_t *ringb, ZPlace *pj, uint32_t *err,
-                                             uint64_t max_tiles, uint32_t &bad, uint32_t spin, Fetch fetch)
+/* A placer warp, number p of N taking turns: for every N-th tile k its byte offset in its stream
+ * (as soon as its size is known, from the scan of the tiles' sizes), then
+ * the chunk offset in the header (a segment's first tile), the stream's size
+ * (its last) and, once the tile is packed, its groups' offsets in the side
+ * index and its bytes, with 16-byte vector stores realigned to that offset.
+ * Its ring bytes are zeroed, so the packers find zeroed space, and
+ * released. */
+template <uint32_t N>
+__device__ __forceinline__ void placer_loop(ZRing *r, uint8_t *ringb, const uint64_t *status, uint64_t max_tiles,
+                                            uint32_t p, uint32_t *err, uint32_t &bad, uint32_t spin)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t cur_job = 0xFFFFFFFFu;
-    for (uint64_t k = 0; k <= max_tiles; k++) {
-        const uint32_t s = (uint32_t)(k % ZR_SLOTS), par = (uint32_t)(k / ZR_SLOTS) & 1u;
+#pragma unroll 1
+    for (uint64_t k = p; k <= max_tiles + N; k += N) {
+        const uint32_t s = (uint32_t)k % ZR_SLOTS, par = (uint32_t)(k / ZR_SLOTS) & 1u;
         mbar_wait(&r->sized[s], par, err);
-        const uint64_t t = r->tile[s];
-        const uint32_t job = r->job[s], total = r->total[s];
+        const ZSlot &S = r->slot[s];
+        const uint64_t t = S.ticket;
         if (t == ZP_NONE) break;
-        if (job != cur_job) {
-            if (lane == 0) fetch(job, pj);
-            __syncwarp();
-            cur_job = job;
-        }
-        const ZGeom &g = pj->g;
-        const uint64_t base = 8ull * g.T + lb_resolve(pj->status, t, total, t == 0, 0, err, spin);
-        const bool fits = base + total <= pj->cap;
+        const uint32_t total = S.total;
+        /* after a wait that gave up, here or in the scan, a sum may be
+         * missing or too small: nothing is written then */
+        const uint64_t sum = scan_wait(status + t, spin, err), base = S.T8 + sum - total;
+        const bool fits = sum != SCAN_NONE && sum >= total && S.T8 + sum <= S.cap;
         if (!fits) bad |= ZERR_CAPACITY;
-        if (lane == 0) {
-            ZTile z;
-            zg_tile(&g, t, &z);
-            pj->idx.tile_off[t] = base;
-            if (fits && z.has_head && z.seg < g.T) {
-                const uint64_t h = base - 8ull * g.T;
-#pragma unroll
-                for (int k8 = 0; k8 < 8; k8++) pj->out[8ull * z.seg + k8] = (uint8_t)(h >> (8 * k8));
-            }
-            if (t == g.ntiles - 1) *pj->idx.size = base + total;
-        }
+        if (lane < 8 && fits && S.hdr) S.hdr[lane] = (uint8_t)((base - S.T8) >> (8u * lane));
+        if (lane == 0 && S.size) *S.size = base + total;
         mbar_wait(&r->packed[s], par, err);
-        const uint32_t pos = r->pos[s], mend = r->mend[s];
-        if (fits) store_realign(pj->out + base, ringb + pos, total, lane, 32);
-        __syncwarp(); /* every lane has read the tile */
+        if (lane < S.ngrp) S.grp_off[lane] = base + S.goff[lane];
+        const uint32_t pos = S.pos, mend = S.mend;
+        if (fits) store_realign(S.out + base, ringb + pos, total, lane, 32);
+        __syncwarp(); /* every lane has read the tile and its slot */
         uint4 *zr = reinterpret_cast<uint4 *>(ringb + pos);
+#pragma unroll 4
         for (uint32_t i = lane; i < zg_ring_need(total) / 16u; i += 32) zr[i] = make_uint4(0, 0, 0, 0);
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0) { /* in order */
+            if (N > 1) ring_wait(&r->placed, (uint32_t)k, err);
             ring_set(&r->tail, mend);
             ring_set(&r->placed, (uint32_t)k + 1);
         }
     }
-}
-
-/* One thread: copy n bytes (a multiple of 16, both 16-byte aligned) one
- * vector at a time, so a job copy holds few registers. */
-__device__ __forceinline__ void copy16(void *dst, const void *src, uint32_t n)
-{
-    uint4 *d = static_cast<uint4 *>(dst);
-    const uint4 *s = static_cast<const uint4 *>(src);
-#pragma unroll 1
-    for (uint32_t i = 0; i < n / 16u; i++) d[i] = s[i];
 }
 
 /* Thread 0: the job and local tile of batch ticket t. */
@@ -497,6 +367,68 @@ __device__ __forceinline__ uint32_t batch_job(const ZBatch &b, uint64_t t, uint6
     const uint32_t j = b.tile_job[t];
     *local = t - b.job_tile0[j];
     return j;
+}
+
+/* All lanes: the words around the widths w[0, n) of a tile's blocks (n <=
+ * 256), requested: blocks 8 lane .. 8 lane + 7 are the eight bytes of v from
+ * bit widths_shift(w) on (those from n on are not 0).  Whole words around
+ * them are read: the index has four bytes before its widths and sixteen
+ * after. */
+__device__ __forceinline__ void load_widths(const uint8_t *w, uint32_t n, uint32_t (&v)[3])
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    v[0] = v[1] = v[2] = 0;
+    if (8u * lane < n) {
+        const uint32_t *p = reinterpret_cast<const uint32_t *>((uintptr_t)(w + 8u * lane) & ~(uintptr_t)3u);
+        v[0] = p[0];
+        v[1] = p[1];
+        v[2] = p[2];
+    }
+}
+__device__ __forceinline__ uint32_t widths_shift(const uint8_t *w) { return ((uint32_t)(uintptr_t)w & 3u) * 8u; }
+
+/* All lanes: the table entries (offset from the tile's first block << 8 |
+ * width) of blocks 8 lane .. 8 lane + 7 of a tile of nblk blocks, the last of
+ * nlast elements and the others of L, from their widths (load_widths); a
+ * width above 32 counts as 0 and sets ZERR_CORRUPT.  Returns the blocks'
+ * bytes. */
+template <bool L32>
+__device__ __forceinline__ uint32_t tile_entries(uint32_t L, uint32_t fmt, uint32_t nblk, uint32_t nlast, uint32_t w0,
+                                                 uint32_t w1, uint4 (&e)[2], uint32_t &bad)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t mine = nblk > 8u * lane ? min(nblk - 8u * lane, 8u) : 0u; /* this lane's blocks */
+    const bool f32 = L32 && fmt == ZG_FASTMODE1;
+    uint32_t ent[8], sum = 0, blast = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++) {
+        uint32_t b = k < mine ? ((k < 4 ? w0 : w1) >> (8 * (k & 3))) & 0xFFu : 0u;
+        if (b > 32) {
+            bad |= ZERR_CORRUPT;
+            b = 0;
+        }
+        ent[k] = sum << 8 | b;
+        blast = k + 1 == mine ? b : blast;
+        if (k < mine) sum += f32 ? block32_bytes(b) : zg_block_bytes_f(fmt, b, L);
+    }
+    if (mine && 8u * lane + mine == nblk) /* the tile's last block may be short */
+        sum += zg_block_bytes_f(fmt, blast, nlast) - zg_block_bytes_f(fmt, blast, L);
+    const uint32_t incl = warp_incl_scan(sum), x = (incl - sum) << 8;
+    e[0] = make_uint4(ent[0] + x, ent[1] + x, ent[2] + x, ent[3] + x);
+    e[1] = make_uint4(ent[4] + x, ent[5] + x, ent[6] + x, ent[7] + x);
+    return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+/* All lanes: each lane's v maximised over its block's G lanes (its octet og
+ * among them), then block `src / G`'s maximum from its first lane. */
+__device__ __forceinline__ uint32_t octet_max(uint32_t v, uint32_t og, uint32_t G, uint32_t src)
+{
+#pragma unroll 1
+    for (uint32_t s = 1; s < G; s <<= 1) {
+        const uint32_t u = __shfl_down_sync(0xffffffffu, v, s);
+        if (og + s < G) v = max(v, u);
+    }
+    return __shfl_sync(0xffffffffu, v, src);
 }
 
 /* Launch-shape queries, remembered per device and kernel: the occupancy
@@ -517,7 +449,7 @@ struct LaunchCache {
     Occ occ[96];
     Attr attr[64];
     int nocc = 0, nattr = 0;
-    int nsm[64] = {0};
+    int nsm[64] = {0}, smem_sm[64] = {0}, smem_rsv[64] = {0};
 };
 
 static inline LaunchCache &launch_cache()
@@ -589,10 +521,46 @@ static inline cudaError_t set_max_smem(const void *fn, size_t smem)
     return cudaSuccess;
 }
 
+/* Ring bytes of a kernel that runs `per_sm` CTAs per SM and needs `fixed`
+ * other bytes of shared memory: at least `least` (one worst-case tile), and
+ * up to the CTA's share of the SM's shared memory less a kilobyte of margin.
+ * The longer the ring, the longer a tile may wait there for its look-back
+ * before the compute warps run out of room. */
+static inline uint32_t ring_bytes(uint32_t per_sm, uint32_t fixed, uint32_t least)
+{
+    LaunchCache &c = launch_cache();
+    int dev = 0, sm = 0, rsv = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && c.smem_sm[dev] > 0) {
+        sm = c.smem_sm[dev];
+        rsv = c.smem_rsv[dev];
+    } else if (cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+               cudaDeviceGetAttribute(&rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return least;
+    } else if (dev >= 0 && dev < 64) {
+        c.smem_rsv[dev] = rsv;
+        c.smem_sm[dev] = sm;
+    }
+    const int share = sm / (int)per_sm - rsv - 1024 - (int)fixed;
+    return share > (int)least ? (uint32_t)share & ~15u : least;
+}
+
 static inline unsigned persistent_grid(const void *fn, int threads, size_t smem, uint64_t ntiles)
 {
     const uint64_t g = (uint64_t)sm_count() * (uint64_t)blocks_per_sm(fn, threads, smem);
     return (unsigned)(g < ntiles ? g : ntiles);
+}
+
+/* Grid of a kernel whose tiles' places come from the scanning CTA: `want`
+ * working CTAs (0: as many as fit, at most one per tile) and, with more than
+ * one tile, the scanner. */
+static inline unsigned scanned_grid(const void *fn, int threads, size_t smem, uint64_t ntiles, unsigned want)
+{
+    unsigned g = persistent_grid(fn, threads, smem, ntiles + 1);
+    if (ntiles == 1) return 1;
+    if (g < 2) g = 2;
+    return want && want + 1 < g ? want + 1 : g;
 }
 
 /* Launchers; each returns the cudaError_t of the launch. */
@@ -629,14 +597,13 @@ cudaError_t sz3_split_compress(uint8_t *out, uint64_t cap, const float *x, const
 cudaError_t sz3_split_decompress(float *y, const uint8_t *in, uint64_t avail, const uint64_t *offs, const Sz3Split3 &sp,
                                  uint32_t bs, double eb, void *ws, cudaStream_t st);
 
-/* Host: a 2-D TMA map of the floats p[0, n) as rows of 32, boxes of
- * box_rows rows (256: a whole tile; 32: one warp's rows), 128-byte swizzle
- * (16-byte chunk k of row r lands at chunk k ^ (r & 7) of a 1024-byte-aligned
- * box).  False when p is not 16-byte aligned, holds fewer than one tile's
- * 256 rows, or the driver's encoder is unavailable. */
-bool zk_rows_map(CUtensorMap *map, const void *p, uint64_t n, uint32_t box_rows);
+/* Host: a 2-D TMA map of the floats p[0, n), from the 16-byte boundary at or
+ * before p on, as rows of 32, boxes of 32 rows, 128-byte swizzle (16-byte
+ * chunk k of row r lands at chunk k ^ (r & 7) of a 1024-byte-aligned box).
+ * False when there are fewer than 256 whole rows or the driver's encoder is
+ * unavailable. */
+bool zk_rows_map(CUtensorMap *map, const void *p, uint64_t n);
 cudaError_t launch_homadd(const HomAddArgs &a, cudaStream_t st);
-cudaError_t launch_decompress_jobs(const DecompressJobsArgs &a, cudaStream_t st);
 cudaError_t launch_walk(const WalkArgs &a, cudaStream_t st);
 
 #endif

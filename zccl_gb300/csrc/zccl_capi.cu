@@ -103,7 +103,7 @@ ZIndex bind_index(void *mem, const ZGeom &g)
  * header-walk scratch.  Only the first part is cleared per call. */
 struct WalkLayout {
     uint32_t M, max_windows, max_groups;
-    size_t seg_P, seg_R, seg_end, seg_ok, win_base, grp_base, wtab, gtab, gentry, gbase, wexit, gwin, total;
+    size_t seg_P, seg_R, seg_end, seg_ok, win_base, grp_base, wtab, gtab, gentry, gbase, gwin, total;
 };
 
 size_t ws_clear_bytes(const ZGeom &g) { return 16 + 8 * g.ntiles; }
@@ -122,7 +122,8 @@ WalkLayout walk_layout(const ZGeom &g)
     WalkLayout l;
     l.M = zg_block_bytes(32, g.L);
     l.max_windows = (uint32_t)(zg_stream_worst(&g) / WALK_WW + g.T + 2);
-    l.max_groups = (l.max_windows + WALK_G - 1) / WALK_G + g.T + 1;
+    const uint32_t G = walk_group(l.M);
+    l.max_groups = (l.max_windows + G - 1) / G + g.T + 1;
     size_t o = align16(ws_clear_bytes(g));
     l.seg_P = o; o = align16(o + 8ull * g.T);
     l.seg_R = o; o = align16(o + 8ull * g.T);
@@ -134,8 +135,7 @@ WalkLayout walk_layout(const ZGeom &g)
     l.gtab = o; o = align16(o + 8ull * l.max_groups * l.M);
     l.gentry = o; o = align16(o + 4ull * l.max_groups);
     l.gbase = o; o = align16(o + 8ull * l.max_groups);
-    l.wexit = o; o = align16(o + (size_t)WALK_WW * l.max_windows * (l.M < 256 ? 1u : 2u));
-    l.gwin = o; o = align16(o + 4ull * l.max_groups * l.M * WALK_G);
+    l.gwin = o; o = align16(o + 4ull * l.max_groups * l.M * G);
     l.total = o + 16;
     return l;
 }
@@ -202,7 +202,6 @@ int walk_stream(zccl_gpu_stream *s, const ZGeom &g, void *ws, cudaStream_t st)
     a.ws.gtab = (uint64_t *)(p + l.gtab);
     a.ws.gentry = (uint32_t *)(p + l.gentry);
     a.ws.gbase = (uint64_t *)(p + l.gbase);
-    a.ws.wexit = p + l.wexit;
     a.ws.gwin = (uint32_t *)(p + l.gwin);
     a.max_windows = l.max_windows;
     a.max_groups = l.max_groups;

@@ -665,6 +665,22 @@ __device__ __forceinline__ float4 ld_shared_v4(uint32_t sa)
                  : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t ld_shared_u8(uint32_t sa)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(sa) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_shared_u16(uint32_t sa)
+{
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(sa) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared_u16(uint32_t sa, uint32_t v)
+{
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(sa), "h"((uint16_t)v) : "memory");
+}
 __device__ __forceinline__ float ld_shared_f32(uint32_t sa)
 {
     float v;

@@ -122,8 +122,17 @@ struct HomAddArgs {
     uint32_t in_ring, in_bytes, ring; /* shared bytes of the input ring, with slack, and of the output ring (filled by the launcher) */
 };
 
-#define WALK_WW 4096u /* bytes per window of the parallel header walk */
-#define WALK_G 32u     /* windows per group */
+#define WALK_WW 2048u /* bytes per window of the parallel header walk */
+#define WALK_GMAX 64u  /* windows per group at most */
+
+/* Windows per group: as many (a power of two) as their tables of M words fit
+ * 128 KB of shared memory. */
+ZG_HD uint32_t walk_group(uint32_t M)
+{
+    uint32_t G = WALK_GMAX;
+    while (G > 1 && G * M * 4u > 128u * 1024u) G >>= 1;
+    return G;
+}
 
 /* Device scratch of the header walk (part of the workspace). */
 struct WalkScratch {
@@ -133,12 +142,11 @@ struct WalkScratch {
     uint32_t *seg_ok;   /* [T]   header entries usable */
     uint32_t *win_base; /* [T+1] first window of each segment (prefix sum) */
     uint32_t *grp_base; /* [T+1] first window group of each segment */
-    uint32_t *wtab;     /* [max_windows * M] exit offset << 16 | blocks, per entry offset */
-    uint64_t *gtab;     /* [max_groups * M]  blocks << 32 | exit offset, per group */
-    uint32_t *gentry;   /* [max_groups] true entry offset of each group */
+    uint32_t *wtab;     /* [max_windows * M] exit offset << 16 | blocks, per entry offset; all ones: dead */
+    uint64_t *gtab;     /* [max_groups * M]  blocks << 32 | exit offset, per group; top bit: dead, with the windows entered */
+    uint32_t *gentry;   /* [max_groups] windows of the group that are entered << 16 | its true entry offset */
     uint64_t *gbase;    /* [max_groups] first block (in its segment) of each group */
-    uint8_t *wexit;     /* [max_windows * WW] per position: exit - end of its sub-window */
-    uint32_t *gwin;     /* [max_groups * M * WALK_G] per group, entry offset and window k of it:
+    uint32_t *gwin;     /* [max_groups * M * G] per group, entry offset and window k of it:
                            blocks before k << 12 | entry offset of k */
 };
 
@@ -151,13 +159,10 @@ struct WalkArgs {
     uint32_t *err;
     WalkScratch ws;
     uint32_t max_windows, max_groups;
-    uint32_t M;             /* largest full block in bytes (filled by launch_walk) */
+    uint32_t M, G;          /* largest full block in bytes, windows per group (filled by launch_walk) */
     uint32_t w1_warp_bytes; /* filled by launch_walk */
     uint32_t seg_batch;     /* group tables staged per step of W2b (filled by launch_walk) */
 };
-
-/* Shared bytes per warp of the window-table kernel. */
-size_t walk_w1_warp_bytes(uint32_t M);
 
 /* Grid of a persistent kernel: every CTA that fits on the device at once,
  * but no more CTAs than tiles. */

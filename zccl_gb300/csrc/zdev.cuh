@@ -648,6 +648,17 @@ __device__ __forceinline__ void bulk_g2s(void *sdst, const void *gsrc, uint32_t 
 }
 
 /* Shared stores by address (a swizzled layout computes its own). */
+/* Four bytes from global to shared memory, asynchronously (both addresses
+ * multiples of 4); cp_async_arrive: one arrival on the barrier when all the
+ * thread's copies so far have landed. */
+__device__ __forceinline__ void cp_async4(uint32_t sdst, const void *gsrc)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sdst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void st_shared_v4(uint32_t sa, float x, float y, float z, float w)
 {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sa), "f"(x), "f"(y), "f"(z), "f"(w)

@@ -27,15 +27,18 @@
  *                (a thread per column, rows loaded in batches), the last one
  *                writing (float)((double)q * (2 eb)) in place
  *                (ZCCLd_float.c:2855-2857).
+ *                For block sides 2, 4 and 8, K3 forms the z and y sums as it
+ *                decodes, and the volume is passed over twice in all.
  * Block sides 2, 4 and 8 (row-mapped kernels): a warp takes a run of 32 / bs
  * blocks along z and walks their rows, coalesced, with the neighbours in
  * registers; compress is one pass (K1-K3 together, quantizing as it loads,
  * the run's place in the stream by decoupled look-back; no quantized
- * volume); decompress K3 stages each run's bytes in shared memory and
- * writes whole rows.  Other block sides: a quantized volume, then
+ * volume).  Other block sides: a quantized volume, then
  * a warp (up to 512 elements) or a CTA per block.
  * Integer sums wrap modulo 2^32 like the reference's int.
  */
+#include <algorithm>
+
 #include "zkern.cuh"
 
 namespace {
@@ -197,6 +200,7 @@ struct Sz3Split {
     double d;
     float hi, lo;
     int ok;
+    int mid; /* 2^-60 <= d <= 2^60: a product with an integer stays far from float's limits */
 };
 
 Sz3Split sz3_split(double d)
@@ -206,6 +210,7 @@ Sz3Split sz3_split(double d)
     s.hi = (float)d;
     s.lo = (float)(d - (double)s.hi);
     s.ok = d >= 0x1p-90 && d <= 0x1p90;
+    s.mid = d >= 0x1p-60 && d <= 0x1p60;
     return s;
 }
 
@@ -249,27 +254,65 @@ __device__ __forceinline__ int32_t sz3_quantize(float x, const Sz3Split &inv, ui
     return (int32_t)v;
 }
 
-/* (float)((double)q * twice) (ZCCLd_float.c:2857): with the product as a
- * float pair (within 2^-22 of an ulp of the result for |q| < 2^24), its
- * nearest float is the reference's unless the pair lies within 2^-18 of
- * half an ulp from it (a midpoint the double rounding could decide) or the
- * result is a power of two or tiny; those take the double steps. */
-__device__ __forceinline__ float sz3_value(int32_t q, const Sz3Split &tw)
+/* (float)((double)q * twice) (ZCCLd_float.c:2857), |q| < 2^24 (`sure` is false
+ * beyond), with tw.mid.
+ * EXACT: twice is a float (as where the caller's bound is one), so the double
+ * product is exact and the float product rounds the same number once.  (Small
+ * q often meet exact ties then, which no rounding test can settle.)
+ * Else the product is formed as a float pair hi + lo, within 2^-46 of it;
+ * r = hi + lo rounded, and d the exact rest (Fast2Sum).  r is the reference's
+ * result unless the product lies so near the middle between r and a neighbour
+ * that the double rounding could decide: if r + d (1 + 2^-17) still rounds to
+ * r, the rest is below half an ulp by 2^-17 of it, far more than both
+ * roundings and the pair's error (the test is exact at powers of two, where
+ * the ulp changes). */
+template <bool EXACT>
+__device__ __forceinline__ float sz3_value(int32_t q, const Sz3Split &tw, bool &sure)
 {
-    if (tw.ok && q == 0) return 0.0f;
-    if (tw.ok && q > -16777216 && q < 16777216) {
-        const float qf = (float)q;
-        const float hi = __fmul_rn(qf, tw.hi);
-        const float lo = __fmaf_rn(qf, tw.lo, __fmaf_rn(qf, tw.hi, -hi));
-        const float r = __fadd_rn(hi, lo);
-        const uint32_t rb = __float_as_uint(r) & 0x7FFFFFFFu, ex = rb >> 23;
-        if (ex > 24u && ex < 254u && (rb & 0x7FFFFFu) != 0u) {
-            const float half = __uint_as_float((ex - 24u) << 23); /* half an ulp of r */
-            const float d = __fadd_rn(__fsub_rn(hi, r), lo);      /* (hi + lo) - r */
-            if (fabsf(d) < __fmul_rn(half, 0.999996185302734375f)) return r; /* 1 - 2^-18 */
+    const float qf = (float)q;
+    const float hi = __fmul_rn(qf, tw.hi);
+    sure = fabsf(qf) < 16777216.0f;
+    if (EXACT) return hi;
+    const float lo = __fmaf_rn(qf, tw.lo, __fmaf_rn(qf, tw.hi, -hi));
+    const float r = __fadd_rn(hi, lo);
+    const float d = __fsub_rn(lo, __fsub_rn(r, hi));
+    sure = sure && __fmaf_rn(d, 1.00000762939453125f, r) == r; /* 1 + 2^-17 */
+    return r;
+}
+
+/* N of them; the unsure ones (about one in 2^17) by the double steps, with
+ * one branch for all. */
+template <bool EXACT, uint32_t N>
+__device__ __forceinline__ void sz3_values(const uint32_t (&q)[N], const Sz3Split &tw, float (&v)[N])
+{
+    bool all = true;
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) {
+        bool sure;
+        v[k] = sz3_value<EXACT>((int32_t)q[k], tw, sure);
+        all &= sure;
+    }
+    if (!all) {
+#pragma unroll
+        for (uint32_t k = 0; k < N; k++) {
+            bool sure;
+            sz3_value<EXACT>((int32_t)q[k], tw, sure);
+            if (!sure) v[k] = (float)__dmul_rn((double)(int32_t)q[k], tw.d);
         }
     }
-    return (float)__dmul_rn((double)q, tw.d);
+}
+
+template <uint32_t N>
+__device__ __forceinline__ void sz3_values(const uint32_t (&q)[N], const Sz3Split &tw, float (&v)[N])
+{
+    if (tw.mid && tw.lo == 0.0f) { /* uniform over the grid */
+        sz3_values<true>(q, tw, v);
+    } else if (tw.mid) {
+        sz3_values<false>(q, tw, v);
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < N; k++) v[k] = (float)__dmul_rn((double)(int32_t)q[k], tw.d);
+    }
 }
 
 /* ---- K0: quantization -------------------------------------------------- */
@@ -757,72 +800,590 @@ __global__ void __launch_bounds__(SZ_THREADS, BS <= 4 ? 4 : 3) k_sz3_compress_ro
     if (full) atomicOr(err, ZERR_CAPACITY);
 }
 
-/* Bytes that hold a unit's blocks at most (every block at rate 32). */
+/* ---- block sides 2, 4 and 8: decompress ---------------------------------
+ * The inverse of the mixed difference is a prefix sum along each axis, in any
+ * order, so the decoder sums along y and z what it decodes and one pass along
+ * x finishes: the volume is written as integers, read and written as floats
+ * (12 bytes of traffic an element instead of the 28 of a pass per axis).
+ * 301 x 450 x 517, side 8: 858 us before (decode 347, z 93, y 120, x 406
+ * alone), 258 now (decode and sums 118, x 103, the carries 15).
+ * 512^3: side 8 382 us, 4 389, 2 558.
+ *
+ * A strip is a row of blocks along z; its bytes are consecutive in the stream.
+ * A part is PARTS strips along y.  Consumer warps take one layer of a part's
+ * blocks each (BS = 8: one plane, 4: one plane, 2: both), a chunk of up to 32
+ * blocks of a strip at a time, a lane per block: a lane decodes octets (8
+ * consecutive elements of its block: one row of 8, two of 4, or the four of 2
+ * with both planes), adds them to its columns' running y sums (registers), and
+ * a warp scan makes the z sums, whose carry along the row sits in shared
+ * memory.  Rows leave through shared memory, coalesced.
+ * A producer warp copies the chunks' bytes into a ring of slots.  Blocks of 512 elements take whole
+ * multiples of 64 bytes, so side by side the lanes' reads would meet in one
+ * bank 16 times over (512^3: 239 us, 94 % of the cycles on shared memory);
+ * they are placed one bank apart, by 4-byte asynchronous copies.  Where a
+ * chunk does not fit a slot (side 8, rates above about 10) it goes in pieces
+ * of 16 or 8 blocks; pieces of up to 16 blocks have 2, 4 or 8 rows decoded
+ * side by side, summed along y by shuffles.
+ * The parts' y sums start at zero; each part's last row is kept (`carry`), and
+ * the pass along x adds the sums of the parts before it. */
 template <uint32_t BS>
-__host__ __device__ constexpr uint32_t sz3_unit_stage()
-{
-    return ((32 / BS) * ((BS * BS * BS + 7) / 8 + 4 * BS * BS * BS) + 15) & ~15u;
-}
+struct Sz3Un {
+    static constexpr uint32_t PI = BS == 2 ? 2 : 1, PJ = BS == 8 ? 1 : 2; /* planes and rows of an octet */
+    static constexpr uint32_t PW = BS / PI, STRIPS = 8 / PW;              /* warps per strip, strips per CTA (along x) */
+    static constexpr uint32_t PARTS = BS == 8 ? 1 : 16 / BS;              /* strips per part: 8 or 16 rows */
+    static constexpr uint32_t ROWS = PARTS * BS, NB = BS * BS * BS;
+    static constexpr uint32_t CAP = BS == 8 ? 24u * 1024u : 32u * ((NB + 7) / 8 + 4 * NB); /* bytes of a chunk in a slot */
+    static constexpr uint32_t AREA = (CAP + 32u + NB / 8 + NB + 24u + 15u) & ~15u; /* phase, rounding, what decode_octet reads on */
+    static constexpr uint32_t SLOTS = BS == 8 ? 2 : 3;
+    static constexpr uint32_t SLOT = 16u + STRIPS * (128u + AREA);        /* blocks in it | block descriptors | bytes */
+    static constexpr uint32_t OUT = 4u * 288u;                            /* a warp's rows on their way out */
+    static constexpr uint32_t SMEM = SLOTS * SLOT + 8u * (OUT + 4u * PI * ROWS) + 4096u; /* margin: reads stay inside whatever a slot holds */
+};
+constexpr uint32_t SZ_UN_THREADS = 9 * 32;
 
-/* decompress K3: a warp per unit; the unit's blocks, consecutive in the
- * stream, come into shared memory in one coalesced copy, then every lane
- * decodes its own elements straight into whole rows of the output */
-template <uint32_t BS>
-__global__ void __launch_bounds__(SZ_THREADS) k_sz3_unpack_rows(const uint8_t *__restrict__ in, uint64_t avail,
-                                                                Sz3Dims g, const uint64_t *__restrict__ offs,
-                                                                uint32_t *__restrict__ vol, uint32_t *err)
+/* Chunks of 32 blocks of the strips, in stream order: their payload bytes (a
+ * warp per chunk). */
+__global__ void __launch_bounds__(SZ_THREADS) k_sz3_chunk_sizes(const uint8_t *__restrict__ in, uint64_t avail, Sz3Dims g,
+                                                                uint64_t nchunks, uint32_t *__restrict__ sizes, uint32_t *err)
 {
-    constexpr uint32_t U = 32 / BS, STAGE = sz3_unit_stage<BS>();
-    extern __shared__ __align__(16) uint8_t st_all[];
-    const uint32_t lane = threadIdx.x & 31u, dz = lane % BS, c = lane / BS;
-    uint8_t *stg = st_all + (threadIdx.x >> 5) * STAGE;
-    const uint64_t units = sz3_units<BS>(g), s0 = g.d2 * g.d3, s1 = g.d3;
+    constexpr uint32_t C = 4; /* chunks at a time */
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nzc = (g.nb3 + 31) / 32;
     uint32_t flag = 0;
-    for (uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units;
-         u += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
-        const Sz3Unit k = sz3_unit<BS>(g, u);
-        uint32_t rate = 0;
-        uint64_t base = 0, end = 0;
-        if (lane < U && k.bk0 + lane < g.nb3) { /* lane c: block c's rate and place */
-            const uint64_t b = (k.bi * g.nb2 + k.bj) * g.nb3 + k.bk0 + lane;
-            const uint32_t n = k.sx * k.sy * sz3_unit_sz<BS>(g, k, lane);
-            rate = b < avail ? in[b] : 0u;
-            base = g.nblocks + offs[b];
-            if (rate > 32 || base + sz3_payload(rate, n) > avail) {
-                flag |= rate > 32 ? ZERR_CORRUPT : ZERR_BOUNDS;
-                rate = 0;
+    for (uint64_t c0 = C * (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); c0 < nchunks;
+         c0 += C * (((uint64_t)gridDim.x * blockDim.x) >> 5)) {
+        uint32_t rate[C], n[C];
+        uint64_t strip = c0 / nzc, zc = c0 % nzc;
+#pragma unroll
+        for (uint32_t u = 0; u < C; u++) {
+            const uint64_t bk = zc * 32 + lane, b = strip * g.nb3 + bk;
+            const bool in_vol = c0 + u < nchunks && bk < g.nb3;
+            const uint64_t bj = strip % g.nb2, bi = strip / g.nb2;
+            rate[u] = in_vol && b < avail ? in[b] : 0u;
+            if (in_vol && b >= avail) flag |= ZERR_BOUNDS;
+            n[u] = in_vol ? (uint32_t)(min((uint64_t)g.bs, g.d1 - bi * g.bs) * min((uint64_t)g.bs, g.d2 - bj * g.bs) *
+                                       min((uint64_t)g.bs, g.d3 - bk * g.bs))
+                          : 0u;
+            if (++zc == nzc) {
+                zc = 0;
+                strip++;
             }
-            end = rate ? base + sz3_payload(rate, n) : 0;
-        }
-        /* blocks follow one another in the stream: the unit's bytes are
-         * [block 0's place, the last end), at most STAGE of them (the places
-         * come from the same rates; checked all the same) */
-        const uint64_t first = __shfl_sync(0xffffffffu, base, 0);
-        if (rate && (base < first || end - first > STAGE)) {
-            flag |= ZERR_CORRUPT;
-            rate = 0;
-            end = 0;
         }
 #pragma unroll
-        for (uint32_t o = 16; o; o >>= 1) end = max(end, __shfl_xor_sync(0xffffffffu, end, o));
-        const uint32_t nbytes = end > first ? (uint32_t)min(end - first, (uint64_t)STAGE) : 0u;
-        __syncwarp(); /* the previous unit is decoded */
-#pragma unroll 8
-        for (uint32_t t = lane; t < nbytes; t += 32) stg[t] = in[first + t];
-        __syncwarp();
-        const uint32_t rl = __shfl_sync(0xffffffffu, rate, c);
-        const uint64_t bl = __shfl_sync(0xffffffffu, base, c);
-        const uint32_t sz = sz3_unit_sz<BS>(g, k, c), n = k.sx * k.sy * sz;
-        if (k.z0 + lane < g.d3) {
-            const uint8_t *sg = stg + (rl ? bl - first : 0);
-            uint32_t *o = vol + k.i0 * s0 + k.j0 * s1 + k.z0 + lane;
-            for (uint32_t di = 0; di < k.sx; di++)
-#pragma unroll
-                for (uint32_t dj = 0; dj < BS; dj++)
-                    if (dj < k.sy) o[di * s0 + dj * s1] = sz3_unpack_elem(sg, rl, n, (di * k.sy + dj) * sz + dz);
+        for (uint32_t u = 0; u < C; u++) {
+            if (rate[u] > 32) {
+                flag |= ZERR_CORRUPT;
+                rate[u] = 0;
+            }
+            const uint32_t size = __reduce_add_sync(0xffffffffu, sz3_payload(rate[u], n[u]));
+            if (lane == 0 && c0 + u < nchunks) sizes[c0 + u] = size;
         }
     }
     if (flag) atomicOr(err, flag);
+}
+
+/* Where a CTA is in its chunks: one of every strip of it at a time. */
+template <uint32_t BS>
+struct Sz3Pos {
+    uint64_t task, ntasks, nparts, nbg;
+    uint64_t cb, bj, bj1, bi0;
+    __device__ __forceinline__ void begin(const Sz3Dims &g)
+    {
+        if (task >= ntasks) return;
+        bi0 = (nbg - 1 - task / nparts) * Sz3Un<BS>::STRIPS;
+        bj = (task % nparts) * Sz3Un<BS>::PARTS;
+        bj1 = min(bj + Sz3Un<BS>::PARTS, g.nb2);
+        cb = 0;
+    }
+    __device__ __forceinline__ void advance(const Sz3Dims &g)
+    {
+        if (++bj < bj1) return;
+        cb += 32;
+        if (cb < g.nb3) {
+            bj = (task % nparts) * Sz3Un<BS>::PARTS;
+            return;
+        }
+        task += gridDim.x;
+        begin(g);
+    }
+};
+
+/* Producer, sides 2 and 4: lane s sends strip s's chunk and lane STRIPS + s
+ * its rates, from which the strip's consumers place its blocks; the next
+ * chunk's place is on its way meanwhile. */
+template <uint32_t BS>
+__device__ __forceinline__ void sz3_produce_small(const uint8_t *__restrict__ in, uint64_t avail, const Sz3Dims &g,
+                                                  const uint64_t *__restrict__ offs, const uint32_t *__restrict__ sizes,
+                                                  uint8_t *slots, uint64_t *full, uint64_t *empty, Sz3Pos<BS> p, uint32_t *err)
+{
+    using U = Sz3Un<BS>;
+    const uint32_t lane = threadIdx.x & 31u, s = lane % U::STRIPS;
+    const uint64_t nzc = (g.nb3 + 31) / 32;
+    if (lane >= 2 * U::STRIPS) return;
+    auto fetch = [&](uint64_t &at, uint32_t &bytes) {
+        const uint64_t bi = p.bi0 + s, strip = bi * g.nb2 + p.bj;
+        at = avail;
+        bytes = 0;
+        if (p.task >= p.ntasks || bi >= g.nb1) return;
+        if (lane < U::STRIPS) {
+            at = g.nblocks + offs[strip * nzc + p.cb / 32];
+            bytes = sizes[strip * nzc + p.cb / 32];
+        } else {
+            at = strip * g.nb3 + p.cb;
+            bytes = (uint32_t)min((uint64_t)32, g.nb3 - p.cb);
+        }
+    };
+    uint64_t nat;
+    uint32_t nbytes, it = 0;
+    fetch(nat, nbytes);
+    for (; p.task < p.ntasks; it++) {
+        const uint64_t at = nat;
+        const uint32_t bytes = at >= avail ? 0u : (uint32_t)min((uint64_t)nbytes, avail - at);
+        p.advance(g);
+        fetch(nat, nbytes);
+        const uint32_t slot = it % U::SLOTS;
+        uint8_t *sl = slots + slot * U::SLOT, *head = sl + 16u + 128u * s;
+        if (it >= U::SLOTS) mbar_wait(empty + slot, (it / U::SLOTS - 1u) & 1u, err);
+        reinterpret_cast<uint64_t *>(head)[lane / U::STRIPS] = at;
+        tma_load_superset(lane < U::STRIPS ? sl + 16u + 128u * U::STRIPS + s * U::AREA : head + 16u, in + at, bytes, full + slot);
+    }
+}
+
+/* Producer, side 8 (one strip): block c at word c (mod 32) of the slot, in as
+ * many pieces as it takes. */
+__device__ __forceinline__ void sz3_produce8(const uint8_t *__restrict__ in, uint64_t avail, const Sz3Dims &g,
+                                             const uint64_t *__restrict__ offs, uint8_t *slots, uint64_t *full,
+                                             uint64_t *empty, Sz3Pos<8> p, uint32_t *err)
+{
+    using U = Sz3Un<8>;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nzc = (g.nb3 + 31) / 32;
+    uint32_t flag = 0, it = 0, nrate = 0;
+    uint64_t nbase = 0;
+    auto fetch = [&]() { /* the next chunk's rates and place */
+        if (p.task >= p.ntasks) return;
+        const uint64_t strip = p.bi0 * g.nb2 + p.bj, at = strip * g.nb3 + p.cb + lane;
+        nrate = p.cb + lane < g.nb3 && at < avail ? in[at] : 0u;
+        nbase = g.nblocks + offs[strip * nzc + p.cb / 32];
+    };
+    fetch();
+    while (p.task < p.ntasks) {
+        const uint32_t kb = (uint32_t)min((uint64_t)32, g.nb3 - p.cb);
+        const uint32_t sx = (uint32_t)min((uint64_t)8, g.d1 - p.bi0 * 8), sy = (uint32_t)min((uint64_t)8, g.d2 - p.bj * 8);
+        const uint32_t sz = lane < kb ? (uint32_t)min((uint64_t)8, g.d3 - (p.cb + lane) * 8) : 0u;
+        uint32_t rate = nrate > 32u ? 0u : nrate; /* reported with the sizes */
+        const uint32_t pay = sz3_payload(rate, sx * sy * sz), inc = warp_incl_scan(pay);
+        const uint64_t at = nbase + (inc - pay);
+        if (rate && at + pay > avail) {
+            flag |= ZERR_BOUNDS;
+            rate = 0;
+        }
+        p.advance(g);
+        fetch();
+        const uint32_t phase = (uint32_t)(reinterpret_cast<uintptr_t>(in) + at) & 3u;
+        const uint32_t words = rate ? (phase + pay + 3u) / 4u : 0u, room = ((words + 31u) & ~31u) + 1u;
+        const uint32_t rinc = warp_incl_scan(room);
+        const uint32_t half = __shfl_sync(0xffffffffu, rinc, 15), all = __shfl_sync(0xffffffffu, rinc, 31);
+        uint32_t kk = 32;
+        if (4u * all > U::CAP) kk = 4u * half <= U::CAP && 4u * (all - half) <= U::CAP ? 16 : 8;
+        const uint8_t *mine = in + (at - phase); /* this lane's block */
+        for (uint32_t sb = 0; sb < kb; sb += kk, it++) {
+            const uint32_t slot = it % U::SLOTS;
+            uint8_t *sl = slots + slot * U::SLOT;
+            if (it >= U::SLOTS) mbar_wait(empty + slot, (it / U::SLOTS - 1u) & 1u, err);
+            const uint32_t lo = __shfl_sync(0xffffffffu, rinc - room, sb), pos = rinc - room - lo;
+            if (lane >= sb && lane < sb + kk)
+                reinterpret_cast<uint32_t *>(sl + 16)[lane - sb] = (4u * pos + phase) | rate << 24;
+            if (lane == 0) *reinterpret_cast<uint32_t *>(sl) = min(kk, kb - sb);
+            const uint32_t area = smem_u32(sl + 16u + 128u) + 4u * lane;
+            const uint32_t last = min(sb + kk, kb);
+#pragma unroll 2
+            for (uint32_t c = sb; c < last; c++) {
+                const uint32_t nw = __shfl_sync(0xffffffffu, words, c), d = area + 4u * __shfl_sync(0xffffffffu, pos, c);
+                const uint8_t *src =
+                    reinterpret_cast<const uint8_t *>(__shfl_sync(0xffffffffu, reinterpret_cast<uintptr_t>(mine), c)) + 4u * lane;
+                for (uint32_t t = 0; t < nw; t += 128) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 128; q += 32)
+                        if (lane + t + q < nw) cp_async4(d + 4u * (t + q), src + 4u * (t + q));
+                }
+            }
+            cp_async_arrive(full + slot); /* every lane, when its copies have landed */
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + slot); /* and the descriptors */
+        }
+    }
+    if (flag) atomicOr(err, flag);
+}
+
+/* What a warp decodes at a time: k blocks of one strip, from block c0 on, in
+ * the planes from i0 on. */
+struct Sz3Piece {
+    const uint8_t *area;
+    uint32_t dsc; /* lane c: block c's place in the area and its rate << 24 (0: no block) */
+    uint32_t *outw, *zc; /* the warp's row buffer; its rows' z sums */
+    uint32_t *o;         /* the volume at (i0, the strip's first row, the first block's z + lane) */
+    uint32_t *co;        /* the same place in the part's kept rows; null if none of these rows is kept */
+    uint64_t s0, s1;     /* strides of the volume along x and y */
+    uint64_t cs;         /* stride of the kept rows along x */
+    uint32_t k, sx, sy, di0, row0, zlim, zleft;
+    bool first;          /* the rows begin here */
+};
+
+/* LK: 2^LK lanes a row (side 8 may take fewer than 32, and 32 >> LK rows side
+ * by side).  WHOLE: the blocks are whole along y and z. */
+template <uint32_t BS, uint32_t LK, bool WHOLE>
+__device__ __forceinline__ void sz3_strip(const Sz3Piece &w, uint32_t (&y)[Sz3Un<BS>::PI * BS])
+{
+    using U = Sz3Un<BS>;
+    constexpr uint32_t PJ = U::PJ, NR = 8 / BS, kk = 1u << LK, RJ = 32u >> LK;
+    const uint32_t lane = threadIdx.x & 31u, c = lane & (kk - 1u), rj = lane >> LK;
+    const uint32_t sy = WHOLE ? BS : w.sy, NJ = (sy + PJ - 1) / PJ;
+    const uint32_t dsc = LK == 5 ? w.dsc : __shfl_sync(0xffffffffu, w.dsc, c);
+    const uint32_t rate = min(dsc >> 24, 32u), off = min(dsc & 0xFFFFFFu, U::CAP + 16u);
+    const uint32_t sz = WHOLE ? BS : c < w.k ? min(BS, w.zleft - c * BS) : 0u, n = w.sx * sy * sz;
+    const bool octets = WHOLE || (sz == BS && sy % PJ == 0); /* every octet is 8 consecutive elements */
+    const uint32_t g0 = BS == 2 ? 0u : (w.di0 * sy) / PJ;
+    uint32_t *o = w.o;
+    uint32_t *src = w.outw + (BS == 8 ? (lane >> 3) * 4u + (lane & 3u) + ((lane >> 2) & 1u) * 144u : lane);
+    constexpr uint32_t STEP = BS == 8 ? 16 : 32; /* words of src per 32 elements */
+#pragma unroll(LK == 5 && BS < 8 ? 4 : 1)
+    for (uint32_t j = 0; j < NJ; j += RJ, o += RJ * PJ * w.s1) {
+        const uint32_t jj = j + rj;
+        uint32_t v[8];
+        if (WHOLE) {
+            decode_octet(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
+        } else {
+#pragma unroll
+            for (uint32_t e = 0; e < 8; e++) v[e] = 0;
+            if (jj < NJ && sz) {
+                if (octets) {
+                    decode_octet(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
+                } else { /* at the volume's end: an element at a time */
+#pragma unroll
+                    for (uint32_t e = 0; e < 8; e++) {
+                        const uint32_t r = e / BS, di = w.di0 + r / PJ, dj = jj * PJ + r % PJ, dz = e % BS;
+                        if (di < w.sx && dj < sy && dz < sz)
+                            v[e] = sz3_unpack_elem(w.area + off, rate, n, (di * sy + dj) * sz + dz);
+                    }
+                }
+            }
+        }
+        /* y sums */
+        if (BS == 8) {
+#pragma unroll
+            for (uint32_t t = kk; t < 32; t <<= 1)
+#pragma unroll
+                for (uint32_t e = 0; e < 8; e++) {
+                    const uint32_t u = __shfl_up_sync(0xffffffffu, v[e], t);
+                    if (lane >= t) v[e] += u;
+                }
+#pragma unroll
+            for (uint32_t e = 0; e < 8; e++) v[e] += y[e % (U::PI * BS)];
+#pragma unroll
+            for (uint32_t e = 0; e < 8; e++)
+                y[e % (U::PI * BS)] = RJ == 1 ? v[e] : __shfl_sync(0xffffffffu, v[e], 32u - kk + c);
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r < NR; r++)
+#pragma unroll
+                for (uint32_t e = 0; e < BS; e++) y[(r / PJ) * BS + e] = v[r * BS + e] += y[(r / PJ) * BS + e];
+        }
+        /* z sums */
+#pragma unroll
+        for (uint32_t r = 0; r < NR; r++) {
+            uint32_t tot = v[r * BS];
+#pragma unroll
+            for (uint32_t e = 1; e < BS; e++) tot += v[r * BS + e];
+            uint32_t run = tot;
+#pragma unroll
+            for (uint32_t t = 1; t < kk; t <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, run, t);
+                if (c >= t) run += u;
+            }
+            uint32_t *z = w.zc + (r / PJ) * U::ROWS + w.row0 + jj * PJ + r % PJ;
+            const uint32_t before = w.first ? 0u : *z;
+            __syncwarp();
+            if (c == kk - 1u) *z = before + run;
+            v[r * BS] += before + run - tot;
+#pragma unroll
+            for (uint32_t e = 1; e < BS; e++) v[r * BS + e] += v[r * BS + e - 1];
+        }
+        /* out, whole rows: word e of the warp's 256 in row order is element e (side 8: the halves of a
+         * block's row 144 words apart, so that neither side meets bank conflicts).  The barriers above
+         * part this from the last row's reads. */
+        if (BS == 8) {
+            *reinterpret_cast<uint4 *>(w.outw + 4u * lane) = make_uint4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<uint4 *>(w.outw + 144u + 4u * lane) = make_uint4(v[4], v[5], v[6], v[7]);
+        } else if (BS == 4) {
+            *reinterpret_cast<uint4 *>(w.outw + 4u * lane) = make_uint4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<uint4 *>(w.outw + 128u + 4u * lane) = make_uint4(v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r < NR; r++)
+                *reinterpret_cast<uint2 *>(w.outw + 64u * r + 2u * lane) = make_uint2(v[2 * r], v[2 * r + 1]);
+        }
+        __syncwarp();
+        if (LK == 5) {
+#pragma unroll
+            for (uint32_t r = 0; r < NR; r++)
+                if ((U::PI == 1 || w.di0 + r / PJ < w.sx) && (WHOLE || j * PJ + r % PJ < sy)) { /* uniform */
+                    uint32_t *p = o + (r / PJ) * w.s0 + (r % PJ) * w.s1;
+                    if (WHOLE && w.zlim == 32u * BS) {
+#pragma unroll
+                        for (uint32_t q = 0; q < BS; q++) p[32u * q] = src[(r * BS + q) * STEP];
+                    } else {
+#pragma unroll
+                        for (uint32_t q = 0; q < BS; q++)
+                            if (lane + 32u * q < w.zlim) p[32u * q] = src[(r * BS + q) * STEP];
+                    }
+                    if (w.co && j * PJ + r % PJ + 1u == sy) { /* the part's last row */
+                        uint32_t *cp = w.co + (r / PJ) * w.cs;
+#pragma unroll
+                        for (uint32_t q = 0; q < BS; q++)
+                            if (lane + 32u * q < w.zlim) cp[32u * q] = src[(r * BS + q) * STEP];
+                    }
+                }
+        } else { /* side 8, RJ rows of kk blocks */
+#pragma unroll
+            for (uint32_t q = 0; q < 8; q++) {
+                const uint32_t r = q / (kk / 4u), z = 32u * (q % (kk / 4u));
+                if ((WHOLE || j + r < sy) && lane + z < w.zlim) {
+                    const uint32_t x = src[q * STEP];
+                    o[r * w.s1 + z] = x;
+                    if (w.co && j + r + 1u == sy) w.co[z] = x;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
+template <uint32_t BS>
+__global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8_t *__restrict__ in, uint64_t avail, Sz3Dims g,
+                                                                     const uint64_t *__restrict__ offs,
+                                                                     const uint32_t *__restrict__ sizes,
+                                                                     uint32_t *__restrict__ vol, uint32_t *__restrict__ carry,
+                                                                     uint32_t *err)
+{
+    using U = Sz3Un<BS>;
+    constexpr uint32_t PI = U::PI;
+    extern __shared__ __align__(16) uint8_t sm[];
+    __shared__ uint64_t full[U::SLOTS], empty[U::SLOTS];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t nparts = (g.nb2 + U::PARTS - 1) / U::PARTS, nbg = (g.nb1 + U::STRIPS - 1) / U::STRIPS, ntasks = nparts * nbg;
+    if (threadIdx.x == 0)
+        for (uint32_t i = 0; i < U::SLOTS; i++) {
+            mbar_init(full + i, BS == 8 ? 33 : 2 * U::STRIPS);
+            mbar_init(empty + i, 8);
+        }
+    __syncthreads();
+    if (warp == 8) {
+        Sz3Pos<BS> p;
+        p.task = blockIdx.x;
+        p.ntasks = ntasks;
+        p.nparts = nparts;
+        p.nbg = nbg;
+        p.begin(g);
+        if constexpr (BS == 8)
+            sz3_produce8(in, avail, g, offs, sm, full, empty, p, err);
+        else
+            sz3_produce_small<BS>(in, avail, g, offs, sizes, sm, full, empty, p, err);
+        return;
+    }
+    const uint32_t s = warp / U::PW;
+    Sz3Piece w;
+    w.outw = reinterpret_cast<uint32_t *>(sm + U::SLOTS * U::SLOT + warp * (U::OUT + 4u * PI * U::ROWS));
+    w.zc = w.outw + U::OUT / 4u; /* [PI][ROWS] */
+    w.di0 = (warp % U::PW) * PI;
+    w.s0 = g.d2 * g.d3;
+    w.s1 = g.d3;
+    w.cs = g.d3;
+    uint32_t it = 0, flag = 0;
+    for (uint64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
+        const uint64_t part = task % nparts, bi = (nbg - 1 - task / nparts) * U::STRIPS + s;
+        const uint64_t bj0 = part * U::PARTS, bj1 = min(bj0 + U::PARTS, g.nb2), i0 = bi * BS + w.di0;
+        w.sx = bi < g.nb1 ? (uint32_t)min((uint64_t)BS, g.d1 - bi * BS) : 0u;
+        for (uint64_t c0 = 0; c0 < g.nb3; c0 += w.k) {
+            uint32_t y[PI * BS]; /* the columns' y sums */
+#pragma unroll
+            for (uint32_t e = 0; e < PI * BS; e++) y[e] = 0;
+            w.first = c0 == 0;
+            for (uint64_t bj = bj0; bj < bj1; bj++, it++) {
+                const uint32_t slot = it % U::SLOTS;
+                const uint8_t *sl = sm + slot * U::SLOT;
+                mbar_wait(full + slot, (it / U::SLOTS) & 1u, err);
+                const uint8_t *head = sl + 16u + 128u * s;
+                if (BS == 8)
+                    w.k = min(max(*reinterpret_cast<const uint32_t *>(sl), 1u), 32u);
+                else
+                    w.k = (uint32_t)min((uint64_t)32, g.nb3 - c0);
+                if (w.di0 < w.sx) {
+                    w.area = sl + 16u + 128u * U::STRIPS + s * U::AREA;
+                    w.sy = (uint32_t)min((uint64_t)BS, g.d2 - bj * BS);
+                    if (BS == 8) {
+                        w.dsc = lane < w.k ? reinterpret_cast<const uint32_t *>(head)[lane] : 0u;
+                    } else { /* the blocks' places, from their rates */
+                        const uint64_t at = reinterpret_cast<const uint64_t *>(head)[0], rat = reinterpret_cast<const uint64_t *>(head)[1];
+                        uint32_t rate = lane < w.k && rat + lane < avail
+                                            ? head[16u + ((uint32_t)(reinterpret_cast<uintptr_t>(in) + rat) & 15u) + lane]
+                                            : 0u;
+                        if (rate > 32u) rate = 0; /* reported with the sizes */
+                        const uint32_t zl = (uint32_t)min(g.d3 - c0 * BS, (uint64_t)(32u * BS));
+                        const uint32_t pay = sz3_payload(rate, w.sx * w.sy * min(BS, zl - min(zl, lane * BS)));
+                        const uint32_t inc = warp_incl_scan(pay);
+                        if (rate && at + inc > avail) {
+                            flag |= ZERR_BOUNDS;
+                            rate = 0;
+                        }
+                        w.dsc = (inc - pay + ((uint32_t)(reinterpret_cast<uintptr_t>(in) + at) & 15u)) | rate << 24;
+                    }
+                    w.row0 = (uint32_t)(bj - bj0) * BS;
+                    w.zleft = (uint32_t)min(g.d3 - c0 * BS, (uint64_t)(32u * BS));
+                    w.zlim = min(w.zleft, w.k * BS);
+                    w.o = vol + i0 * w.s0 + bj * BS * w.s1 + c0 * BS + lane;
+                    w.co = part + 1 < nparts && bj + 1 == bj1 ? carry + (part * g.d1 + i0) * g.d3 + c0 * BS + lane : nullptr;
+                    const bool whole = w.sy == BS && w.zlim == w.k * BS;
+                    if (BS < 8 || w.k > 16) {
+                        if (whole) sz3_strip<BS, 5, true>(w, y);
+                        else sz3_strip<BS, 5, false>(w, y);
+                    } else if constexpr (BS == 8) {
+                        if (w.k > 8) {
+                            if (whole) sz3_strip<8, 4, true>(w, y);
+                            else sz3_strip<8, 4, false>(w, y);
+                        } else if (w.k > 4) {
+                            if (whole) sz3_strip<8, 3, true>(w, y);
+                            else sz3_strip<8, 3, false>(w, y);
+                        } else {
+                            if (whole) sz3_strip<8, 2, true>(w, y);
+                            else sz3_strip<8, 2, false>(w, y);
+                        }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty + slot);
+            }
+        }
+    }
+    if (flag) atomicOr(err, flag);
+}
+
+/* The parts' last rows summed over the parts, in place: a thread per (plane,
+ * z), batches of rows loaded together. */
+__global__ void __launch_bounds__(256) k_sz3_carry(uint32_t *__restrict__ carry, uint64_t columns, uint64_t parts)
+{
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= columns) return;
+    uint32_t run = 0;
+    for (uint64_t p0 = 0; p0 < parts; p0 += SZ_SCAN_BATCH) {
+        uint32_t v[SZ_SCAN_BATCH];
+#pragma unroll
+        for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++) v[u] = p0 + u < parts ? carry[(p0 + u) * columns + t] : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++) {
+            run += v[u];
+            if (p0 + u < parts) carry[(p0 + u) * columns + t] = run;
+        }
+    }
+}
+
+/* The last pass: x sums of the volume and the parts' carries, floats in place.
+ * A CTA takes a run of up to FQ * 288 consecutive elements of a plane (R whole
+ * rows of one part, or a piece of a long row) and walks along x, FQ columns'
+ * sums a thread.  A producer warp keeps a ring of stages of FP planes on their
+ * way (the run, and the carry's row that its rows share).  Bound by memory:
+ * 512^3 194 us (5.5 TB/s), against 351 with the threads themselves loading 4
+ * planes ahead into registers. */
+constexpr uint32_t FQ = 4, FP = 2, FCOLS = FQ * 288;
+
+struct Sz3Run {
+    uint32_t R;      /* rows in a run */
+    uint32_t pieces; /* runs per row where rows are longer than a run */
+    uint32_t cols;   /* elements of a full run */
+    uint32_t cz;     /* carry elements of a full run */
+    uint32_t pb, cb; /* bytes of their places in a stage */
+    uint32_t stages;
+};
+
+__global__ void __launch_bounds__(FCOLS / FQ + 32) k_sz3_finish(uint32_t *vol, const uint32_t *carry, uint64_t d1,
+                                                                uint64_t d2, uint64_t d3, uint32_t rows, Sz3Run f,
+                                                                Sz3Split twice, uint32_t *err)
+{
+    extern __shared__ __align__(16) uint8_t ring[]; /* per stage: FP runs, FP carries */
+    __shared__ uint64_t full[8], empty[8];
+    const uint32_t nth = blockDim.x - 32u, stage = FP * (f.pb + f.cb);
+    const uint64_t j0 = blockIdx.x / f.pieces * f.R, z0 = (uint64_t)(blockIdx.x % f.pieces) * f.cols, plane = d2 * d3;
+    const uint64_t part = j0 / rows; /* parts are whole multiples of R rows */
+    const uint32_t cols = f.pieces > 1 ? (uint32_t)min((uint64_t)f.cols, d3 - z0) : (uint32_t)(min((uint64_t)f.R, d2 - j0) * d3);
+    const bool more = part > 0;
+    const uint64_t nst = (d1 + FP - 1) / FP;
+    uint32_t *p0 = vol + j0 * d3 + z0;
+    const uint32_t *c0 = more ? carry + (part - 1) * d1 * d3 + z0 : nullptr;
+    if (threadIdx.x == 0)
+        for (uint32_t i = 0; i < f.stages; i++) {
+            mbar_init(full + i, 2 * FP);
+            mbar_init(empty + i, nth / 32u);
+        }
+    __syncthreads();
+    if (threadIdx.x >= nth) {
+        const uint32_t l = threadIdx.x - nth, pl = l % FP, c = l / FP;
+        if (c >= 2) return;
+        uint32_t slot = 0, round = 0;
+        for (uint64_t st = 0; st < nst; st++) {
+            const uint64_t i = FP * st + pl;
+            if (round) mbar_wait(empty + slot, (round - 1u) & 1u, err);
+            const uint32_t *g = c ? c0 + i * d3 : p0 + i * plane;
+            const uint32_t bytes = i < d1 && (!c || more) ? 4u * (c ? min(cols, f.cz) : cols) : 0u;
+            tma_load_superset(ring + slot * stage + pl * f.pb + c * (FP * f.pb - pl * f.pb + pl * f.cb),
+                              reinterpret_cast<const uint8_t *>(g), bytes, full + slot);
+            if (++slot == f.stages) {
+                slot = 0;
+                round++;
+            }
+        }
+        return;
+    }
+    uint32_t run[FQ], at[FQ], cz[FQ]; /* the columns' sums; their places in the run and in the carry's row */
+#pragma unroll
+    for (uint32_t q = 0; q < FQ; q++) { /* past the run's end: a column again, so that no value is out of the way */
+        run[q] = 0;
+        at[q] = min(threadIdx.x + nth * q, cols - 1u);
+        cz[q] = at[q] % f.cz;
+    }
+    /* where a copy's first element lies in its 16 bytes: the low bits of its address */
+    const uint32_t pv = (uint32_t)(reinterpret_cast<uintptr_t>(p0) >> 2), pc = (uint32_t)(reinterpret_cast<uintptr_t>(c0) >> 2);
+    float *o = reinterpret_cast<float *>(p0) + threadIdx.x;
+    uint32_t slot = 0, round = 0;
+    for (uint64_t st = 0; st < nst; st++, o += FP * plane) {
+        mbar_wait(full + slot, round & 1u, err);
+        uint32_t v[FP * FQ];
+#pragma unroll
+        for (uint32_t pl = 0; pl < FP; pl++) {
+            const uint32_t i = (uint32_t)st * FP + pl; /* its low bits are enough */
+            const uint32_t *s = reinterpret_cast<const uint32_t *>(ring + slot * stage + pl * f.pb) +
+                                ((pv + i * (uint32_t)plane) & 3u);
+            const uint32_t *e = reinterpret_cast<const uint32_t *>(ring + slot * stage + FP * f.pb + pl * f.cb) +
+                                ((pc + i * (uint32_t)d3) & 3u);
+#pragma unroll
+            for (uint32_t q = 0; q < FQ; q++) /* (a plane that is not there: any value, not written) */
+                v[pl * FQ + q] = run[q] += (more ? e[cz[q]] : 0u) + s[at[q]];
+        }
+        __syncwarp();
+        if ((threadIdx.x & 31u) == 0) mbar_arrive(empty + slot);
+        if (++slot == f.stages) {
+            slot = 0;
+            round++;
+        }
+        float x[FP * FQ];
+        sz3_values(v, twice, x);
+#pragma unroll
+        for (uint32_t pl = 0; pl < FP; pl++)
+            if (FP * st + pl < d1) {
+#pragma unroll
+                for (uint32_t q = 0; q < FQ; q++)
+                    if (threadIdx.x + nth * q < cols) o[pl * plane + nth * q] = x[pl * FQ + q];
+            }
+    }
 }
 
 /* ---- decompress K4-K6: the 3-D prefix sum ------------------------------ */
@@ -873,10 +1434,12 @@ __global__ void k_sz3_scan_x(uint32_t *vol, uint64_t d1, uint64_t plane, Sz3Spli
 #pragma unroll
         for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++) v[u] = i0 + u < d1 ? vol[(i0 + u) * plane + t] : 0u;
 #pragma unroll
-        for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++) {
-            run += v[u];
-            if (i0 + u < d1) reinterpret_cast<float *>(vol)[(i0 + u) * plane + t] = sz3_value((int32_t)run, twice);
-        }
+        for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++) v[u] = run += v[u];
+        float f[SZ_SCAN_BATCH];
+        sz3_values(v, twice, f);
+#pragma unroll
+        for (uint32_t u = 0; u < SZ_SCAN_BATCH; u++)
+            if (i0 + u < d1) reinterpret_cast<float *>(vol)[(i0 + u) * plane + t] = f[u];
     }
 }
 
@@ -889,7 +1452,9 @@ unsigned grid_for(uint64_t items, unsigned per_cta)
     return (unsigned)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-/* Scratch layout: err[4] | sizes[nb] | offs[nb] | sums[nchunks] | total | q volume (compress). */
+/* Scratch layout: err[4] | sizes[nb] | offs[nb] | sums[nchunks] | total |
+ * quantized volume (compress, other block sides) or the parts' carries
+ * (decompress, sides 2, 4 and 8). */
 struct Sz3Ws {
     uint32_t *err, *sizes;
     uint64_t *offs, *sums, *total;
@@ -915,12 +1480,13 @@ Sz3Ws sz3_bind(void *ws, const Sz3Dims &g)
     return w;
 }
 
-cudaError_t sz3_scan(const Sz3Dims &g, const Sz3Ws &w, cudaStream_t st)
+/* Offsets of `count` payload sizes; *total includes the rate table. */
+cudaError_t sz3_scan(const Sz3Dims &g, const Sz3Ws &w, uint64_t count, cudaStream_t st)
 {
-    const uint64_t nch = (g.nblocks + SZ_CHUNK - 1) / SZ_CHUNK;
-    k_sz3_chunk_sums<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, g.nblocks, w.sums);
+    const uint64_t nch = (count + SZ_CHUNK - 1) / SZ_CHUNK;
+    k_sz3_chunk_sums<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, count, w.sums);
     k_sz3_scan_sums<<<1, 1024, 0, st>>>(w.sums, nch, g.nblocks, w.total);
-    k_sz3_offsets<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, g.nblocks, w.sums, w.offs);
+    k_sz3_offsets<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, count, w.sums, w.offs);
     return cudaGetLastError();
 }
 
@@ -956,18 +1522,53 @@ cudaError_t sz3_compress_rows(uint8_t *out, uint64_t cap, const float *x, const 
     return cudaGetLastError();
 }
 
-template <uint32_t BS>
-cudaError_t sz3_unpack_rows(const uint8_t *in, uint64_t avail, const Sz3Dims &g, const Sz3Ws &w, uint32_t *vol,
-                            cudaStream_t st)
+/* Bytes of the parts' carries. */
+size_t sz3_carry_bytes(const Sz3Dims &g)
 {
-    const size_t smem = (size_t)sz3_unit_stage<BS>() * (SZ_THREADS / 32);
+    const uint64_t strips = g.bs == 8 ? Sz3Un<8>::PARTS : g.bs == 4 ? Sz3Un<4>::PARTS : Sz3Un<2>::PARTS;
+    return 4 * (size_t)((g.nb2 + strips - 1) / strips - 1) * g.d1 * g.d3;
+}
+
+template <uint32_t BS>
+cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims &g, const Sz3Ws &w, uint32_t *vol,
+                                const Sz3Split &twice, cudaStream_t st)
+{
+    using U = Sz3Un<BS>;
     cudaError_t e;
-    if (smem > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(k_sz3_unpack_rows<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+    const uint64_t nchunks = g.nb1 * g.nb2 * ((g.nb3 + 31) / 32); /* at most nblocks: sizes and offs hold them */
+    k_sz3_chunk_sizes<<<grid_for(nchunks, SZ_THREADS / 8), SZ_THREADS, 0, st>>>(in, avail, g, nchunks, w.sizes, w.err);
+    if ((e = sz3_scan(g, w, nchunks, st)) != cudaSuccess) return e;
+    const void *fn = (const void *)k_sz3_unpack_sum<BS>;
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::SMEM)) != cudaSuccess) return e;
+    int dev = 0, nsm = 0, per = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SZ_UN_THREADS, U::SMEM)) != cudaSuccess)
         return e;
-    k_sz3_unpack_rows<BS><<<grid_for(sz3_units<BS>(g), SZ_THREADS / 32), SZ_THREADS, smem, st>>>(in, avail, g, w.offs,
-                                                                                                 vol, w.err);
+    const uint64_t nparts = (g.nb2 + U::PARTS - 1) / U::PARTS, tasks = nparts * ((g.nb1 + U::STRIPS - 1) / U::STRIPS);
+    const uint64_t most = (uint64_t)nsm * (per > 0 ? per : 1);
+    uint32_t *carry = reinterpret_cast<uint32_t *>(w.q);
+    k_sz3_unpack_sum<BS><<<(unsigned)(tasks < most ? tasks : most), SZ_UN_THREADS, U::SMEM, st>>>(in, avail, g, w.offs, w.sizes,
+                                                                                                 vol, carry, w.err);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const uint64_t columns = g.d1 * g.d3;
+    if (nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, nparts - 1);
+    Sz3Run f;
+    f.R = 1;
+    while (f.R < 8 && 2 * f.R * g.d3 <= FCOLS && g.d2 / (2 * f.R) >= (uint64_t)nsm) f.R *= 2; /* a power of two: rows of one part */
+    f.pieces = (uint32_t)((g.d3 + FCOLS - 1) / FCOLS);
+    f.cz = (uint32_t)((g.d3 + f.pieces - 1) / f.pieces);
+    if (f.pieces > 1) f.cz = (f.cz + 31u) & ~31u; /* <= FCOLS, a multiple of 32 */
+    f.pieces = (uint32_t)((g.d3 + f.cz - 1) / f.cz);
+    f.cols = f.R * f.cz;
+    f.pb = (4u * f.cols + 47u) & ~15u;
+    f.cb = (4u * f.cz + 47u) & ~15u;
+    const uint32_t nth = (f.cols + 32u * FQ - 1) / (32u * FQ) * 32u, stage = FP * (f.pb + f.cb);
+    f.stages = std::min(8u, std::max(2u, 72u * 1024u / stage));
+    const uint32_t smem = f.stages * stage;
+    if ((e = cudaFuncSetAttribute(k_sz3_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
+    k_sz3_finish<<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, U::ROWS, f, twice, w.err);
     return cudaGetLastError();
 }
 
@@ -978,7 +1579,7 @@ size_t sz3_workspace_bytes(uint64_t d1, uint64_t d2, uint64_t d3, uint32_t bs, b
     const Sz3Dims g = sz3_dims(d1, d2, d3, bs);
     Sz3Ws w = sz3_bind(nullptr, g);
     const size_t head = (size_t)reinterpret_cast<uintptr_t>(w.q);
-    return head + (compress && !sz3_rows(bs) ? 4 * (size_t)(d1 * d2 * d3) : 0) + 256;
+    return head + (sz3_rows(bs) ? sz3_carry_bytes(g) : compress ? 4 * (size_t)(d1 * d2 * d3) : 0) + 256;
 }
 
 size_t sz3_max_stream_bytes(uint64_t d1, uint64_t d2, uint64_t d3, uint32_t bs)
@@ -1010,7 +1611,7 @@ cudaError_t sz3_compress(uint8_t *out, uint64_t cap, const float *x, uint64_t d1
         k_sz3_rates<32><<<grid_for(g.nblocks, SZ_THREADS / 32), SZ_THREADS, 0, st>>>(w.q, g, out, w.sizes);
     else
         k_sz3_rates<SZ_THREADS><<<grid_for(g.nblocks, 1), SZ_THREADS, 0, st>>>(w.q, g, out, w.sizes);
-    if ((e = sz3_scan(g, w, st)) != cudaSuccess) return e;
+    if ((e = sz3_scan(g, w, g.nblocks, st)) != cudaSuccess) return e;
     if (wb) {
         k_sz3_pack<32><<<grid_for(g.nblocks, SZ_THREADS / 32), SZ_THREADS, 4ull * bs * bs * bs * (SZ_THREADS / 32), st>>>(
             w.q, g, out, cap, w.offs, w.err);
@@ -1033,20 +1634,21 @@ cudaError_t sz3_decompress(float *y, const uint8_t *in, uint64_t avail, uint64_t
     const Sz3Ws w = sz3_bind(ws, g);
     cudaError_t e = cudaMemsetAsync(w.err + 2, 0, 8, st); /* the ticket; status words stay until checked */
     if (e != cudaSuccess) return e;
-    k_sz3_sizes<<<grid_for(g.nblocks, 256), 256, 0, st>>>(in, avail, g, w.sizes, w.err);
-    if ((e = sz3_scan(g, w, st)) != cudaSuccess) return e;
     uint32_t *vol = reinterpret_cast<uint32_t *>(y);
-    if (sz3_rows(bs)) {
-        e = bs == 2 ? sz3_unpack_rows<2>(in, avail, g, w, vol, st)
-                    : bs == 4 ? sz3_unpack_rows<4>(in, avail, g, w, vol, st) : sz3_unpack_rows<8>(in, avail, g, w, vol, st);
-        if (e != cudaSuccess) return e;
-    } else if (bs * bs * bs <= 512)
+    const Sz3Split twice = sz3_split(eb * 2);
+    if (sz3_rows(bs))
+        return bs == 2   ? sz3_decompress_rows<2>(in, avail, g, w, vol, twice, st)
+               : bs == 4 ? sz3_decompress_rows<4>(in, avail, g, w, vol, twice, st)
+                         : sz3_decompress_rows<8>(in, avail, g, w, vol, twice, st);
+    k_sz3_sizes<<<grid_for(g.nblocks, 256), 256, 0, st>>>(in, avail, g, w.sizes, w.err);
+    if ((e = sz3_scan(g, w, g.nblocks, st)) != cudaSuccess) return e;
+    if (bs * bs * bs <= 512)
         k_sz3_unpack<32><<<grid_for(g.nblocks, SZ_THREADS / 32), SZ_THREADS, 0, st>>>(in, avail, g, w.offs, vol, w.err);
     else
         k_sz3_unpack<SZ_THREADS><<<grid_for(g.nblocks, 1), SZ_THREADS, 0, st>>>(in, avail, g, w.offs, vol, w.err);
     const uint64_t rows = d1 * d2;
     k_sz3_scan_z<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>(vol, rows, d3);
     k_sz3_scan_y<<<(unsigned)((d1 * d3 + 255) / 256), 256, 0, st>>>(vol, d1, d2, d3);
-    k_sz3_scan_x<<<(unsigned)((d2 * d3 + 255) / 256), 256, 0, st>>>(vol, d1, d2 * d3, sz3_split(eb * 2));
+    k_sz3_scan_x<<<(unsigned)((d2 * d3 + 255) / 256), 256, 0, st>>>(vol, d1, d2 * d3, twice);
     return cudaGetLastError();
 }

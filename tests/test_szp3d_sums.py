@@ -1,6 +1,6 @@
-"""The 3-D codec's decoder where its chunks, pieces, parts and ragged ends can
-go wrong, against the oracle bit for bit, and its float reconstruction against
-the double steps on the CPU."""
+"""The 3-D codec's kernels where their units, chunks, pieces, parts and ragged
+ends can go wrong, against the oracle bit for bit, and the decoder's float
+reconstruction against the double steps on the CPU."""
 from __future__ import annotations
 
 import os
@@ -70,6 +70,29 @@ def test_decode_sums(torch, port, bs, kind, dims):
         assert np.array_equal(y.view(np.uint32), want)
     out, size = codec.compress(torch.from_numpy(x).cuda(), eb)
     assert out[: codec.size(size)].cpu().numpy().tobytes() == s
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bs", [2, 4, 8])
+@pytest.mark.parametrize("scale", [2.0 ** 18, 2.0 ** 19, 2.0 ** 23, 2.0 ** 29])
+def test_encode_past_exact_floats(torch, port, bs, scale):
+    """Quantized values on both sides of what the float steps hold, near ties,
+    in some units of a tile and in all, at any 4-byte phase of the volume."""
+    from zccl_gb300.szp3d import Szp3D
+    dims, eb = (19, 21, 150), 2e-4
+    rng = np.random.default_rng(bs)
+    q = rng.normal(0, 40, dims)
+    q[:, :, 40:70] += scale * rng.choice([-1.0, 0.0, 1.0], (19, 21, 30))
+    q[11:] *= 1 + min(scale / 4000, 2.0)  # within int
+    x = ((np.round(q) - 0.5 * (rng.random(dims) < 0.2)) * 2 * eb).astype(np.float32).ravel()
+    s = port.szp3d_compress(x, dims, bs, eb)
+    codec = Szp3D(dims, bs)
+    for at in range(4):
+        buf = torch.zeros(x.size + 8, dtype=torch.float32, device="cuda")
+        buf[at: at + x.size] = torch.from_numpy(x).cuda()
+        out, size = codec.compress(buf[at: at + x.size], eb)
+        codec.check()
+        assert out[: codec.size(size)].cpu().numpy().tobytes() == s
 
 
 @pytest.mark.gpu

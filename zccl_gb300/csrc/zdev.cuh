@@ -655,6 +655,20 @@ __device__ __forceinline__ void cp_async4(uint32_t sdst, const void *gsrc)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sdst), "l"(gsrc) : "memory");
 }
+/* Sixteen bytes (both addresses multiples of 16), or sixteen zeros where they
+ * are not wanted (gsrc may then be anything). */
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t sdst, const void *gsrc, bool want)
+{
+    asm volatile("{\n .reg .pred p;\n .reg .b32 z;\n"
+                 " setp.ne.u32 p, %2, 0;\n mov.u32 z, 0;\n"
+                 " @p cp.async.cg.shared.global [%0], [%1], 16;\n"
+                 " @!p st.shared.v4.b32 [%0], {z, z, z, z};\n}"
+                 ::"r"(sdst), "l"(gsrc), "r"((uint32_t)want)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <uint32_t N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_arrive(uint64_t *bar)
 {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -29,12 +29,10 @@
  *                (ZCCLd_float.c:2855-2857).
  *                For block sides 2, 4 and 8, K3 forms the z and y sums as it
  *                decodes, and the volume is passed over twice in all.
- * Block sides 2, 4 and 8 (row-mapped kernels): a warp takes a run of 32 / bs
- * blocks along z and walks their rows, coalesced, with the neighbours in
- * registers; compress is one pass (K1-K3 together, quantizing as it loads,
- * the run's place in the stream by decoupled look-back; no quantized
- * volume).  Other block sides: a quantized volume, then
- * a warp (up to 512 elements) or a CTA per block.
+ * Block sides 2, 4 and 8: compress is one pass (K1-K3 together, quantizing as
+ * it loads; the tiles' places in the stream come from one CTA's scan of their
+ * sizes), decompress two.  Other block sides: a quantized volume, then a warp
+ * (up to 512 elements) or a CTA per block.
  * Integer sums wrap modulo 2^32 like the reference's int.
  */
 #include <algorithm>
@@ -42,105 +40,6 @@
 #include "zkern.cuh"
 
 namespace {
-
-/* ---------------------------------------------------------------------
- * Decoupled look-back (Merrill & Garland 2016).  status[t] packs a 2-bit
- * flag (1 = aggregate of tile t only, 2 = inclusive prefix through t) over
- * a 62-bit value; values add modulo 2^62.  Tiles are taken in ticket order,
- * so every tile a CTA waits on belongs to a CTA that is already running and
- * never waits on a later tile.
- * ------------------------------------------------------------------- */
-/* Polls of a predecessor's word before the look-back gives up (about a
- * second at the 32 ns back-off; callers may pass a smaller limit). */
-#define LB_SPIN_LIMIT (1u << 22)
-#define LB_FLAG_A (1ull << 62)
-#define LB_FLAG_P (2ull << 62)
-#define LB_VAL (LB_FLAG_A - 1ull)
-
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-/* Any lane of the publishing warp may call it; lane 0 stores: this tile's
- * aggregate, or, for a first tile (no predecessor in its scan), its
- * inclusive value start + agg. */
-__device__ __forceinline__ void lb_publish(uint64_t *status, uint64_t tile, uint64_t agg, bool first,
-                                           uint64_t start)
-{
-    if ((threadIdx.x & 31u) == 0)
-        st_flag(status + tile, first ? (LB_FLAG_P | ((start + agg) & LB_VAL))
-                                        : (LB_FLAG_A | (agg & LB_VAL)));
-}
-
-/* Called by all lanes of one warp after lb_publish: returns the exclusive
- * prefix of the tile (the sum of every tile back to and including the
- * nearest one that published an inclusive value, or `start` for a first
- * tile) and publishes the tile's inclusive value.  Each round inspects 256
- * predecessors (lane l reads tiles pos - l - 32k, k < 8, all loads in flight
- * together): with a persistent grid several hundred tiles are in flight at
- * once, and the nearest inclusive value is typically that far back.  A
- * predecessor that never publishes makes the wait give up after a bounded
- * number of polls: ZERR_TIMEOUT is set, the missing value counts as 0 and
- * the inclusive value is still published, so successors never hang. */
-static __device__ __noinline__ uint64_t lb_resolve(uint64_t *status, uint64_t tile, uint64_t agg,
-                                                   bool first, uint64_t start, uint32_t *err,
-                                                   uint32_t spin_limit = LB_SPIN_LIMIT)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    if (first) return start;
-    uint64_t prefix = 0;
-    int64_t pos = (int64_t)tile - 1;
-    uint32_t spins = 0;
-    for (;;) {
-        uint64_t v[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            int64_t idx = pos - (int64_t)(lane + 32u * k);
-            v[k] = idx >= 0 ? ld_flag(status + idx) : LB_FLAG_P; /* before tile 0: value 0 */
-        }
-        /* nearest inclusive value: smallest distance lane + 32k flagged P */
-        uint32_t kp = 8, fp = 31, pending = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t flag = (uint32_t)(v[k] >> 62);
-            const uint32_t pm = __ballot_sync(0xffffffffu, flag == 2u);
-            const uint32_t xm = __ballot_sync(0xffffffffu, flag == 0u);
-            if (kp == 8) {
-                if (pm) {
-                    kp = k;
-                    fp = (uint32_t)(__ffs(pm) - 1);
-                    pending |= xm & ((1u << fp) - 1u);
-                } else {
-                    pending |= xm;
-                }
-            }
-        }
-        if (pending) {
-            if (++spins < spin_limit) {
-                __nanosleep(32);
-                continue;
-            }
-            /* give up: missing values count as 0 */
-            if (lane == 0) atomicOr(err, ZERR_TIMEOUT);
-        }
-        uint64_t c = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const bool ready = (v[k] >> 62) != 0;
-            if ((uint32_t)k < kp || ((uint32_t)k == kp && lane <= fp))
-                c += ready ? (v[k] & LB_VAL) : 0ull;
-        }
-        prefix += warp_sum_u64(c);
-        if (kp < 8) break;
-        pos -= 256;
-        spins = 0;
-    }
-    if (lane == 0) st_flag(status + tile, LB_FLAG_P | ((prefix + agg) & LB_VAL));
-    return prefix & LB_VAL;
-}
 
 constexpr uint32_t SZ_THREADS = 256;
 constexpr uint32_t SZ_CHUNK = 2048; /* sizes per CTA in the scan */
@@ -622,17 +521,14 @@ __global__ void __launch_bounds__(SZ_THREADS) k_sz3_unpack(const uint8_t *in, ui
     }
 }
 
-/* ---- block sides 2, 4 and 8: row-mapped kernels -------------------------
- * A warp takes a unit of U = 32 / BS consecutive blocks along z with the
- * same block row and plane: lane l owns z = z0 + l, in block l / BS.  It
- * walks the unit's rows plane by plane, row by row (the order of the
- * elements in a block), loads each row of x once, coalesced, quantizes it
- * and forms the mixed difference from neighbours it holds: the z neighbour
- * by a shuffle (lane 0 loads its own), the previous row's z-difference and
- * the previous plane's 2-D differences in registers.  The row and plane
- * before the unit come in once more for that (zeros outside the volume).
- * So compress reads x twice (rates, then packing) and keeps no quantized
- * volume; decompress writes whole rows. */
+/* ---- block sides 2, 4 and 8: compress ------------------------------------
+ * A unit is U = 32 / BS consecutive blocks along z with the same block row
+ * and plane: lane l owns z = z0 + l, in block l / BS.  A warp takes the unit's
+ * rows plane by plane, quantizes them and forms the mixed difference from
+ * neighbours it holds: the z neighbour by a shuffle (lane r takes row r's
+ * element before z0), the previous row's z-difference and the previous plane's
+ * 2-D differences in registers.  The row and plane before the
+ * unit come in once more for that (zeros outside the volume). */
 struct Sz3Unit {
     uint64_t bi, bj, bk0, i0, j0, z0;
     uint32_t sx, sy;
@@ -642,23 +538,6 @@ template <uint32_t BS>
 __host__ __device__ inline uint64_t sz3_units(const Sz3Dims &g)
 {
     return g.nb1 * g.nb2 * ((g.nb3 + 32 / BS - 1) / (32 / BS));
-}
-
-template <uint32_t BS>
-__device__ __forceinline__ Sz3Unit sz3_unit(const Sz3Dims &g, uint64_t u)
-{
-    constexpr uint32_t U = 32 / BS;
-    const uint64_t nzc = (g.nb3 + U - 1) / U;
-    Sz3Unit k;
-    k.bj = (u / nzc) % g.nb2;
-    k.bi = u / (nzc * g.nb2);
-    k.bk0 = (u % nzc) * U;
-    k.i0 = k.bi * BS;
-    k.j0 = k.bj * BS;
-    k.z0 = k.bk0 * BS;
-    k.sx = (uint32_t)min((uint64_t)BS, g.d1 - k.i0);
-    k.sy = (uint32_t)min((uint64_t)BS, g.d2 - k.j0);
-    return k;
 }
 
 /* Extent along z of the unit's block c (0 past the volume). */
@@ -722,82 +601,423 @@ __device__ __forceinline__ void sz3_walk(const float *__restrict__ x, const Sz3D
     }
 }
 
-/* compress, one pass (quantization included): warps take units in ticket
- * order; a unit's differences go to shared memory in element order while
- * their largest magnitudes give the blocks' rates and payload sizes; the
- * unit's place in the stream comes from a decoupled look-back over the
- * units before it (the unit's bytes are its blocks', consecutive), then
- * its blocks are packed (all at once, BS lanes each, for BS up to 4; else
- * one after another by the whole warp).  The last unit records the
- * stream's size. */
+/* The unit's differences as integers, whatever their size, in the order of
+ * the walk below. */
 template <uint32_t BS>
-__global__ void __launch_bounds__(SZ_THREADS, BS <= 4 ? 4 : 3) k_sz3_compress_rows(const float *__restrict__ x, Sz3Dims g, Sz3Split inv,
-                                                                  uint8_t *out, uint64_t cap, uint64_t *status,
-                                                                  uint32_t *ticket, uint64_t *total, uint32_t *err)
+__device__ __noinline__ void sz3_walk_any(const float *x, const Sz3Dims &g, const Sz3Split &inv, const Sz3Unit &k, uint32_t *d,
+                                          uint32_t &bad)
 {
-    constexpr uint32_t U = 32 / BS, NB = BS * BS * BS;
-    extern __shared__ uint32_t e_all[]; /* U blocks per warp */
-    const uint32_t lane = threadIdx.x & 31u, dz = lane % BS;
-    uint32_t *e = e_all + (threadIdx.x >> 5) * (U * NB);
-    const uint64_t units = sz3_units<BS>(g);
-    uint32_t bad = 0, full = 0;
-    for (;;) {
-        uint32_t u = 0;
-        if (lane == 0) u = atomicAdd(ticket, 1u);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if (u >= units) break; /* uniform */
-        const Sz3Unit k = sz3_unit<BS>(g, u);
-        const uint32_t sz = sz3_unit_sz<BS>(g, k, lane / BS);
-        const bool zin = k.z0 + lane < g.d3;
-        uint32_t *eb = e + (lane / BS) * NB;
-        uint32_t m = 0;
-        __syncwarp(); /* the previous unit is packed */
-        sz3_walk<BS>(x, g, inv, k, bad, [&](uint32_t di, uint32_t dj, uint32_t v) {
-            if (zin) {
-                eb[(di * k.sy + dj) * sz + dz] = v;
-                m = max(m, mag(v));
-            }
-        });
+    sz3_walk<BS>(x, g, inv, k, bad, [&](uint32_t di, uint32_t dj, uint32_t v) { d[di * BS + dj] = v; });
+}
+
+constexpr float SZ_MAGIC = 12582912.0f;         /* 1.5 * 2^23: a float m + this holds the integer m in its low bits, */
+constexpr uint32_t SZ_ZERO = 0x4B400000u;       /* as this + m */
+
+/* (int)floor((double)x * inv + 0.5) on the float pipe.  n is the integer next
+ * to x * hi, d = x * (hi + lo) - n: two roundings of 2^-25 at most, lo's own
+ * error and the reference's two double roundings are together below 2^-23.9
+ * for |n| < 2^19, so n is the reference's result if |d| < 1/2 - 2^-22; else
+ * `sure` becomes false (one value in 2^21).  sq collects n * n, so that one
+ * test finds values out of range or not finite. */
+__device__ __forceinline__ float sz3_quantize_f(float x, const Sz3Split &inv, bool &sure, float &sq)
+{
+    const float n = __fsub_rn(__fmaf_rn(x, inv.hi, SZ_MAGIC), SZ_MAGIC);
+    const float d = __fmaf_rn(x, inv.lo, __fmaf_rn(x, inv.hi, -n));
+    sure = sure && fabsf(d) < 0.499999761581420898f;
+    sq = __fmaf_rn(n, n, sq);
+    return n;
+}
+
+/* A warp's rows on their way, plane by plane through its units, into PD
+ * buffers in turn (a unit's BS + 1 planes are whole rounds of them): row r of a
+ * plane is y = j0 - 1 + r, from the element before z0 on, in the 16-byte chunks
+ * that hold it (160 bytes at any phase).  A lane copies NI chunks a plane;
+ * rows outside the volume are zeros. */
+constexpr uint32_t SZ_ROW = 160, SZ_CH = SZ_ROW / 16;
+template <uint32_t BS>
+struct Sz3Feed {
+    static constexpr uint32_t N = SZ_CH * (BS + 1), NI = (N + 31) / 32, PLANE = SZ_ROW * (BS + 1), PD = BS == 4 ? 5 : 3;
+    uint64_t at[NI]; /* this lane's chunks of the next plane: the element at their start, at any phase */
+    int32_t lim[NI], top[NI]; /* a chunk is wanted where its row's phase is in [lim, top] */
+    uint32_t planes; /* bit pl: plane pl is in the volume */
+    __device__ __forceinline__ void set(const float *x, const Sz3Dims &g, const Sz3Unit &k)
+    {
+        const uint64_t a = reinterpret_cast<uintptr_t>(x) + 4u * ((k.i0 - 1) * (g.d2 * g.d3) + (k.j0 - 1) * g.d3 + k.z0 - 1);
+        const int32_t nz = (int32_t)min((uint64_t)32, g.d3 - k.z0);
+        planes = k.sx ? ((2u << k.sx) - 1u) & (k.i0 ? ~0u : ~1u) : 0u;
 #pragma unroll
-        for (uint32_t o = 1; o < BS; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        /* lane c < U: block c's rate and size */
-        const uint32_t mc = __shfl_sync(0xffffffffu, m, (lane % U) * BS);
-        const uint32_t szc = lane < U ? sz3_unit_sz<BS>(g, k, lane) : 0u;
-        const uint32_t rate = szc ? 32u - __clz(mc) : 0u, size = szc ? sz3_payload(rate, k.sx * k.sy * szc) : 0u;
-        const uint32_t inc = warp_incl_scan(size), agg = __shfl_sync(0xffffffffu, inc, 31);
-        lb_publish(status, u, agg, u == 0, 0);
-        const uint64_t prefix = lb_resolve(status, u, agg, u == 0, 0, err);
-        const uint64_t base = g.nblocks + prefix + (inc - size);
-        if (szc) out[(k.bi * g.nb2 + k.bj) * g.nb3 + k.bk0 + lane] = (uint8_t)rate;
-        if (u == units - 1 && lane == 0) *total = g.nblocks + prefix + agg;
-        __syncwarp();
-        if constexpr (BS <= 4) { /* all blocks of the unit at once, BS lanes each */
-            const uint32_t c = lane / BS;
-            const uint32_t rc = __shfl_sync(0xffffffffu, rate, c);
-            const uint64_t bc = __shfl_sync(0xffffffffu, base, c);
-            const uint32_t n = k.sx * k.sy * sz;
-            if (rc && n) {
-                if (bc + sz3_payload(rc, n) > cap)
-                    full = 1;
-                else
-                    sz3_pack_block<BS>(e + c * NB, n, rc, out + bc, dz);
-            }
-        } else { /* blocks of 512 elements: one after another, the whole warp on each */
-            for (uint32_t c = 0; c < U; c++) {
-                const uint32_t rc = __shfl_sync(0xffffffffu, rate, c);
-                const uint64_t bc = __shfl_sync(0xffffffffu, base, c);
-                const uint32_t n = k.sx * k.sy * sz3_unit_sz<BS>(g, k, c);
-                if (!rc || !n) continue; /* uniform */
-                if (bc + sz3_payload(rc, n) > cap) {
-                    full = 1;
-                    continue;
-                }
-                sz3_pack_block<32>(e + c * NB, n, rc, out + bc, lane);
-            }
+        for (uint32_t s = 0; s < NI; s++) {
+            const uint32_t idx = (threadIdx.x & 31u) + 32u * s, r = idx / SZ_CH, ch = idx % SZ_CH;
+            at[s] = a + 4u * g.d3 * r + 16u * ch; /* wraps only where not read */
+            lim[s] = r >= (k.j0 ? 0u : 1u) && r <= k.sy ? (int32_t)(4u * ch) - nz : 4;
+            top[s] = k.z0 == 0 && ch == 0 ? 2 : 3; /* nothing before the row's first element */
         }
     }
+    /* the next plane, number pl of its unit; one group of copies, in any case */
+    __device__ __forceinline__ void send(uint32_t buf, uint32_t pl, uint64_t stride)
+    {
+        const bool in = (planes >> pl) & 1u;
+#pragma unroll
+        for (uint32_t s = 0; s < NI; s++) {
+            const uint32_t idx = (threadIdx.x & 31u) + 32u * s;
+            if (32u * (s + 1) <= N || idx < N) {
+                const int32_t ph = (int32_t)(((uint32_t)at[s] >> 2) & 3u);
+                cp_async16_or_zero(buf + idx * 16u, reinterpret_cast<const void *>(at[s] & ~(uint64_t)15u),
+                                   in && ph >= lim[s] && ph <= top[s]);
+            }
+            at[s] += stride;
+        }
+        cp_async_commit();
+    }
+};
+
+/* The unit's differences, SZ_ZERO + d at w[di * BS + dj] (rows and planes
+ * outside the volume: any), and this lane's largest magnitude; the next
+ * unit's rows are sent for meanwhile, into the buffers that this one leaves.
+ * In floats, which hold every step exactly while the quantized values are
+ * below 2^19 (the differences below 2^22); false if they are not, or where a
+ * value needs the double steps (one unit in thousands; they hold up the tiles
+ * after them): any w then. */
+template <uint32_t BS>
+__device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
+                                           const Sz3Unit &k, const Sz3Unit &next, Sz3Feed<BS> &feed, uint32_t (&w)[BS * BS],
+                                           uint32_t &mx)
+{
+    using F = Sz3Feed<BS>;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t d3 = (uint32_t)g.d3, dpl = (uint32_t)(g.d2 * g.d3); /* phases: low bits are enough */
+    const uint32_t a0 = ((uint32_t)reinterpret_cast<uintptr_t>(x) >> 2) + ((uint32_t)k.i0 - 1u) * dpl + ((uint32_t)k.j0 - 1u) * d3 +
+                        (uint32_t)k.z0 - 1u;
+    const bool even = (d3 & 3u) == 0; /* every row at the same phase */
+    const bool lin = k.z0 && lane <= BS;
+    const uint64_t stride = 4u * g.d2 * g.d3;
+    float dp[BS], sq = 0.0f, top = 0.0f;
+    bool sure = true;
+#pragma unroll
+    for (uint32_t pl = 0; pl <= BS; pl++) {
+        cp_async_wait<F::PD - 1>(); /* all but the PD - 1 planes after this one */
+        __syncwarp();
+        const uint32_t buf = sbuf + pl % F::PD * F::PLANE, ap = a0 + pl * dpl;
+        float cv[BS + 1], cl;
+        if (even) {
+            const uint32_t at = buf + 4u * ((a0 & 3u) + 1u + lane);
+#pragma unroll
+            for (uint32_t r = 0; r <= BS; r++) cv[r] = ld_shared_f32(at + r * SZ_ROW);
+        } else {
+#pragma unroll
+            for (uint32_t r = 0; r <= BS; r++) cv[r] = ld_shared_f32(buf + r * SZ_ROW + 4u * (((ap + r * d3) & 3u) + 1u + lane));
+        }
+        cl = lin ? ld_shared_f32(buf + lane * SZ_ROW + 4u * ((ap + lane * d3) & 3u)) : 0.0f; /* lane r: before row r */
+        __syncwarp();
+        if (pl + F::PD == BS + 1) feed.set(x, g, next);
+        feed.send(buf, (pl + F::PD) % (BS + 1), stride);
+        float q[BS + 1], ql = sz3_quantize_f(cl, inv, sure, sq);
+#pragma unroll
+        for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_f(cv[r], inv, sure, sq);
+        float rp = 0.0f;
+#pragma unroll
+        for (uint32_t r = 0; r <= BS; r++) {
+            const float up = __shfl_up_sync(0xffffffffu, q[r], 1), l0 = __shfl_sync(0xffffffffu, ql, r);
+            const float rc = q[r] - (lane ? up : l0); /* q(z) - q(z - 1) */
+            if (r) {
+                const float d = rc - rp;
+                if (pl) {
+                    const float e = d - dp[r - 1];
+                    w[(pl - 1) * BS + r - 1] = __float_as_uint(e + SZ_MAGIC);
+                    top = fmaxf(top, fabsf(e));
+                }
+                dp[r - 1] = d;
+            }
+            rp = rc;
+        }
+    }
+    mx = (uint32_t)top;
+    return sure && sq < 274877906944.0f; /* 2^38; NaN is not */
+}
+
+/* Octet g of a block of n elements at byte o of the zeroed buffer: w[k] =
+ * SZ_ZERO + difference (0 past the block's end). */
+__device__ __forceinline__ void sz3_put_octet(uint32_t sbase, uint32_t o, uint32_t rate, uint32_t n, uint32_t g,
+                                              const uint32_t (&w)[8])
+{
+    if (!rate) return;
+    const uint32_t B = rate >> 3, r = rate & 7u, h = o + ((n + 7u) >> 3), at = o + g;
+    uint32_t m[8], s8 = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint32_t v = w[k] - SZ_ZERO;
+        s8 = __funnelshift_l(v, s8, 1);
+        m[k] = (uint32_t)abs((int32_t)v);
+    }
+    if (s8) sh_or(sbase + (at & ~3u), s8 << (8u * (at & 3u)));
+    if (B == 1) {
+        const uint32_t lo = __byte_perm(__byte_perm(m[0] >> r, m[1] >> r, 0x0040), __byte_perm(m[2] >> r, m[3] >> r, 0x0040), 0x5410);
+        const uint32_t hi = __byte_perm(__byte_perm(m[4] >> r, m[5] >> r, 0x0040), __byte_perm(m[6] >> r, m[7] >> r, 0x0040), 0x5410);
+        or_bytes(sbase, h + 8u * g, (uint64_t)hi << 32 | lo);
+    } else if (B > 1) {
+        const uint32_t keep = B >= 4 ? 0xFFFFFFFFu : (1u << (8u * B)) - 1u;
+#pragma unroll
+        for (int k = 0; k < 8; k++) or_bytes(sbase, h + (8u * g + (uint32_t)k) * B, (m[k] >> r) & keep);
+    }
+    if (r) { /* r bytes, most significant bit first: two halves of 4 r bits */
+        const uint32_t mask = (1u << r) - 1u;
+        uint32_t a = m[0] & mask, b = m[4] & mask;
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+            a = a << r | (m[k] & mask);
+            b = b << r | (m[4 + k] & mask);
+        }
+        /* the 8 r bits at the top of 64, bytes first to last upward */
+        const uint32_t s = 32u - 4u * r, at2 = a << s, bt = b << s;
+        const uint32_t hi = at2 | (bt >> (4u * r)), lo = bt << s;
+        or_bytes(sbase, h + n * B + g * r, (uint64_t)(s ? bswap32(lo) : 0u) << 32 | bswap32(hi));
+    }
+}
+
+/* One pass.  Tiles of NW * UPW units in stream order, handed out by tickets:
+ * each of NW compute warps takes UPW units, keeps their differences in
+ * registers while the blocks' rates, sizes and places in the tile are found
+ * (the tile's one barrier), and packs them into a ring in shared memory, an
+ * octet of 8 consecutive elements a lane: 256 elements at a time change from
+ * rows to octets through a small buffer.  The ring, its placer warps (which
+ * write the tiles out) and the scan of the tiles' sizes by one CTA are the
+ * 1-D compressor's.
+ * Bound by issue, 80 instructions per 32 elements at side 4 (252 with exact
+ * integer quantization, byte-wise packing and a look-back per warp).  512^3:
+ * side 8 485 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
+ * side 4 take 440, three CTAs an SM 470 (spills), 10 or 12 compute warps the
+ * same 408. */
+template <uint32_t BS>
+struct Sz3Cm {
+    static constexpr uint32_t NW = 8;                                        /* compute warps */
+    static constexpr uint32_t U = 32 / BS, NB = BS * BS * BS, UPW = BS == 2 ? 2 : 1;
+    static constexpr uint32_t BPW = U * UPW;                                 /* blocks per warp, at most 32 */
+    static constexpr uint32_t ROWS = BS * BS < 8 ? BS * BS : 8;              /* rows of a unit changed at a time */
+    static constexpr uint32_t PER = ROWS * BS, BST = PER + (BS == 2 ? 4 : BS); /* a block's elements in them, its stride */
+    static constexpr uint32_t WORST = NW * BPW * ((NB + 7) / 8 + 4 * NB);    /* a tile's bytes */
+    static constexpr uint32_t THREADS = 32 * (NW + 2);                       /* and the placer and the one that claims */
+    static constexpr uint32_t FEED = Sz3Feed<BS>::PLANE * Sz3Feed<BS>::PD;   /* a warp's rows */
+    static constexpr uint32_t OWN = FEED + 4 * U * BST;                      /* a warp's shared bytes */
+};
+constexpr uint32_t SZ_CM_PLACERS = 1;
+
+struct Sz3CmShared {
+    uint64_t full[2], empty[2];
+    uint64_t ticket[2];
+    uint4 place[2][16]; /* compute warps' first units: z chunk, block row, block plane */
+    uint32_t ws[2][34];
+    ZRing ring;
+    uint32_t scanner;
+};
+constexpr uint32_t SZ_CM_HEAD = (sizeof(Sz3CmShared) + 15u) / 16u * 16u;
+
+template <uint32_t BS>
+__global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(const float *__restrict__ x, Sz3Dims g, Sz3Split inv,
+                                                                        uint8_t *out, uint64_t cap, uint64_t *status,
+                                                                        uint32_t *ticket, uint64_t *total_out, uint32_t R,
+                                                                        uint32_t *err)
+{
+    using C = Sz3Cm<BS>;
+    constexpr uint32_t U = C::U, UPW = C::UPW, NW = C::NW;
+    extern __shared__ __align__(16) uint8_t sm[];
+    Sz3CmShared *sh = reinterpret_cast<Sz3CmShared *>(sm);
+    uint8_t *outs = sm + SZ_CM_HEAD + NW * C::OWN;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t nzc = (uint32_t)((g.nb3 + U - 1) / U), nb2 = (uint32_t)g.nb2;
+    const uint32_t units = (uint32_t)sz3_units<BS>(g), ntiles = (units + NW * UPW - 1u) / (NW * UPW);
+    uint32_t bad = 0;
+    if (tid == 0) {
+        for (uint32_t i = 0; i < 2; i++) {
+            mbar_init(&sh->full[i], 1);
+            mbar_init(&sh->empty[i], NW);
+        }
+        ring_init(&sh->ring, NW);
+        sh->scanner = gridDim.x > 1 && atomicAdd(ticket + 1, 1u) == 0;
+    }
+#pragma unroll 1
+    for (uint32_t i = tid; i < (R + 48u) / 16u; i += C::THREADS) reinterpret_cast<uint4 *>(outs)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    if (sh->scanner) {
+        if (warp == 0) scan_tiles(status, ntiles, ticket, err, SCAN_SPIN_LIMIT);
+        return;
+    }
+    if (warp >= NW && warp < NW + SZ_CM_PLACERS) {
+        placer_loop<SZ_CM_PLACERS>(&sh->ring, outs, status, ntiles, warp - NW, err, bad, SCAN_SPIN_LIMIT);
+        if (bad) atomicOr(err, bad);
+        return;
+    }
+    if (warp == NW + SZ_CM_PLACERS) { /* claims the tiles */
+        for (uint32_t it = 0;; it++) {
+            uint32_t t = lane ? 0u : atomicAdd(ticket, 1u);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            const uint32_t s = it & 1u, u = t * (NW * UPW) + lane * UPW, strip = u / nzc;
+            if (it >= 2) mbar_wait(&sh->empty[s], (it / 2u - 1u) & 1u, err);
+            if (lane < NW)
+                sh->place[s][lane] = make_uint4(u - strip * nzc, strip % nb2, t < ntiles ? strip / nb2 : (uint32_t)g.nb1, 0u);
+            __syncwarp();
+            if (lane == 0) {
+                if (t < ntiles) {
+                    ZSlot &S = ring_slot(&sh->ring, it, err);
+                    S.ticket = t;
+                    S.out = out;
+                    S.cap = cap;
+                    S.hdr = nullptr;
+                    S.size = t == ntiles - 1u ? total_out : nullptr;
+                    S.T8 = g.nblocks; /* the rate table */
+                    S.ngrp = 0;
+                }
+                sh->ticket[s] = t < ntiles ? t : ZP_NONE;
+                mbar_arrive(&sh->full[s]);
+            }
+            if (t >= ntiles) return;
+        }
+    }
+
+    uint8_t *own = sm + SZ_CM_HEAD + warp * C::OWN;
+    uint32_t *st = reinterpret_cast<uint32_t *>(own + C::FEED);
+    const uint32_t sbuf = smem_u32(own);
+    const uint32_t c = lane / BS, dz = lane % BS; /* this lane's block and place in a unit */
+    uint32_t H = 0, hp = 0;
+    /* tile number it's ticket (once for each it) and this warp's first unit of it */
+    uint4 at;
+    auto claim = [&](uint32_t it) {
+        mbar_wait(&sh->full[it & 1u], (it / 2u) & 1u, err);
+        const uint64_t t = sh->ticket[it & 1u];
+        at = sh->place[it & 1u][warp];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->empty[it & 1u]);
+        return t;
+    };
+    auto unit = [&]() { /* the unit at `at` (no rows or planes where there is none), which moves on */
+        Sz3Unit K;
+        K.bk0 = (uint64_t)at.x * U;
+        K.bj = at.y;
+        K.bi = at.z;
+        K.i0 = K.bi * BS;
+        K.j0 = K.bj * BS;
+        K.z0 = K.bk0 * BS;
+        K.sx = at.z < (uint32_t)g.nb1 ? (uint32_t)min((uint64_t)BS, g.d1 - K.i0) : 0u;
+        K.sy = K.sx ? (uint32_t)min((uint64_t)BS, g.d2 - K.j0) : 0u;
+        if (++at.x == nzc) {
+            at.x = 0;
+            if (++at.y == nb2) {
+                at.y = 0;
+                at.z++;
+            }
+        }
+        return K;
+    };
+    uint64_t t = claim(0);
+    Sz3Unit nextu = unit();
+    Sz3Feed<BS> feed;
+    feed.set(x, g, nextu);
+#pragma unroll 1
+    for (uint32_t pl = 0; pl < Sz3Feed<BS>::PD; pl++) feed.send(sbuf + pl * Sz3Feed<BS>::PLANE, pl, 4u * g.d2 * g.d3);
+#pragma unroll 1
+    for (uint32_t it = 0; it <= ntiles; it++) {
+        if (t == ZP_NONE) {
+            if (tid == 0) ring_end(&sh->ring, it, SZ_CM_PLACERS, err);
+            break;
+        }
+        uint64_t tn = ZP_NONE;
+        uint32_t w[UPW][BS * BS];
+        Sz3Unit k[UPW];
+        uint32_t rate = 0, n = 0; /* lane b: block b of the warp's */
+#pragma unroll
+        for (uint32_t i = 0; i < UPW; i++) {
+            Sz3Unit &K = k[i];
+            K = nextu;
+            if (i + 1 == UPW) tn = claim(it + 1);
+            nextu = unit();
+            uint32_t mx = 0;
+            if (__any_sync(0xffffffffu, !sz3_walk_f<BS>(sbuf, x, g, inv, K, nextu, feed, w[i], mx)) || !inv.mid) {
+                uint32_t d[BS * BS];
+                for (uint32_t e = 0; e < BS * BS; e++) d[e] = 0;
+                if (K.sx) sz3_walk_any<BS>(x, g, inv, K, d, bad);
+                mx = 0;
+#pragma unroll
+                for (uint32_t e = 0; e < BS * BS; e++) {
+                    w[i][e] = SZ_ZERO + d[e];
+                    mx = max(mx, mag(d[e]));
+                }
+            }
+            if (K.sx < BS || K.sy < BS) { /* rows outside the volume count for nothing */
+                mx = 0;
+#pragma unroll
+                for (uint32_t e = 0; e < BS * BS; e++)
+                    if (e / BS < K.sx && e % BS < K.sy) mx = max(mx, mag(w[i][e] - SZ_ZERO));
+            }
+            if (K.z0 + lane >= g.d3) mx = 0;
+#pragma unroll
+            for (uint32_t o = 1; o < BS; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const uint32_t mc = __shfl_sync(0xffffffffu, mx, (lane % U) * BS);
+            if (lane / U == i && K.sx) {
+                n = K.sx * K.sy * sz3_unit_sz<BS>(g, K, lane % U);
+                rate = n ? 32u - __clz(mc) : 0u;
+                if (n) out[(K.bi * g.nb2 + K.bj) * g.nb3 + K.bk0 + lane % U] = (uint8_t)rate;
+            }
+        }
+        uint32_t total;
+        const uint32_t off = grp_excl_scan1(sz3_payload(rate, n), sh->ws[it & 1u], &total, 32u * NW, 1);
+        if (tid == 0) {
+            scan_publish(status, t, total, t == 0);
+            ring_sized(&sh->ring, it, total);
+        }
+        uint32_t mend;
+        const uint32_t pos = ring_space(&sh->ring, zg_ring_need(total), R, H, hp, mend, err);
+        const uint32_t pk = smem_u32(outs + pos);
+#pragma unroll
+        for (uint32_t i = 0; i < UPW; i++) {
+            const Sz3Unit &K = k[i];
+            if (K.sx == BS && K.sy == BS && K.z0 + 32 <= g.d3) { /* whole blocks: rows are octets, or halves or quarters */
+#pragma unroll
+                for (uint32_t e0 = 0; e0 < BS * BS; e0 += C::ROWS) {
+                    __syncwarp();
+#pragma unroll
+                    for (uint32_t e = 0; e < C::ROWS; e++) st[c * C::BST + e * BS + dz] = w[i][e0 + e];
+                    __syncwarp();
+                    constexpr uint32_t OCT = C::PER / 8; /* octets of a block in this lot */
+                    const uint32_t b = lane / OCT, go = lane % OCT;
+                    const uint32_t at = __shfl_sync(0xffffffffu, off, (i * U + b) & 31u), rb = __shfl_sync(0xffffffffu, rate, (i * U + b) & 31u);
+                    if (b < U) {
+                        const uint4 *p = reinterpret_cast<const uint4 *>(st + b * C::BST + 8u * go);
+                        const uint4 lo = p[0], hi = p[1];
+                        const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                        sz3_put_octet(pk, at, rb, C::NB, e0 * BS / 8u + go, v);
+                    }
+                }
+            } else if (K.sx) { /* at the volume's end: 256 elements at a time in their blocks' own order */
+                constexpr uint32_t NB = C::NB, LB = NB > 256 ? 256 : NB, LOTS = U * NB > 256 ? U * NB / 256 : 1; /* a lot's elements of a block */
+                const uint32_t sz = K.z0 + lane < g.d3 ? sz3_unit_sz<BS>(g, K, c) : 0u;
+#pragma unroll 1
+                for (uint32_t lot = 0; lot < LOTS; lot++) {
+                    const uint32_t b0 = lot * 256u / NB, e0 = lot * 256u % NB; /* its first block, and first element of it */
+                    __syncwarp();
+                    if (sz && c - b0 < 256u / LB)
+#pragma unroll
+                        for (uint32_t e = 0; e < BS * BS; e++) {
+                            const uint32_t di = e / BS, dj = e % BS, at = (di * K.sy + dj) * sz + dz - e0;
+                            if (di < K.sx && dj < K.sy && at < LB) st[(c - b0) * LB + at] = w[i][e];
+                        }
+                    __syncwarp();
+                    const uint32_t b = b0 + lane / (LB / 8u), go = lane % (LB / 8u), ln = (i * U + b) & 31u;
+                    const uint32_t at = __shfl_sync(0xffffffffu, off, ln), rb = __shfl_sync(0xffffffffu, rate, ln), nb = __shfl_sync(0xffffffffu, n, ln);
+                    if (b < U && e0 + 8u * go < nb) {
+                        uint32_t v[8];
+#pragma unroll
+                        for (uint32_t e = 0; e < 8; e++) v[e] = e0 + 8u * go + e < nb ? st[(b - b0) * LB + 8u * go + e] : SZ_ZERO;
+                        sz3_put_octet(pk, at, rb, nb, e0 / 8u + go, v);
+                    }
+                }
+            }
+        }
+        if (tid == 0) ring_where(&sh->ring, it, pos, mend);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->ring.packed[it % ZR_SLOTS]);
+        t = tn;
+    }
+    cp_async_wait<0>();
     if (bad) atomicOr(err, ZERR_RANGE);
-    if (full) atomicOr(err, ZERR_CAPACITY);
 }
 
 /* ---- block sides 2, 4 and 8: decompress ---------------------------------
@@ -1493,32 +1713,26 @@ cudaError_t sz3_scan(const Sz3Dims &g, const Sz3Ws &w, uint64_t count, cudaStrea
 /* Block sides with the row-mapped kernels. */
 bool sz3_rows(uint32_t bs) { return bs == 2 || bs == 4 || bs == 8; }
 
-/* One pass; the units' look-back flags use the offsets array (8 bytes a
- * block, at least 8 a unit) and the ticket the third of the four scratch
- * words before it (the first two are error words the status check reads),
- * both zeroed first. */
+/* One pass; the tiles' sizes and places use the offsets array (8 bytes a
+ * block, at least 8 a tile), and the ticket and the scanner's word the last
+ * two of the four scratch words before it (the first two are error words the
+ * status check reads), all zeroed first. */
 template <uint32_t BS>
 cudaError_t sz3_compress_rows(uint8_t *out, uint64_t cap, const float *x, const Sz3Dims &g, const Sz3Ws &w,
                               const Sz3Split &inv, cudaStream_t st)
 {
+    using C = Sz3Cm<BS>;
     const uint64_t units = sz3_units<BS>(g);
-    if (units >> 32) return cudaErrorInvalidValue; /* tickets are 32-bit */
-    uint64_t *status = w.offs;
-    cudaError_t e = cudaMemsetAsync(status, 0, 8 * units, st);
+    if ((units + 16) >> 32) return cudaErrorInvalidValue; /* units are counted in 32 bits */
+    const uint64_t ntiles = (units + C::NW * C::UPW - 1) / (C::NW * C::UPW);
+    cudaError_t e = cudaMemsetAsync(w.offs, 0, 8 * ntiles, st);
     if (e != cudaSuccess) return e;
-    const size_t smem = 4ull * 32 * BS * BS * (SZ_THREADS / 32);
+    const uint32_t fixed = SZ_CM_HEAD + C::NW * C::OWN + 48u, R = ring_bytes(2, fixed, zg_ring_need(C::WORST));
+    const size_t smem = fixed + R;
     const void *fn = (const void *)k_sz3_compress_rows<BS>;
-    if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                                cudaSuccess)
-        return e;
-    int dev = 0, nsm = 0, per = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SZ_THREADS, smem)) != cudaSuccess)
-        return e;
-    const uint64_t want = (units + SZ_THREADS / 32 - 1) / (SZ_THREADS / 32), most = (uint64_t)nsm * (per > 0 ? per : 1);
-    const unsigned grid = (unsigned)(want < most ? want : most);
-    k_sz3_compress_rows<BS><<<grid, SZ_THREADS, smem, st>>>(x, g, inv, out, cap, status, w.err + 2, w.total, w.err);
+    if ((e = set_max_smem(fn, smem)) != cudaSuccess) return e;
+    const unsigned grid = scanned_grid(fn, C::THREADS, smem, ntiles, 0);
+    k_sz3_compress_rows<BS><<<grid, C::THREADS, smem, st>>>(x, g, inv, out, cap, w.offs, w.err + 2, w.total, R, w.err);
     return cudaGetLastError();
 }
 

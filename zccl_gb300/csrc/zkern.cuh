@@ -196,7 +196,8 @@ struct ZSlot {
     uint64_t *grp_off;  /* index: the tile's first group's offset */
     uint8_t *hdr;       /* a segment's first tile: its chunk offset in the header, else null */
     uint64_t *size;     /* the stream's last tile: where its size goes, else null */
-    uint32_t T8, ngrp;  /* bytes of the header; the tile's groups */
+    uint64_t T8;        /* bytes before the first tile's: the header */
+    uint32_t ngrp;      /* the tile's groups */
     uint32_t total, pos, mend;
     uint16_t goff[ZG_SUB]; /* where each of its groups starts in it (a tile is below 64 KB) */
 };

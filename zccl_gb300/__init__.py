@@ -456,8 +456,8 @@ def check_all(objs) -> None:
     objs = list(objs)
     if not objs:
         return
-    words = torch.stack([o._status_words() for o in objs]).cpu()
-    bad = [o for o, w in zip(objs, words) if bool(w.any())]
+    words = torch.stack([o._status_words() for o in objs]).cpu().numpy()
+    bad = [o for o, w in zip(objs, words.any(axis=1)) if w]
     if bad:
         for o in objs:
             if o is not bad[0]:

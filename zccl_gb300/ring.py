@@ -166,9 +166,11 @@ class RingAllreduce:
         return b
 
     def _plan(self, key, kind, jobs):
+        """The batch planned under key; jobs() lists its jobs when it is not
+        there yet (8 ranks' P x P chunk views alone take 0.2 ms to make)."""
         b = self._plans.get(key)
         if b is None:
-            b = Batch(kind, jobs, self.L, device=self.device)
+            b = Batch(kind, jobs(), self.L, device=self.device)
             self._plans[key] = b
         return b
 
@@ -184,7 +186,7 @@ class RingAllreduce:
             return ys
         y = self._buffers(tag)["y"]
         self._plan((tag, "gather", eb), BATCH_DECOMPRESS,
-                   [(reduced[c], eb, self.T, self._chunk(y, c), False) for c in range(P)]).run()
+                   lambda: [(reduced[c], eb, self.T, self._chunk(y, c), False) for c in range(P)]).run()
         self._check()
         return y
 
@@ -198,13 +200,11 @@ class RingAllreduce:
             for k in [k for k in self._plans if k[:2] == ("ho", "compress")]:
                 del self._plans[k]
         self._plan(key, BATCH_COMPRESS,
-                   [(self._chunk(xs[r], c), eb, self.T, S[r][c]) for r in range(P) for c in range(P)]).run()
+                   lambda: [(self._chunk(xs[r], c), eb, self.T, S[r][c]) for r in range(P) for c in range(P)]).run()
         for i in range(P - 1):
-            jobs = []
-            for r in range(P):
-                src, c = (r - 1) % P, (r - 2 - i) % P
-                jobs.append(([S[src][c], S[r][c]], self.T, spare[c]))
-            self._plan(("ho", "step", i), BATCH_HOMADD, jobs).run()
+            pairs = [((r - 1) % P, r, (r - 2 - i) % P) for r in range(P)]  # sender, rank, chunk
+            self._plan(("ho", "step", i), BATCH_HOMADD,
+                       lambda: [([S[src][c], S[r][c]], self.T, spare[c]) for src, r, c in pairs]).run()
             for r in range(P):  # the sums become the ranks' chunks; the old chunks the spares
                 c = (r - 2 - i) % P
                 S[r][c], spare[c] = spare[c], S[r][c]
@@ -220,17 +220,15 @@ class RingAllreduce:
         for i in range(P - 1):
             # every rank compresses the chunk it sends (a message per chunk:
             # the P ranks send P different chunks in a step) ...
+            sent = [(r, (r - 1 - i) % P) for r in range(P)]
             self._plan(("doc", "send", i, eb), BATCH_COMPRESS,
-                       [(self._chunk(acc[r], (r - 1 - i) % P), eb, self.T, msg[(r - 1 - i) % P])
-                        for r in range(P)]).run()
+                       lambda: [(self._chunk(acc[r], c), eb, self.T, msg[c]) for r, c in sent]).run()
             # ... and adds the one it receives, decompressed, into its own
-            jobs = []
-            for r in range(P):
-                c = (r - 2 - i) % P
-                jobs.append((msg[c], eb, self.T, self._chunk(acc[r], c), True))
-            self._plan(("doc", "add", i, eb), BATCH_DECOMPRESS, jobs).run()
+            got = [(r, (r - 2 - i) % P) for r in range(P)]
+            self._plan(("doc", "add", i, eb), BATCH_DECOMPRESS,
+                       lambda: [(msg[c], eb, self.T, self._chunk(acc[r], c), True) for r, c in got]).run()
         self._plan(("doc", "reduced", eb), BATCH_COMPRESS,
-                   [(self._chunk(acc[c], c), eb, self.T, red[c]) for c in range(P)]).run()
+                   lambda: [(self._chunk(acc[c], c), eb, self.T, red[c]) for c in range(P)]).run()
         self.reduced = red[:]
         return self._gather_batched(self.reduced, eb, per_rank_outputs, "doc")
 

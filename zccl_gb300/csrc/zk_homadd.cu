@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(ADD_THREADS, 2) k_homadd(const __grid_constant
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
                     smask = __funnelshift_l(acc[j], smask, 1); /* (smask << 1) | sign of element j */
-                    mf = fmaxf(mf, fabsf(__uint_as_float(acc[j])));
+                    if (j & 1) mf = max3_abs(mf, __uint_as_float(acc[j - 1]), __uint_as_float(acc[j]));
                 }
                 mx = (uint32_t)mf;
                 if (__builtin_expect(mx < (1u << 22), 1)) { /* 2^23 + |sum|: the magnitude in the low 23 bits */

@@ -714,7 +714,7 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
         float q[BS + 1], ql = sz3_quantize_f(cl, inv, sure, sq);
 #pragma unroll
         for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_f(cv[r], inv, sure, sq);
-        float rp = 0.0f;
+        float rp = 0.0f, ep = 0.0f;
 #pragma unroll
         for (uint32_t r = 0; r <= BS; r++) {
             const float up = __shfl_up_sync(0xffffffffu, q[r], 1), l0 = __shfl_sync(0xffffffffu, ql, r);
@@ -724,7 +724,8 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
                 if (pl) {
                     const float e = d - dp[r - 1];
                     w[(pl - 1) * BS + r - 1] = __float_as_uint(e + SZ_MAGIC);
-                    top = fmaxf(top, fabsf(e));
+                    if (r % 2 == 0) top = max3_abs(top, ep, e);
+                    ep = e;
                 }
                 dp[r - 1] = d;
             }

@@ -602,12 +602,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-/* `n` arrivals at once (release at CTA scope). */
-__device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
-}
-
 /* One try for phase `parity` of the barrier (the hardware may hold the
  * thread for up to the given time, in ns, before it answers). */
 __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity, uint32_t ns)
@@ -734,22 +728,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t sa, const void *map, int32_
         "l"((uint64_t)(uintptr_t)map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
         : "memory");
 }
-
-/* Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned)
- * from shared memory to global, in the issuing thread's bulk group.  The
- * writers of the shared bytes run fence_proxy_async_smem() and a barrier
- * before it. */
-__device__ __forceinline__ void bulk_s2g(void *gdst, const void *ssrc, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-/* The issuing thread's bulk stores have read their shared source (the
- * buffer may be written again) / have completed. */
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 /* One thread: TMA bulk copy of the 16-byte-aligned superset
  * [floor16(g), ceil16(g + nbytes)) into the 16-byte-aligned buffer s, arming
@@ -884,29 +862,7 @@ __device__ __forceinline__ uint32_t grp_excl_scan1(uint32_t v, uint32_t *ws, uin
     return __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u) + inc - v;
 }
 
-/* Two exclusive scans at once (v0 with scratch ws0, v1 with ws1, 33 words
- * each) over the first n threads, with one barrier: every warp reads all
- * warp sums.  Callers alternate between two pairs of scratch arrays on
- * consecutive calls, as for grp_excl_scan1. */
-__device__ __forceinline__ void grp_excl_scan2_1(uint32_t v0, uint32_t v1, uint32_t *ws0, uint32_t *ws1,
-                                                 uint32_t &r0, uint32_t &r1, uint32_t &t0, uint32_t &t1,
-                                                 uint32_t n, uint32_t id)
-{
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = n >> 5;
-    const uint32_t i0 = warp_incl_scan(v0), i1 = warp_incl_scan(v1);
-    if (lane == 31) {
-        ws0[warp] = i0;
-        ws1[warp] = i1;
-    }
-    named_sync(id, n);
-    const uint32_t a = lane < nw ? ws0[lane] : 0u, b = lane < nw ? ws1[lane] : 0u;
-    t0 = __reduce_add_sync(0xffffffffu, a);
-    t1 = __reduce_add_sync(0xffffffffu, b);
-    r0 = __reduce_add_sync(0xffffffffu, lane < warp ? a : 0u) + i0 - v0;
-    r1 = __reduce_add_sync(0xffffffffu, lane < warp ? b : 0u) + i1 - v1;
-}
-
-/* The same over the whole CTA. */
+/* grp_excl_scan over the whole CTA. */
 __device__ __forceinline__ uint32_t cta_excl_scan(uint32_t v, uint32_t *wsum, uint32_t *total)
 {
     return grp_excl_scan(v, wsum, total, blockDim.x, 0);

@@ -52,7 +52,6 @@ typedef struct ZGeom {
     uint32_t fmt;     /* block magnitude layout: ZG_FASTMODE1 or ZG_FIXED_BYTES */
     uint32_t GB;      /* blocks per index group */
     uint32_t nt_rcp;  /* floor(2^32 / nt_reg) (2^32 - 1 for 1): division of tile numbers */
-    uint32_t small;   /* n < 2^31: every element, block and group number fits 32 bits */
 } ZGeom;
 
 /* Block magnitude layouts.  fastmode1: B = b/8 whole bytes per magnitude
@@ -124,7 +123,6 @@ ZG_HD int zg_init(ZGeom *g, uint64_t n, uint32_t L, uint32_t T)
     g->T = T;
     g->L = L;
     g->fmt = ZG_FASTMODE1;
-    g->small = n < (1ull << 31);
     g->GB = zg_tile_blocks(L) / ZG_SUB;
     g->tbs = n / T;
     g->rem = (uint32_t)(n % T);
@@ -180,54 +178,6 @@ ZG_HD void zg_tile(const ZGeom *g, uint64_t t, ZTile *z)
     uint64_t last = (z->blk0 + z->nblk) * g->L; /* elements after the head, capped below */
     if (last > z->seg_len - 1) last = z->seg_len - 1;
     z->e_end = z->seg_start + 1 + last;
-}
-
-/* Group `sub` of tile t: blocks [gblk, gblk + nblk) of the stream, the last of
- * nlast elements, the first starting at element e_first. */
-typedef struct ZGroup {
-    uint64_t e_first, gblk, grp;
-    uint32_t nblk, nlast, has_head;
-} ZGroup;
-
-ZG_HD void zg_group(const ZGeom *g, uint64_t t, uint32_t sub, ZGroup *c)
-{
-    const uint32_t GB = g->GB, L = g->L, b0 = sub * GB;
-    if (g->small) { /* the same in 32 bits: a warp of the decompressor does this for every group */
-        const uint32_t reg = g->T * (uint32_t)g->nt_reg;
-        uint32_t s, k, nb, len;
-        if ((uint32_t)t < reg) {
-            s = zg_seg_of(g, (uint32_t)t);
-            k = (uint32_t)t - s * (uint32_t)g->nt_reg;
-            nb = (uint32_t)g->nb_reg;
-            len = (uint32_t)g->tbs;
-        } else {
-            s = g->T;
-            k = (uint32_t)t - reg;
-            nb = (uint32_t)g->nb_rm;
-            len = g->rem;
-        }
-        const uint32_t blk = k * g->TB + b0, left = nb > blk ? nb - blk : 0u;
-        c->nblk = left < GB ? left : GB;
-        c->has_head = k == 0 && sub == 0;
-        c->gblk = s * (uint32_t)g->nb_reg + blk;
-        c->grp = s * (uint32_t)g->gr_reg + k * ZG_SUB + sub;
-        c->e_first = s * (uint32_t)g->tbs + 1u + blk * L;
-        c->nlast = left > GB || !left ? L : len - 1u - (blk + c->nblk - 1u) * L;
-        if (c->nlast > L) c->nlast = L;
-        return;
-    }
-    ZTile z;
-    zg_tile(g, t, &z);
-    c->nblk = z.nblk > b0 ? (z.nblk - b0 < GB ? z.nblk - b0 : GB) : 0u;
-    c->has_head = z.has_head && sub == 0;
-    c->gblk = z.gblk0 + b0;
-    c->grp = z.grp0 + sub;
-    c->e_first = z.e_first + (uint64_t)b0 * L;
-    c->nlast = L;
-    if (c->nblk) {
-        const uint32_t rest = (uint32_t)(z.e_end - z.e_first) - (b0 + c->nblk - 1u) * L;
-        if (rest < L) c->nlast = rest;
-    }
 }
 
 /* Elements of block j (index within the segment) of a segment of len. */

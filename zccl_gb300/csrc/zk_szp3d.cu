@@ -1513,7 +1513,7 @@ __global__ void __launch_bounds__(256) k_sz3_carry(uint32_t *__restrict__ carry,
  * rows of one part, or a piece of a long row) and walks along x, FQ columns'
  * sums a thread.  A producer warp keeps a ring of stages of FP planes on their
  * way (the run, and the carry's row that its rows share).  Bound by memory:
- * 512^3 194 us (5.5 TB/s), against 351 with the threads themselves loading 4
+ * 512^3 176 us (6.1 TB/s), against 351 with the threads themselves loading 4
  * planes ahead into registers. */
 constexpr uint32_t FQ = 4, FP = 2, FCOLS = FQ * 288;
 
@@ -1768,9 +1768,14 @@ cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const uint64_t columns = g.d1 * g.d3;
     if (nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, nparts - 1);
+    /* the most rows a run (they share the carry's row) that leave no SM short of
+     * runs: 384^3 with two rows, 192 runs on 152 SMs, 107 us, with one 89; 512^3
+     * with two, 256 runs, 176, with one 193 */
     Sz3Run f;
-    f.R = 1;
-    while (f.R < 8 && 2 * f.R * g.d3 <= FCOLS && g.d2 / (2 * f.R) >= (uint64_t)nsm) f.R *= 2; /* a power of two: rows of one part */
+    const uint64_t sms = (uint64_t)nsm;
+    auto even = [&](uint64_t runs) { return runs >= 8 * sms || 5 * runs >= 4 * sms * ((runs + sms - 1) / sms); };
+    for (f.R = 8; f.R > 1; f.R /= 2) /* a power of two: rows of one part */
+        if (f.R * g.d3 <= FCOLS && even((g.d2 + f.R - 1) / f.R)) break;
     f.pieces = (uint32_t)((g.d3 + FCOLS - 1) / FCOLS);
     f.cz = (uint32_t)((g.d3 + f.pieces - 1) / f.pieces);
     if (f.pieces > 1) f.cz = (f.cz + 31u) & ~31u; /* <= FCOLS, a multiple of 32 */
@@ -1779,10 +1784,11 @@ cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims
     f.pb = (4u * f.cols + 47u) & ~15u;
     f.cb = (4u * f.cz + 47u) & ~15u;
     const uint32_t nth = (f.cols + 32u * FQ - 1) / (32u * FQ) * 32u, stage = FP * (f.pb + f.cb);
-    f.stages = std::min(8u, std::max(2u, 72u * 1024u / stage));
+    const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
+    /* three CTAs an SM, or four where that takes them all at once */
+    f.stages = std::min(8u, std::max(2u, (runs > 3 * sms && runs <= 4 * sms ? 54u : 72u) * 1024u / stage));
     const uint32_t smem = f.stages * stage;
     if ((e = cudaFuncSetAttribute(k_sz3_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-    const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
     k_sz3_finish<<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, U::ROWS, f, twice, w.err);
     return cudaGetLastError();
 }

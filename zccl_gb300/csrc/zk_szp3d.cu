@@ -610,6 +610,9 @@ __device__ __noinline__ void sz3_walk_any(const float *x, const Sz3Dims &g, cons
     sz3_walk<BS>(x, g, inv, k, bad, [&](uint32_t di, uint32_t dj, uint32_t v) { d[di * BS + dj] = v; });
 }
 
+/* The double steps for a value below 2^19. */
+__device__ __noinline__ float sz3_quantize_d(float x, double inv) { return (float)floor(__dadd_rn(__dmul_rn((double)x, inv), 0.5)); }
+
 constexpr float SZ_MAGIC = 12582912.0f;         /* 1.5 * 2^23: a float m + this holds the integer m in its low bits, */
 constexpr uint32_t SZ_ZERO = 0x4B400000u;       /* as this + m */
 
@@ -676,8 +679,11 @@ struct Sz3Feed {
  * unit's rows are sent for meanwhile, into the buffers that this one leaves.
  * In floats, which hold every step exactly while the quantized values are
  * below 2^19 (the differences below 2^22); false if they are not, or where a
- * value needs the double steps (one unit in thousands; they hold up the tiles
- * after them): any w then. */
+ * value needs the double steps (one unit in thousands): any w then.
+ * Side 8 takes the planes in a loop, with w in local memory, and the double
+ * steps by the plane: as straight code for its 81 rows, a volume of 57 x 51 x 306
+ * took 63 us, most of it the code's way from L2, and 38 so; 512^3 489 us and
+ * 426. */
 template <uint32_t BS>
 __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
                                            const Sz3Unit &k, const Sz3Unit &next, Sz3Feed<BS> &feed, uint32_t (&w)[BS * BS],
@@ -693,11 +699,12 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
     const uint64_t stride = 4u * g.d2 * g.d3;
     float dp[BS], sq = 0.0f, top = 0.0f;
     bool sure = true;
-#pragma unroll
-    for (uint32_t pl = 0; pl <= BS; pl++) {
+    uint32_t slot = 0; /* pl % PD */
+#pragma unroll(BS == 8 ? 1 : BS + 1)
+    for (uint32_t pl = 0; pl <= BS; pl++, slot = slot + 1 == F::PD ? 0 : slot + 1) {
         cp_async_wait<F::PD - 1>(); /* all but the PD - 1 planes after this one */
         __syncwarp();
-        const uint32_t buf = sbuf + pl % F::PD * F::PLANE, ap = a0 + pl * dpl;
+        const uint32_t buf = sbuf + slot * F::PLANE, ap = a0 + pl * dpl;
         float cv[BS + 1], cl;
         if (even) {
             const uint32_t at = buf + 4u * ((a0 & 3u) + 1u + lane);
@@ -710,10 +717,16 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
         cl = lin ? ld_shared_f32(buf + lane * SZ_ROW + 4u * ((ap + lane * d3) & 3u)) : 0.0f; /* lane r: before row r */
         __syncwarp();
         if (pl + F::PD == BS + 1) feed.set(x, g, next);
-        feed.send(buf, (pl + F::PD) % (BS + 1), stride);
+        feed.send(buf, pl + F::PD <= BS ? pl + F::PD : pl + F::PD - BS - 1, stride);
         float q[BS + 1], ql = sz3_quantize_f(cl, inv, sure, sq);
 #pragma unroll
         for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_f(cv[r], inv, sure, sq);
+        if (BS == 8 && __any_sync(0xffffffffu, !sure)) { /* the double steps, for this plane */
+            ql = sz3_quantize_d(cl, inv.d);
+#pragma unroll
+            for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_d(cv[r], inv.d);
+            sure = true; /* (out of range: sq shows it) */
+        }
         float rp = 0.0f, ep = 0.0f;
 #pragma unroll
         for (uint32_t r = 0; r <= BS; r++) {
@@ -785,7 +798,7 @@ __device__ __forceinline__ void sz3_put_octet(uint32_t sbase, uint32_t o, uint32
  * 1-D compressor's.
  * Bound by issue, 80 instructions per 32 elements at side 4 (252 with exact
  * integer quantization, byte-wise packing and a look-back per warp).  512^3:
- * side 8 485 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
+ * side 8 426 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
  * side 4 take 440, three CTAs an SM 470 (spills), 10 or 12 compute warps the
  * same 408. */
 template <uint32_t BS>
@@ -936,7 +949,7 @@ __global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(con
                 for (uint32_t e = 0; e < BS * BS; e++) d[e] = 0;
                 if (K.sx) sz3_walk_any<BS>(x, g, inv, K, d, bad);
                 mx = 0;
-#pragma unroll
+#pragma unroll(BS == 8 ? 1 : BS * BS)
                 for (uint32_t e = 0; e < BS * BS; e++) {
                     w[i][e] = SZ_ZERO + d[e];
                     mx = max(mx, mag(d[e]));
@@ -944,7 +957,7 @@ __global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(con
             }
             if (K.sx < BS || K.sy < BS) { /* rows outside the volume count for nothing */
                 mx = 0;
-#pragma unroll
+#pragma unroll(BS == 8 ? 1 : BS * BS)
                 for (uint32_t e = 0; e < BS * BS; e++)
                     if (e / BS < K.sx && e % BS < K.sy) mx = max(mx, mag(w[i][e] - SZ_ZERO));
             }
@@ -970,7 +983,47 @@ __global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(con
 #pragma unroll
         for (uint32_t i = 0; i < UPW; i++) {
             const Sz3Unit &K = k[i];
-            if (K.sx == BS && K.sy == BS && K.z0 + 32 <= g.d3) { /* whole blocks: rows are octets, or halves or quarters */
+            if constexpr (BS == 8) {
+                /* blocks whole along y and z go plane by plane, 8 octets of each; the others of a unit, from
+                 * `whole` on, in their own order, 256 elements at a time */
+                const uint32_t zleft = (uint32_t)min((uint64_t)32, g.d3 - K.z0);
+                const uint32_t there = K.sx ? (zleft + 7u) / 8u : 0u, whole = K.sx && K.sy == 8 ? zleft / 8u : 0u;
+#pragma unroll 1
+                for (uint32_t di = 0; whole && di < K.sx; di++) {
+                    __syncwarp();
+#pragma unroll
+                    for (uint32_t e = 0; e < 8; e++) st[c * C::BST + e * 8u + dz] = w[i][di * 8u + e];
+                    __syncwarp();
+                    const uint32_t b = lane / 8u, at = __shfl_sync(0xffffffffu, off, b), rb = __shfl_sync(0xffffffffu, rate, b);
+                    if (b < whole) {
+                        const uint4 *p = reinterpret_cast<const uint4 *>(st + b * C::BST + 8u * (lane % 8u));
+                        const uint4 lo = p[0], hi = p[1];
+                        const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                        sz3_put_octet(pk, at, rb, K.sx * 64u, di * 8u + lane % 8u, v);
+                    }
+                }
+                const uint32_t sz = K.z0 + lane < g.d3 ? sz3_unit_sz<BS>(g, K, c) : 0u;
+#pragma unroll 1
+                for (uint32_t lot = 2u * whole; lot < 2u * there; lot++) {
+                    const uint32_t b = lot / 2u, e0 = (lot & 1u) * 256u; /* its block, and first element of it */
+                    if (e0 >= K.sx * K.sy * 8u) continue;
+                    __syncwarp();
+                    if (sz && c == b)
+#pragma unroll 4
+                        for (uint32_t e = 0; e < 64; e++) {
+                            const uint32_t at = (e / 8u * K.sy + e % 8u) * sz + dz - e0;
+                            if (e / 8u < K.sx && e % 8u < K.sy && at < 256u) st[at] = w[i][e];
+                        }
+                    __syncwarp();
+                    const uint32_t at = __shfl_sync(0xffffffffu, off, b), rb = __shfl_sync(0xffffffffu, rate, b), nb = __shfl_sync(0xffffffffu, n, b);
+                    if (e0 + 8u * lane < nb) {
+                        uint32_t v[8];
+#pragma unroll
+                        for (uint32_t e = 0; e < 8; e++) v[e] = e0 + 8u * lane + e < nb ? st[8u * lane + e] : SZ_ZERO;
+                        sz3_put_octet(pk, at, rb, nb, e0 / 8u + lane, v);
+                    }
+                }
+            } else if (K.sx == BS && K.sy == BS && K.z0 + 32 <= g.d3) { /* whole blocks: rows are octets, or halves or quarters */
 #pragma unroll
                 for (uint32_t e0 = 0; e0 < BS * BS; e0 += C::ROWS) {
                     __syncwarp();

@@ -1567,8 +1567,10 @@ __global__ void __launch_bounds__(256) k_sz3_carry(uint32_t *__restrict__ carry,
  * sums a thread.  A producer warp keeps a ring of stages of FP planes on their
  * way (the run, and the carry's row that its rows share).  Bound by memory:
  * 512^3 176 us (6.1 TB/s), against 351 with the threads themselves loading 4
- * planes ahead into registers. */
-constexpr uint32_t FQ = 4, FP = 2, FCOLS = FQ * 288;
+ * planes ahead into registers.  Small planes leave an SM few warps, and a
+ * stage's chain of waits, sums and stores sets the pace: eight planes a stage
+ * and one column a thread then. */
+constexpr uint32_t FTH = 288; /* summing threads at most */
 
 struct Sz3Run {
     uint32_t R;      /* rows in a run */
@@ -1579,7 +1581,8 @@ struct Sz3Run {
     uint32_t stages;
 };
 
-__global__ void __launch_bounds__(FCOLS / FQ + 32) k_sz3_finish(uint32_t *vol, const uint32_t *carry, uint64_t d1,
+template <uint32_t FQ, uint32_t FP>
+__global__ void __launch_bounds__(FTH + 32) k_sz3_finish(uint32_t *vol, const uint32_t *carry, uint64_t d1,
                                                                 uint64_t d2, uint64_t d3, uint32_t rows, Sz3Run f,
                                                                 Sz3Split twice, uint32_t *err)
 {
@@ -1797,6 +1800,36 @@ size_t sz3_carry_bytes(const Sz3Dims &g)
     return 4 * (size_t)((g.nb2 + strips - 1) / strips - 1) * g.d1 * g.d3;
 }
 
+template <uint32_t FQ, uint32_t FP>
+cudaError_t sz3_finish(const Sz3Dims &g, uint32_t *vol, const uint32_t *carry, uint32_t rows, const Sz3Split &twice,
+                       uint64_t sms, uint32_t *err, cudaStream_t st)
+{
+    constexpr uint32_t FCOLS = FQ * FTH;
+    /* the most rows a run (they share the carry's row) that leave no SM short of
+     * runs: 384^3 with two rows, 192 runs on 152 SMs, 107 us, with one 89; 512^3
+     * with two, 256 runs, 176, with one 193 */
+    Sz3Run f;
+    auto even = [&](uint64_t runs) { return runs >= 8 * sms || 5 * runs >= 4 * sms * ((runs + sms - 1) / sms); };
+    for (f.R = 8; f.R > 1; f.R /= 2) /* a power of two: rows of one part */
+        if (f.R * g.d3 <= FCOLS && even((g.d2 + f.R - 1) / f.R)) break;
+    f.pieces = (uint32_t)((g.d3 + FCOLS - 1) / FCOLS);
+    f.cz = (uint32_t)((g.d3 + f.pieces - 1) / f.pieces);
+    if (f.pieces > 1) f.cz = (f.cz + 31u) & ~31u; /* <= FCOLS, a multiple of 32 */
+    f.pieces = (uint32_t)((g.d3 + f.cz - 1) / f.cz);
+    f.cols = f.R * f.cz;
+    f.pb = (4u * f.cols + 47u) & ~15u;
+    f.cb = (4u * f.cz + 47u) & ~15u;
+    const uint32_t nth = (f.cols + 32u * FQ - 1) / (32u * FQ) * 32u, stage = FP * (f.pb + f.cb);
+    const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
+    /* three CTAs an SM, or four where that takes them all at once */
+    f.stages = std::min(8u, std::max(2u, (runs > 3 * sms && runs <= 4 * sms ? 54u : 72u) * 1024u / stage));
+    const uint32_t smem = f.stages * stage;
+    const cudaError_t e = cudaFuncSetAttribute(k_sz3_finish<FQ, FP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_sz3_finish<FQ, FP><<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, rows, f, twice, err);
+    return cudaGetLastError();
+}
+
 template <uint32_t BS>
 cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims &g, const Sz3Ws &w, uint32_t *vol,
                                 const Sz3Split &twice, cudaStream_t st)
@@ -1821,29 +1854,10 @@ cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const uint64_t columns = g.d1 * g.d3;
     if (nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, nparts - 1);
-    /* the most rows a run (they share the carry's row) that leave no SM short of
-     * runs: 384^3 with two rows, 192 runs on 152 SMs, 107 us, with one 89; 512^3
-     * with two, 256 runs, 176, with one 193 */
-    Sz3Run f;
-    const uint64_t sms = (uint64_t)nsm;
-    auto even = [&](uint64_t runs) { return runs >= 8 * sms || 5 * runs >= 4 * sms * ((runs + sms - 1) / sms); };
-    for (f.R = 8; f.R > 1; f.R /= 2) /* a power of two: rows of one part */
-        if (f.R * g.d3 <= FCOLS && even((g.d2 + f.R - 1) / f.R)) break;
-    f.pieces = (uint32_t)((g.d3 + FCOLS - 1) / FCOLS);
-    f.cz = (uint32_t)((g.d3 + f.pieces - 1) / f.pieces);
-    if (f.pieces > 1) f.cz = (f.cz + 31u) & ~31u; /* <= FCOLS, a multiple of 32 */
-    f.pieces = (uint32_t)((g.d3 + f.cz - 1) / f.cz);
-    f.cols = f.R * f.cz;
-    f.pb = (4u * f.cols + 47u) & ~15u;
-    f.cb = (4u * f.cz + 47u) & ~15u;
-    const uint32_t nth = (f.cols + 32u * FQ - 1) / (32u * FQ) * 32u, stage = FP * (f.pb + f.cb);
-    const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
-    /* three CTAs an SM, or four where that takes them all at once */
-    f.stages = std::min(8u, std::max(2u, (runs > 3 * sms && runs <= 4 * sms ? 54u : 72u) * 1024u / stage));
-    const uint32_t smem = f.stages * stage;
-    if ((e = cudaFuncSetAttribute(k_sz3_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
-    k_sz3_finish<<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, U::ROWS, f, twice, w.err);
-    return cudaGetLastError();
+    /* small planes (see k_sz3_finish): 45 x 60, 500 planes, 38 us against 86; 300 x 300 44 against 64;
+     * 384 x 384 108 against 90 */
+    return g.d2 * g.d3 <= 800 * (uint64_t)nsm ? sz3_finish<1, 8>(g, vol, carry, U::ROWS, twice, (uint64_t)nsm, w.err, st)
+                                         : sz3_finish<4, 2>(g, vol, carry, U::ROWS, twice, (uint64_t)nsm, w.err, st);
 }
 
 } // namespace

@@ -682,8 +682,8 @@ struct Sz3Feed {
  * value needs the double steps (one unit in thousands): any w then.
  * Side 8 takes the planes in a loop, with w in local memory, and the double
  * steps by the plane: as straight code for its 81 rows, a volume of 57 x 51 x 306
- * took 63 us, most of it the code's way from L2, and 38 so; 512^3 489 us and
- * 426. */
+ * took 63 us, most of it the code's way from L2, and 36 so; 512^3 489 us and
+ * 412. */
 template <uint32_t BS>
 __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
                                            const Sz3Unit &k, const Sz3Unit &next, Sz3Feed<BS> &feed, uint32_t (&w)[BS * BS],
@@ -798,12 +798,11 @@ __device__ __forceinline__ void sz3_put_octet(uint32_t sbase, uint32_t o, uint32
  * 1-D compressor's.
  * Bound by issue, 80 instructions per 32 elements at side 4 (252 with exact
  * integer quantization, byte-wise packing and a look-back per warp).  512^3:
- * side 8 426 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
+ * side 8 412 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
  * side 4 take 440, three CTAs an SM 470 (spills), 10 or 12 compute warps the
  * same 408. */
-template <uint32_t BS>
+template <uint32_t BS, uint32_t NW> /* NW: compute warps */
 struct Sz3Cm {
-    static constexpr uint32_t NW = 8;                                        /* compute warps */
     static constexpr uint32_t U = 32 / BS, NB = BS * BS * BS, UPW = BS == 2 ? 2 : 1;
     static constexpr uint32_t BPW = U * UPW;                                 /* blocks per warp, at most 32 */
     static constexpr uint32_t ROWS = BS * BS < 8 ? BS * BS : 8;              /* rows of a unit changed at a time */
@@ -825,14 +824,14 @@ struct Sz3CmShared {
 };
 constexpr uint32_t SZ_CM_HEAD = (sizeof(Sz3CmShared) + 15u) / 16u * 16u;
 
-template <uint32_t BS>
-__global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(const float *__restrict__ x, Sz3Dims g, Sz3Split inv,
+template <uint32_t BS, uint32_t NW>
+__global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows(const float *__restrict__ x, Sz3Dims g, Sz3Split inv,
                                                                         uint8_t *out, uint64_t cap, uint64_t *status,
                                                                         uint32_t *ticket, uint64_t *total_out, uint32_t R,
                                                                         uint32_t *err)
 {
-    using C = Sz3Cm<BS>;
-    constexpr uint32_t U = C::U, UPW = C::UPW, NW = C::NW;
+    using C = Sz3Cm<BS, NW>;
+    constexpr uint32_t U = C::U, UPW = C::UPW;
     extern __shared__ __align__(16) uint8_t sm[];
     Sz3CmShared *sh = reinterpret_cast<Sz3CmShared *>(sm);
     uint8_t *outs = sm + SZ_CM_HEAD + NW * C::OWN;
@@ -957,9 +956,12 @@ __global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(con
             }
             if (K.sx < BS || K.sy < BS) { /* rows outside the volume count for nothing */
                 mx = 0;
-#pragma unroll(BS == 8 ? 1 : BS * BS)
-                for (uint32_t e = 0; e < BS * BS; e++)
-                    if (e / BS < K.sx && e % BS < K.sy) mx = max(mx, mag(w[i][e] - SZ_ZERO));
+#pragma unroll(BS == 8 ? 1 : BS)
+                for (uint32_t di = 0; di < BS; di++)
+                    if (di < K.sx)
+#pragma unroll
+                        for (uint32_t dj = 0; dj < BS; dj++)
+                            if (dj < K.sy) mx = max(mx, mag(w[i][di * BS + dj] - SZ_ZERO));
             }
             if (K.z0 + lane >= g.d3) mx = 0;
 #pragma unroll
@@ -1009,10 +1011,13 @@ __global__ void __launch_bounds__(Sz3Cm<BS>::THREADS, 2) k_sz3_compress_rows(con
                     if (e0 >= K.sx * K.sy * 8u) continue;
                     __syncwarp();
                     if (sz && c == b)
-#pragma unroll 4
-                        for (uint32_t e = 0; e < 64; e++) {
-                            const uint32_t at = (e / 8u * K.sy + e % 8u) * sz + dz - e0;
-                            if (e / 8u < K.sx && e % 8u < K.sy && at < 256u) st[at] = w[i][e];
+#pragma unroll 1
+                        for (uint32_t di = 0; di < K.sx; di++) {
+                            const uint32_t at = di * K.sy * sz + dz - e0; /* its row 0 */
+                            if ((int32_t)at >= 256 || (int32_t)(at + K.sy * sz) <= 0) continue;
+#pragma unroll
+                            for (uint32_t dj = 0; dj < 8; dj++)
+                                if (dj < K.sy && at + dj * sz < 256u) st[at + dj * sz] = w[i][di * 8u + dj];
                         }
                     __syncwarp();
                     const uint32_t at = __shfl_sync(0xffffffffu, off, b), rb = __shfl_sync(0xffffffffu, rate, b), nb = __shfl_sync(0xffffffffu, n, b);
@@ -1774,22 +1779,25 @@ bool sz3_rows(uint32_t bs) { return bs == 2 || bs == 4 || bs == 8; }
  * block, at least 8 a tile), and the ticket and the scanner's word the last
  * two of the four scratch words before it (the first two are error words the
  * status check reads), all zeroed first. */
-template <uint32_t BS>
+template <uint32_t BS, uint32_t NW = 8>
 cudaError_t sz3_compress_rows(uint8_t *out, uint64_t cap, const float *x, const Sz3Dims &g, const Sz3Ws &w,
                               const Sz3Split &inv, cudaStream_t st)
 {
-    using C = Sz3Cm<BS>;
+    using C = Sz3Cm<BS, NW>;
     const uint64_t units = sz3_units<BS>(g);
     if ((units + 16) >> 32) return cudaErrorInvalidValue; /* units are counted in 32 bits */
-    const uint64_t ntiles = (units + C::NW * C::UPW - 1) / (C::NW * C::UPW);
+    if constexpr (BS == 8 && NW == 8) { /* too few units for tiles of eight on every SM: 57 x 51 x 306 36 us, with four 33 */
+        if (units < 8 * (uint64_t)sm_count()) return sz3_compress_rows<8, 4>(out, cap, x, g, w, inv, st);
+    }
+    const uint64_t ntiles = (units + NW * C::UPW - 1) / (NW * C::UPW);
     cudaError_t e = cudaMemsetAsync(w.offs, 0, 8 * ntiles, st);
     if (e != cudaSuccess) return e;
-    const uint32_t fixed = SZ_CM_HEAD + C::NW * C::OWN + 48u, R = ring_bytes(2, fixed, zg_ring_need(C::WORST));
+    const uint32_t fixed = SZ_CM_HEAD + NW * C::OWN + 48u, R = ring_bytes(2, fixed, zg_ring_need(C::WORST));
     const size_t smem = fixed + R;
-    const void *fn = (const void *)k_sz3_compress_rows<BS>;
+    const void *fn = (const void *)k_sz3_compress_rows<BS, NW>;
     if ((e = set_max_smem(fn, smem)) != cudaSuccess) return e;
     const unsigned grid = scanned_grid(fn, C::THREADS, smem, ntiles, 0);
-    k_sz3_compress_rows<BS><<<grid, C::THREADS, smem, st>>>(x, g, inv, out, cap, w.offs, w.err + 2, w.total, R, w.err);
+    k_sz3_compress_rows<BS, NW><<<grid, C::THREADS, smem, st>>>(x, g, inv, out, cap, w.offs, w.err + 2, w.total, R, w.err);
     return cudaGetLastError();
 }
 

@@ -165,14 +165,14 @@ typedef struct zccl_gpu_stream {
 
 /* Largest stream of n floats (every block at width 32). */
 size_t zccl_gpu_max_stream_bytes(size_t n, int L, int T);
-/* Bytes of the side index of one stream (about n/L + 12 per 8192 floats). */
+/* Bytes of the side index of one stream (about n/L + 12 per 1024 floats). */
 size_t zccl_gpu_index_bytes(size_t n, int L, int T);
-/* Bytes of device scratch one call needs (look-back state, error word, and
- * for streams that arrive without an index the header walk's tables, about
- * one byte per byte of the largest stream of this geometry).
+/* Bytes of device scratch one call needs (the tiles' size words, error words,
+ * and for streams that arrive without an index the header walk's tables, about
+ * half a byte per byte of the largest stream of this geometry at L = 32).
  * Its first 8 bytes are two status words: zero them once when the
  * workspace is allocated.  Every call leaves them alone (it zeroes only its
- * own look-back state) and ORs the errors it detects into them, so the
+ * own size words and tickets) and ORs the errors it detects into them, so the
  * errors of every call on a workspace since the last zccl_gpu_check() are
  * reported by that check, which then clears them. */
 size_t zccl_gpu_workspace_bytes(size_t n, int L, int T);

@@ -109,7 +109,7 @@ struct WalkLayout {
 size_t ws_clear_bytes(const ZGeom &g) { return 16 + 8 * g.ntiles; }
 
 /* Zero what a call needs zeroed at launch: the tile ticket and the
- * look-back words.  The two status words in front of them are left alone,
+ * tiles' size words.  The two status words in front of them are left alone,
  * so errors of earlier calls on the workspace stay visible until
  * zccl_gpu_check() reads and clears them. */
 cudaError_t ws_clear(void *ws, const ZGeom &g, cudaStream_t st)
@@ -157,7 +157,7 @@ ZWork bind_ws(void *ws)
 
 /* Test hook: with ZCCL_GPU_TEST_STALL_TILE0=1 in the environment a
  * compression hands out tiles from 1 on, so tile 0 never publishes its size
- * and its successor's look-back must give up, after 4096 polls instead of
+ * and the scan of the sizes must give up on it, after 4096 polls instead of
  * the usual limit.  The call then reports ZCCL_GPU_ETIMEOUT; nothing waits
  * without bound on the way. */
 bool test_stall_tile0()

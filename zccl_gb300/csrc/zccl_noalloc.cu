@@ -4,7 +4,7 @@
  * that must not allocate device memory.
  *
  * The compressor needs, per call, an error word, a tile ticket and one
- * look-back status word per tile, all zero at launch: 16 + 8 * tiles bytes.
+ * size word per tile, all zero at launch: 16 + 8 * tiles bytes.
  * Here they live in g_scratch, a file-scope __device__ array that exists
  * once per device from the moment the library's device code is loaded.
  * Its address is looked up with cudaGetSymbolAddress the first time a call

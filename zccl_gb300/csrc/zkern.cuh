@@ -183,8 +183,8 @@ struct WalkArgs {
  * count of released bytes, `tail`, shows that the space is free.  Up to
  * ZR_SLOTS tiles are between sizing and write-out at once (the ring's bytes
  * hold one worst-case tile, far more typical ones), so the packing warps do
- * not wait for a placer delayed by a slow look-back; 16 measured 3.7 %
- * faster than 4 on the two-way add.  All waits are bounded: on time-out
+ * not wait for a placer whose tile's place is late; 16 measured 3.7 % faster
+ * than 4 on the two-way add.  All waits are bounded: on time-out
  * ZERR_TIMEOUT is set and the caller goes on.
  * ------------------------------------------------------------------ */
 #define ZR_SLOTS 16u
@@ -530,7 +530,7 @@ static inline cudaError_t set_max_smem(const void *fn, size_t smem)
 /* Ring bytes of a kernel that runs `per_sm` CTAs per SM and needs `fixed`
  * other bytes of shared memory: at least `least` (one worst-case tile), and
  * up to the CTA's share of the SM's shared memory less a kilobyte of margin.
- * The longer the ring, the longer a tile may wait there for its look-back
+ * The longer the ring, the longer a tile may wait there for its place
  * before the compute warps run out of room. */
 static inline uint32_t ring_bytes(uint32_t per_sm, uint32_t fixed, uint32_t least)
 {

@@ -486,6 +486,37 @@ __device__ __forceinline__ void or_bytes(uint32_t sbase, uint32_t at, uint64_t v
     if (w2) sh_or(q + 8u, w2);
 }
 
+/* The magnitudes m of octet g of a block of n elements whose high bytes begin
+ * at byte h of the zeroed buffer at sbase: B high bytes each, then (from
+ * h + n B on) r low bits each, most significant first.  Four elements' low
+ * bits at a time are joined in 32 bits. */
+__device__ __forceinline__ void put_octet(uint32_t sbase, uint32_t h, uint32_t n, uint32_t g, uint32_t B, uint32_t r,
+                                          const uint32_t (&m)[8])
+{
+    if (B == 1) {
+        const uint32_t lo = __byte_perm(__byte_perm(m[0] >> r, m[1] >> r, 0x0040), __byte_perm(m[2] >> r, m[3] >> r, 0x0040), 0x5410);
+        const uint32_t hi = __byte_perm(__byte_perm(m[4] >> r, m[5] >> r, 0x0040), __byte_perm(m[6] >> r, m[7] >> r, 0x0040), 0x5410);
+        or_bytes(sbase, h + 8u * g, (uint64_t)hi << 32 | lo);
+    } else if (B > 1) {
+        const uint32_t keep = B >= 4 ? 0xFFFFFFFFu : (1u << (8u * B)) - 1u;
+#pragma unroll
+        for (int k = 0; k < 8; k++) or_bytes(sbase, h + (8u * g + (uint32_t)k) * B, (m[k] >> r) & keep);
+    }
+    if (r) { /* r bytes */
+        const uint32_t mask = (1u << r) - 1u;
+        uint32_t a = m[0] & mask, b = m[4] & mask;
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+            a = a << r | (m[k] & mask);
+            b = b << r | (m[4 + k] & mask);
+        }
+        /* the 8 r bits at the top of 64, bytes first to last upward */
+        const uint32_t s = 32u - 4u * r, at = a << s, bt = b << s;
+        const uint32_t hi = at | (bt >> (4u * r)), lo = bt << s;
+        or_bytes(sbase, h + n * B + g * r, (uint64_t)bswap32(lo) << 32 | bswap32(hi));
+    }
+}
+
 /* The inverse of decode_octet: octet g of a block of n elements and width b
  * into the zeroed buffer at sbase from byte o on; s8: its signs (element k at
  * bit 7 - k); m: its magnitudes (bits from the 24th on are ignored for
@@ -500,25 +531,7 @@ __device__ __forceinline__ void encode_octet(uint32_t sbase, uint32_t o, uint32_
         or_bytes(sbase, o, b | s8 << 8);
     else
         or_bytes(sbase, o + 1u + g, s8);
-    const uint32_t hb = o + 1u + ((n + 7u) >> 3), at = hb + 8u * B * g;
-    if (B == 1) {
-        uint64_t v = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) v |= (uint64_t)((m[k] >> r) & 0xFFu) << (8 * k);
-        or_bytes(sbase, at, v);
-    } else if (B > 1) {
-        const uint32_t keep = B == 2 ? 0xFFFFu : B == 3 ? 0xFFFFFFu : 0xFFFFFFFFu;
-#pragma unroll
-        for (int k = 0; k < 8; k++) or_bytes(sbase, at + (uint32_t)k * B, (m[k] >> r) & keep);
-    }
-    if (r) { /* r bytes, most significant bit first */
-        const uint32_t mask = (1u << r) - 1u;
-        uint64_t v = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) v = v << r | (m[k] & mask);
-        v <<= 64u - 8u * r;
-        or_bytes(sbase, hb + B * n + g * r, (uint64_t)bswap32((uint32_t)v) << 32 | bswap32((uint32_t)(v >> 32)));
-    }
+    put_octet(sbase, o + 1u + ((n + 7u) >> 3), n, g, B, r, m);
 }
 
 /* A block of n elements, one element at a time: separate streams for the

@@ -764,28 +764,7 @@ __device__ __forceinline__ void sz3_put_octet(uint32_t sbase, uint32_t o, uint32
         m[k] = (uint32_t)abs((int32_t)v);
     }
     if (s8) sh_or(sbase + (at & ~3u), s8 << (8u * (at & 3u)));
-    if (B == 1) {
-        const uint32_t lo = __byte_perm(__byte_perm(m[0] >> r, m[1] >> r, 0x0040), __byte_perm(m[2] >> r, m[3] >> r, 0x0040), 0x5410);
-        const uint32_t hi = __byte_perm(__byte_perm(m[4] >> r, m[5] >> r, 0x0040), __byte_perm(m[6] >> r, m[7] >> r, 0x0040), 0x5410);
-        or_bytes(sbase, h + 8u * g, (uint64_t)hi << 32 | lo);
-    } else if (B > 1) {
-        const uint32_t keep = B >= 4 ? 0xFFFFFFFFu : (1u << (8u * B)) - 1u;
-#pragma unroll
-        for (int k = 0; k < 8; k++) or_bytes(sbase, h + (8u * g + (uint32_t)k) * B, (m[k] >> r) & keep);
-    }
-    if (r) { /* r bytes, most significant bit first: two halves of 4 r bits */
-        const uint32_t mask = (1u << r) - 1u;
-        uint32_t a = m[0] & mask, b = m[4] & mask;
-#pragma unroll
-        for (int k = 1; k < 4; k++) {
-            a = a << r | (m[k] & mask);
-            b = b << r | (m[4 + k] & mask);
-        }
-        /* the 8 r bits at the top of 64, bytes first to last upward */
-        const uint32_t s = 32u - 4u * r, at2 = a << s, bt = b << s;
-        const uint32_t hi = at2 | (bt >> (4u * r)), lo = bt << s;
-        or_bytes(sbase, h + n * B + g * r, (uint64_t)(s ? bswap32(lo) : 0u) << 32 | bswap32(hi));
-    }
+    put_octet(sbase, h, n, g, B, r, m);
 }
 
 /* One pass.  Tiles of NW * UPW units in stream order, handed out by tickets:

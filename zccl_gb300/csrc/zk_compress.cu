@@ -291,19 +291,17 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
             }
             b = own ? width_of(mx, a.wt) : 0u;
         } else {
-            const uint32_t last = nblk ? (nblk - 1u) * L + (b0 + nblk == tb ? D.nlast : L) : 0u; /* the group's last float, the one before it being 0 */
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
                 const uint32_t k = i * BPI + bi;
                 const bool has = bi < BPI && k < nblk;
                 const uint32_t nk = !has ? 0u : b0 + k + 1u < tb ? L : D.nlast;
-                const uint32_t e = k * L + 8u * og; /* the octet's first element is float e + 1 */
+                /* the octet's first element is float e + 1 of the group's, the block's last is float `end`: past
+                 * it copies, no delta */
+                const uint32_t end = has ? k * L + nk : 0u, e = min(k * L + 8u * og, end);
                 float x[9];
 #pragma unroll
-                for (uint32_t j = 0; j < 9; j++) { /* past the block's end copies: no delta */
-                    const float f = nblk || warp == 0 ? lin[D.at + min(e + j, last)] : 0.f;
-                    x[j] = j == 0 || 8u * og + j <= nk ? f : x[j - 1];
-                }
+                for (uint32_t j = 0; j < 9; j++) x[j] = nblk || warp == 0 ? lin[D.at + min(e + j, end)] : 0.f;
                 uint32_t mi[8], s8, mx;
                 int32_t qi;
                 if (__builtin_expect(!quantize_deltas<8>(x, inv, mi, s8, mx, qi), 0))

@@ -1810,8 +1810,8 @@ cudaError_t sz3_finish(const Sz3Dims &g, uint32_t *vol, const uint32_t *carry, u
     const uint64_t runs = (g.d2 + f.R - 1) / f.R * f.pieces;
     /* three CTAs an SM, or four where that takes them all at once */
     f.stages = std::min(8u, std::max(2u, (runs > 3 * sms && runs <= 4 * sms ? 54u : 72u) * 1024u / stage));
-    const uint32_t smem = f.stages * stage;
-    const cudaError_t e = cudaFuncSetAttribute(k_sz3_finish<FQ, FP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const uint32_t smem = f.stages * stage; /* at most 72 KB; the limit is the same in every call, from any thread */
+    const cudaError_t e = set_max_smem((const void *)k_sz3_finish<FQ, FP>, 72u * 1024u);
     if (e != cudaSuccess) return e;
     k_sz3_finish<FQ, FP><<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, rows, f, twice, err);
     return cudaGetLastError();
@@ -1827,24 +1827,19 @@ cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims
     k_sz3_chunk_sizes<<<grid_for(nchunks, SZ_THREADS / 8), SZ_THREADS, 0, st>>>(in, avail, g, nchunks, w.sizes, w.err);
     if ((e = sz3_scan(g, w, nchunks, st)) != cudaSuccess) return e;
     const void *fn = (const void *)k_sz3_unpack_sum<BS>;
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::SMEM)) != cudaSuccess) return e;
-    int dev = 0, nsm = 0, per = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SZ_UN_THREADS, U::SMEM)) != cudaSuccess)
-        return e;
+    if ((e = set_max_smem(fn, U::SMEM)) != cudaSuccess) return e;
+    const uint64_t nsm = (uint64_t)sm_count();
     const uint64_t nparts = (g.nb2 + U::PARTS - 1) / U::PARTS, tasks = nparts * ((g.nb1 + U::STRIPS - 1) / U::STRIPS);
-    const uint64_t most = (uint64_t)nsm * (per > 0 ? per : 1);
     uint32_t *carry = reinterpret_cast<uint32_t *>(w.q);
-    k_sz3_unpack_sum<BS><<<(unsigned)(tasks < most ? tasks : most), SZ_UN_THREADS, U::SMEM, st>>>(in, avail, g, w.offs, w.sizes,
-                                                                                                 vol, carry, w.err);
+    k_sz3_unpack_sum<BS><<<persistent_grid(fn, SZ_UN_THREADS, U::SMEM, tasks), SZ_UN_THREADS, U::SMEM, st>>>(
+        in, avail, g, w.offs, w.sizes, vol, carry, w.err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const uint64_t columns = g.d1 * g.d3;
     if (nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, nparts - 1);
     /* small planes (see k_sz3_finish): 45 x 60, 500 planes, 38 us against 86; 300 x 300 44 against 64;
      * 384 x 384 108 against 90 */
-    return g.d2 * g.d3 <= 800 * (uint64_t)nsm ? sz3_finish<1, 8>(g, vol, carry, U::ROWS, twice, (uint64_t)nsm, w.err, st)
-                                         : sz3_finish<4, 2>(g, vol, carry, U::ROWS, twice, (uint64_t)nsm, w.err, st);
+    return g.d2 * g.d3 <= 800 * nsm ? sz3_finish<1, 8>(g, vol, carry, U::ROWS, twice, nsm, w.err, st)
+                                    : sz3_finish<4, 2>(g, vol, carry, U::ROWS, twice, nsm, w.err, st);
 }
 
 } // namespace

@@ -510,20 +510,16 @@ static inline cudaError_t set_max_smem(const void *fn, size_t smem)
     LaunchCache &c = launch_cache();
     int dev = 0;
     cudaGetDevice(&dev);
-    {
-        std::lock_guard<std::mutex> lk(c.mu);
-        for (int i = 0; i < c.nattr; i++)
-            if (c.attr[i].fn == fn && c.attr[i].dev == dev && c.attr[i].smem >= smem) return cudaSuccess;
-    }
+    std::lock_guard<std::mutex> lk(c.mu); /* held while setting: a call that wants less must not undo one that wants more */
+    int i = 0;
+    while (i < c.nattr && !(c.attr[i].fn == fn && c.attr[i].dev == dev)) i++;
+    if (i < c.nattr && c.attr[i].smem >= smem) return cudaSuccess;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(c.mu);
-    for (int i = 0; i < c.nattr; i++)
-        if (c.attr[i].fn == fn && c.attr[i].dev == dev) {
-            c.attr[i].smem = smem;
-            return cudaSuccess;
-        }
-    if (c.nattr < 64) c.attr[c.nattr++] = {fn, dev, smem};
+    if (i < c.nattr)
+        c.attr[i].smem = smem;
+    else if (c.nattr < 64)
+        c.attr[c.nattr++] = {fn, dev, smem};
     return cudaSuccess;
 }
 

@@ -694,7 +694,6 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
     const uint32_t d3 = (uint32_t)g.d3, dpl = (uint32_t)(g.d2 * g.d3); /* phases: low bits are enough */
     const uint32_t a0 = ((uint32_t)reinterpret_cast<uintptr_t>(x) >> 2) + ((uint32_t)k.i0 - 1u) * dpl + ((uint32_t)k.j0 - 1u) * d3 +
                         (uint32_t)k.z0 - 1u;
-    const bool even = (d3 & 3u) == 0; /* every row at the same phase */
     const bool lin = k.z0 && lane <= BS;
     const uint64_t stride = 4u * g.d2 * g.d3;
     float dp[BS], sq = 0.0f, top = 0.0f;
@@ -706,14 +705,8 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
         __syncwarp();
         const uint32_t buf = sbuf + slot * F::PLANE, ap = a0 + pl * dpl;
         float cv[BS + 1], cl;
-        if (even) {
-            const uint32_t at = buf + 4u * ((a0 & 3u) + 1u + lane);
 #pragma unroll
-            for (uint32_t r = 0; r <= BS; r++) cv[r] = ld_shared_f32(at + r * SZ_ROW);
-        } else {
-#pragma unroll
-            for (uint32_t r = 0; r <= BS; r++) cv[r] = ld_shared_f32(buf + r * SZ_ROW + 4u * (((ap + r * d3) & 3u) + 1u + lane));
-        }
+        for (uint32_t r = 0; r <= BS; r++) cv[r] = ld_shared_f32(buf + r * SZ_ROW + 4u * (((ap + r * d3) & 3u) + 1u + lane));
         cl = lin ? ld_shared_f32(buf + lane * SZ_ROW + 4u * ((ap + lane * d3) & 3u)) : 0.0f; /* lane r: before row r */
         __syncwarp();
         if (pl + F::PD == BS + 1) feed.set(x, g, next);

@@ -845,10 +845,13 @@ struct PinBuf {
 constexpr uint32_t kMaxGroups = 8;
 constexpr uint32_t kLanes = 4;
 constexpr uint32_t kWalkLanes = 2 * kLanes; /* workspaces: the add's second walk of lane l uses l + kLanes */
-/* groups per call: compression has no walk, so finer groups overlap more;
- * decompression and the add walk each group's headers, whose kernels carry
- * a fixed cost per launch */
-constexpr uint32_t kGroupsCompress = 8, kGroupsDecompress = 8, kGroupsHomadd = 8;
+/* The least elements of a group.  A group costs some ten launches and a
+ * status read, 50 us with a walk, whatever its size, and the host waits for
+ * each copy from pageable memory; only groups whose copies take longer gain by
+ * overlapping.  Compress, add and decompress of 4M floats, pageable: 1360 us
+ * in eight groups, 800 in one; 16M: 2830 and, in two, 2000; pinned 16M 454 +
+ * 546 + 554 and 460 + 538 + 550 (with 2^24: 512 + 551 + 626). */
+constexpr uint64_t kLeastGroup = 1ull << 23;
 
 /* Cached device buffers of the drop-in layer, one set per device. */
 struct DropCtx {
@@ -1051,15 +1054,15 @@ bool overlaps(const void *a, size_t na, const void *b, size_t nb)
 }
 
 /* The chunk groups of a call on geometry g, or none when the call is not
- * worth cutting (one chunk, or fewer than 2^22 elements).  The last group
+ * worth cutting (one chunk, or fewer elements than two groups hold).  The last group
  * holds more chunks than the remainder segment has elements, so its stream
  * splits exactly like the whole one's tail. */
-std::vector<Group> chunk_groups(const ZGeom &g, uint32_t most)
+std::vector<Group> chunk_groups(const ZGeom &g)
 {
     std::vector<Group> out;
     const uint32_t T = g.T;
-    if (T < 2 || g.n < (1ull << 22)) return out;
-    const uint32_t G = std::min<uint32_t>(T, std::min<uint32_t>(most, kMaxGroups));
+    const uint32_t G = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(T, kMaxGroups), g.n / kLeastGroup);
+    if (G < 2) return out;
     std::vector<uint32_t> cut;
     for (uint32_t k = 0; k <= G; k++) cut.push_back((uint32_t)((uint64_t)T * k / G));
     while (cut.size() > 2 && T - cut[cut.size() - 2] <= g.rem) cut.erase(cut.end() - 2);
@@ -1552,7 +1555,7 @@ int dropin_compress(unsigned char *outputBytes, const float *oriData, size_t *ou
     if (!nz_out && !is_device_ptr(oriData) && !is_device_ptr(outputBytes) &&
         !overlaps(outputBytes, (size_t)zg_stream_worst(&g), oriData, 4 * n)) {
         g.fmt = fmt;
-        const std::vector<Group> gr = chunk_groups(g, kGroupsCompress);
+        const std::vector<Group> gr = chunk_groups(g);
         if (!gr.empty()) return pipe_compress(c, outputBytes, oriData, outSize, eb, g, gr);
     }
     if (!is_device_ptr(oriData)) {
@@ -1604,7 +1607,7 @@ int dropin_decompress(float *newData, size_t n, float eb, int L, const unsigned 
     if (!dout && !nz_out && !size_out && !is_device_ptr(cmp) &&
         !overlaps(newData, 4 * n, cmp, (size_t)zg_stream_worst(&g))) {
         g.fmt = fmt;
-        const std::vector<Group> gr = chunk_groups(g, kGroupsDecompress);
+        const std::vector<Group> gr = chunk_groups(g);
         if (!gr.empty()) {
             bool capped = false;
             int rc = pipe_decompress(c, newData, cmp, eb, g, gr, false, &capped);
@@ -1654,7 +1657,7 @@ int dropin_homadd(unsigned char *final_cmp, size_t *final_size, size_t n, float 
     if (!c) return ZCCL_GPU_ECUDA;
     std::lock_guard<std::mutex> lk(c->mu);
     if (!cases_out && !is_device_ptr(final_cmp) && !is_device_ptr(cmp1) && !is_device_ptr(cmp2)) {
-        const std::vector<Group> gr = chunk_groups(g, kGroupsHomadd);
+        const std::vector<Group> gr = chunk_groups(g);
         if (!gr.empty()) {
             bool capped = false;
             int rc = pipe_homadd(c, final_cmp, final_size, cmp1, cmp2, g, gr, false, &capped);

@@ -108,8 +108,9 @@ struct WalkLayout {
 
 size_t ws_clear_bytes(const ZGeom &g) { return 16 + 8 * g.ntiles; }
 
-/* Zero what a call needs zeroed at launch: the tile ticket and the
- * tiles' size words.  The two status words in front of them are left alone,
+/* Zero what a compression or an add needs zeroed at launch (the header walk
+ * and the decompressor use none of it): the tile ticket and the tiles' size
+ * words.  The two status words in front of them are left alone,
  * so errors of earlier calls on the workspace stay visible until
  * zccl_gpu_check() reads and clears them. */
 cudaError_t ws_clear(void *ws, const ZGeom &g, cudaStream_t st)
@@ -301,7 +302,6 @@ extern "C" int zccl_gpu_build_index(zccl_gpu_stream *s, size_t n, int L, int T, 
     ZGeom g;
     if (make_geom(n, L, T, &g) || !valid_stream(s) || !d_ws) return ZCCL_GPU_EINVAL;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     return walk_stream(s, g, d_ws, st);
 }
 
@@ -313,7 +313,6 @@ static int decompress_fmt(float *d_out, zccl_gpu_stream *in, size_t n, float eb,
     if (make_geom(n, L, T, &g) || !valid_stream(in) || !d_out || !d_ws) return ZCCL_GPU_EINVAL;
     g.fmt = fmt;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     ZWork w = bind_ws(d_ws);
     if (!in->indexed) {
         int rc = walk_stream(in, g, d_ws, st);
@@ -354,7 +353,6 @@ extern "C" int zccl_gpu_decompress_accumulate(float *d_acc, const zccl_gpu_strea
         !(eb > 0.0f) || !isfinite(eb))
         return ZCCL_GPU_EINVAL;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     DecompressArgs a;
     memset(&a, 0, sizeof(a));
     a.job.g = g;
@@ -370,7 +368,7 @@ extern "C" int zccl_gpu_decompress_accumulate(float *d_acc, const zccl_gpu_strea
 }
 
 /* The add of P inputs given by their bytes and index arrays (which need
- * not sit in one stream's index layout), on a cleared workspace. */
+ * not sit in one stream's index layout). */
 static int homadd_inputs(zccl_gpu_stream *out, const HomInput *in, int P, int qv, const ZGeom &g, void *d_ws,
                          unsigned long long *d_cases, cudaStream_t st)
 {
@@ -406,7 +404,6 @@ extern "C" int zccl_gpu_homadd_cases(zccl_gpu_stream *out, zccl_gpu_stream *ins,
     for (int p = 0; p < P; p++)
         if (!valid_stream(&ins[p]) || ins[p].bytes == out->bytes) return ZCCL_GPU_EINVAL;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    if (ws_clear(d_ws, g, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     HomInput in[ZH_MAXP];
     int qv = 1;
     for (int p = 0; p < P; p++) {
@@ -674,7 +671,9 @@ extern "C" int zccl_gpu_batch_run(const zccl_gpu_batch *b, void *cuda_stream)
     cudaStream_t st = (cudaStream_t)cuda_stream;
     uint8_t *base = static_cast<uint8_t *>(b->d_mem);
     /* the status words stay until zccl_gpu_batch_check() reads them */
-    if (cudaMemsetAsync(base + 8, 0, b->clear_bytes - 8, st) != cudaSuccess) return ZCCL_GPU_ECUDA;
+    if (b->kind != ZCCL_GPU_BATCH_DECOMPRESS && /* (takes its tiles in a fixed order) */
+        cudaMemsetAsync(base + 8, 0, b->clear_bytes - 8, st) != cudaSuccess)
+        return ZCCL_GPU_ECUDA;
     ZBatch bt;
     bt.jobs = base + b->jobs_off;
     bt.tile_job = reinterpret_cast<const uint16_t *>(base + b->map_off);
@@ -1484,7 +1483,7 @@ int pipe_homadd(DropCtx *c, unsigned char *out, size_t *out_size, const unsigned
             both.index = c->lix[l][0].p;
             both.indexed = 0;
             both.qprev_valid = 0;
-            if (cudaStreamWaitEvent(st, c->ev_in[k], 0) != cudaSuccess || ws_clear(ws, gc[k], st) != cudaSuccess) {
+            if (cudaStreamWaitEvent(st, c->ev_in[k], 0) != cudaSuccess) {
                 rc = ZCCL_GPU_ECUDA;
                 break;
             }
@@ -1514,8 +1513,7 @@ int pipe_homadd(DropCtx *c, unsigned char *out, size_t *out_size, const unsigned
             if (st2 != st && pl.next + NL == k + 1 && (rc = pl.place(st2))) break;
             if (cudaStreamWaitEvent(st, c->ev_in[k], 0) != cudaSuccess ||
                 cudaStreamWaitEvent(st2, c->ev_in[k], 0) != cudaSuccess ||
-                (k >= NL && cudaStreamWaitEvent(st2, c->ev_k[k - NL], 0) != cudaSuccess) ||
-                ws_clear(ws, q.g, st) != cudaSuccess || ws_clear(ws2, q.g, st2) != cudaSuccess) {
+                (k >= NL && cudaStreamWaitEvent(st2, c->ev_k[k - NL], 0) != cudaSuccess)) {
                 rc = ZCCL_GPU_ECUDA;
                 break;
             }
@@ -1678,7 +1676,6 @@ int dropin_homadd(unsigned char *final_cmp, size_t *final_size, size_t n, float 
         /* the first input's index walk runs while the second input is
          * copied on the other stream; then the second's walk, a check of
          * both, and the add of the indexed inputs */
-        if (ws_clear(c->ws.p, g, c->st) != cudaSuccess) return ZCCL_GPU_ECUDA;
         if (int rc = stage_stream(c, 0, cmp1, g, &in[0], pass > 0, &cap1)) return rc;
         if (int rc = walk_stream(&in[0], g, c->ws.p, c->st)) return rc;
         if (int rc = stage_stream(c, 1, cmp2, g, &in[1], pass > 0, &cap2, c->st2)) return rc;

@@ -1895,8 +1895,6 @@ cudaError_t sz3_decompress(float *y, const uint8_t *in, uint64_t avail, uint64_t
 {
     const Sz3Dims g = sz3_dims(d1, d2, d3, bs);
     const Sz3Ws w = sz3_bind(ws, g);
-    cudaError_t e = cudaMemsetAsync(w.err + 2, 0, 8, st); /* the ticket; status words stay until checked */
-    if (e != cudaSuccess) return e;
     uint32_t *vol = reinterpret_cast<uint32_t *>(y);
     const Sz3Split twice = sz3_split(eb * 2);
     if (sz3_rows(bs))
@@ -1904,7 +1902,8 @@ cudaError_t sz3_decompress(float *y, const uint8_t *in, uint64_t avail, uint64_t
                : bs == 4 ? sz3_decompress_rows<4>(in, avail, g, w, vol, twice, st)
                          : sz3_decompress_rows<8>(in, avail, g, w, vol, twice, st);
     k_sz3_sizes<<<grid_for(g.nblocks, 256), 256, 0, st>>>(in, avail, g, w.sizes, w.err);
-    if ((e = sz3_scan(g, w, g.nblocks, st)) != cudaSuccess) return e;
+    const cudaError_t e = sz3_scan(g, w, g.nblocks, st);
+    if (e != cudaSuccess) return e;
     if (bs * bs * bs <= 512)
         k_sz3_unpack<32><<<grid_for(g.nblocks, SZ_THREADS / 32), SZ_THREADS, 0, st>>>(in, avail, g, w.offs, vol, w.err);
     else

@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
         const bool own = lane < nblk;
         const uint32_t n = !own ? 0u : b0 + lane + 1u < tb ? L : D.nlast;
         uint32_t b = 0, smask = 0, m[32];
+        uint32_t ints = 0; /* not L32, bit i: octet i's magnitudes are integers, without the float form's exponent above them */
         int32_t q0 = 0; /* lane 0: the value before the group */
 
         if (L32) {
@@ -304,8 +305,10 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
                 for (uint32_t j = 0; j < 9; j++) x[j] = nblk || warp == 0 ? lin[D.at + min(e + j, end)] : 0.f;
                 uint32_t mi[8], s8, mx;
                 int32_t qi;
-                if (__builtin_expect(!quantize_deltas<8>(x, inv, mi, s8, mx, qi), 0))
+                if (__builtin_expect(!quantize_deltas<8>(x, inv, mi, s8, mx, qi), 0)) {
                     quantize_exact<8>([&](int j) { return x[j]; }, inv, mi, s8, mx, qi, bad);
+                    ints |= 1u << i;
+                }
                 if (!has) mx = 0;
                 if (i == 0) q0 = qi;
 #pragma unroll
@@ -362,6 +365,11 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
                     uint32_t mi[8];
 #pragma unroll
                     for (int j = 0; j < 8; j++) mi[j] = 8u * og + (uint32_t)j < nk ? m[8 * i + j] : 0u;
+                    /* another octet may have made the block so wide that bits from the 24th on are packed */
+                    if (__builtin_expect((e & 0xFFu) >= 24u && !((ints >> i) & 1u), 0)) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) mi[j] &= 0x7FFFFFu;
+                    }
                     encode_octet(pk, e >> 8, e & 0xFFu, nk, og, (smask >> (8 * i)) & 0xFFu, mi, fmt);
                 }
             }

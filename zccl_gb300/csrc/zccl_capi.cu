@@ -122,9 +122,9 @@ WalkLayout walk_layout(const ZGeom &g)
 {
     WalkLayout l;
     l.M = zg_block_bytes(32, g.L);
-    l.max_windows = (uint32_t)(zg_stream_worst(&g) / WALK_WW + g.T + 2);
+    l.max_windows = walk_max_windows(&g);
+    l.max_groups = walk_max_groups(&g);
     const uint32_t G = walk_group(l.M);
-    l.max_groups = (l.max_windows + G - 1) / G + g.T + 1;
     size_t o = align16(ws_clear_bytes(g));
     l.seg_P = o; o = align16(o + 8ull * g.T);
     l.seg_R = o; o = align16(o + 8ull * g.T);

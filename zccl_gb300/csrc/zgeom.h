@@ -25,6 +25,8 @@
 
 #include <stdint.h>
 
+#include "zccl_err.h"
+
 #ifdef __CUDACC__
 #define ZG_HD __host__ __device__ __forceinline__
 #else
@@ -200,6 +202,61 @@ ZG_HD uint64_t zg_seg_worst(uint64_t len, uint32_t L)
 ZG_HD uint64_t zg_stream_worst(const ZGeom *g)
 {
     return 8ull * g->T + (uint64_t)g->T * zg_seg_worst(g->tbs, g->L) + zg_seg_worst(g->rem, g->L);
+}
+
+/* The header walk of a stream without an index reads every chunk's bytes in
+ * windows of WALK_WW bytes, which it handles in groups. */
+#define WALK_WW 2048u /* bytes per window */
+#define WALK_GMAX 64u /* windows per group at most */
+
+/* Windows per group: as many (a power of two) as their tables of M words fit
+ * 128 KB of shared memory. */
+ZG_HD uint32_t walk_group(uint32_t M)
+{
+    uint32_t G = WALK_GMAX;
+    while (G > 1 && G * M * 4u > 128u * 1024u) G >>= 1;
+    return G;
+}
+
+/* Windows of a chunk whose blocks lie in bytes [P, R). */
+ZG_HD uint32_t walk_windows(uint64_t P, uint64_t R) { return (uint32_t)zg_div_up(R - P, WALK_WW); }
+
+/* Most windows, and most groups of them, that the chunks of one header have:
+ * walk_chunk takes no chunk above its worst size, and every chunk may end in
+ * a part of a window and of a group. */
+ZG_HD uint32_t walk_max_windows(const ZGeom *g) { return (uint32_t)(zg_stream_worst(g) / WALK_WW + g->T + 2); }
+
+ZG_HD uint32_t walk_max_groups(const ZGeom *g)
+{
+    const uint32_t G = walk_group(zg_block_bytes(32, g->L));
+    return (walk_max_windows(g) + G - 1) / G + g->T + 1;
+}
+
+/* Chunk s of a stream of `avail` readable bytes, none of them used from
+ * end_bound on, whose header gives its offset `rel` and the next chunk's
+ * `next` (s + 1 < T): *P its first block's byte, *R the end of the bytes its
+ * blocks may take.  ZERR_* bits, 0 for a chunk that can be walked.  No chunk
+ * takes more than a segment's worst size: a header whose offsets do not
+ * increase could otherwise give many chunks the same bytes, and more windows
+ * than walk_max_windows(). */
+ZG_HD uint32_t walk_chunk(const ZGeom *g, uint32_t s, uint64_t rel, uint64_t next, uint64_t avail, uint64_t end_bound,
+                          uint64_t *P, uint64_t *R)
+{
+    const uint64_t hdr = 8ull * g->T;
+    uint32_t bad = s == 0 && rel != 0 ? ZERR_CORRUPT : 0u;
+    *P = *R = 0;
+    if (hdr > avail || rel > avail - hdr || hdr + rel + 4 > avail) return bad | ZERR_BOUNDS;
+    const uint64_t worst = hdr + rel + zg_seg_worst(g->tbs, g->L); /* where its blocks end at the latest */
+    *P = hdr + rel + 4;
+    if (s + 1 < g->T) {
+        *R = hdr + next;
+        if (next > avail - hdr || *R < *P || *R > end_bound || *R > worst) bad |= ZERR_CORRUPT;
+    } else { /* no later start bounds it (a remainder segment follows it and is walked apart) */
+        *R = avail < end_bound ? avail : end_bound;
+        if (*R > worst) *R = worst;
+        if (*R < *P) *R = *P;
+    }
+    return bad;
 }
 
 ZG_HD uint32_t zg_a16(uint32_t v) { return (v + 15u) & ~15u; }

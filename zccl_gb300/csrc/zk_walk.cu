@@ -90,39 +90,16 @@ __global__ void k_walk_setup(const WalkArgs a)
         const uint32_t s = s0 + threadIdx.x;
         uint32_t nwin = 0;
         if (s < g.T) {
-            uint64_t P = 0, R = 0;
-            bool ok = hdr <= a.avail;
-            if (!ok) atomicOr(a.err, ZERR_BOUNDS);
-            if (ok) {
-                uint64_t rel = load_u64(a.in + 8ull * s);
-                if (s == 0 && rel != 0) atomicOr(a.err, ZERR_CORRUPT);
-                if (rel > a.avail - hdr || hdr + rel + 4 > a.avail) {
-                    atomicOr(a.err, ZERR_BOUNDS);
-                    ok = false;
-                } else {
-                    a.idx.grp_off[(uint64_t)s * g.gr_reg] = hdr + rel;
-                    P = hdr + rel + 4;
-                    if (s + 1 < g.T) {
-                        uint64_t rn = load_u64(a.in + 8ull * (s + 1));
-                        R = hdr + rn;
-                        /* chunk starts increase and a stream never exceeds end_bound,
-                         * which keeps the window count within the scratch */
-                        if (rn > a.avail - hdr || R < P || R > a.end_bound) {
-                            atomicOr(a.err, ZERR_CORRUPT);
-                            ok = false;
-                        }
-                    } else {
-                        /* the last chunk: no later start bounds it, but its
-                         * blocks take at most a segment's worst size (a
-                         * remainder segment follows them and is walked apart) */
-                        R = a.avail < a.end_bound ? a.avail : a.end_bound;
-                        const uint64_t worst = P - 4 + zg_seg_worst(g.tbs, g.L);
-                        if (R > worst) R = worst;
-                        if (R < P) R = P;
-                    }
-                }
+            uint64_t P, R, rel = 0, next = 0;
+            if (hdr <= a.avail) {
+                rel = load_u64(a.in + 8ull * s);
+                if (s + 1 < g.T) next = load_u64(a.in + 8ull * (s + 1));
             }
-            if (ok && g.nb_reg > 0) nwin = (uint32_t)zg_div_up(R - P, WALK_WW);
+            const uint32_t bad = walk_chunk(&g, s, rel, next, a.avail, a.end_bound, &P, &R);
+            bool ok = !bad;
+            if (bad) atomicOr(a.err, bad);
+            if (ok) a.idx.grp_off[(uint64_t)s * g.gr_reg] = hdr + rel;
+            if (ok && g.nb_reg > 0) nwin = walk_windows(P, R);
             if (ok && g.nb_reg > 0 && nwin == 0) {
                 atomicOr(a.err, ZERR_BOUNDS);
                 ok = false;

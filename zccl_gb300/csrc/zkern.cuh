@@ -122,18 +122,6 @@ struct HomAddArgs {
     uint32_t in_ring, in_bytes, ring; /* shared bytes of the input ring, with slack, and of the output ring (filled by the launcher) */
 };
 
-#define WALK_WW 2048u /* bytes per window of the parallel header walk */
-#define WALK_GMAX 64u  /* windows per group at most */
-
-/* Windows per group: as many (a power of two) as their tables of M words fit
- * 128 KB of shared memory. */
-ZG_HD uint32_t walk_group(uint32_t M)
-{
-    uint32_t G = WALK_GMAX;
-    while (G > 1 && G * M * 4u > 128u * 1024u) G >>= 1;
-    return G;
-}
-
 /* Device scratch of the header walk (part of the workspace). */
 struct WalkScratch {
     uint64_t *seg_P;    /* [T]   first block byte of each regular segment */

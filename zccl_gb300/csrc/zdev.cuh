@@ -265,8 +265,8 @@ __device__ __forceinline__ void decode_add_any(const uint32_t *w, uint32_t o, ui
  * as floats, their signs in sg (element j at bit 31 - j): each(j, m, sg) for
  * all 32, garbage from element n on.  The same instructions for every
  * such width, so a warp whose blocks mix them does not split; a zero-width
- * block reads (and discards) what follows its header.  Reads up to 150 bytes
- * past a block's first byte (buffers carry slack). */
+ * block reads (and discards) what follows its header.  All 32 elements are
+ * read, whatever n: see zg_lane_slack. */
 template <class Each>
 __device__ __forceinline__ void decode_small_f(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, Each each)
 {
@@ -413,7 +413,8 @@ __device__ __forceinline__ void quantize_exact(X x, float inv, uint32_t (&m)[N],
  *     by funnel shifts; for B = 0 the byte permute selects a zero byte, so
  *     lanes whose blocks mix B = 0 and 1 take the same instructions, and a
  *     zero-width block reads (and discards) whatever follows its header.
- * Reads up to n / 8 + 8G + 20 bytes past a block's end (buffers carry slack). */
+ * Reads up to zg_octet_slack(L) bytes past a block's end (a lane whose octet is
+ * past it reads octet 0). */
 __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, uint32_t g,
                                              uint32_t fmt, uint32_t (&d)[8])
 {
@@ -423,8 +424,9 @@ __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint
         r = 0;
     }
     const uint32_t ns = (n + 7u) >> 3; /* a segment's last block may be shorter than L */
-    const uint32_t sg = (uint32_t)reinterpret_cast<const uint8_t *>(w)[o + 1u + g] << 24; /* element k: bit 31 - k */
-    const uint32_t hb = o + 1u + ns, la = hb + B * n + g * r;
+    const uint32_t gr = 8u * g < n ? g : 0u; /* the octet that is read */
+    const uint32_t sg = (uint32_t)reinterpret_cast<const uint8_t *>(w)[o + 1u + gr] << 24; /* element k: bit 31 - k */
+    const uint32_t hb = o + 1u + ns, la = hb + B * n + gr * r;
     uint32_t F0, F1;
     {
         const uint32_t k = la >> 2, sh = (la & 3u) * 8u;
@@ -441,14 +443,14 @@ __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint
         d[k] = (m ^ s) - s;
     };
     if (B <= 1) {
-        const uint32_t a = hb + 8u * g, k0 = a >> 2, sh = (a & 3u) * 8u;
+        const uint32_t a = hb + 8u * gr, k0 = a >> 2, sh = (a & 3u) * 8u;
         const uint32_t w0 = w[k0], w1 = w[k0 + 1], w2 = w[k0 + 2];
         const uint32_t A0 = __funnelshift_r(w0, w1, sh), A1 = __funnelshift_r(w1, w2, sh);
         const uint32_t zsel = B ? 0x4440u : 0x4444u; /* selector nibble 4: a byte of the zero operand */
 #pragma unroll
         for (int k = 0; k < 8; k++) put(k, __byte_perm(k < 4 ? A0 : A1, 0, B ? 0x4440u | (uint32_t)(k & 3) : zsel));
     } else if (B == 2) {
-        const uint32_t a = hb + 16u * g, k0 = a >> 2, sh = (a & 3u) * 8u;
+        const uint32_t a = hb + 16u * gr, k0 = a >> 2, sh = (a & 3u) * 8u;
         uint32_t prev = w[k0];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -462,7 +464,7 @@ __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint
         const uint32_t bmask = B >= 4 ? 0xFFFFFFFFu : 0xFFFFFFu;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            const uint32_t a = hb + (8u * g + (uint32_t)k) * B;
+            const uint32_t a = hb + (8u * gr + (uint32_t)k) * B;
             put(k, __funnelshift_r(w[a >> 2], w[(a >> 2) + 1], (a & 3u) * 8u) & bmask);
         }
     }
@@ -472,9 +474,6 @@ __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint
             if (8u * g + (uint32_t)k >= n) d[k] = 0;
     }
 }
-
-/* Bytes decode_octet may read past the last byte of a tile's last block. */
-__host__ __device__ __forceinline__ uint32_t octet_slack(uint32_t L) { return (L + 7u) / 8u + 8u * ((L + 7u) / 8u) + 24u; }
 
 /* v (its low bytes first) ORed into the zeroed buffer from byte at on. */
 __device__ __forceinline__ void or_bytes(uint32_t sbase, uint32_t at, uint64_t v)

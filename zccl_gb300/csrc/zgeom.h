@@ -264,6 +264,12 @@ ZG_HD uint32_t zg_a16(uint32_t v) { return (v + 15u) & ~15u; }
 /* Largest tile in bytes: head + TB blocks at width 32. */
 ZG_HD uint32_t zg_tile_worst(uint32_t L, uint32_t TB) { return TB * zg_block_bytes(32, L) + 4u; }
 
+/* Bytes past a tile's last block that its decoders may read, and discard:
+ * decode_octet (eight elements a lane), and the forms that take 32 elements a
+ * lane also of a short block (its first bytes, then 31 elements of four bytes). */
+ZG_HD uint32_t zg_octet_slack(uint32_t L) { return (L + 7u) / 8u + 8u * ((L + 7u) / 8u) + 24u; }
+ZG_HD uint32_t zg_lane_slack(void) { return 136u; }
+
 /* Bytes a packed tile of `total` bytes takes in the output ring (its bytes,
  * the packer's zeroed tail, 16-byte granularity), and the ring's size: the
  * largest tile fits; readers may look 32 bytes past a tile, so the region

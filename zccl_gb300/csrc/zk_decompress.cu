@@ -426,7 +426,7 @@ cudaError_t launch_decompress(const DecompressArgs &a0, cudaStream_t st)
     /* two typical tiles (at least one of the largest), room for the reads
      * past a tile's end, and the floats */
     a.room = zg_a16(zg_tile_worst(L, a.job.g.TB) + 15u);
-    a.in_bytes = (a.room + octet_slack(L) + 127u) / 128u * 128u;
+    a.in_bytes = (a.room + zg_octet_slack(L) + 127u) / 128u * 128u;
     const size_t smem = DEC_HEAD + a.in_bytes + DEC_WARPS * ((GB * L + 31u) / 32u * 128u);
     const bool batch = a.batch.jobs != nullptr;
     const uint64_t tiles = batch ? a.batch.ntiles : a.job.g.ntiles;

@@ -464,7 +464,7 @@ cudaError_t launch_homadd(const HomAddArgs &a0, cudaStream_t st)
     /* two CTAs share an SM (registers allow no more): the ring takes the
      * shared memory they leave */
     a.in_ring = 2u * zg_a16(zg_tile_worst(L, TB) + 15u);
-    a.in_bytes = zg_a16(a.in_ring + octet_slack(L)); /* and room for reads past a block's end */
+    a.in_bytes = zg_a16(a.in_ring + (L == 32 ? zg_lane_slack() : zg_octet_slack(L))); /* and room for reads past a block's end */
     const uint32_t fixed = ADD_HEAD + a.in_bytes + 48u;
     a.ring = ring_bytes(2, fixed, zg_ring_bytes(L, TB));
     const size_t smem = fixed + a.ring;

@@ -1880,10 +1880,7 @@ cudaError_t sz3_compress(uint8_t *out, uint64_t cap, const float *x, uint64_t d1
             w.q, g, out, cap, w.offs, w.err);
     } else {
         const size_t smem = 4ull * bs * bs * bs;
-        if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(k_sz3_pack<SZ_THREADS>,
-                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                                    cudaSuccess)
-            return e;
+        if ((e = set_max_smem((const void *)k_sz3_pack<SZ_THREADS>, smem)) != cudaSuccess) return e;
         k_sz3_pack<SZ_THREADS><<<grid_for(g.nblocks, 1), SZ_THREADS, smem, st>>>(w.q, g, out, cap, w.offs, w.err);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

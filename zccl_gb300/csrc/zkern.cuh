@@ -9,10 +9,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <mutex>
-
 #include "zdev.cuh"
 #include "zgeom.h"
+#include "zlaunch.h"
 
 #define ZH_MAXP 32 /* most inputs one homomorphic-add launch accepts */
 
@@ -423,134 +422,6 @@ __device__ __forceinline__ uint32_t octet_max(uint32_t v, uint32_t og, uint32_t 
         if (og + s < G) v = max(v, u);
     }
     return __shfl_sync(0xffffffffu, v, src);
-}
-
-/* Launch-shape queries, remembered per device and kernel: the occupancy
- * calculator and the shared-memory attribute cost host time on every
- * launch, and a pipelined host-buffer call launches a hundred kernels. */
-struct LaunchCache {
-    struct Occ {
-        const void *fn;
-        int dev, threads, per;
-        size_t smem;
-    };
-    struct Attr {
-        const void *fn;
-        int dev;
-        size_t smem;
-    };
-    std::mutex mu;
-    Occ occ[96];
-    Attr attr[64];
-    int nocc = 0, nattr = 0;
-    int nsm[64] = {0}, smem_sm[64] = {0}, smem_rsv[64] = {0};
-};
-
-static inline LaunchCache &launch_cache()
-{
-    static LaunchCache c;
-    return c;
-}
-
-/* Blocks of fn per SM at this block size and shared memory (at least 1). */
-static inline int blocks_per_sm(const void *fn, int threads, size_t smem)
-{
-    LaunchCache &c = launch_cache();
-    int dev = 0;
-    cudaGetDevice(&dev);
-    {
-        std::lock_guard<std::mutex> lk(c.mu);
-        for (int i = 0; i < c.nocc; i++)
-            if (c.occ[i].fn == fn && c.occ[i].dev == dev && c.occ[i].threads == threads && c.occ[i].smem == smem)
-                return c.occ[i].per;
-    }
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        per = 0;
-    }
-    if (per < 1) per = 1;
-    std::lock_guard<std::mutex> lk(c.mu);
-    if (c.nocc < 96) c.occ[c.nocc++] = {fn, dev, threads, per, smem};
-    return per;
-}
-
-/* SMs of the current device. */
-static inline int sm_count()
-{
-    LaunchCache &c = launch_cache();
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && c.nsm[dev] > 0) return c.nsm[dev];
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
-        cudaGetLastError();
-        return 1;
-    }
-    if (dev >= 0 && dev < 64) c.nsm[dev] = n;
-    return n;
-}
-
-/* cudaFuncSetAttribute(fn, MaxDynamicSharedMemorySize, smem), skipped when
- * an equal or larger value is already set for fn on this device. */
-static inline cudaError_t set_max_smem(const void *fn, size_t smem)
-{
-    LaunchCache &c = launch_cache();
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(c.mu); /* held while setting: a call that wants less must not undo one that wants more */
-    int i = 0;
-    while (i < c.nattr && !(c.attr[i].fn == fn && c.attr[i].dev == dev)) i++;
-    if (i < c.nattr && c.attr[i].smem >= smem) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (i < c.nattr)
-        c.attr[i].smem = smem;
-    else if (c.nattr < 64)
-        c.attr[c.nattr++] = {fn, dev, smem};
-    return cudaSuccess;
-}
-
-/* Ring bytes of a kernel that runs `per_sm` CTAs per SM and needs `fixed`
- * other bytes of shared memory: at least `least` (one worst-case tile), and
- * up to the CTA's share of the SM's shared memory less a kilobyte of margin.
- * The longer the ring, the longer a tile may wait there for its place
- * before the compute warps run out of room. */
-static inline uint32_t ring_bytes(uint32_t per_sm, uint32_t fixed, uint32_t least)
-{
-    LaunchCache &c = launch_cache();
-    int dev = 0, sm = 0, rsv = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && c.smem_sm[dev] > 0) {
-        sm = c.smem_sm[dev];
-        rsv = c.smem_rsv[dev];
-    } else if (cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-               cudaDeviceGetAttribute(&rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
-        cudaGetLastError();
-        return least;
-    } else if (dev >= 0 && dev < 64) {
-        c.smem_rsv[dev] = rsv;
-        c.smem_sm[dev] = sm;
-    }
-    const int share = sm / (int)per_sm - rsv - 1024 - (int)fixed;
-    return share > (int)least ? (uint32_t)share & ~15u : least;
-}
-
-static inline unsigned persistent_grid(const void *fn, int threads, size_t smem, uint64_t ntiles)
-{
-    const uint64_t g = (uint64_t)sm_count() * (uint64_t)blocks_per_sm(fn, threads, smem);
-    return (unsigned)(g < ntiles ? g : ntiles);
-}
-
-/* Grid of a kernel whose tiles' places come from the scanning CTA: `want`
- * working CTAs (0: as many as fit, at most one per tile) and, with more than
- * one tile, the scanner. */
-static inline unsigned scanned_grid(const void *fn, int threads, size_t smem, uint64_t ntiles, unsigned want)
-{
-    unsigned g = persistent_grid(fn, threads, smem, ntiles + 1);
-    if (ntiles == 1) return 1;
-    if (g < 2) g = 2;
-    return want && want + 1 < g ? want + 1 : g;
 }
 
 /* Launchers; each returns the cudaError_t of the launch. */

@@ -414,7 +414,8 @@ __device__ __forceinline__ void quantize_exact(X x, float inv, uint32_t (&m)[N],
  *     lanes whose blocks mix B = 0 and 1 take the same instructions, and a
  *     zero-width block reads (and discards) whatever follows its header.
  * Reads up to zg_octet_slack(L) bytes past a block's end (a lane whose octet is
- * past it reads octet 0). */
+ * past it reads octet 0; INSIDE: there is none). */
+template <bool INSIDE = false>
 __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint32_t b, uint32_t n, uint32_t g,
                                              uint32_t fmt, uint32_t (&d)[8])
 {
@@ -424,7 +425,7 @@ __device__ __forceinline__ void decode_octet(const uint32_t *w, uint32_t o, uint
         r = 0;
     }
     const uint32_t ns = (n + 7u) >> 3; /* a segment's last block may be shorter than L */
-    const uint32_t gr = 8u * g < n ? g : 0u; /* the octet that is read */
+    const uint32_t gr = INSIDE || 8u * g < n ? g : 0u; /* the octet that is read */
     const uint32_t sg = (uint32_t)reinterpret_cast<const uint8_t *>(w)[o + 1u + gr] << 24; /* element k: bit 31 - k */
     const uint32_t hb = o + 1u + ns, la = hb + B * n + gr * r;
     uint32_t F0, F1;

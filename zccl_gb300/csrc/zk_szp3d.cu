@@ -363,8 +363,10 @@ __global__ void __launch_bounds__(1024) k_sz3_scan_sums(uint64_t *sums, uint64_t
     if (threadIdx.x == 0) *total = head + carry;
 }
 
+/* sums: the chunks' exclusive sums; null for a single chunk, whose *total (all
+ * bytes, with the rate table's `head`) is found here. */
 __global__ void __launch_bounds__(1024) k_sz3_offsets(const uint32_t *sizes, uint64_t nb, const uint64_t *sums,
-                                                      uint64_t *offs)
+                                                      uint64_t *offs, uint64_t head, uint64_t *total)
 {
     __shared__ uint64_t ws[33];
     const uint64_t c = blockIdx.x, lo = c * SZ_CHUNK;
@@ -394,7 +396,8 @@ __global__ void __launch_bounds__(1024) k_sz3_offsets(const uint32_t *sizes, uin
         ws[lane] = ti - t;
     }
     __syncthreads();
-    uint64_t run = sums[c] + ws[warp] + inc - s;
+    uint64_t run = (sums ? sums[c] : 0) + ws[warp] + inc - s;
+    if (!sums && threadIdx.x == blockDim.x - 1) *total = head + run + s;
     for (uint32_t r = 0; r < per; r++) {
         const uint64_t i = lo + (uint64_t)threadIdx.x * per + r;
         if (i < nb) offs[i] = run;
@@ -1133,25 +1136,37 @@ __global__ void __launch_bounds__(SZ_THREADS) k_sz3_chunk_sizes(const uint8_t *_
     if (flag) atomicOr(err, flag);
 }
 
-/* Where a CTA is in its chunks: one of every strip of it at a time. */
-template <uint32_t BS>
+/* How a volume's chunks go to CTAs: a task is a part of STRIPS strips and one
+ * of nseg pieces of it along z. */
+struct Sz3Tasks {
+    uint64_t ntasks, nparts, nbg, nseg;
+    uint64_t seg; /* blocks along z in a piece: a multiple of 32 */
+};
+
+/* Where a CTA is in its chunks: one of every strip of it at a time.  PIECES:
+ * the strips are cut along z. */
+template <uint32_t BS, bool PIECES>
 struct Sz3Pos {
-    uint64_t task, ntasks, nparts, nbg;
-    uint64_t cb, bj, bj1, bi0;
+    Sz3Tasks t;
+    uint64_t task;
+    uint64_t cb, cb1, bj, bj1, bi0;
+    __device__ __forceinline__ uint64_t strips() const { return PIECES ? task / t.nseg : task; } /* the task's, in all */
+    __device__ __forceinline__ uint64_t first() const { return strips() % t.nparts * Sz3Un<BS>::PARTS; }
     __device__ __forceinline__ void begin(const Sz3Dims &g)
     {
-        if (task >= ntasks) return;
-        bi0 = (nbg - 1 - task / nparts) * Sz3Un<BS>::STRIPS;
-        bj = (task % nparts) * Sz3Un<BS>::PARTS;
+        if (task >= t.ntasks) return;
+        bi0 = (t.nbg - 1 - strips() / t.nparts) * Sz3Un<BS>::STRIPS;
+        bj = first();
         bj1 = min(bj + Sz3Un<BS>::PARTS, g.nb2);
-        cb = 0;
+        cb = PIECES ? task % t.nseg * t.seg : 0;
+        cb1 = PIECES ? min(cb + t.seg, g.nb3) : g.nb3;
     }
     __device__ __forceinline__ void advance(const Sz3Dims &g)
     {
         if (++bj < bj1) return;
         cb += 32;
-        if (cb < g.nb3) {
-            bj = (task % nparts) * Sz3Un<BS>::PARTS;
+        if (cb < (PIECES ? cb1 : g.nb3)) {
+            bj = first();
             return;
         }
         task += gridDim.x;
@@ -1162,10 +1177,10 @@ struct Sz3Pos {
 /* Producer, sides 2 and 4: lane s sends strip s's chunk and lane STRIPS + s
  * its rates, from which the strip's consumers place its blocks; the next
  * chunk's place is on its way meanwhile. */
-template <uint32_t BS>
+template <uint32_t BS, bool PIECES>
 __device__ __forceinline__ void sz3_produce_small(const uint8_t *__restrict__ in, uint64_t avail, const Sz3Dims &g,
                                                   const uint64_t *__restrict__ offs, const uint32_t *__restrict__ sizes,
-                                                  uint8_t *slots, uint64_t *full, uint64_t *empty, Sz3Pos<BS> p, uint32_t *err)
+                                                  uint8_t *slots, uint64_t *full, uint64_t *empty, Sz3Pos<BS, PIECES> p, uint32_t *err)
 {
     using U = Sz3Un<BS>;
     const uint32_t lane = threadIdx.x & 31u, s = lane % U::STRIPS;
@@ -1175,7 +1190,7 @@ __device__ __forceinline__ void sz3_produce_small(const uint8_t *__restrict__ in
         const uint64_t bi = p.bi0 + s, strip = bi * g.nb2 + p.bj;
         at = avail;
         bytes = 0;
-        if (p.task >= p.ntasks || bi >= g.nb1) return;
+        if (p.task >= p.t.ntasks || bi >= g.nb1) return;
         if (lane < U::STRIPS) {
             at = g.nblocks + offs[strip * nzc + p.cb / 32];
             bytes = sizes[strip * nzc + p.cb / 32];
@@ -1187,7 +1202,7 @@ __device__ __forceinline__ void sz3_produce_small(const uint8_t *__restrict__ in
     uint64_t nat;
     uint32_t nbytes, it = 0;
     fetch(nat, nbytes);
-    for (; p.task < p.ntasks; it++) {
+    for (; p.task < p.t.ntasks; it++) {
         const uint64_t at = nat;
         const uint32_t bytes = at >= avail ? 0u : (uint32_t)min((uint64_t)nbytes, avail - at);
         p.advance(g);
@@ -1202,9 +1217,10 @@ __device__ __forceinline__ void sz3_produce_small(const uint8_t *__restrict__ in
 
 /* Producer, side 8 (one strip): block c at word c (mod 32) of the slot, in as
  * many pieces as it takes. */
+template <bool PIECES>
 __device__ __forceinline__ void sz3_produce8(const uint8_t *__restrict__ in, uint64_t avail, const Sz3Dims &g,
                                              const uint64_t *__restrict__ offs, uint8_t *slots, uint64_t *full,
-                                             uint64_t *empty, Sz3Pos<8> p, uint32_t *err)
+                                             uint64_t *empty, Sz3Pos<8, PIECES> p, uint32_t *err)
 {
     using U = Sz3Un<8>;
     const uint32_t lane = threadIdx.x & 31u;
@@ -1212,13 +1228,13 @@ __device__ __forceinline__ void sz3_produce8(const uint8_t *__restrict__ in, uin
     uint32_t flag = 0, it = 0, nrate = 0;
     uint64_t nbase = 0;
     auto fetch = [&]() { /* the next chunk's rates and place */
-        if (p.task >= p.ntasks) return;
+        if (p.task >= p.t.ntasks) return;
         const uint64_t strip = p.bi0 * g.nb2 + p.bj, at = strip * g.nb3 + p.cb + lane;
         nrate = p.cb + lane < g.nb3 && at < avail ? in[at] : 0u;
         nbase = g.nblocks + offs[strip * nzc + p.cb / 32];
     };
     fetch();
-    while (p.task < p.ntasks) {
+    while (p.task < p.t.ntasks) {
         const uint32_t kb = (uint32_t)min((uint64_t)32, g.nb3 - p.cb);
         const uint32_t sx = (uint32_t)min((uint64_t)8, g.d1 - p.bi0 * 8), sy = (uint32_t)min((uint64_t)8, g.d2 - p.bj * 8);
         const uint32_t sz = lane < kb ? (uint32_t)min((uint64_t)8, g.d3 - (p.cb + lane) * 8) : 0u;
@@ -1303,13 +1319,13 @@ __device__ __forceinline__ void sz3_strip(const Sz3Piece &w, uint32_t (&y)[Sz3Un
         const uint32_t jj = j + rj;
         uint32_t v[8];
         if (WHOLE) {
-            decode_octet(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
+            decode_octet<true>(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
         } else {
 #pragma unroll
             for (uint32_t e = 0; e < 8; e++) v[e] = 0;
             if (jj < NJ && sz) {
                 if (octets) {
-                    decode_octet(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
+                    decode_octet<true>(reinterpret_cast<const uint32_t *>(w.area), off - 1u, rate, n, g0 + jj, ZG_FASTMODE1, v);
                 } else { /* at the volume's end: an element at a time */
 #pragma unroll
                     for (uint32_t e = 0; e < 8; e++) {
@@ -1410,8 +1426,8 @@ __device__ __forceinline__ void sz3_strip(const Sz3Piece &w, uint32_t (&y)[Sz3Un
     __syncwarp();
 }
 
-template <uint32_t BS>
-__global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8_t *__restrict__ in, uint64_t avail, Sz3Dims g,
+template <uint32_t BS, bool PIECES>
+__global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8_t *__restrict__ in, uint64_t avail, Sz3Dims g, Sz3Tasks tk,
                                                                      const uint64_t *__restrict__ offs,
                                                                      const uint32_t *__restrict__ sizes,
                                                                      uint32_t *__restrict__ vol, uint32_t *__restrict__ carry,
@@ -1422,7 +1438,6 @@ __global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8
     extern __shared__ __align__(16) uint8_t sm[];
     __shared__ uint64_t full[U::SLOTS], empty[U::SLOTS];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t nparts = (g.nb2 + U::PARTS - 1) / U::PARTS, nbg = (g.nb1 + U::STRIPS - 1) / U::STRIPS, ntasks = nparts * nbg;
     if (threadIdx.x == 0)
         for (uint32_t i = 0; i < U::SLOTS; i++) {
             mbar_init(full + i, BS == 8 ? 33 : 2 * U::STRIPS);
@@ -1430,16 +1445,14 @@ __global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8
         }
     __syncthreads();
     if (warp == 8) {
-        Sz3Pos<BS> p;
+        Sz3Pos<BS, PIECES> p;
+        p.t = tk;
         p.task = blockIdx.x;
-        p.ntasks = ntasks;
-        p.nparts = nparts;
-        p.nbg = nbg;
         p.begin(g);
         if constexpr (BS == 8)
-            sz3_produce8(in, avail, g, offs, sm, full, empty, p, err);
+            sz3_produce8<PIECES>(in, avail, g, offs, sm, full, empty, p, err);
         else
-            sz3_produce_small<BS>(in, avail, g, offs, sizes, sm, full, empty, p, err);
+            sz3_produce_small<BS, PIECES>(in, avail, g, offs, sizes, sm, full, empty, p, err);
         return;
     }
     const uint32_t s = warp / U::PW;
@@ -1451,15 +1464,17 @@ __global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8
     w.s1 = g.d3;
     w.cs = g.d3;
     uint32_t it = 0, flag = 0;
-    for (uint64_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
-        const uint64_t part = task % nparts, bi = (nbg - 1 - task / nparts) * U::STRIPS + s;
+    for (uint64_t task = blockIdx.x; task < tk.ntasks; task += gridDim.x) {
+        const uint64_t strips = PIECES ? task / tk.nseg : task, z0 = PIECES ? task % tk.nseg * tk.seg : 0;
+        const uint64_t part = strips % tk.nparts, bi = (tk.nbg - 1 - strips / tk.nparts) * U::STRIPS + s;
         const uint64_t bj0 = part * U::PARTS, bj1 = min(bj0 + U::PARTS, g.nb2), i0 = bi * BS + w.di0;
+        const uint64_t z1 = PIECES ? min(z0 + tk.seg, g.nb3) : g.nb3;
         w.sx = bi < g.nb1 ? (uint32_t)min((uint64_t)BS, g.d1 - bi * BS) : 0u;
-        for (uint64_t c0 = 0; c0 < g.nb3; c0 += w.k) {
+        for (uint64_t c0 = z0; c0 < z1; c0 += w.k) {
             uint32_t y[PI * BS]; /* the columns' y sums */
 #pragma unroll
             for (uint32_t e = 0; e < PI * BS; e++) y[e] = 0;
-            w.first = c0 == 0;
+            w.first = c0 == z0;
             for (uint64_t bj = bj0; bj < bj1; bj++, it++) {
                 const uint32_t slot = it % U::SLOTS;
                 const uint8_t *sl = sm + slot * U::SLOT;
@@ -1493,7 +1508,7 @@ __global__ void __launch_bounds__(SZ_UN_THREADS, 3) k_sz3_unpack_sum(const uint8
                     w.zleft = (uint32_t)min(g.d3 - c0 * BS, (uint64_t)(32u * BS));
                     w.zlim = min(w.zleft, w.k * BS);
                     w.o = vol + i0 * w.s0 + bj * BS * w.s1 + c0 * BS + lane;
-                    w.co = part + 1 < nparts && bj + 1 == bj1 ? carry + (part * g.d1 + i0) * g.d3 + c0 * BS + lane : nullptr;
+                    w.co = part + 1 < tk.nparts && bj + 1 == bj1 ? carry + (part * g.d1 + i0) * g.d3 + c0 * BS + lane : nullptr;
                     const bool whole = w.sy == BS && w.zlim == w.k * BS;
                     if (BS < 8 || w.k > 16) {
                         if (whole) sz3_strip<BS, 5, true>(w, y);
@@ -1538,6 +1553,27 @@ __global__ void __launch_bounds__(256) k_sz3_carry(uint32_t *__restrict__ carry,
     }
 }
 
+/* Rows whose z sums start anew in each of nseg pieces of `seg` elements: what is
+ * still to be added to each (pre[row * nseg + s]), the sums at the ends of the
+ * pieces before it, of the row and of the carry's row that belongs to it; a
+ * warp per row of the volume. */
+__global__ void __launch_bounds__(256) k_sz3_piece_sums(const uint32_t *__restrict__ vol, const uint32_t *__restrict__ carry,
+                                                        uint64_t d1, uint64_t d2, uint64_t d3, uint32_t part_rows, uint64_t seg,
+                                                        uint64_t nseg, uint32_t *__restrict__ pre)
+{
+    const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= d1 * d2) return;
+    const uint64_t i = row / d2, part = row % d2 / part_rows;
+    const uint32_t *v = vol + row * d3, *c = part ? carry + ((part - 1) * d1 + i) * d3 : nullptr;
+    uint32_t run = 0;
+    for (uint64_t s0 = 0; s0 < nseg; s0 += 32) {
+        const uint64_t s = s0 + (threadIdx.x & 31u), z = (s + 1) * seg - 1;
+        const uint32_t e = s + 1 < nseg ? v[z] + (c ? c[z] : 0u) : 0u, inc = warp_incl_scan(e);
+        if (s < nseg) pre[row * nseg + s] = run + inc - e;
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+}
+
 /* The last pass: x sums of the volume and the parts' carries, floats in place.
  * A CTA takes a run of up to FQ * 288 consecutive elements of a plane (R whole
  * rows of one part, or a piece of a long row) and walks along x, FQ columns'
@@ -1556,9 +1592,11 @@ struct Sz3Run {
     uint32_t cz;     /* carry elements of a full run */
     uint32_t pb, cb; /* bytes of their places in a stage */
     uint32_t stages;
+    const uint32_t *pre; /* PIECES: what the rows' pieces along z lack (k_sz3_piece_sums) */
+    uint64_t seg, nseg;
 };
 
-template <uint32_t FQ, uint32_t FP>
+template <uint32_t FQ, uint32_t FP, bool PIECES>
 __global__ void __launch_bounds__(FTH + 32) k_sz3_finish(uint32_t *vol, const uint32_t *carry, uint64_t d1,
                                                                 uint64_t d2, uint64_t d3, uint32_t rows, Sz3Run f,
                                                                 Sz3Split twice, uint32_t *err)
@@ -1607,8 +1645,23 @@ __global__ void __launch_bounds__(FTH + 32) k_sz3_finish(uint32_t *vol, const ui
     /* where a copy's first element lies in its 16 bytes: the low bits of its address */
     const uint32_t pv = (uint32_t)(reinterpret_cast<uintptr_t>(p0) >> 2), pc = (uint32_t)(reinterpret_cast<uintptr_t>(c0) >> 2);
     float *o = reinterpret_cast<float *>(p0) + threadIdx.x;
+    const uint32_t *zp[FQ]; /* PIECES: the columns' places in f.pre, in the next plane */
+    if (PIECES) {
+#pragma unroll
+        for (uint32_t q = 0; q < FQ; q++) zp[q] = f.pre + (j0 + at[q] / f.cz) * f.nseg + (z0 + cz[q]) / f.seg;
+    }
     uint32_t slot = 0, round = 0;
     for (uint64_t st = 0; st < nst; st++, o += FP * plane) {
+        uint32_t zv[FP * FQ];
+        if (PIECES) {
+#pragma unroll
+            for (uint32_t pl = 0; pl < FP; pl++)
+#pragma unroll
+                for (uint32_t q = 0; q < FQ; q++) {
+                    zv[pl * FQ + q] = FP * st + pl < d1 ? *zp[q] : 0u;
+                    zp[q] += d2 * f.nseg;
+                }
+        }
         mbar_wait(full + slot, round & 1u, err);
         uint32_t v[FP * FQ];
 #pragma unroll
@@ -1620,7 +1673,7 @@ __global__ void __launch_bounds__(FTH + 32) k_sz3_finish(uint32_t *vol, const ui
                                 ((pc + i * (uint32_t)d3) & 3u);
 #pragma unroll
             for (uint32_t q = 0; q < FQ; q++) /* (a plane that is not there: any value, not written) */
-                v[pl * FQ + q] = run[q] += (more ? e[cz[q]] : 0u) + s[at[q]];
+                v[pl * FQ + q] = run[q] += (more ? e[cz[q]] : 0u) + s[at[q]] + (PIECES ? zv[pl * FQ + q] : 0u);
         }
         __syncwarp();
         if ((threadIdx.x & 31u) == 0) mbar_arrive(empty + slot);
@@ -1738,9 +1791,13 @@ Sz3Ws sz3_bind(void *ws, const Sz3Dims &g)
 cudaError_t sz3_scan(const Sz3Dims &g, const Sz3Ws &w, uint64_t count, cudaStream_t st)
 {
     const uint64_t nch = (count + SZ_CHUNK - 1) / SZ_CHUNK;
+    if (nch == 1) {
+        k_sz3_offsets<<<1, 1024, 0, st>>>(w.sizes, count, nullptr, w.offs, g.nblocks, w.total);
+        return cudaGetLastError();
+    }
     k_sz3_chunk_sums<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, count, w.sums);
     k_sz3_scan_sums<<<1, 1024, 0, st>>>(w.sums, nch, g.nblocks, w.total);
-    k_sz3_offsets<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, count, w.sums, w.offs);
+    k_sz3_offsets<<<(unsigned)nch, 1024, 0, st>>>(w.sizes, count, w.sums, w.offs, g.nblocks, w.total);
     return cudaGetLastError();
 }
 
@@ -1773,22 +1830,54 @@ cudaError_t sz3_compress_rows(uint8_t *out, uint64_t cap, const float *x, const 
     return cudaGetLastError();
 }
 
-/* Bytes of the parts' carries. */
+/* The tasks of a volume: strips are cut along z where there are fewer than half
+ * of SZ_TASKS of them, into pieces that make at most SZ_TASKS tasks (three CTAs
+ * on each of 152 SMs).  Otherwise a task goes along the whole row, and a few long
+ * rows leave the device idle: 8 x 8 x 100000, side 8, 2247 us in whole rows, 54
+ * in pieces; 64 x 64 x 3000, side 4, 193 and 80 (start of the sums in the
+ * decoder: 345 and 113). */
+constexpr uint64_t SZ_TASKS = 456;
+template <uint32_t BS>
+Sz3Tasks sz3_tasks(const Sz3Dims &g)
+{
+    using U = Sz3Un<BS>;
+    Sz3Tasks t;
+    t.nparts = (g.nb2 + U::PARTS - 1) / U::PARTS;
+    t.nbg = (g.nb1 + U::STRIPS - 1) / U::STRIPS;
+    const uint64_t strips = t.nparts * t.nbg, chunks = (g.nb3 + 31) / 32;
+    const uint64_t want = strips < SZ_TASKS ? std::min(chunks, SZ_TASKS / strips) : 1;
+    const uint64_t per = (chunks + want - 1) / want; /* chunks of a piece */
+    t.seg = 32 * per;
+    t.nseg = (chunks + per - 1) / per;
+    t.ntasks = strips * t.nseg;
+    return t;
+}
+
+/* Bytes of the parts' carries, and of what the pieces of the volume's rows
+ * lack: no less than any smaller volume's (the sub-volumes of the OpenMP form
+ * share one scratch), so there are as many pieces as any volume's rows have. */
+template <uint32_t BS>
 size_t sz3_carry_bytes(const Sz3Dims &g)
 {
-    const uint64_t strips = g.bs == 8 ? Sz3Un<8>::PARTS : g.bs == 4 ? Sz3Un<4>::PARTS : Sz3Un<2>::PARTS;
-    return 4 * (size_t)((g.nb2 + strips - 1) / strips - 1) * g.d1 * g.d3;
+    using U = Sz3Un<BS>;
+    const uint64_t crows = ((g.nb2 + U::PARTS - 1) / U::PARTS - 1) * g.d1, chunks = (g.nb3 + 31) / 32;
+    const uint64_t most = SZ_TASKS * U::STRIPS * BS * U::ROWS; /* rows of a task, all tasks' */
+    return 4 * (size_t)(crows * g.d3 + (chunks > 1 ? std::min(g.d1 * g.d2 * chunks, most) : 0));
+}
+
+size_t sz3_carry_bytes(const Sz3Dims &g)
+{
+    return g.bs == 8 ? sz3_carry_bytes<8>(g) : g.bs == 4 ? sz3_carry_bytes<4>(g) : sz3_carry_bytes<2>(g);
 }
 
 template <uint32_t FQ, uint32_t FP>
-cudaError_t sz3_finish(const Sz3Dims &g, uint32_t *vol, const uint32_t *carry, uint32_t rows, const Sz3Split &twice,
+cudaError_t sz3_finish(const Sz3Dims &g, uint32_t *vol, const uint32_t *carry, uint32_t rows, Sz3Run f, const Sz3Split &twice,
                        uint64_t sms, uint32_t *err, cudaStream_t st)
 {
     constexpr uint32_t FCOLS = FQ * FTH;
     /* the most rows a run (they share the carry's row) that leave no SM short of
      * runs: 384^3 with two rows, 192 runs on 152 SMs, 107 us, with one 89; 512^3
      * with two, 256 runs, 176, with one 193 */
-    Sz3Run f;
     auto even = [&](uint64_t runs) { return runs >= 8 * sms || 5 * runs >= 4 * sms * ((runs + sms - 1) / sms); };
     for (f.R = 8; f.R > 1; f.R /= 2) /* a power of two: rows of one part */
         if (f.R * g.d3 <= FCOLS && even((g.d2 + f.R - 1) / f.R)) break;
@@ -1804,9 +1893,10 @@ cudaError_t sz3_finish(const Sz3Dims &g, uint32_t *vol, const uint32_t *carry, u
     /* three CTAs an SM, or four where that takes them all at once */
     f.stages = std::min(8u, std::max(2u, (runs > 3 * sms && runs <= 4 * sms ? 54u : 72u) * 1024u / stage));
     const uint32_t smem = f.stages * stage; /* at most 72 KB; the limit is the same in every call, from any thread */
-    const cudaError_t e = set_max_smem((const void *)k_sz3_finish<FQ, FP>, 72u * 1024u);
+    auto *k = f.pre ? k_sz3_finish<FQ, FP, true> : k_sz3_finish<FQ, FP, false>;
+    const cudaError_t e = set_max_smem((const void *)k, 72u * 1024u);
     if (e != cudaSuccess) return e;
-    k_sz3_finish<FQ, FP><<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, rows, f, twice, err);
+    k<<<(unsigned)runs, nth + 32u, smem, st>>>(vol, carry, g.d1, g.d2, g.d3, rows, f, twice, err);
     return cudaGetLastError();
 }
 
@@ -1819,20 +1909,29 @@ cudaError_t sz3_decompress_rows(const uint8_t *in, uint64_t avail, const Sz3Dims
     const uint64_t nchunks = g.nb1 * g.nb2 * ((g.nb3 + 31) / 32); /* at most nblocks: sizes and offs hold them */
     k_sz3_chunk_sizes<<<grid_for(nchunks, SZ_THREADS / 8), SZ_THREADS, 0, st>>>(in, avail, g, nchunks, w.sizes, w.err);
     if ((e = sz3_scan(g, w, nchunks, st)) != cudaSuccess) return e;
-    const void *fn = (const void *)k_sz3_unpack_sum<BS>;
-    if ((e = set_max_smem(fn, U::SMEM)) != cudaSuccess) return e;
     const uint64_t nsm = (uint64_t)sm_count();
-    const uint64_t nparts = (g.nb2 + U::PARTS - 1) / U::PARTS, tasks = nparts * ((g.nb1 + U::STRIPS - 1) / U::STRIPS);
+    const Sz3Tasks tk = sz3_tasks<BS>(g);
+    auto *unpack = tk.nseg > 1 ? k_sz3_unpack_sum<BS, true> : k_sz3_unpack_sum<BS, false>;
+    const void *fn = (const void *)unpack;
+    if ((e = set_max_smem(fn, U::SMEM)) != cudaSuccess) return e;
     uint32_t *carry = reinterpret_cast<uint32_t *>(w.q);
-    k_sz3_unpack_sum<BS><<<persistent_grid(fn, SZ_UN_THREADS, U::SMEM, tasks), SZ_UN_THREADS, U::SMEM, st>>>(
-        in, avail, g, w.offs, w.sizes, vol, carry, w.err);
+    unpack<<<persistent_grid(fn, SZ_UN_THREADS, U::SMEM, tk.ntasks), SZ_UN_THREADS, U::SMEM, st>>>(
+        in, avail, g, tk, w.offs, w.sizes, vol, carry, w.err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const uint64_t columns = g.d1 * g.d3;
-    if (nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, nparts - 1);
+    const uint64_t columns = g.d1 * g.d3, rows = g.d1 * g.d2;
+    if (tk.nparts > 2) k_sz3_carry<<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(carry, columns, tk.nparts - 1);
+    Sz3Run f = {};
+    if (tk.nseg > 1) {
+        uint32_t *pre = carry + (tk.nparts - 1) * columns;
+        f.pre = pre;
+        f.seg = tk.seg * BS;
+        f.nseg = tk.nseg;
+        k_sz3_piece_sums<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(vol, carry, g.d1, g.d2, g.d3, U::ROWS, f.seg, f.nseg, pre);
+    }
     /* small planes (see k_sz3_finish): 45 x 60, 500 planes, 38 us against 86; 300 x 300 44 against 64;
      * 384 x 384 108 against 90 */
-    return g.d2 * g.d3 <= 800 * nsm ? sz3_finish<1, 8>(g, vol, carry, U::ROWS, twice, nsm, w.err, st)
-                                    : sz3_finish<4, 2>(g, vol, carry, U::ROWS, twice, nsm, w.err, st);
+    return g.d2 * g.d3 <= 800 * nsm ? sz3_finish<1, 8>(g, vol, carry, U::ROWS, f, twice, nsm, w.err, st)
+                                    : sz3_finish<4, 2>(g, vol, carry, U::ROWS, f, twice, nsm, w.err, st);
 }
 
 } // namespace

@@ -1,7 +1,8 @@
 """The 3-D decoder on volumes with few rows of blocks, whose rows are summed in
-pieces along z: rows of one piece's length and around it, pieces with and
+pieces along z (rows of one piece's length and around it, pieces with and
 without the carry of the rows before them, planes of both sizes of the last
-pass, outputs at every phase.  Floats must equal the oracle's bit for bit."""
+pass, outputs at every phase), and on flat volumes, some of which take another
+decoder.  Floats must equal the oracle's bit for bit."""
 from __future__ import annotations
 
 import numpy as np
@@ -40,6 +41,23 @@ def test_rows_in_pieces(port, bs, dims):
             got = buf.cpu().numpy()
             assert np.array_equal(got[p: p + n].view(np.uint32), want)
             assert (got[:p] == 7).all() and (got[p + n:] == 7).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bs", [2, 4, 8])
+@pytest.mark.parametrize("dims", [(1500, 1501, 2), (600, 500, 5), (601, 603, 5), (380, 390, 8), (340, 340, 9), (3001, 3003, 1)])
+def test_flat_volumes(port, bs, dims):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zccl_gb300.szp3d import Szp3D
+    x, eb = volume(dims, False, bs), 1e-3
+    codec = Szp3D(dims, bs)
+    wire = port.szp3d_compress(x, dims, bs, eb)
+    b = torch.from_numpy(np.frombuffer(wire, np.uint8).copy()).cuda()
+    y = codec.decompress(b, eb, avail=len(wire))
+    codec.check()
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), port.szp3d_decompress(wire, dims, bs, eb).view(np.uint32).ravel())
 
 
 @pytest.mark.gpu

@@ -1804,6 +1804,16 @@ cudaError_t sz3_scan(const Sz3Dims &g, const Sz3Ws &w, uint64_t count, cudaStrea
 /* Block sides with the row-mapped kernels. */
 bool sz3_rows(uint32_t bs) { return bs == 2 || bs == 4 || bs == 8; }
 
+/* ... and what their decoder takes: not wide flat volumes in blocks of 4^3, one
+ * or two along z, which leave 30 of its lanes idle.  Side 4, with it and with a
+ * warp a block: 2000 x 2000 x 3 1482 and 775 us, 1500 x 1500 x 6 916 and 572,
+ * 1000 x 1000 x 12 298 and 343, but 100 x 3000 x 3 144 and 297 (few columns to
+ * sum); sides 2 and 8, 2000 x 2000 x 3: 1095 and 1347, 568 and 713. */
+bool sz3_decode_rows(const Sz3Dims &g)
+{
+    return sz3_rows(g.bs) && !(g.bs == 4 && g.nb3 <= 2 && std::min(g.d1, g.d2) * g.d3 >= 3000);
+}
+
 /* One pass; the tiles' sizes and places use the offsets array (8 bytes a
  * block, at least 8 a tile), and the ticket and the scanner's word the last
  * two of the four scratch words before it (the first two are error words the
@@ -1993,7 +2003,7 @@ cudaError_t sz3_decompress(float *y, const uint8_t *in, uint64_t avail, uint64_t
     const Sz3Ws w = sz3_bind(ws, g);
     uint32_t *vol = reinterpret_cast<uint32_t *>(y);
     const Sz3Split twice = sz3_split(eb * 2);
-    if (sz3_rows(bs))
+    if (sz3_decode_rows(g))
         return bs == 2   ? sz3_decompress_rows<2>(in, avail, g, w, vol, twice, st)
                : bs == 4 ? sz3_decompress_rows<4>(in, avail, g, w, vol, twice, st)
                          : sz3_decompress_rows<8>(in, avail, g, w, vol, twice, st);

@@ -342,6 +342,14 @@ __device__ __forceinline__ float max3_abs(float a, float b, float c)
     return d;
 }
 
+/* The same, NaN if one of them is. */
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c)
+{
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 /* 1.0f with the sign of bit 31 of s. */
 __device__ __forceinline__ float sign_of(uint32_t s) { return __uint_as_float((s & 0x80000000u) | 0x3F800000u); }
 

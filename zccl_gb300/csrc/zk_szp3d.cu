@@ -551,87 +551,186 @@ __device__ __forceinline__ uint32_t sz3_unit_sz(const Sz3Dims &g, const Sz3Unit 
     return bk < g.nb3 ? (uint32_t)min((uint64_t)BS, g.d3 - bk * BS) : 0u;
 }
 
-/* row(di, dj, e): the difference at (i0 + di, j0 + dj, z0 + lane) for every
- * lane (meaningless where z0 + lane >= d3); called by the whole warp. */
-template <uint32_t BS, class Row>
-__device__ __forceinline__ void sz3_walk(const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
-                                         const Sz3Unit &k, uint32_t &bad, Row row)
+constexpr float SZ_MAGIC = 12582912.0f;         /* 1.5 * 2^23: a float m + this holds the integer m in its low bits, */
+constexpr uint32_t SZ_ZERO = 0x4B400000u;       /* as this + m */
+
+/* The unit's rows again, from memory: planes i0 - 1 .. and rows j0 - 1 .. of
+ * each, z0 + lane, and in lane r the element before z0 of row r, zeros outside
+ * the volume; plane(pl, v, l) for all BS + 1 planes, by the whole warp.  Sides 2
+ * and 4 have all rows on their way at once, side 8 (81 rows) a plane ahead. */
+template <uint32_t BS, class Plane>
+__device__ __forceinline__ void sz3_reload(const float *__restrict__ x, const Sz3Dims &g, const Sz3Unit &k, Plane plane)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t s0 = g.d2 * g.d3, s1 = g.d3, z = k.z0 + lane;
     const bool zin = z < g.d3;
-    auto live = [&](uint32_t r) { return r == 0 ? k.j0 > 0 : r - 1 < k.sy; }; /* row j0 - 1 + r */
-    /* plane i's rows j0 - 1 .. j0 + BS - 1 (v), and in lane r the element
-     * before z0 of row r (l), which lane 0 needs; all loads issued before
-     * any is used; rows outside read as 0 */
-    auto load = [&](uint64_t i, float (&v)[BS + 1], float &l) {
+    auto load = [&](uint32_t pl, float (&v)[BS + 1], float &l) {
+        const bool in = pl ? pl <= k.sx : k.i0 > 0 && k.sx > 0; /* (no unit: sx = 0) */
+        const uint64_t o = (k.i0 + pl - 1) * s0; /* wraps only where not read */
 #pragma unroll
-        for (uint32_t r = 0; r <= BS; r++) {
-            const uint64_t o = i * s0 + (k.j0 + r - 1) * s1; /* wraps only where not live */
-            v[r] = live(r) && zin ? x[o + z] : 0.0f;
-        }
-        const uint64_t o = i * s0 + (k.j0 + lane - 1) * s1;
-        l = lane <= BS && live(lane) && k.z0 ? x[o + k.z0 - 1] : 0.0f;
+        for (uint32_t r = 0; r <= BS; r++) v[r] = in && zin && (r ? r <= k.sy : k.j0 > 0) ? x[o + (k.j0 + r - 1) * s1 + z] : 0.0f;
+        l = in && k.z0 && lane <= BS && (lane ? lane <= k.sy : k.j0 > 0) ? x[o + (k.j0 + lane - 1) * s1 + k.z0 - 1] : 0.0f;
     };
-    uint32_t dp[BS]; /* the previous plane's 2-D differences, row by row */
+    if constexpr (BS == 8) {
+        float v[BS + 1], nv[BS + 1], l, nl;
+        load(0, v, l);
+#pragma unroll 1
+        for (uint32_t pl = 0; pl <= BS; pl++) {
+            load(pl + 1, nv, nl); /* (zeros past the last) */
+            plane(pl, v, l);
 #pragma unroll
-    for (uint32_t dj = 0; dj < BS; dj++) dp[dj] = 0;
-    int di = k.i0 ? -1 : 0;
-    float cv[BS + 1], nv[BS + 1], cl, nl = 0.0f;
-    load((uint64_t)((int64_t)k.i0 + di), cv, cl);
-    for (; di < (int)k.sx; di++) {
-        if (di + 1 < (int)k.sx) load(k.i0 + (uint64_t)(di + 1), nv, nl); /* the next plane, in flight meanwhile */
-        const uint32_t qleft = (uint32_t)sz3_quantize(cl, inv, bad); /* 0 where cl is */
-        auto zdiff = [&](uint32_t r) -> uint32_t {                   /* q(z) - q(z - 1) of row r */
-            const uint32_t q = zin ? (uint32_t)sz3_quantize(cv[r], inv, bad) : 0u;
-            const uint32_t up = __shfl_up_sync(0xffffffffu, q, 1), l0 = __shfl_sync(0xffffffffu, qleft, r);
-            return q - (lane ? up : l0);
-        };
-        uint32_t rp = k.j0 ? zdiff(0) : 0u;
-#pragma unroll
-        for (uint32_t dj = 0; dj < BS; dj++) {
-            if (dj < k.sy) {
-                const uint32_t rc = zdiff(dj + 1);
-                const uint32_t d = rc - rp;
-                rp = rc;
-                if (di >= 0) row((uint32_t)di, dj, d - dp[dj]);
-                dp[dj] = d;
-            }
+            for (uint32_t r = 0; r <= BS; r++) v[r] = nv[r];
+            l = nl;
         }
+    } else {
+        float v[BS + 1][BS + 1], l[BS + 1];
 #pragma unroll
-        for (uint32_t r = 0; r <= BS; r++) cv[r] = nv[r];
-        cl = nl;
+        for (uint32_t pl = 0; pl <= BS; pl++) load(pl, v[pl], l[pl]);
+#pragma unroll
+        for (uint32_t pl = 0; pl <= BS; pl++) plane(pl, v[pl], l[pl]);
     }
 }
 
-/* The unit's differences as integers, whatever their size, in the order of
- * the walk below. */
-template <uint32_t BS>
-__device__ __noinline__ void sz3_walk_any(const float *x, const Sz3Dims &g, const Sz3Split &inv, const Sz3Unit &k, uint32_t *d,
-                                          uint32_t &bad)
+/* sz3_quantize out of line. */
+__device__ __noinline__ int32_t sz3_quantize_far(float x, const Sz3Split &inv, uint32_t &bad) { return sz3_quantize(x, inv, bad); }
+
+/* The same: n is the integer next to the float x * hi and d the rest, x * (hi +
+ * lo) - n, |d| < 2, which moves n on to the integer next to x * inv.  For |n| < 2^24
+ * d's roundings (2^-25, 2^-24), lo's error (2^-24) and the reference's are together
+ * below 2^-22.5; the others, and what lies within 2^-22 of a middle, go the long
+ * way. */
+__device__ __forceinline__ uint32_t sz3_quantize_wide(float x, const Sz3Split &inv, uint32_t &bad)
 {
-    sz3_walk<BS>(x, g, inv, k, bad, [&](uint32_t di, uint32_t dj, uint32_t v) { d[di * BS + dj] = v; });
+    const float p = __fmul_rn(x, inv.hi), n = rintf(p);
+    const float d = __fmaf_rn(x, inv.lo, __fmaf_rn(x, inv.hi, -n)), c = __fsub_rn(__fadd_rn(d, SZ_MAGIC), SZ_MAGIC);
+    if (inv.mid && fabsf(p) < 16777200.0f && fabsf(__fsub_rn(d, c)) < 0.499999761581420898f) /* NaN is not */
+        return (uint32_t)__float2int_rn(__fadd_rn(n, c));
+    return (uint32_t)sz3_quantize_far(x, inv, bad);
 }
 
-/* The double steps for a value below 2^19. */
-__device__ __noinline__ float sz3_quantize_d(float x, double inv) { return (float)floor(__dadd_rn(__dmul_rn((double)x, inv), 0.5)); }
-
-constexpr float SZ_MAGIC = 12582912.0f;         /* 1.5 * 2^23: a float m + this holds the integer m in its low bits, */
-constexpr uint32_t SZ_ZERO = 0x4B400000u;       /* as this + m */
+/* The unit's differences from integers, whatever their size: SZ_ZERO + difference
+ * at w[di * BS + dj] (outside the volume: any), the largest magnitude to mx.
+ * True, for the whole warp, if values or differences pass 2^22. */
+template <uint32_t BS>
+__device__ __forceinline__ bool sz3_walk_any(const float *x, const Sz3Dims &g, const Sz3Split &inv, const Sz3Unit &k, uint32_t *w,
+                                          uint32_t &mx, uint32_t &bad)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t dp[BS]; /* the plane's 2-D differences, row by row */
+#pragma unroll
+    for (uint32_t dj = 0; dj < BS; dj++) dp[dj] = 0;
+    uint32_t far = 0;
+    mx = 0;
+    sz3_reload<BS>(x, g, k, [&](uint32_t pl, const float (&v)[BS + 1], float l) {
+        const uint32_t ql = sz3_quantize_wide(l, inv, bad); /* 0 where l is */
+        uint32_t rp = 0;
+#pragma unroll
+        for (uint32_t r = 0; r <= BS; r++) {
+            const uint32_t q = sz3_quantize_wide(v[r], inv, bad);
+            far = max(far, mag(q));
+            const uint32_t up = __shfl_up_sync(0xffffffffu, q, 1), l0 = __shfl_sync(0xffffffffu, ql, r);
+            const uint32_t rc = q - (lane ? up : l0); /* q(z) - q(z - 1) */
+            if (r) {
+                if (pl) {
+                    const uint32_t e = rc - rp - dp[r - 1];
+                    w[(pl - 1) * BS + r - 1] = SZ_ZERO + e;
+                    mx = max(mx, mag(e));
+                }
+                dp[r - 1] = rc - rp;
+            }
+            rp = rc;
+        }
+    });
+    return __any_sync(0xffffffffu, max(far, mx) >= 1u << 22) || !inv.mid;
+}
 
 /* (int)floor((double)x * inv + 0.5) on the float pipe.  n is the integer next
  * to x * hi, d = x * (hi + lo) - n: two roundings of 2^-25 at most, lo's own
- * error and the reference's two double roundings are together below 2^-23.9
- * for |n| < 2^19, so n is the reference's result if |d| < 1/2 - 2^-22; else
- * `sure` becomes false (one value in 2^21).  sq collects n * n, so that one
- * test finds values out of range or not finite. */
-__device__ __forceinline__ float sz3_quantize_f(float x, const Sz3Split &inv, bool &sure, float &sq)
+ * error and the reference's two double roundings are together below 2^-23.5
+ * for |n| < 2^22, so n is the reference's result if |d| < SZ_SURE, 1/2 - 2^-22.
+ * If x * lo moves it past n's middle (one value in 2^25 / |n|), n + round(d)
+ * is, unless a value lies next to a middle all the same (one in 2^21). */
+constexpr float SZ_SURE = 0.499999761581420898f;
+__device__ __forceinline__ float sz3_quantize_f(float x, const Sz3Split &inv, float &d)
 {
     const float n = __fsub_rn(__fmaf_rn(x, inv.hi, SZ_MAGIC), SZ_MAGIC);
-    const float d = __fmaf_rn(x, inv.lo, __fmaf_rn(x, inv.hi, -n));
-    sure = sure && fabsf(d) < 0.499999761581420898f;
-    sq = __fmaf_rn(n, n, sq);
+    d = __fmaf_rn(x, inv.lo, __fmaf_rn(x, inv.hi, -n));
     return n;
+}
+
+/* The same for any value: n moves on to the integer next to x * (hi + lo), and
+ * what then still lies next to a middle takes the double steps.  Past 2^22, or
+ * not finite: something past 2^22. */
+__device__ __forceinline__ float sz3_quantize_any(float x, const Sz3Split &inv)
+{
+    float d;
+    const float n = sz3_quantize_f(x, inv, d), c = __fsub_rn(__fadd_rn(d, SZ_MAGIC), SZ_MAGIC);
+    if (!(fabsf(n) < 4194304.0f)) return 8388608.0f; /* NaN too */
+    if (fabsf(__fsub_rn(d, c)) < SZ_SURE) return __fadd_rn(n, c);
+    return (float)floor(__dadd_rn(__dmul_rn((double)x, inv.d), 0.5));
+}
+/* Four at a time, out of line. */
+__device__ __noinline__ float4 sz3_quantize_any4(float4 x, const Sz3Split &inv)
+{
+    return make_float4(sz3_quantize_any(x.x, inv), sz3_quantize_any(x.y, inv), sz3_quantize_any(x.z, inv), sz3_quantize_any(x.w, inv));
+}
+
+/* One plane of a unit in floats, from its quantized rows q and, in lane r, the
+ * element before row r's first: its differences to w (from the second plane on)
+ * as SZ_ZERO + d, and the largest magnitudes of the values (far) and of the
+ * differences (top). */
+template <uint32_t BS>
+__device__ __forceinline__ void sz3_plane_f(uint32_t pl, const float (&q)[BS + 1], float ql, float (&dp)[BS], uint32_t *w,
+                                            float &far, float &top)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    far = max3_abs(far, ql, q[0]);
+#pragma unroll
+    for (uint32_t r = 1; r < BS; r += 2) far = max3_abs(far, q[r], q[r + 1]);
+    float rp = 0.0f, ep = 0.0f;
+#pragma unroll
+    for (uint32_t r = 0; r <= BS; r++) {
+        const float up = __shfl_up_sync(0xffffffffu, q[r], 1), l0 = __shfl_sync(0xffffffffu, ql, r);
+        const float rc = q[r] - (lane ? up : l0); /* q(z) - q(z - 1) */
+        if (r) {
+            const float d = rc - rp;
+            if (pl) {
+                const float e = d - dp[r - 1];
+                w[(pl - 1) * BS + r - 1] = __float_as_uint(e + SZ_MAGIC);
+                if (r % 2 == 0) top = max3_abs(top, ep, e);
+                ep = e;
+            }
+            dp[r - 1] = d;
+        }
+        rp = rc;
+    }
+}
+
+/* The unit once more from memory, every value by sz3_quantize_any; false (for
+ * the whole warp) if values or differences pass 2^22. */
+template <uint32_t BS>
+__device__ __forceinline__ bool sz3_walk_again(const float *x, const Sz3Dims &g, const Sz3Split &inv, const Sz3Unit &k, uint32_t *w,
+                                            uint32_t &mx)
+{
+    float dp[BS], far = 0.0f, top = 0.0f;
+    sz3_reload<BS>(x, g, k, [&](uint32_t pl, const float (&v)[BS + 1], float l) {
+        float q[BS + 1];
+#pragma unroll
+        for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_any(v[r], inv);
+        sz3_plane_f<BS>(pl, q, sz3_quantize_any(l, inv), dp, w, far, top);
+    });
+    mx = (uint32_t)top;
+    return __all_sync(0xffffffffu, far < 4194304.0f && top < 4194304.0f);
+}
+
+/* A unit that sz3_walk_f leaves, with the most that it returned.  True if its
+ * values or differences pass 2^22. */
+template <uint32_t BS>
+__device__ __noinline__ bool sz3_walk_slow(const float *x, const Sz3Dims &g, const Sz3Split &inv, const Sz3Unit &k, uint32_t left,
+                                           uint32_t *w, uint32_t &mx, uint32_t &bad)
+{
+    if (BS < 8 && left == 1u && sz3_walk_again<BS>(x, g, inv, k, w, mx)) return false;
+    return sz3_walk_any<BS>(x, g, inv, k, w, mx, bad);
 }
 
 /* A warp's rows on their way, plane by plane through its units, into PD
@@ -680,17 +779,22 @@ struct Sz3Feed {
 /* The unit's differences, SZ_ZERO + d at w[di * BS + dj] (rows and planes
  * outside the volume: any), and this lane's largest magnitude; the next
  * unit's rows are sent for meanwhile, into the buffers that this one leaves.
- * In floats, which hold every step exactly while the quantized values are
- * below 2^19 (the differences below 2^22); false if they are not, or where a
- * value needs the double steps (one unit in thousands): any w then.
- * Side 8 takes the planes in a loop, with w in local memory, and the double
- * steps by the plane: as straight code for its 81 rows, a volume of 57 x 51 x 306
- * took 63 us, most of it the code's way from L2, and 36 so; 512^3 489 us and
- * 412. */
+ * In floats, which hold every step exactly while the quantized values and the
+ * differences are below 2^22 (a difference of such values that passes 2^24, and
+ * may be rounded, shows as one past 2^22).  Returns 0; or, by the lane, 2 if they
+ * are not, and 1 where sz3_quantize_f leaves a value open: any w then.
+ * Values of some 10^5 steps leave one open in nearly every unit: 256^3, side 4,
+ * 150000 steps from zero, 282 us with integer steps for them, 131 with
+ * sz3_walk_again (188 with integers for all).  A test after every plane keeps such units to their second form
+ * for the plane alone (79 us), but parts the planes' code: 512^3, side 4, 413 and
+ * 423 us, side 2 834 and 858.
+ * Side 8 takes the planes in a loop, with w in local memory, and has that test: as
+ * straight code for its 81 rows, a volume of 57 x 51 x 306 took 63 us, most of it
+ * the code's way from L2, and 36 so; 512^3 489 us and 382. */
 template <uint32_t BS>
-__device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
-                                           const Sz3Unit &k, const Sz3Unit &next, Sz3Feed<BS> &feed, uint32_t (&w)[BS * BS],
-                                           uint32_t &mx)
+__device__ __forceinline__ uint32_t sz3_walk_f(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Split &inv,
+                                               const Sz3Unit &k, const Sz3Unit &next, Sz3Feed<BS> &feed, uint32_t (&w)[BS * BS],
+                                               uint32_t &mx)
 {
     using F = Sz3Feed<BS>;
     const uint32_t lane = threadIdx.x & 31u;
@@ -699,8 +803,7 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
                         (uint32_t)k.z0 - 1u;
     const bool lin = k.z0 && lane <= BS;
     const uint64_t stride = 4u * g.d2 * g.d3;
-    float dp[BS], sq = 0.0f, top = 0.0f;
-    bool sure = true;
+    float dp[BS], far = 0.0f, top = 0.0f, open = 0.0f; /* open: the widest rest */
     uint32_t slot = 0; /* pl % PD */
 #pragma unroll(BS == 8 ? 1 : BS + 1)
     for (uint32_t pl = 0; pl <= BS; pl++, slot = slot + 1 == F::PD ? 0 : slot + 1) {
@@ -714,35 +817,46 @@ __device__ __forceinline__ bool sz3_walk_f(uint32_t sbuf, const float *__restric
         __syncwarp();
         if (pl + F::PD == BS + 1) feed.set(x, g, next);
         feed.send(buf, pl + F::PD <= BS ? pl + F::PD : pl + F::PD - BS - 1, stride);
-        float q[BS + 1], ql = sz3_quantize_f(cl, inv, sure, sq);
+        float q[BS + 1], d[BS + 1], dl, ql = sz3_quantize_f(cl, inv, dl);
 #pragma unroll
-        for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_f(cv[r], inv, sure, sq);
-        if (BS == 8 && __any_sync(0xffffffffu, !sure)) { /* the double steps, for this plane */
-            ql = sz3_quantize_d(cl, inv.d);
+        for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_f(cv[r], inv, d[r]);
+        open = max3_abs_nan(open, dl, d[0]);
 #pragma unroll
-            for (uint32_t r = 0; r <= BS; r++) q[r] = sz3_quantize_d(cv[r], inv.d);
-            sure = true; /* (out of range: sq shows it) */
-        }
-        float rp = 0.0f, ep = 0.0f;
+        for (uint32_t r = 1; r < BS; r += 2) open = max3_abs_nan(open, d[r], d[r + 1]);
+        if (BS == 8 && __any_sync(0xffffffffu, !(open < SZ_SURE))) { /* the plane again */
+            open = 0.0f;
+            auto at = [&](uint32_t r) { return r == 0 ? cl : cv[r <= BS + 1 ? r - 1 : 0]; };
 #pragma unroll
-        for (uint32_t r = 0; r <= BS; r++) {
-            const float up = __shfl_up_sync(0xffffffffu, q[r], 1), l0 = __shfl_sync(0xffffffffu, ql, r);
-            const float rc = q[r] - (lane ? up : l0); /* q(z) - q(z - 1) */
-            if (r) {
-                const float d = rc - rp;
-                if (pl) {
-                    const float e = d - dp[r - 1];
-                    w[(pl - 1) * BS + r - 1] = __float_as_uint(e + SZ_MAGIC);
-                    if (r % 2 == 0) top = max3_abs(top, ep, e);
-                    ep = e;
-                }
-                dp[r - 1] = d;
+            for (uint32_t r = 0; r < BS + 2; r += 4) {
+                const float4 a = sz3_quantize_any4(make_float4(at(r), at(r + 1), at(r + 2), at(r + 3)), inv);
+                if (r == 0) ql = a.x;
+                else q[r - 1] = a.x;
+                if (r < BS + 1) q[r < BS + 1 ? r : 0] = a.y;
+                if (r + 1 < BS + 1) q[r + 1 < BS + 1 ? r + 1 : 0] = a.z;
+                if (r + 2 < BS + 1) q[r + 2 < BS + 1 ? r + 2 : 0] = a.w;
             }
-            rp = rc;
         }
+        sz3_plane_f<BS>(pl, q, ql, dp, w, far, top);
     }
     mx = (uint32_t)top;
-    return sure && sq < 274877906944.0f; /* 2^38; NaN is not */
+    return !(far < 4194304.0f && top < 4194304.0f) ? 2u : BS < 8 && !(open < SZ_SURE) ? 1u : 0u;
+}
+
+/* In sz3_walk_f's place, for a warp whose last unit it could not take: the feed
+ * moves on.  (Side 8, 256^3, 6 million steps from zero, 252 us without and 216;
+ * sides 2 and 4 lose 4 % of every volume by it.) */
+template <uint32_t BS>
+__device__ __forceinline__ void sz3_pass(uint32_t sbuf, const float *__restrict__ x, const Sz3Dims &g, const Sz3Unit &next,
+                                         Sz3Feed<BS> &feed)
+{
+    using F = Sz3Feed<BS>;
+#pragma unroll 1
+    for (uint32_t pl = 0; pl <= BS; pl++) {
+        cp_async_wait<F::PD - 1>();
+        __syncwarp();
+        if (pl + F::PD == BS + 1) feed.set(x, g, next);
+        feed.send(sbuf + pl % F::PD * F::PLANE, pl + F::PD <= BS ? pl + F::PD : pl + F::PD - BS - 1, 4u * g.d2 * g.d3);
+    }
 }
 
 /* Octet g of a block of n elements at byte o of the zeroed buffer: w[k] =
@@ -896,6 +1010,7 @@ __global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows
         return K;
     };
     uint64_t t = claim(0);
+    bool far = !inv.mid; /* side 8: sz3_walk_f would not take the next unit, as it seems (uniform over the warp) */
     Sz3Unit nextu = unit();
     Sz3Feed<BS> feed;
     feed.set(x, g, nextu);
@@ -918,15 +1033,21 @@ __global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows
             if (i + 1 == UPW) tn = claim(it + 1);
             nextu = unit();
             uint32_t mx = 0;
-            if (__any_sync(0xffffffffu, !sz3_walk_f<BS>(sbuf, x, g, inv, K, nextu, feed, w[i], mx)) || !inv.mid) {
-                uint32_t d[BS * BS];
-                for (uint32_t e = 0; e < BS * BS; e++) d[e] = 0;
-                if (K.sx) sz3_walk_any<BS>(x, g, inv, K, d, bad);
-                mx = 0;
-#pragma unroll(BS == 8 ? 1 : BS * BS)
-                for (uint32_t e = 0; e < BS * BS; e++) {
-                    w[i][e] = SZ_ZERO + d[e];
-                    mx = max(mx, mag(d[e]));
+            uint32_t left = 2;
+            if (BS == 8 && far)
+                sz3_pass<BS>(sbuf, x, g, nextu, feed);
+            else
+                left = sz3_walk_f<BS>(sbuf, x, g, inv, K, nextu, feed, w[i], mx);
+            if (BS < 8 && !inv.mid) left = 2;
+            if (__any_sync(0xffffffffu, left != 0u)) {
+                left = __reduce_max_sync(0xffffffffu, left);
+                if constexpr (BS == 8) {
+                    far = sz3_walk_slow<BS>(x, g, inv, K, left, w[i], mx, bad);
+                } else {
+                    uint32_t d[BS * BS];
+                    sz3_walk_slow<BS>(x, g, inv, K, left, d, mx, bad);
+#pragma unroll
+                    for (uint32_t e = 0; e < BS * BS; e++) w[i][e] = d[e];
                 }
             }
             if (K.sx < BS || K.sy < BS) { /* rows outside the volume count for nothing */
@@ -1844,8 +1965,8 @@ cudaError_t sz3_compress_rows(uint8_t *out, uint64_t cap, const float *x, const 
  * of SZ_TASKS of them, into pieces that make at most SZ_TASKS tasks (three CTAs
  * on each of 152 SMs).  Otherwise a task goes along the whole row, and a few long
  * rows leave the device idle: 8 x 8 x 100000, side 8, 2247 us in whole rows, 54
- * in pieces; 64 x 64 x 3000, side 4, 193 and 80 (start of the sums in the
- * decoder: 345 and 113). */
+ * in pieces; 64 x 64 x 3000, side 4, 193 and 80 (with a pass per axis
+ * 345 and 113). */
 constexpr uint64_t SZ_TASKS = 456;
 template <uint32_t BS>
 Sz3Tasks sz3_tasks(const Sz3Dims &g)

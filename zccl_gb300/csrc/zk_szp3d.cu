@@ -1082,10 +1082,10 @@ __global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows
         for (uint32_t i = 0; i < UPW; i++) {
             const Sz3Unit &K = k[i];
             if constexpr (BS == 8) {
-                /* blocks whole along y and z go plane by plane, 8 octets of each; the others of a unit, from
-                 * `whole` on, in their own order, 256 elements at a time */
+                /* blocks whole along z go plane by plane, an octet a row; the last one of a unit, from `whole` on,
+                 * where it is not, in its own order, 256 elements at a time */
                 const uint32_t zleft = (uint32_t)min((uint64_t)32, g.d3 - K.z0);
-                const uint32_t there = K.sx ? (zleft + 7u) / 8u : 0u, whole = K.sx && K.sy == 8 ? zleft / 8u : 0u;
+                const uint32_t there = K.sx ? (zleft + 7u) / 8u : 0u, whole = K.sx ? zleft / 8u : 0u;
 #pragma unroll 1
                 for (uint32_t di = 0; whole && di < K.sx; di++) {
                     __syncwarp();
@@ -1093,11 +1093,11 @@ __global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows
                     for (uint32_t e = 0; e < 8; e++) st[c * C::BST + e * 8u + dz] = w[i][di * 8u + e];
                     __syncwarp();
                     const uint32_t b = lane / 8u, at = __shfl_sync(0xffffffffu, off, b), rb = __shfl_sync(0xffffffffu, rate, b);
-                    if (b < whole) {
+                    if (b < whole && lane % 8u < K.sy) {
                         const uint4 *p = reinterpret_cast<const uint4 *>(st + b * C::BST + 8u * (lane % 8u));
                         const uint4 lo = p[0], hi = p[1];
                         const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-                        sz3_put_octet(pk, at, rb, K.sx * 64u, di * 8u + lane % 8u, v);
+                        sz3_put_octet(pk, at, rb, K.sx * K.sy * 8u, di * K.sy + lane % 8u, v);
                     }
                 }
                 const uint32_t sz = K.z0 + lane < g.d3 ? sz3_unit_sz<BS>(g, K, c) : 0u;

@@ -716,6 +716,12 @@ __device__ __forceinline__ float4 ld_shared_v4(uint32_t sa)
                  : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t sa)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(sa) : "memory");
+    return v;
+}
 __device__ __forceinline__ uint32_t ld_shared_u8(uint32_t sa)
 {
     uint32_t v;

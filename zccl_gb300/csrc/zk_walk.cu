@@ -65,8 +65,8 @@ struct Sizer {
 };
 
 /* Segment of a window / group index: last s with base[s] <= i, by all lanes,
- * 32 of the remaining parts a step (131072 chunks of one window each: 25 us a
- * thousand windows by halves, 105 by 32 bases a step from the first on). */
+ * 32 parts of what is left a step (131072 chunks of 64 floats, from wire bytes:
+ * 4.5 ms; by halves 25, 32 bases a step from the first on 105). */
 __device__ __forceinline__ uint32_t find_seg(const uint32_t *base, uint32_t T, uint32_t i)
 {
     uint32_t lo = 0, n = T; /* base[lo] <= i; the last such is in [lo, lo + n) */
@@ -128,28 +128,37 @@ __global__ void k_walk_setup(const WalkArgs a)
 }
 
 /* Bytes of a warp's window area: the window and the M bytes after it, with
- * alignment slack. */
-__host__ __device__ inline uint32_t win_area(uint32_t M) { return (WALK_WW + M + 32u + 15u) & ~15u; }
+ * alignment slack; and then a bit for every 16-byte line of it. */
+__host__ __device__ inline uint32_t win_lines(uint32_t M) { return (WALK_WW + M + 32u + 15u) & ~15u; }
+__host__ __device__ inline uint32_t win_area(uint32_t M) { return win_lines(M) + ((win_lines(M) / 512u + 1u) * 4u + 15u & ~15u); }
+
+/* A window in a warp's area, loaded. */
+struct Window {
+    uint32_t at, buf; /* shared addresses of its first byte and of the area */
+    uint32_t bits;    /* of the lines' bits, set where a line is not all zero; 0: no line is */
+    bool zeros;       /* every line is zero (sparse data: zero-width blocks) */
+};
 
 /* The window [start, start + WW + M) of the stream into the 16-byte-aligned
- * area buf (bytes past avail read as 0xFF, no header), by aligned 16-byte loads that the
- * warp issues together; returns where the window's first byte landed.  zeros:
- * everything loaded is zero (sparse data: zero-width blocks). */
-__device__ __forceinline__ uint32_t load_window(const WalkArgs &a, uint64_t start, uint8_t *buf, bool &zeros)
+ * area (bytes past avail read as 0xFF, no header), by aligned 16-byte loads that the
+ * warp issues together. */
+__device__ __forceinline__ Window load_window(const WalkArgs &a, uint64_t start, uint8_t *area)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uintptr_t base = reinterpret_cast<uintptr_t>(a.in), end = base + a.avail;
     const uintptr_t lo = (base + start) & ~(uintptr_t)15;
     const uint32_t ph = (uint32_t)(base + start - lo), nl = (ph + WALK_WW + a.M + 15u) / 16u;
-    uint4 *d = reinterpret_cast<uint4 *>(buf);
+    uint4 *d = reinterpret_cast<uint4 *>(area);
     uint32_t any = 0;
+    bool gap = false; /* a zero line */
 #pragma unroll 8
     for (uint32_t i = lane; i < nl; i += 32) {
         const uintptr_t p = lo + 16u * i;
+        uint32_t o;
         if (p >= base && p + 16u <= end) {
             const uint4 v = *reinterpret_cast<const uint4 *>(p);
             d[i] = v;
-            any |= v.x | v.y | v.z | v.w;
+            o = v.x | v.y | v.z | v.w;
         } else { /* a line across either end of the readable bytes */
             uint32_t v[4] = {~0u, ~0u, ~0u, ~0u};
             for (uint32_t k = 0; k < 16; k++) {
@@ -158,11 +167,38 @@ __device__ __forceinline__ uint32_t load_window(const WalkArgs &a, uint64_t star
                     v[k >> 2] ^= (uint32_t)(uint8_t)~*reinterpret_cast<const uint8_t *>(q) << (8 * (k & 3));
             }
             d[i] = make_uint4(v[0], v[1], v[2], v[3]);
-            any |= v[0] | v[1] | v[2] | v[3];
+            o = v[0] | v[1] | v[2] | v[3];
+        }
+        any |= o;
+        gap |= o == 0;
+    }
+    Window w;
+    w.buf = smem_u32(area);
+    w.at = w.buf + ph;
+    w.zeros = !__any_sync(0xffffffffu, any != 0);
+    w.bits = 0;
+    if (__any_sync(0xffffffffu, gap) && !w.zeros) {
+        uint32_t *bits = reinterpret_cast<uint32_t *>(area + win_lines(a.M));
+        w.bits = smem_u32(bits);
+        for (uint32_t i0 = 0; i0 < nl; i0 += 32) { /* each lane reads what it wrote */
+            const uint4 v = i0 + lane < nl ? d[i0 + lane] : make_uint4(0, 0, 0, 0);
+            const uint32_t m = __ballot_sync(0xffffffffu, (v.x | v.y | v.z | v.w) != 0);
+            if (lane == 0) bits[i0 / 32u] = m;
         }
     }
-    zeros = !__any_sync(0xffffffffu, any != 0);
-    return smem_u32(buf) + ph;
+    __syncwarp();
+    return w;
+}
+
+/* One thread, at a zero byte, number pos of a window that has lines of zeros:
+ * how many zeros they show from there on, up to byte `end`; 1 if its line is none. */
+__device__ __forceinline__ uint32_t zero_run(const Window &w, uint32_t pos, uint32_t end)
+{
+    const uint32_t a = w.at + pos - w.buf, l = a >> 4, last = (w.at + end - w.buf + 15u) >> 4; /* lines that matter */
+    uint32_t k = l >> 5, m = ld_shared_u32(w.bits + 4u * k) >> (l & 31u) << (l & 31u);
+    while (!m && 32u * (k + 1u) < last) m = ld_shared_u32(w.bits + 4u * ++k);
+    const uint32_t next = m ? 32u * k + (uint32_t)__ffs(m) - 1u : last; /* the next line that is not zero */
+    return next == l ? 1u : min(16u * next - a, end - pos);
 }
 
 /* ---- W1 --------------------------------------------------------------
@@ -176,6 +212,9 @@ __device__ __forceinline__ uint32_t load_window(const WalkArgs &a, uint64_t star
  * chain of dependent shared loads of about as many steps as the window has
  * blocks, in few instructions each.  Per warp: the window, then per place a
  * flag and a result.
+ * In windows that have lines of zeros, their blocks go at once: a field of 1M
+ * zeros, whose windows end in such a stretch, 150 us for the whole walk with a
+ * step a block here and in W3, 62 so (a pass over every position, 80).
  * 64M floats' 77 MB of signal data: 80 us, bound by issue (a window's few
  * long walks leave most lanes of their warp idle); a backward pass over every
  * position of every window, which this replaces, took 176.  A stream of 0.6 MB:
@@ -185,24 +224,32 @@ constexpr uint32_t HEAD = 128, HEAD_DEAD = WALK_WW - 1; /* HEAD + M - 1 < HEAD_D
 
 __host__ __device__ inline uint32_t w1_warp_bytes(uint32_t M) { return win_area(M) + ((6u * M + 15u) & ~15u); }
 
-/* One thread: the walk of the window at shared address `win` from pos until
- * it is at `end` or past it; cnt counts its blocks.  False when it dies.  Runs
- * of zero-width blocks (1-byte zeros) go sixteen at a time where the alignment
- * allows. */
-__device__ __forceinline__ bool walk_to(uint32_t win, uint32_t &pos, uint32_t &cnt, uint32_t end, const Sizer &size)
+/* One thread: the walk of a window from pos to its end: where it leaves it
+ * (offset into the next) << 16 | its blocks, or DEAD. */
+__device__ __forceinline__ uint32_t walk_out(uint32_t win, uint32_t pos, const Sizer &size)
 {
-    while (pos < end) {
+    uint32_t cnt = 0;
+    while (pos < WALK_WW) {
         const uint32_t b = ld_shared_u8(win + pos);
-        if (b > 32u) return false;
-        uint32_t n = 1;
-        if (b == 0 && ((win + pos) & 15u) == 0 && pos + 16u <= end) {
-            const float4 v = ld_shared_v4(win + pos);
-            if (!(__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w))) n = 16;
-        }
-        pos += n > 1 ? n : size(b);
+        if (b > 32u) return DEAD;
+        pos += size(b);
+        cnt++;
+    }
+    return (pos - WALK_WW) << 16 | cnt;
+}
+
+/* The same in a window that has lines of zeros: their zero-width blocks at once. */
+__device__ __noinline__ uint32_t walk_out_runs(Window w, uint32_t pos, Sizer size)
+{
+    uint32_t cnt = 0;
+    while (pos < WALK_WW) {
+        const uint32_t b = ld_shared_u8(w.at + pos);
+        if (b > 32u) return DEAD;
+        const uint32_t n = b ? 1u : zero_run(w, pos, WALK_WW);
+        pos += b ? size(b) : n;
         cnt += n;
     }
-    return true;
+    return (pos - WALK_WW) << 16 | cnt;
 }
 
 __global__ void __launch_bounds__(32 * WARPS_W1) k_walk_tables(const WalkArgs a)
@@ -221,10 +268,10 @@ __global__ void __launch_bounds__(32 * WARPS_W1) k_walk_tables(const WalkArgs a)
     for (uint32_t wg = blockIdx.x * WARPS_W1 + warp; wg < nwin; wg += gridDim.x * WARPS_W1) {
         const uint32_t s = find_seg(w.win_base, g.T, wg);
         const uint64_t start = w.seg_P[s] + (uint64_t)(wg - w.win_base[s]) * WALK_WW;
-        bool zeros;
-        const uint32_t win = load_window(a, start, area, zeros);
+        const Window w1 = load_window(a, start, area);
+        const uint32_t win = w1.at;
         uint32_t *tab = a.ws.wtab + (uint64_t)wg * M;
-        if (zeros) { /* a block a byte */
+        if (w1.zeros) { /* a block a byte */
             for (uint32_t e = lane; e < M; e += 32) tab[e] = WALK_WW - e;
             continue;
         }
@@ -274,10 +321,10 @@ __global__ void __launch_bounds__(32 * WARPS_W1) k_walk_tables(const WalkArgs a)
             n += __popc(m);
         }
         __syncwarp();
-        for (uint32_t i = lane; i < n; i += 32) {
-            uint32_t pos = HEAD + list[i], cnt = 0;
-            fin[list[i]] = walk_to(win, pos, cnt, WALK_WW, size) ? (pos - WALK_WW) << 16 | cnt : DEAD;
-        }
+        if (w1.bits)
+            for (uint32_t i = lane; i < n; i += 32) fin[list[i]] = walk_out_runs(w1, HEAD + list[i], size);
+        else
+            for (uint32_t i = lane; i < n; i += 32) fin[list[i]] = walk_out(win, HEAD + list[i], size);
         __syncwarp();
         for (uint32_t e = lane; e < M; e += 32) {
             const uint32_t t = tab[e];
@@ -378,14 +425,35 @@ __global__ void __launch_bounds__(1024) k_walk_segments(const WalkArgs a)
  * One warp per window: its true entry and first block are one load (gwin at
  * its group's true entry); lane 0 follows the headers from the entry and
  * lists where they are, PATH at a time, and all lanes write the blocks' widths
- * (neighbouring bytes) and group offsets.  Shared bytes per warp: the window,
+ * (neighbouring bytes) and group offsets.  Lines of zeros, one zero-width block a
+ * byte, need no list.  Shared bytes per warp: the window,
  * the list.  64M floats' 77 MB: 65 us; a stream of 0.6 MB: 12 us, against 18
  * with a lane per 128-byte part of the window. */
 constexpr uint32_t PATH = 256;
 
 __host__ __device__ inline uint32_t w3_warp_bytes(uint32_t M) { return win_area(M) + 2u * PATH; }
 
-__global__ void __launch_bounds__(32 * WARPS_W3) k_walk_final(const WalkArgs a)
+/* One thread, in a window that has lines of zeros: the next headers, up to and
+ * with a byte that is none or up to a line of zeros, at most PATH of them, into
+ * the list: the position behind them and their number; or, where such a line
+ * starts at pos, pos and 1 << 16 | the zeros from there on. */
+__device__ __noinline__ uint2 list_runs(Window w, uint32_t pos, uint32_t list, Sizer size)
+{
+    uint32_t n = 0, b = 0;
+    while (pos < WALK_WW && n < PATH && b <= 32u) {
+        b = ld_shared_u8(w.at + pos);
+        if (b == 0) {
+            const uint32_t z = zero_run(w, pos, WALK_WW);
+            if (z > 1u) return make_uint2(pos, n ? n : 1u << 16 | z);
+        }
+        st_shared_u16(list + 2u * n, pos);
+        n++;
+        pos += size(min(b, 32u));
+    }
+    return make_uint2(b > 32u ? WALK_WW : pos, n);
+}
+
+__global__ void __launch_bounds__(32 * WARPS_W3, 6) k_walk_final(const WalkArgs a)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const ZGeom &g = a.g;
@@ -411,39 +479,44 @@ __global__ void __launch_bounds__(32 * WARPS_W3) k_walk_final(const WalkArgs a)
         if (blk0 >= nb) continue;
         const uint64_t gblk0 = (uint64_t)s * g.nb_reg, grp0 = (uint64_t)s * g.gr_reg;
         const uint64_t start = w.seg_P[s] + (uint64_t)k * WALK_WW;
-        bool zeros;
-        const uint32_t win = load_window(a, start, area, zeros);
-        __syncwarp();
+        const Window win = load_window(a, start, area);
         uint32_t pos = v & 0xFFFu; /* lane 0's walk */
         while (blk0 < nb) {
-            /* the next headers, up to and with a byte that is none */
-            uint32_t n = 0;
-            if (zeros) {
-                n = min(WALK_WW - pos, 4096u); /* one a byte: no list */
-            } else {
-                if (lane == 0) {
+            /* the next headers, up to and with a byte that is none; or a run of zeros, which needs no list */
+            uint32_t n = 0; /* 1 << 16 | blocks: a run */
+            if (win.zeros) {
+                n = 1u << 16 | (WALK_WW - pos);
+            } else if (lane == 0) {
+                if (win.bits) {
+                    const uint2 r = list_runs(win, pos, list, size);
+                    pos = r.x;
+                    n = r.y;
+                } else {
                     uint32_t b = 0;
                     while (pos < WALK_WW && n < PATH && b <= 32u) {
-                        b = ld_shared_u8(win + pos);
+                        b = ld_shared_u8(win.at + pos);
                         st_shared_u16(list + 2u * n, pos);
                         n++;
                         pos += size(min(b, 32u));
                     }
                     if (b > 32u) pos = WALK_WW;
                 }
-                n = __shfl_sync(0xffffffffu, n, 0);
-                __syncwarp();
             }
+            n = __shfl_sync(0xffffffffu, n, 0);
+            const bool run = n >> 16;
+            n &= 0xFFFFu;
+            const uint32_t from = __shfl_sync(0xffffffffu, pos, 0); /* the run's first byte */
+            __syncwarp();
             if (n == 0) break;
             const uint64_t q = (blk0 + lane) >> 32 ? (blk0 + lane) / g.GB : (uint32_t)(blk0 + lane) / g.GB;
             uint32_t in_grp = (uint32_t)(blk0 + lane - q * g.GB);
             uint64_t grp = grp0 + q;
             for (uint32_t i = lane; i < n; i += 32) {
                 const uint64_t blk = blk0 + i;
-                const uint32_t p = zeros ? pos + i : ld_shared_u16(list + 2u * i);
+                const uint32_t p = run ? from + i : ld_shared_u16(list + 2u * i);
                 if (blk < nb) {
                     const uint64_t gpos = start + p;
-                    const uint32_t b = ld_shared_u8(win + p);
+                    const uint32_t b = ld_shared_u8(win.at + p);
                     if (gpos >= a.avail) {
                         atomicOr(a.err, ZERR_BOUNDS);
                     } else if (b > 32) {
@@ -462,7 +535,7 @@ __global__ void __launch_bounds__(32 * WARPS_W3) k_walk_final(const WalkArgs a)
                 for (in_grp += 32; in_grp >= g.GB; in_grp -= g.GB) grp++;
             }
             blk0 += n;
-            if (zeros) break;
+            if (run) pos += n;
             __syncwarp(); /* the list is reused */
         }
         __syncwarp();

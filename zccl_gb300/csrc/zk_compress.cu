@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
         } else {
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
+                if (i && i * BPI >= nblk) break; /* uniform: a group may fill fewer rounds */
                 const uint32_t k = i * BPI + bi;
                 const bool has = bi < BPI && k < nblk;
                 const uint32_t nk = !has ? 0u : b0 + k + 1u < tb ? L : D.nlast;
@@ -358,6 +359,7 @@ __global__ void __launch_bounds__(CMP_THREADS, 2) k_compress(const __grid_consta
             const uint32_t ent = off << 8 | b;
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
+                if (i * BPI >= nblk) break;
                 const uint32_t k = i * BPI + bi, e = __shfl_sync(0xffffffffu, ent, k & 31u);
                 const bool has = bi < BPI && k < nblk;
                 const uint32_t nk = !has ? 0u : b0 + k + 1u < tb ? L : D.nlast;

@@ -333,6 +333,7 @@ __global__ void __launch_bounds__(ADD_THREADS, 2) k_homadd(const __grid_constant
             } else {
 #pragma unroll
                 for (uint32_t i = 0; i < 4; i++) {
+                    if (i * BPI >= nblk) break; /* uniform: a group may fill fewer rounds */
                     const uint32_t k = i * BPI + bi, ek = __shfl_sync(0xffffffffu, e, k & 31u);
                     const bool has = bi < BPI && k < nblk;
                     const uint32_t nk = !has ? 0u : b0 + k + 1u < tb ? L : D.nlast;
@@ -391,6 +392,7 @@ __global__ void __launch_bounds__(ADD_THREADS, 2) k_homadd(const __grid_constant
         } else {
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
+                if (i * BPI >= nblk) break;
                 uint32_t mx = 0, s8 = 0;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(ADD_THREADS, 2) k_homadd(const __grid_constant
             const uint32_t ent = off << 8 | b;
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
+                if (i * BPI >= nblk) break;
                 const uint32_t k = i * BPI + bi, ek = __shfl_sync(0xffffffffu, ent, k & 31u);
                 const bool has = bi < BPI && k < nblk;
                 const uint32_t nk = !has ? 0u : b0 + k + 1u < tb ? L : D.nlast;

@@ -409,6 +409,10 @@ int zccl_gpu_batch_check(const zccl_gpu_batch *b, void *cuda_stream);
 /* Status of the last drop-in call made by this thread. */
 int zccl_gpu_last_status(void);
 
+/* Groups of chunks into which the drop-ins cut a call on host buffers, so that
+ * its copies and kernels overlap; 1: not cut, 0: no such geometry. */
+int zccl_gpu_dropin_groups(size_t n, int L, int T);
+
 /* Text for a status code. */
 const char *zccl_gpu_strerror(int status);
 

@@ -140,6 +140,7 @@ def lib() -> ctypes.CDLL:
         "zccl_gpu_szp3d_decompress_split": (i, [vp, vp, sz, sz, sz, sz, i, ctypes.c_double, i, vp, vp]),
         "zccl_gpu_check": (i, [vp, vp]),
         "zccl_gpu_last_status": (i, []),
+        "zccl_gpu_dropin_groups": (i, [sz, i, i]),
         "zccl_gpu_strerror": (ctypes.c_char_p, [i]),
         "zccl_gpu_width_table": (None, [ctypes.POINTER(ctypes.c_uint32)]),
         "zccl_gpu_compress_noalloc": (i, [sp, vp, sz, f, i, i, vp, ctypes.POINTER(vp)]),

@@ -852,6 +852,15 @@ constexpr uint32_t kWalkLanes = 2 * kLanes; /* workspaces: the add's second walk
  * 546 + 554 and 460 + 538 + 550 (with 2^24: 512 + 551 + 626). */
 constexpr uint64_t kLeastGroup = 1ull << 23;
 
+/* Test hook: ZCCL_GPU_TEST_LEAST_GROUP in the environment, in elements, so that
+ * small calls take the grouped path. */
+uint64_t least_group()
+{
+    const char *e = getenv("ZCCL_GPU_TEST_LEAST_GROUP");
+    const unsigned long long v = e ? strtoull(e, nullptr, 10) : 0;
+    return v ? v : kLeastGroup;
+}
+
 /* Cached device buffers of the drop-in layer, one set per device. */
 struct DropCtx {
     std::mutex mu;
@@ -1060,7 +1069,7 @@ std::vector<Group> chunk_groups(const ZGeom &g)
 {
     std::vector<Group> out;
     const uint32_t T = g.T;
-    const uint32_t G = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(T, kMaxGroups), g.n / kLeastGroup);
+    const uint32_t G = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(T, kMaxGroups), g.n / least_group());
     if (G < 2) return out;
     std::vector<uint32_t> cut;
     for (uint32_t k = 0; k <= G; k++) cut.push_back((uint32_t)((uint64_t)T * k / G));
@@ -1898,6 +1907,14 @@ int dropin_szp3d_decompress_split(float *y, const unsigned char *cmp, size_t d1,
 } // namespace
 
 extern "C" int zccl_gpu_last_status(void) { return t_last_status; }
+
+extern "C" int zccl_gpu_dropin_groups(size_t n, int L, int T)
+{
+    ZGeom g;
+    if (make_geom(n, L, T, &g)) return 0;
+    const size_t k = chunk_groups(g).size();
+    return k ? (int)k : 1;
+}
 
 extern "C" void ZCCL_float_openmp_threadblock_arg(unsigned char *outputBytes, float *oriData,
                                                   size_t *outSize, float absErrBound, size_t nbEle,

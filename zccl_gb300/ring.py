@@ -60,10 +60,13 @@ class RingAllreduce:
     decompress-and-accumulate batch, then the allgather's compression and
     decompression batches.  The streams and float buffers the steps pass
     around belong to the ring object and the batches are planned once per
-    input and error bound, so repeated calls replay the same launches; the
-    returned floats live in a buffer the next call reuses.
+    input and error bound (the last four bounds' plans are kept), so repeated
+    calls replay the same launches; the returned floats live in a buffer the
+    next call reuses.
     batched=False: one C-ABI call per chunk and step, the reference's call
     sequence (the results are the same bytes)."""
+
+    BOUNDS = 4  # error bounds per variant whose plans are kept
 
     def __init__(self, count: int, P: int, L: int = 32, T: int = 1, device: str = "cuda", batched: bool = True):
         self.count, self.P, self.L, self.T = int(count), int(P), int(L), int(T)
@@ -74,6 +77,7 @@ class RingAllreduce:
         self.batched = bool(batched)
         self._codecs: dict[int, Codec] = {}
         self._plans: dict = {}
+        self._bounds: dict[str, list] = {}  # per variant, the bounds it has plans for, the last used last
         self._bufs = None
 
     def codec(self, c: int) -> Codec:
@@ -174,6 +178,19 @@ class RingAllreduce:
             self._plans[key] = b
         return b
 
+    def _use_bound(self, variant, eb):
+        """The plans of a variant's oldest bound go when it has more than BOUNDS
+        of them: a caller whose bound follows the data has a new one every time."""
+        bounds = self._bounds.setdefault(variant, [])
+        if eb in bounds:
+            bounds.remove(eb)
+        bounds.append(eb)
+        if len(bounds) > self.BOUNDS:
+            old = bounds.pop(0)
+            for k in [k for k in self._plans if k[0] == variant and k[1] != "step"]:
+                if old == (k[2] if k[1] == "compress" else k[-1]):
+                    del self._plans[k]
+
     def _gather_batched(self, reduced, eb, per_rank_outputs, tag):
         import torch
         P = self.P
@@ -191,7 +208,14 @@ class RingAllreduce:
         return y
 
     def _homomorphic_batched(self, xs, eb, per_rank_outputs):
+        import torch
         P = self.P
+        # a plan holds the inputs' addresses only: what lies there is looked at in every call
+        for x in xs:
+            if x.dtype != torch.float32 or not x.is_contiguous() or x.dim() < 1 or x.numel() != x.shape[0] \
+                    or x.numel() < self.count:
+                raise ValueError(f"every rank's buffer must be a contiguous float32 tensor of {self.count} elements")
+        self._use_bound("ho", eb)
         B = self._buffers("ho")
         S = [row[:] for row in B["S"]]
         spare = B["spare"][:]
@@ -213,6 +237,7 @@ class RingAllreduce:
 
     def _doc_batched(self, xs, eb, per_rank_outputs):
         P = self.P
+        self._use_bound("doc", eb)
         B = self._buffers("doc")
         acc, msg, red = B["acc"], B["msg"], B["red"]
         for a, x in zip(acc, xs):

@@ -167,6 +167,14 @@ bool test_stall_tile0()
     return v && v[0] == '1' && v[1] == 0;
 }
 
+/* Test hook: with ZCCL_GPU_TEST_NO_SCANNER=1 no CTA of a compression scans the
+ * tiles' sizes, as in a launch whose scanner has left its place to others. */
+bool test_no_scanner()
+{
+    const char *v = getenv("ZCCL_GPU_TEST_NO_SCANNER");
+    return v && v[0] == '1' && v[1] == 0;
+}
+
 int status_of_bits(uint32_t bits)
 {
     if (bits & ZERR_TIMEOUT) return ZCCL_GPU_ETIMEOUT;
@@ -275,6 +283,12 @@ static int compress_fmt(zccl_gpu_stream *out, const float *d_in, size_t n, float
             cudaStreamSynchronize(st) != cudaSuccess)
             return ZCCL_GPU_ECUDA;
         a.w.spin = 4096;
+    }
+    if (test_no_scanner()) {
+        static const uint32_t one = 1;
+        if (cudaMemcpyAsync(a.w.role, &one, 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return ZCCL_GPU_ECUDA;
     }
     int rc = cuda_status(launch_compress(a, st));
     if (rc == ZCCL_GPU_OK) {

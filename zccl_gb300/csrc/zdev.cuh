@@ -911,6 +911,7 @@ __device__ __forceinline__ uint32_t cta_excl_scan(uint32_t v, uint32_t *wsum, ui
 /* Polls before a wait gives up (a second or more; callers may pass a
  * smaller limit). */
 #define SCAN_SPIN_LIMIT (1u << 22)
+#define SCAN_ALONE (1u << 20) /* polls without any tile handed out */
 #define SCAN_SIZE (1ull << 62)
 #define SCAN_SUM (2ull << 62)
 #define SCAN_VAL (SCAN_SIZE - 1ull)
@@ -938,32 +939,56 @@ __device__ __forceinline__ void scan_publish(uint64_t *status, uint64_t t, uint3
     st_flag(status + t, (first ? SCAN_SUM : SCAN_SIZE) | size);
 }
 
-/* All lanes of a warp: the inclusive sum through a tile, waiting for it;
- * SCAN_NONE and ZERR_TIMEOUT after `limit` polls. */
+/* All lanes of a warp: the inclusive sum through a tile of `size` bytes, waiting
+ * for it; SCAN_NONE and ZERR_TIMEOUT after `limit` polls.  With no scanner (see
+ * scan_tiles) the tile before gives it, which is looked at too from the
+ * SCAN_HELP-th poll on (the add of two 512^3 streams 307 us, 309 with 64 polls,
+ * 314 with 16, which the scanner's usual delay reaches). */
 #define SCAN_NONE (~0ull)
-__device__ __forceinline__ uint64_t scan_wait(const uint64_t *word, uint32_t limit, uint32_t *err)
+#define SCAN_HELP 64u
+static __device__ __noinline__ uint64_t scan_wait_slow(uint64_t *word, uint32_t size, uint32_t limit, uint32_t *err)
 {
     uint64_t v = ld_flag(word);
-    uint32_t i = 0;
 #pragma unroll 1
-    while ((v >> 62) != 2u) { /* every lane reads the same word, but not at the same time */
-        if (++i >= limit) {
+    for (uint32_t i = 0; (v >> 62) != 2u; i++) {
+        if (i >= limit) {
             atomicOr(err, ZERR_TIMEOUT);
             break;
+        }
+        if ((v >> 62) == 1u) { /* not a stream's first tile */
+            const uint64_t before = ld_flag(word - 1);
+            if ((before >> 62) == 2u) {
+                v = SCAN_SUM | ((before & SCAN_VAL) + size); /* as the scanner would have it */
+                st_flag(word, v);
+                break;
+            }
         }
         __nanosleep(64);
         v = ld_flag(word);
     }
-    return __shfl_sync(0xffffffffu, (v >> 62) == 2u ? v & SCAN_VAL : SCAN_NONE, 0);
+    return v;
 }
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v);
+__device__ __forceinline__ uint64_t scan_wait(uint64_t *word, uint32_t size, uint32_t limit, uint32_t *err)
+{
+    uint64_t v = ld_flag(word);
+#pragma unroll 1
+    for (uint32_t i = 0; i < SCAN_HELP && (v >> 62) != 2u; i++) { /* every lane reads the same word, but not at the same time */
+        __nanosleep(64);
+        v = ld_flag(word);
+    }
+    if ((v >> 62) != 2u) v = scan_wait_slow(word, size, limit, err);
+    return __shfl_sync(0xffffffffu, (v >> 62) == 2u ? v & SCAN_VAL : SCAN_NONE, 0);
+}
 
 /* The scanning warp, over n tiles.  A tile that never publishes makes it
  * give up after `limit` polls: ZERR_TIMEOUT is set, the tile's size counts
  * as 0 and the scan goes on, so that no placer waits forever.  While the tile
  * waited for is not yet handed out (its CTA is still waiting for room on the
- * device), polls count 64-fold less. */
+ * device), polls count 64-fold less.
+ * If no tile at all has been handed out for a second or more, other work may hold
+ * all of the device but this CTA's place: the scanner leaves it to a CTA that
+ * works, and the placers take their sums from one another (scan_wait). */
 static __device__ __noinline__ void scan_tiles(uint64_t *status, uint64_t n, const uint32_t *ticket, uint32_t *err,
                                                uint32_t limit)
 {
@@ -1002,6 +1027,7 @@ static __device__ __noinline__ void scan_tiles(uint64_t *status, uint64_t n, con
             continue;
         }
         __nanosleep(32);
+        if (pos == 0 && polls >= SCAN_ALONE && *(volatile const uint32_t *)ticket == 0u) return;
         if (++polls < limit) continue;
         if (limit == SCAN_SPIN_LIMIT && *(volatile const uint32_t *)ticket <= pos && ++idle < 64u) {
             polls = 0;

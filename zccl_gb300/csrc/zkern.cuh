@@ -314,7 +314,7 @@ __device__ __forceinline__ void ring_end(ZRing *r, uint32_t k, uint32_t placers,
  * Its ring bytes are zeroed, so the packers find zeroed space, and
  * released. */
 template <uint32_t N>
-__device__ __forceinline__ void placer_loop(ZRing *r, uint8_t *ringb, const uint64_t *status, uint64_t max_tiles,
+__device__ __forceinline__ void placer_loop(ZRing *r, uint8_t *ringb, uint64_t *status, uint64_t max_tiles,
                                             uint32_t p, uint32_t *err, uint32_t &bad, uint32_t spin)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -328,7 +328,7 @@ __device__ __forceinline__ void placer_loop(ZRing *r, uint8_t *ringb, const uint
         const uint32_t total = S.total;
         /* after a wait that gave up, here or in the scan, a sum may be
          * missing or too small: nothing is written then */
-        const uint64_t sum = scan_wait(status + t, spin, err), base = S.T8 + sum - total;
+        const uint64_t sum = scan_wait(status + t, total, spin, err), base = S.T8 + sum - total;
         const bool fits = sum != SCAN_NONE && sum >= total && S.T8 + sum <= S.cap;
         if (!fits) bad |= ZERR_CAPACITY;
         if (lane < 8 && fits && S.hdr) S.hdr[lane] = (uint8_t)((base - S.T8) >> (8u * lane));

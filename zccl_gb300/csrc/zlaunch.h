@@ -8,6 +8,7 @@
 #include <cuda_runtime_api.h>
 #include <stddef.h>
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <mutex>
 #include <vector>
@@ -139,12 +140,13 @@ static inline unsigned persistent_grid(const void *fn, int threads, size_t smem,
 
 /* Grid of a kernel whose tiles' places come from the scanning CTA: `want`
  * working CTAs (0: as many as fit, at most one per tile) and, with more than
- * one tile, the scanner. */
+ * one tile, the scanner (none where only one CTA fits).  Test hook:
+ * ZCCL_GPU_TEST_ONE_CTA=1 in the environment launches a single CTA. */
 static inline unsigned scanned_grid(const void *fn, int threads, size_t smem, uint64_t ntiles, unsigned want)
 {
-    unsigned g = persistent_grid(fn, threads, smem, ntiles + 1);
-    if (ntiles == 1) return 1;
-    if (g < 2) g = 2;
+    const char *one = getenv("ZCCL_GPU_TEST_ONE_CTA");
+    if (ntiles == 1 || (one && one[0] == '1' && !one[1])) return 1;
+    const unsigned g = persistent_grid(fn, threads, smem, ntiles + 1);
     return want && want + 1 < g ? want + 1 : g;
 }
 

@@ -199,9 +199,12 @@ ZG_HD uint64_t zg_seg_worst(uint64_t len, uint32_t L)
     return s;
 }
 
+/* Bytes of the header: an offset per chunk (up to 2^31 of them). */
+ZG_HD uint64_t zg_header_bytes(const ZGeom *g) { return 8ull * g->T; }
+
 ZG_HD uint64_t zg_stream_worst(const ZGeom *g)
 {
-    return 8ull * g->T + (uint64_t)g->T * zg_seg_worst(g->tbs, g->L) + zg_seg_worst(g->rem, g->L);
+    return zg_header_bytes(g) + (uint64_t)g->T * zg_seg_worst(g->tbs, g->L) + zg_seg_worst(g->rem, g->L);
 }
 
 /* The header walk of a stream without an index reads every chunk's bytes in
@@ -242,7 +245,7 @@ ZG_HD uint32_t walk_max_groups(const ZGeom *g)
 ZG_HD uint32_t walk_chunk(const ZGeom *g, uint32_t s, uint64_t rel, uint64_t next, uint64_t avail, uint64_t end_bound,
                           uint64_t *P, uint64_t *R)
 {
-    const uint64_t hdr = 8ull * g->T;
+    const uint64_t hdr = zg_header_bytes(g);
     uint32_t bad = s == 0 && rel != 0 ? ZERR_CORRUPT : 0u;
     *P = *R = 0;
     if (hdr > avail || rel > avail - hdr || hdr + rel + 4 > avail) return bad | ZERR_BOUNDS;

@@ -84,7 +84,7 @@ __global__ void k_walk_setup(const WalkArgs a)
 {
     const ZGeom &g = a.g;
     const WalkScratch &w = a.ws;
-    const uint64_t hdr = 8ull * g.T;
+    const uint64_t hdr = zg_header_bytes(&g);
     __shared__ uint32_t wsum[33];
     uint32_t carry_w = 0, carry_g = 0;
     for (uint32_t s0 = 0; s0 < g.T; s0 += blockDim.x) {

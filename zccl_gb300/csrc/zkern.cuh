@@ -252,7 +252,7 @@ __device__ __forceinline__ void ring_describe(ZSlot &S, uint64_t t, uint64_t loc
     S.grp_off = idx.grp_off + z.grp0;
     S.hdr = z.has_head && z.seg < g.T ? out + 8ull * z.seg : nullptr;
     S.size = local == g.ntiles - 1 ? idx.size : nullptr;
-    S.T8 = 8u * g.T;
+    S.T8 = zg_header_bytes(&g);
     S.ngrp = z.nblk ? (z.nblk + g.GB - 1u) / g.GB : 1u;
 }
 

@@ -157,6 +157,9 @@ __device__ __forceinline__ void load_tiles(const CompressArgs &a, CShared *sh, u
         if (it >= 1)
 #pragma unroll 1
             for (uint32_t w = 0; w < CMP_WARPS; w++) mbar_wait(&sh->empty[w], (it - 1u) & 1u, a.w.err);
+        /* in every lane: a warp with nothing to read is done with this tile as soon as its lane here has sent for
+         * it, and a lane that still waited for the tile before would not see that phase any more */
+        __syncwarp();
         if (lane < CMP_WARPS) load_floats<L32>(f, map, in + lane * CMP_IN, sh->full + lane);
     }
 }

@@ -8,11 +8,14 @@
  */
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <errno.h>
 #include <math.h>
 #include <omp.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -99,8 +102,9 @@ ZIndex bind_index(void *mem, const ZGeom &g)
     return z;
 }
 
-/* Workspace: err u32 | walk_err u32 | ticket u32 | pad | status[ntiles] |
- * header-walk scratch.  Only the first part is cleared per call. */
+/* Workspace: err u32 | walk_err u32 | ticket u32 | role u32 | status[ntiles] |
+ * header-walk scratch.  Of these a compression or an add clears the ticket, the
+ * role (which CTA scans) and the status words. */
 struct WalkLayout {
     uint32_t M, max_windows, max_groups;
     size_t seg_P, seg_R, seg_end, seg_ok, win_base, grp_base, wtab, gtab, gentry, gbase, gwin, total;
@@ -109,8 +113,8 @@ struct WalkLayout {
 size_t ws_clear_bytes(const ZGeom &g) { return 16 + 8 * g.ntiles; }
 
 /* Zero what a compression or an add needs zeroed at launch (the header walk
- * and the decompressor use none of it): the tile ticket and the tiles' size
- * words.  The two status words in front of them are left alone,
+ * and the decompressor use none of it): the tile ticket, the scanner's word
+ * and the tiles' size words.  The two status words in front of them are left alone,
  * so errors of earlier calls on the workspace stay visible until
  * zccl_gpu_check() reads and clears them. */
 cudaError_t ws_clear(void *ws, const ZGeom &g, cudaStream_t st)
@@ -861,9 +865,10 @@ constexpr uint32_t kWalkLanes = 2 * kLanes; /* workspaces: the add's second walk
 /* The least elements of a group.  A group costs some ten launches and a
  * status read, 50 us with a walk, whatever its size, and the host waits for
  * each copy from pageable memory; only groups whose copies take longer gain by
- * overlapping.  Compress, add and decompress of 4M floats, pageable: 1360 us
- * in eight groups, 800 in one; 16M: 2830 and, in two, 2000; pinned 16M 454 +
- * 546 + 554 and 460 + 538 + 550 (with 2^24: 512 + 551 + 626). */
+ * overlapping.  Compress, add and decompress together, groups of 2^19 floats and
+ * more (up to eight) and of 2^23: 4M floats, pageable, 1300 to 2200 us and 750,
+ * pinned 1070 and 720; 12M 2850 and 1410, 1460 and 1395; 16M (two groups) 3250 and
+ * 1990, 1715 and 1590. */
 constexpr uint64_t kLeastGroup = 1ull << 23;
 
 /* Test hook: ZCCL_GPU_TEST_LEAST_GROUP in the environment, in elements, so that
@@ -972,6 +977,44 @@ size_t device_room(const void *p)
     size_t size = 0;
     if (!fn || fn(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return 0;
     return (size_t)(base + size - (CUdeviceptr)p);
+}
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23 /* Linux 5.14 */
+#endif
+
+uintptr_t page_size()
+{
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    return page;
+}
+
+/* Whether an output array in host memory looks as if nothing had touched its pages
+ * yet: the whole page from byte `at` on, well inside what is to be written, is not
+ * present (an array's first pages may be, from the allocator's earlier use).  A few
+ * microseconds, asked for while kernels run. */
+bool untouched(const void *p, size_t at)
+{
+    if (at < 64 * 1024) return false;
+    const uintptr_t a = ((uintptr_t)p + at + page_size() - 1) & ~(page_size() - 1);
+    const int keep = errno;
+    unsigned char in = 1;
+    const bool absent = mincore((void *)a, page_size(), &in) == 0 && !(in & 1);
+    errno = keep;
+    return absent;
+}
+
+/* The whole pages of host range [p, p + n), which a copy from the device is about
+ * to write, made present, their contents untouched.  Into pages that are not, a copy
+ * may fault its way one by one, 60 us for each 64 KB: compress, add and decompress of
+ * 4M floats into arrays just allocated 24 ms, and 3.6 so.  Where the kernel cannot,
+ * the copy does as before. */
+void touch_pages(void *p, size_t n)
+{
+    const uintptr_t a = ((uintptr_t)p + page_size() - 1) & ~(page_size() - 1), b = ((uintptr_t)p + n) & ~(page_size() - 1);
+    const int keep = errno;
+    if (b > a) madvise((void *)a, b - a, MADV_POPULATE_WRITE);
+    errno = keep;
 }
 
 int finish(DropCtx *c, void *ws)
@@ -1175,6 +1218,7 @@ struct Placer {
     unsigned char *out;
     uint32_t T;
     bool after_inputs;
+    bool fresh;       /* out is in pages that nothing has touched */
     uint64_t run = 0; /* chunk bytes placed */
     size_t next = 0;  /* the next group to place */
 
@@ -1194,6 +1238,7 @@ struct Placer {
             e += run;
             memcpy(out + 8ull * (q.s0 + i), &e, 8);
         }
+        if (fresh) touch_pages(out + 8ull * T + run, size - hdr);
         if ((after_inputs && cudaStreamWaitEvent(st, c->ev, 0) != cudaSuccess) ||
             cudaMemcpyAsync(out + 8ull * T + run, dev[k] + hdr, size - hdr, cudaMemcpyDeviceToHost, st) !=
                 cudaSuccess)
@@ -1239,7 +1284,7 @@ int pipe_compress(DropCtx *c, unsigned char *out, const float *x, size_t *outSiz
     const bool upfront = is_pinned_ptr(x);
     for (size_t k = 0; upfront && k < G && !rc; k++) rc = copy_in(k);
     for (size_t k = 0; k < G; k++) dev[k] = (uint8_t *)c->s[0].p + soff[k];
-    Placer pl{c, gr, dev, cap, poff, out, g.T, false};
+    Placer pl{c, gr, dev, cap, poff, out, g.T, false, untouched(out, g.n / 4)};
     for (size_t k = 0; k < G && !rc; k++) {
         const Group &q = gr[k];
         const uint32_t l = (uint32_t)(k % NL);
@@ -1336,6 +1381,7 @@ int pipe_decompress(DropCtx *c, float *y, const unsigned char *cmp, float eb, co
         if (int rc = c->lws[l].ensure(max_ws_bytes(gr))) return rc;
     }
     if (int rc = c->pin.ensure(poff[G])) return rc;
+    const bool fresh = untouched(y, 2 * g.n);
     float *fout = (float *)c->fout.p;
     uint8_t *pin = (uint8_t *)c->pin.p;
     const unsigned char *body = cmp + 8ull * g.T;
@@ -1368,6 +1414,7 @@ int pipe_decompress(DropCtx *c, float *y, const unsigned char *cmp, float eb, co
             break;
         /* the floats leave on the group's lane: a separate copy stream may
          * share a hardware queue with a busy lane (see drop_ctx) */
+        if (fresh) touch_pages(y + q.e0, 4 * q.n);
         if (cudaMemcpyAsync(y + q.e0, fout + q.e0, 4 * q.n, cudaMemcpyDeviceToHost, st) != cudaSuccess)
             rc = ZCCL_GPU_ECUDA;
     }
@@ -1482,7 +1529,7 @@ int pipe_homadd(DropCtx *c, unsigned char *out, size_t *out_size, const unsigned
     if (!rc && after_inputs && cudaEventRecord(c->ev, c->st_in) != cudaSuccess) rc = ZCCL_GPU_ECUDA;
     const bool per_group = !upfront && !after_inputs;
     for (size_t k = 0; k < G; k++) dev[k] = (uint8_t *)c->s[2].p + soff[k];
-    Placer pl{c, gr, dev, cap, poff, out, g.T, after_inputs};
+    Placer pl{c, gr, dev, cap, poff, out, g.T, after_inputs, untouched(out, g.n / 4)};
     for (size_t k = 0; k < G && !rc; k++) {
         const Group &q = gr[k];
         const uint32_t Ts = q.s1 - q.s0;
@@ -1601,6 +1648,7 @@ int dropin_compress(unsigned char *outputBytes, const float *oriData, size_t *ou
         s.capacity = worst;
     }
     if (int rc = compress_fmt(&s, d_in, n, eb, L, T, c->ws.p, c->st, fmt)) return rc;
+    const bool fresh = !dout && untouched(outputBytes, n / 4); /* the middle of a stream an eighth as large */
     if (int rc = finish(c, c->ws.p)) return rc;
     size_t size = 0;
     if (int rc = zccl_gpu_stream_size(&s, n, L, T, &size, c->st)) return rc;
@@ -1609,6 +1657,7 @@ int dropin_compress(unsigned char *outputBytes, const float *oriData, size_t *ou
     if (s.bytes != outputBytes) {
         if (dout && size > room) return ZCCL_GPU_ECAPACITY;
         cudaMemcpyKind k = dout ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+        if (fresh) touch_pages(outputBytes, size);
         if (cudaMemcpyAsync(outputBytes, s.bytes, size, k, c->st) != cudaSuccess) return ZCCL_GPU_ECUDA;
         if (cudaStreamSynchronize(c->st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     }
@@ -1650,6 +1699,7 @@ int dropin_decompress(float *newData, size_t n, float eb, int L, const unsigned 
         bool capped;
         if (int rc = stage_stream(c, 0, cmp, g, &s, pass > 0, &capped)) return rc;
         if (int rc = decompress_fmt(d_out, &s, n, eb, L, T, c->ws.p, c->st, fmt)) return rc;
+        if (!dout && pass == 0 && untouched(newData, 2 * n)) touch_pages(newData, 4 * n); /* while the kernels run */
         int rc = finish(c, c->ws.p);
         if (rc == ZCCL_GPU_EBOUNDS && capped && pass == 0) continue;
         if (rc) return rc;
@@ -1694,6 +1744,8 @@ int dropin_homadd(unsigned char *final_cmp, size_t *final_size, size_t n, float 
     out.bytes = (unsigned char *)c->s[2].p;
     out.capacity = worst;
     out.index = c->ix[2].p;
+    const bool dout = is_device_ptr(final_cmp);
+    bool fresh = false;
     for (int pass = 0;; pass++) { /* second pass: see dropin_decompress */
         bool cap1, cap2;
         /* the first input's index walk runs while the second input is
@@ -1714,6 +1766,7 @@ int dropin_homadd(unsigned char *final_cmp, size_t *final_size, size_t n, float 
         }
         if (rc == ZCCL_GPU_OK) {
             if ((rc = zccl_gpu_homadd_cases(&out, in, 2, n, L, T, c->ws.p, d_cases, c->st))) return rc;
+            fresh = !dout && untouched(final_cmp, n / 4);
             rc = finish(c, c->ws.p);
         }
         if (rc == ZCCL_GPU_OK && d_cases &&
@@ -1726,9 +1779,9 @@ int dropin_homadd(unsigned char *final_cmp, size_t *final_size, size_t n, float 
     }
     size_t size = 0;
     if (int rc = zccl_gpu_stream_size(&out, n, L, T, &size, c->st)) return rc;
-    const bool dout = is_device_ptr(final_cmp);
     if (dout && size > device_room(final_cmp)) return ZCCL_GPU_ECAPACITY;
     cudaMemcpyKind k = dout ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    if (fresh) touch_pages(final_cmp, size);
     if (cudaMemcpyAsync(final_cmp, out.bytes, size, k, c->st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     if (cudaStreamSynchronize(c->st) != cudaSuccess) return ZCCL_GPU_ECUDA;
     *final_size += size;

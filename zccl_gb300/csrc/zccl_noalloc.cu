@@ -3,8 +3,9 @@
  * its scratch in a fixed array of this library's device image, for callers
  * that must not allocate device memory.
  *
- * The compressor needs, per call, an error word, a tile ticket and one
- * size word per tile, all zero at launch: 16 + 8 * tiles bytes.
+ * The compressor needs, per call, two error words, a tile ticket, a word that
+ * tells which CTA scans the sizes and one size word per tile, all but the first
+ * two zero at launch: 16 + 8 * tiles bytes.
  * Here they live in g_scratch, a file-scope __device__ array that exists
  * once per device from the moment the library's device code is loaded.
  * Its address is looked up with cudaGetSymbolAddress the first time a call
@@ -66,7 +67,7 @@ extern "C" int zccl_gpu_compress_noalloc(zccl_gpu_stream *out, const float *d_in
     ZGeom g;
     if (L < 1 || T < 1 || zg_init(&g, (uint64_t)n, (uint32_t)L, (uint32_t)T) != 0)
         return ZCCL_GPU_EINVAL;
-    /* error word, ticket, padding, one status word per tile */
+    /* two error words, ticket, the scanner's word, one size word per tile */
     if (16ull + 8ull * g.ntiles > (uint64_t)ZCCL_GPU_NOALLOC_SCRATCH_BYTES) return ZCCL_GPU_ESCRATCH;
     void *scratch = nullptr;
     if (int rc = scratch_address(&scratch)) return rc;

@@ -7,8 +7,9 @@
  *   decode_small_f/decode_mid_f   its inverse as floats, widths below 16 / 16..23
  *   decode_add_any       any width, added to integers
  *   decode_octet         eight elements of any block
- *   encode_any/decode_any     any block, one element at a time
- *   Packer / Reader      MSB-first bit streams in shared memory
+ *   encode_octet         its inverse
+ *   encode_any           any block, one element at a time
+ *   Packer               MSB-first bit streams in shared memory
  *   tma_load_superset()  TMA bulk copy global -> shared
  *   store_realign()      shared -> global at any byte alignment
  *   cta_excl_scan()      block-wide exclusive scan
@@ -673,7 +674,6 @@ __device__ __forceinline__ void bulk_g2s(void *sdst, const void *gsrc, uint32_t 
         : "memory");
 }
 
-/* Shared stores by address (a swizzled layout computes its own). */
 /* Four bytes from global to shared memory, asynchronously (both addresses
  * multiples of 4); cp_async_arrive: one arrival on the barrier when all the
  * thread's copies so far have landed. */
@@ -699,6 +699,7 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t *bar)
 {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+/* Shared accesses by address (a swizzled layout computes its own). */
 __device__ __forceinline__ void st_shared_v4(uint32_t sa, float x, float y, float z, float w)
 {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sa), "f"(x), "f"(y), "f"(z), "f"(w)

@@ -15,8 +15,9 @@
 
 #define ZH_MAXP 32 /* most inputs one homomorphic-add launch accepts */
 
-/* Per-call scratch in device memory, zeroed before every call:
- * err | walk_err | ticket | role | status[ntiles]. */
+/* Per-call scratch in device memory: err | walk_err | ticket | role |
+ * status[ntiles].  The first two stay until they are checked, the others are
+ * zeroed before every compression and add. */
 struct ZWork {
     uint32_t *err;      /* ZERR_* bits of the codec kernels */
     uint32_t *walk_err; /* ZERR_* bits of the index walk that ran before, if any */
@@ -64,7 +65,7 @@ struct ZBatch {
 struct CompressArgs {
     CompressJob job; /* the single job (batch.jobs == null) */
     ZBatch batch;
-    ZWork w; /* err and ticket; status is per job */
+    ZWork w;
     ZWidthTable wt;
     uint32_t grid; /* CTAs to launch, 0 = as many as fit */
     uint32_t ring; /* bytes of the ring of packed tiles (filled by the launcher) */

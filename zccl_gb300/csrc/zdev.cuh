@@ -943,8 +943,8 @@ __device__ __forceinline__ void scan_publish(uint64_t *status, uint64_t t, uint3
 /* All lanes of a warp: the inclusive sum through a tile of `size` bytes, waiting
  * for it; SCAN_NONE and ZERR_TIMEOUT after `limit` polls.  With no scanner (see
  * scan_tiles) the tile before gives it, which is looked at too from the
- * SCAN_HELP-th poll on (the add of two 512^3 streams 307 us, 309 with 64 polls,
- * 314 with 16, which the scanner's usual delay reaches). */
+ * SCAN_HELP-th poll on (64: the add of two 512^3 streams 0.6 % slower than
+ * without this look; 16, which the scanner's usual delay reaches, 2 %). */
 #define SCAN_NONE (~0ull)
 #define SCAN_HELP 64u
 static __device__ __noinline__ uint64_t scan_wait_slow(uint64_t *word, uint32_t size, uint32_t limit, uint32_t *err)

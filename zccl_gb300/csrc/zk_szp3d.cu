@@ -885,11 +885,11 @@ __device__ __forceinline__ void sz3_put_octet(uint32_t sbase, uint32_t o, uint32
  * rows to octets through a small buffer.  The ring, its placer warps (which
  * write the tiles out) and the scan of the tiles' sizes by one CTA are the
  * 1-D compressor's.
- * Bound by issue, 80 instructions per 32 elements at side 4 (252 with exact
+ * Bound by issue, 85 instructions per 32 elements at side 4 (252 with exact
  * integer quantization, byte-wise packing and a look-back per warp).  512^3:
- * side 8 412 us, 4 407, 2 828, against 706, 1216 and 3662.  Two units a warp at
- * side 4 take 440, three CTAs an SM 470 (spills), 10 or 12 compute warps the
- * same 408. */
+ * side 8 388 us, 4 410, 2 820, against 706, 1216 and 3662.  At side 4, from
+ * 407, two units a warp took 440, three CTAs an SM 470 (spills), 10 or 12
+ * compute warps the same 408. */
 template <uint32_t BS, uint32_t NW> /* NW: compute warps */
 struct Sz3Cm {
     static constexpr uint32_t U = 32 / BS, NB = BS * BS * BS, UPW = BS == 2 ? 2 : 1;
@@ -1182,7 +1182,7 @@ __global__ void __launch_bounds__(Sz3Cm<BS, NW>::THREADS, 2) k_sz3_compress_rows
  * (12 bytes of traffic an element instead of the 28 of a pass per axis).
  * 301 x 450 x 517, side 8: 858 us before (decode 347, z 93, y 120, x 406
  * alone), 258 now (decode and sums 118, x 103, the carries 15).
- * 512^3: side 8 382 us, 4 389, 2 558.
+ * 512^3: side 8 408 us, 4 425, 2 590.
  *
  * A strip is a row of blocks along z; its bytes are consecutive in the stream.
  * A part is PARTS strips along y.  Consumer warps take one layer of a part's

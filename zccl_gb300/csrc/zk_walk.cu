@@ -215,7 +215,7 @@ __device__ __forceinline__ uint32_t zero_run(const Window &w, uint32_t pos, uint
  * In windows that have lines of zeros, their blocks go at once: a field of 1M
  * zeros, whose windows end in such a stretch, 150 us for the whole walk with a
  * step a block here and in W3, 62 so (a pass over every position, 80).
- * 64M floats' 77 MB of signal data: 80 us, bound by issue (a window's few
+ * 64M floats' 77 MB of signal data: 76 us, bound by issue (a window's few
  * long walks leave most lanes of their warp idle); a backward pass over every
  * position of every window, which this replaces, took 176.  A stream of 0.6 MB:
  * 15 us against 23; windows of 4096 bytes 64 / 23, four windows a warp in turn
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(1024) k_walk_segments(const WalkArgs a)
  * lists where they are, PATH at a time, and all lanes write the blocks' widths
  * (neighbouring bytes) and group offsets.  Lines of zeros, one zero-width block a
  * byte, need no list.  Shared bytes per warp: the window,
- * the list.  64M floats' 77 MB: 65 us; a stream of 0.6 MB: 12 us, against 18
+ * the list.  64M floats' 77 MB: 66 us; a stream of 0.6 MB: 12 us, against 18
  * with a lane per 128-byte part of the window. */
 constexpr uint32_t PATH = 256;
 

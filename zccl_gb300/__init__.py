@@ -41,6 +41,7 @@ EXPORTS = [
     "zccl_gpu_compress", "zccl_gpu_decompress", "zccl_gpu_homadd", "zccl_gpu_homadd_cases",
     "zccl_gpu_decompress_accumulate",
     "zccl_gpu_build_index", "zccl_gpu_stream_size", "zccl_gpu_frame_size", "zccl_gpu_check", "zccl_gpu_last_status",
+    "zccl_gpu_dropin_groups",
     "zccl_gpu_strerror", "zccl_gpu_width_table", "zccl_gpu_compress_noalloc",
     "zccl_gpu_batch_bytes", "zccl_gpu_batch_plan", "zccl_gpu_batch_run", "zccl_gpu_batch_tune",
     "zccl_gpu_batch_check",
